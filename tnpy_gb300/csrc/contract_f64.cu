@@ -6,6 +6,7 @@
 //
 // Every contraction is L x MPS -> MPO -> R split into two GEMMs (K = chi and K = chi*D)
 // around a small dense MPO step (K = D*d), i.e. 4*chi^3*D*d + 2*chi^2*D^2*d^2 flops.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cstring>
@@ -13,108 +14,206 @@
 
 #include "tnx_internal.cuh"
 
+namespace cg = cooperative_groups;
+
 namespace tnx {
 
 // ---------------------------------------------------------------------------------
-// FP64 SIMT GEMM: 64x64 tile, 16-deep K slab, 256 threads, 4x4 outputs per thread
-// interleaved by 16 so that shared-memory reads of a warp hit distinct banks.
-// GB300 runs FP64 at ~1/64 of the FP32 rate, so this kernel is bound by the FP64 pipe
-// for every shape that matters; the tiling only has to keep that pipe fed.
+// FP64 SIMT GEMM. GB300 issues 2 FP64 FMAs per clock and SM (one warp instruction occupies its
+// sub-partition's pipe for 64 clocks), so the pipe is the bound at every shape, a tile of any
+// size keeps it fed, and the time of a product is the FMA count of the busiest SM: what matters
+// is that the work spreads over all 152 SMs with little padding. Hence three tiles (64 x 64,
+// 32 x 32, 16 x 16) and a split of K over the CTAs of a thread-block cluster, whose partial tiles
+// are summed through distributed shared memory in rank order (deterministic, no workspace);
+// f64_plan picks the pair with the least FMAs on the busiest SM. The next 16-deep K slab is
+// loaded into registers while the current one is multiplied. Threads own interleaved outputs, so
+// the shared-memory reads of a warp hit distinct banks.
 // ---------------------------------------------------------------------------------
 namespace {
-constexpr int GB_M = 64, GB_N = 64, GB_K = 16, GB_T = 256;
+constexpr int GB_K = 16;
 
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(GB_T) gemm_f64_kernel(int64_t M, int64_t N, int64_t K, double alpha,
+template <bool TA, bool TB, int BM, int BN, int NT>
+__global__ void __launch_bounds__(NT) gemm_f64_kernel(int64_t M, int64_t N, int64_t K, double alpha,
                                                      const double* __restrict__ A, int64_t lda,
                                                      int64_t sa, const double* __restrict__ B,
                                                      int64_t ldb, int64_t sb, double beta,
                                                      double* __restrict__ C, int64_t ldc,
                                                      int64_t sc, int64_t k_total,
-                                                     const int* __restrict__ bmask) {
-  __shared__ double As[GB_K][GB_M + 1];
-  __shared__ double Bs[GB_K][GB_N + 1];
-  const int64_t bz = blockIdx.z;
-  if (bmask && !bmask[bz]) return;  // a batch entry the caller masked out
+                                                     const int* __restrict__ bmask, int nsplit, int64_t kslice) {
+  constexpr int TY = NT / 16, RI = BM / TY, RJ = BN / 16;  // outputs per thread
+  constexpr int LA = BM * GB_K / NT, LB = BN * GB_K / NT;  // slab elements per thread
+  static_assert(BM % TY == 0 && BN % 16 == 0 && LA * NT == BM * GB_K && LB * NT == BN * GB_K, "FP64 GEMM tile");
+  constexpr int STAGE = GB_K * (BM + 1 + BN + 1), TILE = BM * BN;
+  __shared__ double sm[STAGE > TILE ? STAGE : TILE];  // slab, then the partial tile of a split product
+  double(*As)[BM + 1] = reinterpret_cast<double(*)[BM + 1]>(sm);
+  double(*Bs)[BN + 1] = reinterpret_cast<double(*)[BN + 1]>(sm + GB_K * (BM + 1));
+  const int64_t bz = blockIdx.z / nsplit;
+  const int rank = int(blockIdx.z % nsplit);  // = the CTA's rank in its 1 x 1 x nsplit cluster
+  if (bmask && !bmask[bz]) return;  // a batch entry the caller masked out (all of its cluster)
   A += bz * sa;
   B += bz * sb;
   C += bz * sc;
-  const int64_t m0 = int64_t(blockIdx.y) * GB_M, n0 = int64_t(blockIdx.x) * GB_N;
+  const int64_t m0 = int64_t(blockIdx.y) * BM, n0 = int64_t(blockIdx.x) * BN;
   // split-K mode (k_total > 0): batch index bz owns K range [bz*K, min((bz+1)*K, k_total))
   if (k_total > 0) {
     const int64_t rem = k_total - bz * K;
     K = rem < K ? rem : K;
   }
+  const int64_t kb = rank * kslice, ke = kb + kslice < K ? kb + kslice : K;
   const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-  double acc[4][4];
+  double acc[RI][RJ];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < RI; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
+    for (int j = 0; j < RJ; ++j) acc[i][j] = 0.0;
 
-  for (int64_t k0 = 0; k0 < K; k0 += GB_K) {
-    // A tile: As[kk][mm] = op(A)[m0+mm][k0+kk]
+  double pa[LA], pb[LB];
+  // global -> registers for the slab at k0 (zero outside the matrix and the slice); consecutive
+  // threads walk the unit-stride index
+  auto fetch = [&](int64_t k0) {
 #pragma unroll
-    for (int r = 0; r < (GB_M * GB_K) / GB_T; ++r) {
-      int e = tid + r * GB_T;
-      int mm, kk;
-      if (TA) {  // stored K x M: consecutive threads walk m
-        mm = e % GB_M;
-        kk = e / GB_M;
-      } else {  // stored M x K: consecutive threads walk k
-        kk = e % GB_K;
-        mm = e / GB_K;
-      }
-      int64_t gm = m0 + mm, gk = k0 + kk;
-      double v = 0.0;
-      if (gm < M && gk < K) v = TA ? A[gk * lda + gm] : A[gm * lda + gk];
-      As[kk][mm] = v;
+    for (int r = 0; r < LA; ++r) {
+      const int e = tid + r * NT;
+      const int mm = TA ? e % BM : e / GB_K, kk = TA ? e / BM : e % GB_K;
+      const int64_t gm = m0 + mm, gk = k0 + kk;
+      pa[r] = (gm < M && gk < ke) ? (TA ? A[gk * lda + gm] : A[gm * lda + gk]) : 0.0;
     }
-    // B tile: Bs[kk][nn] = op(B)[k0+kk][n0+nn]
 #pragma unroll
-    for (int r = 0; r < (GB_N * GB_K) / GB_T; ++r) {
-      int e = tid + r * GB_T;
-      int nn, kk;
-      if (TB) {  // stored N x K
-        kk = e % GB_K;
-        nn = e / GB_K;
-      } else {  // stored K x N
-        nn = e % GB_N;
-        kk = e / GB_N;
-      }
-      int64_t gn = n0 + nn, gk = k0 + kk;
-      double v = 0.0;
-      if (gn < N && gk < K) v = TB ? B[gn * ldb + gk] : B[gk * ldb + gn];
-      Bs[kk][nn] = v;
+    for (int r = 0; r < LB; ++r) {
+      const int e = tid + r * NT;
+      const int nn = TB ? e / GB_K : e % BN, kk = TB ? e % GB_K : e / BN;
+      const int64_t gn = n0 + nn, gk = k0 + kk;
+      pb[r] = (gn < N && gk < ke) ? (TB ? B[gn * ldb + gk] : B[gk * ldb + gn]) : 0.0;
     }
+  };
+  auto stage = [&]() {
+#pragma unroll
+    for (int r = 0; r < LA; ++r) {
+      const int e = tid + r * NT;
+      As[TA ? e / BM : e % GB_K][TA ? e % BM : e / GB_K] = pa[r];
+    }
+#pragma unroll
+    for (int r = 0; r < LB; ++r) {
+      const int e = tid + r * NT;
+      Bs[TB ? e % GB_K : e / BN][TB ? e / GB_K : e % BN] = pb[r];
+    }
+  };
+  if (kb < ke) {
+    fetch(kb);
+    stage();
     __syncthreads();
+    for (int64_t k0 = kb; k0 < ke; k0 += GB_K) {
+      const bool more = k0 + GB_K < ke;
+      if (more) fetch(k0 + GB_K);
+      const int kn = ke - k0 < GB_K ? int(ke - k0) : GB_K;  // no FMAs on the padding of a short slab
+#pragma unroll 4
+      for (int kk = 0; kk < kn; ++kk) {
+        double a[RI], b[RJ];
 #pragma unroll
-    for (int kk = 0; kk < GB_K; ++kk) {
-      double a[4], b[4];
+        for (int i = 0; i < RI; ++i) a[i] = As[kk][ty + TY * i];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty + 16 * i];
+        for (int j = 0; j < RJ; ++j) b[j] = Bs[kk][tx + 16 * j];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx + 16 * j];
+        for (int i = 0; i < RI; ++i)
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    int64_t gm = m0 + ty + 16 * i;
-    if (gm >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      int64_t gn = n0 + tx + 16 * j;
-      if (gn >= N) continue;
-      double v = alpha * acc[i][j];
-      if (beta != 0.0) v = fma(beta, C[gm * ldc + gn], v);
-      C[gm * ldc + gn] = v;
+          for (int j = 0; j < RJ; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+      }
+      __syncthreads();
+      if (more) {
+        stage();
+        __syncthreads();
+      }
     }
   }
+  auto put = [&](int64_t gm, int64_t gn, double v) {
+    if (gm >= M || gn >= N) return;
+    v *= alpha;
+    if (beta != 0.0) v = fma(beta, C[gm * ldc + gn], v);
+    C[gm * ldc + gn] = v;
+  };
+  if (nsplit == 1) {
+#pragma unroll
+    for (int i = 0; i < RI; ++i)
+#pragma unroll
+      for (int j = 0; j < RJ; ++j) put(m0 + ty + TY * i, n0 + tx + 16 * j, acc[i][j]);
+    return;
+  }
+  // the slices' partial tiles, summed in rank order; each rank finishes its share of the elements
+  cg::cluster_group cluster = cg::this_cluster();
+#pragma unroll
+  for (int i = 0; i < RI; ++i)
+#pragma unroll
+    for (int j = 0; j < RJ; ++j) sm[(ty + TY * i) * BN + tx + 16 * j] = acc[i][j];
+  cluster.sync();
+  for (int e = rank * NT + tid; e < TILE; e += NT * nsplit) {
+    double v = 0.0;
+    for (int r = 0; r < nsplit; ++r) v += cluster.map_shared_rank(sm, r)[e];
+    put(m0 + e / BN, n0 + e % BN, v);
+  }
+  cluster.sync();  // no CTA leaves while another may still read its tile
+}
+
+// Tile (64, 32 or 16 rows and columns) and K split of one product. The cost of a candidate is the
+// number of FMA clocks of the busiest SM, ceil(CTAs / 152) * tile * slice / 2, plus its fixed part
+// (launch, first loads, the cluster's sum). Measured (GB300, per call): 402 x 168 x 840, 886 us
+// with 64 x 64 tiles (21 CTAs) and 120 us planned (286 of 16 x 16; the pipe alone: 90 us);
+// 64 x 32 x 160, 172 us (one CTA) and 7.7 us planned; 512^3, 538 and 237 us; 2048 x 1024 x 5120,
+// 20.6 ms without the prefetch and 17.4 ms with it (1.235 of 1.26 TFLOP/s).
+struct F64Plan {
+  int tile, nsplit;
+  int64_t kslice;
+};
+
+F64Plan f64_plan(int64_t m, int64_t n, int64_t k, int64_t batch) {
+  static const int tiles[3] = {64, 32, 16};
+  static const int splits[4] = {1, 2, 4, 8};  // 8: the largest portable cluster
+  F64Plan best{64, 1, (k + GB_K - 1) / GB_K * GB_K};
+  double best_cost = 1e300;
+  for (int t : tiles) {
+    const int64_t my = (m + t - 1) / t, nx = (n + t - 1) / t;
+    if (my > 65535 && t < 64) continue;  // beyond the grid's y limit
+    for (int s : splits) {
+      if (batch * s > 65535 || (s > 1 && t == 64)) break;
+      const int64_t ks = ((k + s - 1) / s + GB_K - 1) / GB_K * GB_K;
+      if (s > 1 && ks * (s - 1) >= k) break;  // an empty slice
+      const double ctas = double(my) * double(nx) * double(batch) * s;
+      const double waves = double(int64_t((ctas + 151) / 152));
+      const double per = double(t) * t * double(ks < k ? ks : k) / 2.0;
+      // fixed clocks per CTA: first slab, store (and the cluster's barriers and sum)
+      const double cost = waves * (per + t * t / 2.0) + 2000.0 + (s > 1 ? 3000.0 + waves * t * t / 2.0 : 0.0);
+      if (cost < best_cost) {
+        best_cost = cost;
+        best = {t, s, ks};
+      }
+    }
+  }
+  return best;
+}
+
+template <int BM, int BN, int NT>
+int launch_f64(bool ta, bool tb, const F64Plan& p, dim3 grid, int64_t m, int64_t n, int64_t k, double alpha,
+               const double* A, int64_t lda, int64_t sa, const double* B, int64_t ldb, int64_t sb, double beta,
+               double* C, int64_t ldc, int64_t sc, cudaStream_t st, int64_t k_total, const int* bmask) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 1;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = unsigned(p.nsplit);
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(NT);
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = p.nsplit > 1 ? 1 : 0;
+  auto go = [&](auto kernel) {
+    return cudaLaunchKernelEx(&cfg, kernel, m, n, k, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc, k_total, bmask,
+                              p.nsplit, p.kslice);
+  };
+  if (!ta && !tb) TNX_CUDA(go(gemm_f64_kernel<false, false, BM, BN, NT>));
+  else if (ta && !tb) TNX_CUDA(go(gemm_f64_kernel<true, false, BM, BN, NT>));
+  else if (!ta && tb) TNX_CUDA(go(gemm_f64_kernel<false, true, BM, BN, NT>));
+  else TNX_CUDA(go(gemm_f64_kernel<true, true, BM, BN, NT>));
+  return TNX_OK;
 }
 }  // namespace
 
@@ -131,23 +230,22 @@ int gemm_f64(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha, co
     return TNX_OK;
   }
   TNX_CHECK_SHAPE(batch <= 65535, "gemm_f64: batch %lld > 65535", (long long)batch);
-  dim3 grid((unsigned)((n + GB_N - 1) / GB_N), (unsigned)((m + GB_M - 1) / GB_M), (unsigned)batch);
+  const F64Plan p = f64_plan(m, n, k, batch);
+  dim3 grid((unsigned)((n + p.tile - 1) / p.tile), (unsigned)((m + p.tile - 1) / p.tile),
+            (unsigned)(batch * p.nsplit));
   TNX_CHECK_SHAPE(grid.y <= 65535, "gemm_f64: m too large");
   profile_mark(KF_F64_GEMM, st, true);
-  if (!ta && !tb)
-    gemm_f64_kernel<false, false><<<grid, GB_T, 0, st>>>(m, n, k, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc, k_total,
-                                                          bmask);
-  else if (ta && !tb)
-    gemm_f64_kernel<true, false><<<grid, GB_T, 0, st>>>(m, n, k, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc, k_total,
-                                                          bmask);
-  else if (!ta && tb)
-    gemm_f64_kernel<false, true><<<grid, GB_T, 0, st>>>(m, n, k, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc, k_total,
-                                                          bmask);
+  if (p.tile == 64)
+    TNX_TRY((launch_f64<64, 64, 256>(ta, tb, p, grid, m, n, k, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc, st,
+                                     k_total, bmask)));
+  else if (p.tile == 32)
+    TNX_TRY((launch_f64<32, 32, 128>(ta, tb, p, grid, m, n, k, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc, st,
+                                     k_total, bmask)));
   else
-    gemm_f64_kernel<true, true><<<grid, GB_T, 0, st>>>(m, n, k, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc, k_total,
-                                                          bmask);
+    TNX_TRY((launch_f64<16, 16, 128>(ta, tb, p, grid, m, n, k, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc, st,
+                                     k_total, bmask)));
   profile_mark(KF_F64_GEMM, st, false);
-  profile_work(KF_F64_GEMM, 2.0 * double(m) * n * k * batch, 8.0 * (double(m) * k + double(k) * n + double(m) * n) * batch);
+  profile_work(KF_F64_GEMM, 2.0 * double(m) * n * k * batch, 8.0 * batch * (double(m) * k + double(k) * n + double(m) * n));
   TNX_LAUNCH_CHECK();
   return TNX_OK;
 }
@@ -171,7 +269,9 @@ __global__ void splitk_reduce_kernel(const double* __restrict__ P, int nsplit, i
 int gemm_f64_splitk(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha, const double* A, int64_t lda,
                     const double* B, int64_t ldb, double beta, double* C, int64_t ldc, int nsplit, double* part,
                     cudaStream_t st, bool df) {
-  if (nsplit <= 1) return gemm_fp64_class(df, ta, tb, m, n, k, alpha, A, lda, 0, B, ldb, 0, beta, C, ldc, 0, 1, st);
+  // FP64 products split K inside gemm_f64 (clusters), without partials in memory
+  if (!df || nsplit <= 1)
+    return gemm_fp64_class(df, ta, tb, m, n, k, alpha, A, lda, 0, B, ldb, 0, beta, C, ldc, 0, 1, st);
   const int64_t kc = (k + nsplit - 1) / nsplit;
   nsplit = int((k + kc - 1) / kc);
   const int64_t sa = ta ? kc * lda : kc, sb = tb ? kc : kc * ldb;
