@@ -20,6 +20,7 @@
 #include <cmath>
 
 #include "tnx_internal.cuh"
+#include "wcontract.cuh"
 
 namespace tnx {
 namespace {
@@ -32,66 +33,6 @@ inline unsigned bgrid(int64_t total, int threads, int64_t cap) {
   int64_t b = (total + threads - 1) / threads;
   if (b > cap) b = cap;
   return unsigned(b < 1 ? 1 : b);
-}
-
-// ---- batched MPO contraction (blockIdx.y = chain) ---------------------------------------
-__global__ void bw_left_kernel(const double* __restrict__ T1, int64_t sT1, const double* __restrict__ W, int64_t sW,
-                               double* __restrict__ T2, int64_t sT2, int64_t chi_l, int d, int64_t chi_r, int dl,
-                               int dr, const int* __restrict__ mask = nullptr) {
-  extern __shared__ double ws[];
-  const int b = blockIdx.y;
-  if (mask && !mask[b]) return;
-  T1 += b * sT1;
-  W += b * sW;
-  T2 += b * sT2;
-  const int wn = dl * dr * d * d;
-  for (int i = threadIdx.x; i < wn; i += blockDim.x) ws[i] = W[i];
-  __syncthreads();
-  const int64_t total = chi_l * chi_r;
-  for (int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
-       idx += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t ap = idx / chi_r, c = idx % chi_r;
-    double in[BWMAX];
-    for (int w = 0; w < dl; ++w)
-      for (int s = 0; s < d; ++s) in[w * d + s] = T1[((w * chi_l + ap) * d + s) * chi_r + c];
-    for (int sp = 0; sp < d; ++sp) {
-      double* out = T2 + ((ap * d + sp) * chi_r + c) * dr;
-      for (int v = 0; v < dr; ++v) {
-        double acc = 0.0;
-        for (int w = 0; w < dl; ++w)
-          for (int s = 0; s < d; ++s) acc = fma(in[w * d + s], ws[((w * dr + v) * d + s) * d + sp], acc);
-        out[v] = acc;
-      }
-    }
-  }
-}
-
-__global__ void bw_right_kernel(const double* __restrict__ T1, int64_t sT1, const double* __restrict__ W, int64_t sW,
-                                double* __restrict__ T2, int64_t sT2, int64_t chi_l, int d, int64_t chi_r, int dl,
-                                int dr) {
-  extern __shared__ double ws[];
-  const int b = blockIdx.y;
-  T1 += b * sT1;
-  W += b * sW;
-  T2 += b * sT2;
-  const int wn = dl * dr * d * d;
-  for (int i = threadIdx.x; i < wn; i += blockDim.x) ws[i] = W[i];
-  __syncthreads();
-  const int64_t total = chi_l * chi_r;
-  for (int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
-       idx += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t a = idx / chi_r, cp = idx % chi_r;
-    double in[BWMAX];
-    for (int s = 0; s < d; ++s)
-      for (int v = 0; v < dr; ++v) in[v * d + s] = T1[((a * d + s) * dr + v) * chi_r + cp];
-    for (int w = 0; w < dl; ++w)
-      for (int sp = 0; sp < d; ++sp) {
-        double acc = 0.0;
-        for (int v = 0; v < dr; ++v)
-          for (int s = 0; s < d; ++s) acc = fma(in[v * d + s], ws[((w * dr + v) * d + s) * d + sp], acc);
-        T2[((a * dl + w) * d + sp) * chi_r + cp] = acc;
-      }
-  }
 }
 
 __global__ void bdiag_kernel(const double* __restrict__ L, int64_t sL, const double* __restrict__ W, int64_t sW,
@@ -499,10 +440,8 @@ int bmatvec(const double* L, int64_t sL, const double* W, int64_t sW, const doub
   // T1[(w,a'),(s,c)] = sum_a L[a,(w,a')] x[a,(s,c)]
   TNX_TRY(bgemm(df, true, false, g.dl * g.chi_l, g.d * g.chi_r, g.chi_l, 1.0, L, g.dl * g.chi_l, sL, x,
                 g.d * g.chi_r, sx, 0.0, T1, g.d * g.chi_r, ne, B, st, mask, oz, ozb));
-  const size_t smem = size_t(g.dl * g.dr * g.d * g.d) * sizeof(double);
-  bw_left_kernel<<<dim3(bgrid(g.chi_l * g.chi_r, 128, 64), B), 128, smem, st>>>(
-      T1, ne, W, sW, T2, ne, g.chi_l, int(g.d), g.chi_r, int(g.dl), int(g.dr), mask);
-  TNX_LAUNCH_CHECK();
+  TNX_TRY(wc::launch_left<double>(T1, ne, W, sW, wc::OutF64{T2}, ne, g.chi_l, g.d, g.chi_r, g.dl, g.dr,
+                                  g.chi_r * g.dr, B, mask, st));
   // y[(a',s'),c'] = sum_{(c,v)} T2[(a',s'),(c,v)] R[(c,v),c']
   TNX_TRY(bgemm(df, false, false, g.chi_l * g.d, g.chi_r, g.chi_r * g.dr, 1.0, T2, g.chi_r * g.dr, ne, R, g.chi_r,
                 sR, 0.0, y, g.chi_r, sy, B, st, mask, oz, ozb));
@@ -640,21 +579,17 @@ int tnx_batched_env_update(int direction, const double* E_in, int64_t sE, const 
   double* T2 = reinterpret_cast<double*>(static_cast<char*>(workspace) + align_up(size_t(batch) * ne * 8));
   const size_t ozb = bmatvec_oz_bytes(g, batch);
   void* oz = ozb ? static_cast<char*>(workspace) + 2 * align_up(size_t(batch) * ne * 8) : nullptr;
-  const size_t smem = size_t(dl * dr * d * d) * sizeof(double);
   if (direction == 1) {
     TNX_TRY(bgemm(df, true, false, dl * chi_l, d * chi_r, chi_l, 1.0, E_in, dl * chi_l, sE, A, d * chi_r, sA, 0.0, T1,
                   d * chi_r, ne, batch, st, nullptr, oz, ozb));
-    bw_left_kernel<<<dim3(bgrid(chi_l * chi_r, 128, 64), batch), 128, smem, st>>>(T1, ne, W, sW, T2, ne, chi_l,
-                                                                                  int(d), chi_r, int(dl), int(dr));
-    TNX_LAUNCH_CHECK();
+    TNX_TRY(wc::launch_left<double>(T1, ne, W, sW, wc::OutF64{T2}, ne, chi_l, d, chi_r, dl, dr, chi_r * dr, batch,
+                                    nullptr, st));
     TNX_TRY(bgemm(df, true, false, chi_r * dr, chi_r, chi_l * d, 1.0, T2, chi_r * dr, ne, A, chi_r, sA, 0.0, E_out,
                   chi_r, sO, batch, st, nullptr, oz, ozb));
   } else {
     TNX_TRY(bgemm(df, false, false, chi_l * d, dr * chi_r, chi_r, 1.0, A, chi_r, sA, E_in, dr * chi_r, sE, 0.0, T1,
                   dr * chi_r, ne, batch, st, nullptr, oz, ozb));
-    bw_right_kernel<<<dim3(bgrid(chi_l * chi_r, 128, 64), batch), 128, smem, st>>>(T1, ne, W, sW, T2, ne, chi_l,
-                                                                                   int(d), chi_r, int(dl), int(dr));
-    TNX_LAUNCH_CHECK();
+    TNX_TRY(wc::launch_right<double>(T1, ne, W, sW, T2, ne, chi_l, d, chi_r, dl, dr, batch, st));
     TNX_TRY(bgemm(df, false, true, chi_l * dl, chi_l, d * chi_r, 1.0, T2, d * chi_r, ne, A, d * chi_r, sA, 0.0, E_out,
                   chi_l, sO, batch, st, nullptr, oz, ozb));
   }

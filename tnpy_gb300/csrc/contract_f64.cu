@@ -13,6 +13,7 @@
 #include <mutex>
 
 #include "tnx_internal.cuh"
+#include "wcontract.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -283,93 +284,17 @@ int gemm_f64_splitk(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double al
   return TNX_OK;
 }
 
-// ---------------------------------------------------------------------------------
-// MPO step. The MPO tensor (at most 32 x 32 x 2 x 2 here) is staged in shared memory;
-// each thread owns one (a', c) [left form] or (a, c') [right form] fibre and produces
-// all dr*d (dl*d) outputs from its dl*d (dr*d) inputs.
-// ---------------------------------------------------------------------------------
-namespace {
-constexpr int WMAX = 64;  // max dl*d and dr*d handled per thread
-
-__global__ void wcontract_left_kernel(const double* __restrict__ T1, const double* __restrict__ W,
-                                      double* __restrict__ T2, int64_t chi_l, int d, int64_t chi_r,
-                                      int dl, int dr) {
-  extern __shared__ double ws[];
-  const int wn = dl * dr * d * d;
-  for (int i = threadIdx.x; i < wn; i += blockDim.x) ws[i] = W[i];
-  __syncthreads();
-  const int64_t total = chi_l * chi_r;
-  for (int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
-       idx += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t ap = idx / chi_r, c = idx % chi_r;
-    double in[WMAX];
-    // T1[(w,a'),(s,c)] at ((w*chi_l + a')*d + s)*chi_r + c
-    for (int w = 0; w < dl; ++w)
-      for (int s = 0; s < d; ++s) in[w * d + s] = T1[((w * chi_l + ap) * d + s) * chi_r + c];
-    // T2[(a',s'),(c,v)] at ((a'*d + s')*chi_r + c)*dr + v
-    for (int sp = 0; sp < d; ++sp) {
-      double* out = T2 + ((ap * d + sp) * chi_r + c) * dr;
-      for (int v = 0; v < dr; ++v) {
-        double acc = 0.0;
-        for (int w = 0; w < dl; ++w)
-          for (int s = 0; s < d; ++s) acc = fma(in[w * d + s], ws[((w * dr + v) * d + s) * d + sp], acc);
-        out[v] = acc;
-      }
-    }
-  }
-}
-
-__global__ void wcontract_right_kernel(const double* __restrict__ T1, const double* __restrict__ W,
-                                       double* __restrict__ T2, int64_t chi_l, int d, int64_t chi_r,
-                                       int dl, int dr) {
-  extern __shared__ double ws[];
-  const int wn = dl * dr * d * d;
-  for (int i = threadIdx.x; i < wn; i += blockDim.x) ws[i] = W[i];
-  __syncthreads();
-  const int64_t total = chi_l * chi_r;
-  for (int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
-       idx += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t a = idx / chi_r, cp = idx % chi_r;
-    double in[WMAX];
-    // T1[(a,s),(v,c')] at ((a*d + s)*dr + v)*chi_r + c'
-    for (int s = 0; s < d; ++s)
-      for (int v = 0; v < dr; ++v) in[v * d + s] = T1[((a * d + s) * dr + v) * chi_r + cp];
-    // T2[(a,w),(s',c')] at ((a*dl + w)*d + s')*chi_r + c'
-    for (int w = 0; w < dl; ++w)
-      for (int sp = 0; sp < d; ++sp) {
-        double acc = 0.0;
-        for (int v = 0; v < dr; ++v)
-          for (int s = 0; s < d; ++s) acc = fma(in[v * d + s], ws[((w * dr + v) * d + s) * d + sp], acc);
-        T2[((a * dl + w) * d + sp) * chi_r + cp] = acc;
-      }
-  }
-}
-
-inline unsigned grid_for(int64_t total, int threads) {
-  int64_t b = (total + threads - 1) / threads;
-  if (b > 152 * 16) b = 152 * 16;
-  return (unsigned)(b < 1 ? 1 : b);
-}
-}  // namespace
-
+// MPO step of one site (wcontract.cuh)
 int wcontract_left(const double* T1, const double* W, double* T2, int64_t chi_l, int64_t d,
                    int64_t chi_r, int64_t dl, int64_t dr, cudaStream_t st) {
-  TNX_CHECK_SHAPE(dl * d <= WMAX && dr * d <= WMAX, "MPO bond too large (dl*d, dr*d <= %d)", WMAX);
-  size_t smem = size_t(dl * dr * d * d) * sizeof(double);
-  wcontract_left_kernel<<<grid_for(chi_l * chi_r, 128), 128, smem, st>>>(T1, W, T2, chi_l, (int)d, chi_r,
-                                                                          (int)dl, (int)dr);
-  TNX_LAUNCH_CHECK();
-  return TNX_OK;
+  TNX_CHECK_SHAPE(dl * d <= 64 && dr * d <= 64, "MPO bond too large (dl*d, dr*d <= %d)", 64);
+  return wc::launch_left<double>(T1, 0, W, 0, wc::OutF64{T2}, 0, chi_l, d, chi_r, dl, dr, chi_r * dr, 1, nullptr, st);
 }
 
 int wcontract_right(const double* T1, const double* W, double* T2, int64_t chi_l, int64_t d,
                     int64_t chi_r, int64_t dl, int64_t dr, cudaStream_t st) {
-  TNX_CHECK_SHAPE(dl * d <= WMAX && dr * d <= WMAX, "MPO bond too large (dl*d, dr*d <= %d)", WMAX);
-  size_t smem = size_t(dl * dr * d * d) * sizeof(double);
-  wcontract_right_kernel<<<grid_for(chi_l * chi_r, 128), 128, smem, st>>>(T1, W, T2, chi_l, (int)d, chi_r,
-                                                                           (int)dl, (int)dr);
-  TNX_LAUNCH_CHECK();
-  return TNX_OK;
+  TNX_CHECK_SHAPE(dl * d <= 64 && dr * d <= 64, "MPO bond too large (dl*d, dr*d <= %d)", 64);
+  return wc::launch_right<double>(T1, 0, W, 0, T2, 0, chi_l, d, chi_r, dl, dr, 1, st);
 }
 
 int64_t matvec1_scratch_elems(int64_t chi_l, int64_t d, int64_t chi_r, int64_t dl, int64_t dr) {

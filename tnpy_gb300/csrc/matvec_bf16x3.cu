@@ -30,6 +30,7 @@
 
 #include "tc_ptx.cuh"
 #include "tnx_internal.cuh"
+#include "wcontract.cuh"
 
 namespace tnx {
 namespace {
@@ -214,35 +215,6 @@ __global__ void split_transpose_kernel(const T* __restrict__ src, int64_t rows, 
       const __nv_bfloat16 h = __double2bfloat16(v);
       hi[c * ldp + r] = h;
       lo[c * ldp + r] = __double2bfloat16(v - double(__bfloat162float(h)));
-    }
-  }
-}
-
-// T2 split operand: A3[(a',s')][(c,v)] (row pitch ldp) from T1 (FP32, [(w,a')][(s,c)]).
-__global__ void wcontract_split_kernel(const float* __restrict__ T1, const double* __restrict__ W,
-                                       __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo,
-                                       int64_t chi_l, int d, int64_t chi_r, int dl, int dr, int64_t ldp) {
-  extern __shared__ float wsf[];
-  const int wn = dl * dr * d * d;
-  for (int i = threadIdx.x; i < wn; i += blockDim.x) wsf[i] = float(W[i]);
-  __syncthreads();
-  const int64_t total = chi_l * chi_r;
-  for (int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
-       idx += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t ap = idx / chi_r, c = idx % chi_r;
-    float in[64];
-    for (int w = 0; w < dl; ++w)
-      for (int s = 0; s < d; ++s) in[w * d + s] = T1[((w * chi_l + ap) * d + s) * chi_r + c];
-    for (int sp = 0; sp < d; ++sp) {
-      const int64_t o = (ap * d + sp) * ldp + c * dr;
-      for (int v = 0; v < dr; ++v) {
-        float acc = 0.f;
-        for (int w = 0; w < dl; ++w)
-          for (int s = 0; s < d; ++s) acc = fmaf(in[w * d + s], wsf[((w * dr + v) * d + s) * d + sp], acc);
-        const __nv_bfloat16 h = __float2bfloat16_rn(acc);
-        hi[o + v] = h;
-        lo[o + v] = __float2bfloat16_rn(acc - __bfloat162float(h));
-      }
     }
   }
 }
@@ -449,16 +421,9 @@ int mixed_apply_t(const double* W, const T* x, T* y, int64_t chi_l, int64_t d, i
     };
     TNX_TRY(autotuned(TuneKey{3, m.M1, m.N1, m.K1p, 0, 0}, 2, m.N1 >= 256 ? 0 : 1, m.N1 >= 256, st, run));
   }
-  // step 2: MPO contraction into the split A3 operand
-  {
-    int64_t total = chi_l * chi_r;
-    int64_t blocks = (total + 127) / 128;
-    if (blocks > 152 * 16) blocks = 152 * 16;
-    size_t smem = size_t(dl * dr * d * d) * sizeof(float);
-    wcontract_split_kernel<<<unsigned(blocks), 128, smem, st>>>(m.T1, W, m.a3h, m.a3l, chi_l, int(d), chi_r,
-                                                                 int(dl), int(dr), m.K3p);
-    TNX_LAUNCH_CHECK();
-  }
+  // step 2: MPO contraction into the split A3 operand, [(a',s')][(c,v)] with row pitch K3p (wcontract.cuh)
+  TNX_TRY((wc::launch_left<float>(m.T1, 0, W, 0, wc::OutSplit{m.a3h, m.a3l}, 0, chi_l, d, chi_r, dl, dr, m.K3p, 1,
+                                  nullptr, st)));
   // step 3: y = A3 . B3^T (FP32 accumulators written as T); tiles autotuned per shape
   {
     auto run = [&](int v) -> int {
