@@ -295,8 +295,11 @@ __global__ void __launch_bounds__(DT) lincomb_kernel(const T* __restrict__ V, co
   }
 }
 
+// CTAs of a vector kernel: one element per thread until two CTAs fill every SM. The FP64 pipe takes
+// a warp's FMA in 64 clocks, so a Ritz vector over 24 basis vectors at n = 2048 took 18 us on 2 CTAs
+// (four elements per thread) and takes 6.5 us on 8.
 inline int nchunk_for(int64_t n) {
-  int64_t c = (n + DT * 4 - 1) / (DT * 4);
+  int64_t c = (n + DT - 1) / DT;
   if (c > 2 * 152) c = 2 * 152;
   return int(c < 1 ? 1 : c);
 }

@@ -198,7 +198,7 @@ int tnx_eigh_batched(double* A, const int64_t* offsets, const int* sizes, int ba
     set_error("tnx_eigh_batched: workspace %zu bytes < required %zu", workspace_bytes, need);
     return TNX_ERR_WORKSPACE;
   }
-  if (batch == 1 && keep == 1 && max_size <= 64)  // one small matrix, lowest pair: one-warp path
+  if (batch == 1 && keep == 1 && max_size <= 64)  // one small matrix, lowest pair
     return rr_lowest_f64(A, max_size, max_size, evals, evecs, as_stream(stream));
   return eigh_small_f64(A, offsets, sizes, batch, max_size, keep, evals, evecs,
                         static_cast<double*>(workspace), as_stream(stream));
@@ -207,65 +207,72 @@ int tnx_eigh_batched(double* A, const int64_t* offsets, const int* sizes, int ba
 }  // extern "C"
 
 // ---------------------------------------------------------------------------------------
-// Lowest eigenpair of a small symmetric matrix (n <= 64) with one warp.
+// Lowest eigenpair of small symmetric matrices (n <= 64), one CTA of 256 threads each: the
+// Davidson Rayleigh-Ritz problem and the dense effective Hamiltonians of the chain ends.
 //
-// GB300 issues FP64 at ~2 FMA/clock/SM, so an FP64 Jacobi on one SM costs ~n^3 * sweeps
-// FP64 clocks (~100 us at n = 24). Here the Jacobi sweeps run in FP32 (64x the issue
-// rate), and the lowest eigenpair is then refined in FP64 against the FP64 matrix:
+// An FP64 instruction holds its sub-partition's pipe for 64 clocks on GB300 (2 FMAs per clock and
+// SM), an FP32 one for one, so the Jacobi sweeps run in FP32 and the lowest pair is then refined
+// against the FP64 matrix,
 //   s <- s - sum_{j != 0} v_j (v_j . r) / (lambda_j - theta),  r = A s - theta s,
 // which contracts the error by ~(FP32 eigenvector error) per step; three steps reach
 // FP64 accuracy for a non-degenerate lowest eigenvalue, and theta = s^T A s is FP64.
-// Used for the Davidson Rayleigh-Ritz problem and the dense effective Hamiltonians
-// of the chain ends.
+// Only s, r, theta and the norm are FP64: the correction's relative error of ~1e-6 is what the
+// FP32 eigenvectors leave it anyway, and the next step works it off.
+//
+// A round of the sweep is two barriers long: the angles (one thread per pair), then every 2 x 2
+// block (pair k, pair l) of A <- J^T A J by one thread, columns first as in the two-pass form, so
+// each entry sees the operations of the two-pass form. A random 24 x 24 matrix: 211 us with a pass and a barrier each for
+// columns, rows and zeroing, exact divisions and the correction in FP64, 87 us so; 64 x 64: 1.90 ms
+// and 0.54 ms; the mean over a chi = 32 eigensolve's 68 problems 93 and 50 us.
 // ---------------------------------------------------------------------------------------
 namespace tnx {
 namespace {
 
 constexpr int RW_MAX = 64;
 
-constexpr int RR_T = 128;  // threads of the Rayleigh-Ritz kernel
+constexpr int RR_T = 256;  // threads of the Rayleigh-Ritz kernel
+constexpr int RR_G = RR_T / 32;
 
-// Lowest eigenpair of a small symmetric matrix (n <= 64): parallel-ordered cyclic Jacobi in
-// FP32 (the rotation angles of one round by one thread per pair, the row and column updates
-// spread over all threads), then three FP64 correction steps of the lowest Ritz vector against
-// the FP32 eigenbasis, s <- s - sum_j v_j (v_j . r) / (l_j - theta), and the FP64 Rayleigh
-// quotient. FP32 rounding keeps regenerating off-diagonal entries at ~6e-8 |A|_F, so the sweeps
+// FP32 rounding keeps regenerating off-diagonal entries at ~6e-8 |A|_F, so the sweeps
 // stop once every off-diagonal entry is below 1e-6 |A|_F; the FP64 steps take it from there.
-// Batched form: block b solves the matrix at A + b sA into eval[b sE], evec + b sV, and returns at
+// Block b solves the matrix at A + b sA into eval[b sE], evec + b sV, and returns at
 // once when active is given and active[b] == 0.
-__global__ void __launch_bounds__(RR_T) rr_lowest_warp_kernel(const double* __restrict__ A, int n, int ld,
-                                                            double* __restrict__ eval, double* __restrict__ evec,
-                                                            int64_t sA, int64_t sE, int64_t sV,
-                                                            const int* __restrict__ active) {
+__global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restrict__ A, int n, int ld,
+                                                         double* __restrict__ eval, double* __restrict__ evec,
+                                                         int64_t sA, int64_t sE, int64_t sV,
+                                                         const int* __restrict__ active) {
   if (active && !active[blockIdx.x]) return;
   A += int64_t(blockIdx.x) * sA;
   eval += int64_t(blockIdx.x) * sE;
   evec += int64_t(blockIdx.x) * sV;
   extern __shared__ double sm_d[];
-  double* Ad = sm_d;                                      // n x n FP64
-  float* Af = reinterpret_cast<float*>(Ad + n * n);       // n x (n+1) FP32
-  float* Vf = Af + n * (n + 1);                           // n x (n+1) FP32
-  double* s = reinterpret_cast<double*>(Vf + n * (n + 1) + ((n * (n + 1)) & 1));  // n FP64 (8-byte aligned)
-  double* r = s + n;                                      // n
-  double* f = r + n;                                      // n correction coefficients
+  const int nf = n + 1;
+  double* Ad = sm_d;                                      // n x (n+1) FP64
+  double* s = Ad + n * nf;                                // n
+  double* rp = s + n;                                     // partial products, RR_G x n
+  float* Af = reinterpret_cast<float*>(rp + RR_G * n);       // n x (n+1) FP32
+  float* Vf = Af + n * nf;                                // n x (n+1) FP32
+  float* rf = Vf + n * nf;                                // n: residual
+  float* fp = rf + n;                                     // partial projections, RR_G x n
   __shared__ float cs[32], ss[32];
   __shared__ int pp[32], qq[32];
   __shared__ float red[RR_T / 32];
   __shared__ double redd[RR_T / 32];
   __shared__ int s_any, s_imin;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nf = n + 1;
   float fro = 0.f;
   for (int e = tid; e < n * n; e += RR_T) {
-    const int i = e / n, j = e % n;
+    const int i = e / n, j = e - i * n;
     const double v = A[int64_t(i) * ld + j];
-    Ad[e] = v;
-    Af[i * nf + j] = float(v);
+    const float f = float(v);
+    Ad[i * nf + j] = v;
+    Af[i * nf + j] = f;
     Vf[i * nf + j] = (i == j) ? 1.f : 0.f;
-    fro += float(v) * float(v);
+    fro += f * f;
   }
   for (int o = 16; o > 0; o >>= 1) fro += __shfl_xor_sync(0xffffffffu, fro, o);
   if (lane == 0) red[warp] = fro;
+  if (tid == 0) s_any = 0;
   __syncthreads();
   fro = 0.f;
   for (int w = 0; w < RR_T / 32; ++w) fro += red[w];
@@ -273,21 +280,25 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_warp_kernel(const double* __re
   const float thresh = 1e-6f * fro;
   if (n > 1) {
     const int np = n + (n & 1), npairs = np / 2;
-    if (tid == 0) s_any = 0;
-    __syncthreads();
+    const int tx = tid & 15, ty = tid >> 4;
     for (int sweep = 0; sweep < 30; ++sweep) {
       for (int rnd = 0; rnd < np - 1; ++rnd) {
         if (tid < npairs) {
-          int p = tid == 0 ? 0 : 1 + (tid - 1 + rnd) % (np - 1);
-          int q = 1 + (np - 1 - tid - 1 + rnd) % (np - 1);
+          // round robin: 0 stays, the others turn by one player a round
+          const int m1 = np - 1;
+          int p = tid - 1 + rnd, q = np - 2 - tid + rnd;
+          p = tid == 0 ? 0 : 1 + (p >= m1 ? p - m1 : p);
+          q = 1 + (q >= m1 ? q - m1 : q);
           if (p > q) { int t = p; p = q; q = t; }
           float c = 1.f, sn = 0.f;
           if (q < n) {
             const float apq = Af[p * nf + q], app = Af[p * nf + p], aqq = Af[q * nf + q];
-            if (fabsf(apq) > thresh) {
-              const float th = (aqq - app) / (2.f * apq);
-              const float t = (th >= 0.f ? 1.f : -1.f) / (fabsf(th) + sqrtf(1.f + th * th));
-              c = 1.f / sqrtf(1.f + t * t);
+            if (fabsf(apq) > thresh) {  // |th| < 1e6 then, and th^2 is far from overflow
+              // approximate reciprocals (a few ulp): the FP64 steps correct what the sweeps leave
+              const float th = __fdividef(0.5f * (aqq - app), apq);
+              const float h2 = fmaf(th, th, 1.f);
+              const float t = copysignf(__fdividef(1.f, fmaf(h2, rsqrtf(h2), fabsf(th))), th);
+              c = rsqrtf(fmaf(t, t, 1.f));
               sn = t * c;
               s_any = 1;
             }
@@ -295,36 +306,46 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_warp_kernel(const double* __re
           pp[tid] = p; qq[tid] = q; cs[tid] = c; ss[tid] = sn;
         }
         __syncthreads();
-        // A <- A J: columns p, q (pairs touch disjoint columns)
-        for (int e = tid; e < npairs * n; e += RR_T) {
-          const int k = e / n, i = e % n;
-          const float sn = ss[k];
-          if (sn == 0.f) continue;
-          const int p = pp[k], q = qq[k];
-          const float c = cs[k];
-          const float a = Af[i * nf + p], b = Af[i * nf + q];
-          Af[i * nf + p] = c * a - sn * b;
-          Af[i * nf + q] = sn * a + c * b;
+        // A <- J^T (A J): block (rows of pair k, columns of pair l); the padding player of an odd n
+        // (index n) has no entries
+        for (int k = ty; k < npairs; k += RR_T / 16) {
+          const float sk = ss[k], ck = cs[k];
+          const int pk = pp[k], qk = qq[k];
+          for (int l = tx; l < npairs; l += 16) {
+            const float sl = ss[l], cl = cs[l];
+            if (sk == 0.f && sl == 0.f) continue;
+            const int pl = pp[l], ql = qq[l];
+            const bool row2 = qk < n, col2 = ql < n;
+            float* r0 = Af + pk * nf;
+            float* r1 = Af + qk * nf;
+            float a = r0[pl], b = col2 ? r0[ql] : 0.f, c = row2 ? r1[pl] : 0.f, d = row2 && col2 ? r1[ql] : 0.f;
+            if (sl != 0.f) {
+              const float a1 = cl * a - sl * b, b1 = sl * a + cl * b;
+              const float c1 = cl * c - sl * d, d1 = sl * c + cl * d;
+              a = a1; b = b1; c = c1; d = d1;
+            }
+            if (sk != 0.f) {
+              const float a1 = ck * a - sk * c, c1 = sk * a + ck * c;
+              const float b1 = ck * b - sk * d, d1 = sk * b + ck * d;
+              a = a1; b = b1; c = c1; d = d1;
+            }
+            if (k == l) b = c = 0.f;  // the entry this rotation removes
+            r0[pl] = a;
+            if (col2) r0[ql] = b;
+            if (row2) r1[pl] = c;
+            if (row2 && col2) r1[ql] = d;
+          }
         }
-        __syncthreads();
-        // A <- J^T A: rows p, q (disjoint rows); V <- V J
-        for (int e = tid; e < npairs * n; e += RR_T) {
-          const int k = e / n, j = e % n;
-          const float sn = ss[k];
-          if (sn == 0.f) continue;
-          const int p = pp[k], q = qq[k];
-          const float c = cs[k];
-          const float a = Af[p * nf + j], b = Af[q * nf + j];
-          Af[p * nf + j] = c * a - sn * b;
-          Af[q * nf + j] = sn * a + c * b;
-          const float va = Vf[j * nf + p], vb = Vf[j * nf + q];
-          Vf[j * nf + p] = c * va - sn * vb;
-          Vf[j * nf + q] = sn * va + c * vb;
-        }
-        __syncthreads();
-        if (tid < npairs && ss[tid] != 0.f) {
-          Af[pp[tid] * nf + qq[tid]] = 0.f;
-          Af[qq[tid] * nf + pp[tid]] = 0.f;
+        // V <- V J
+        for (int l = ty; l < npairs; l += RR_T / 16) {
+          const float sl = ss[l], cl = cs[l];
+          if (sl == 0.f) continue;
+          const int pl = pp[l], ql = qq[l];
+          for (int j = tx; j < n; j += 16) {
+            const float va = Vf[j * nf + pl], vb = Vf[j * nf + ql];
+            Vf[j * nf + pl] = cl * va - sl * vb;
+            Vf[j * nf + ql] = sl * va + cl * vb;
+          }
         }
         __syncthreads();
       }
@@ -336,69 +357,113 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_warp_kernel(const double* __re
       __syncthreads();
     }
   }
-  // lowest FP32 eigenvalue
-  if (tid == 0) {
-    int imin = 0;
-    float dmin = Af[0];
-    for (int i = 1; i < n; ++i)
-      if (Af[i * nf + i] < dmin) { dmin = Af[i * nf + i]; imin = i; }
-    s_imin = imin;
+  // lowest FP32 eigenvalue (the first of equal ones), by warp 0
+  if (warp == 0) {
+    int im = lane < n ? lane : 0;
+    float dm = Af[im * nf + im];
+    if (lane + 32 < n && Af[(lane + 32) * nf + lane + 32] < dm) {
+      im = lane + 32;
+      dm = Af[im * nf + im];
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const float od = __shfl_xor_sync(0xffffffffu, dm, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, im, o);
+      if (od < dm || (od == dm && oi < im)) {
+        dm = od;
+        im = oi;
+      }
+    }
+    if (lane == 0) s_imin = im;
   }
   __syncthreads();
   const int imin = s_imin;
   for (int i = tid; i < n; i += RR_T) s[i] = double(Vf[i * nf + imin]);
   __syncthreads();
-  const double floor = 1e-6 * (double(fro) + 1e-300);
-  double theta = 0.0;
+  const float floor = 1e-6f * fro;
+  // warp g takes columns g, g + RR_G, ... of a product; the partial sums are added in group order
+  auto sum_d = [&](int i) {
+    double t = rp[i];
+#pragma unroll
+    for (int g = 1; g < RR_G; ++g) t += rp[g * n + i];
+    return t;
+  };
+  auto sum_f = [&](int i) {
+    float t = fp[i];
+#pragma unroll
+    for (int g = 1; g < RR_G; ++g) t += fp[g * n + i];
+    return t;
+  };
   for (int step = 0; step < 4; ++step) {
-    // normalise s (n <= 64 entries: summed by every warp redundantly), r = A s, theta = s . r
-    double nn = 0.0;
-    for (int i = lane; i < n; i += 32) nn += s[i] * s[i];
-    for (int o = 16; o > 0; o >>= 1) nn += __shfl_xor_sync(0xffffffffu, nn, o);
-    __syncthreads();
-    const double inv = 1.0 / sqrt(nn);
-    for (int i = tid; i < n; i += RR_T) s[i] *= inv;
-    __syncthreads();
-    double th = 0.0;
-    for (int i = tid; i < n; i += RR_T) {
+    // y = A s, then |s|^2 and s . y together (n <= 64: the entries sit in warps 0 and 1)
+    for (int i = lane; i < n; i += 32) {
       double acc = 0.0;
-      for (int j = 0; j < n; ++j) acc = fma(Ad[i * n + j], s[j], acc);
-      r[i] = acc;
-      th = fma(acc, s[i], th);
-    }
-    for (int o = 16; o > 0; o >>= 1) th += __shfl_xor_sync(0xffffffffu, th, o);
-    if (lane == 0) redd[warp] = th;
-    __syncthreads();
-    th = 0.0;
-    for (int w = 0; w < RR_T / 32; ++w) th += redd[w];
-    theta = th;
-    if (step == 3) break;
-    for (int i = tid; i < n; i += RR_T) r[i] -= theta * s[i];
-    __syncthreads();
-    // f_j = (v_j . r) / (l_j - theta), one warp per j; (near-)degenerate partners keep f_j = 0
-    for (int j = warp; j < n; j += RR_T / 32) {
-      double dot = 0.0;
-      for (int i = lane; i < n; i += 32) dot = fma(double(Vf[i * nf + j]), r[i], dot);
-      for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-      const double den = double(Af[j * nf + j]) - theta;
-      if (lane == 0) f[j] = (j != imin && fabs(den) >= floor) ? dot / den : 0.0;
+      for (int j = warp; j < n; j += RR_G) acc = fma(Ad[i * nf + j], s[j], acc);
+      rp[warp * n + i] = acc;
     }
     __syncthreads();
-    for (int i = tid; i < n; i += RR_T) {
-      double acc = s[i];
-      for (int j = 0; j < n; ++j) acc = fma(-f[j], double(Vf[i * nf + j]), acc);
-      s[i] = acc;
+    double yi = 0.0, si = 0.0;
+    if (warp < 2) {
+      if (tid < n) {
+        yi = sum_d(tid);
+        si = s[tid];
+      }
+      double nn = 0.0, sy = 0.0;
+      if (warp * 32 < n) {
+        nn = si * si;
+        sy = si * yi;
+        for (int o = 16; o > 0; o >>= 1) {
+          nn += __shfl_xor_sync(0xffffffffu, nn, o);
+          sy += __shfl_xor_sync(0xffffffffu, sy, o);
+        }
+      }
+      if (lane == 0) {
+        redd[warp] = nn;
+        redd[2 + warp] = sy;
+      }
     }
+    __syncthreads();
+    const double nn = redd[0] + redd[1];
+    // 1 / sqrt(nn) from an FP32 seed by two Newton steps
+    double inv = double(rsqrtf(float(nn)));
+    inv = inv * fma(-0.5 * nn * inv, inv, 1.5);
+    inv = inv * fma(-0.5 * nn * inv, inv, 1.5);
+    const double theta = (redd[2] + redd[3]) * (inv * inv);
+    if (tid < n) s[tid] = si * inv;
+    if (step == 3) {
+      if (tid == 0) eval[0] = theta;
+      break;
+    }
+    if (tid < n) rf[tid] = float(fma(-theta, si, yi) * inv);
+    __syncthreads();
+    // f_j = (v_j . r) / (l_j - theta); (near-)degenerate partners keep f_j = 0
+    for (int j = lane; j < n; j += 32) {
+      float acc = 0.f;
+      for (int i = warp; i < n; i += RR_G) acc = fmaf(Vf[i * nf + j], rf[i], acc);
+      fp[warp * n + j] = acc;
+    }
+    __syncthreads();
+    for (int j = tid; j < n; j += RR_T) {
+      const float den = float(double(Af[j * nf + j]) - theta);
+      const float dot = sum_f(j);
+      rf[j] = (j != imin && fabsf(den) >= floor) ? dot / den : 0.f;
+    }
+    __syncthreads();
+    for (int i = lane; i < n; i += 32) {
+      float acc = 0.f;
+      for (int j = warp; j < n; j += RR_G) acc = fmaf(Vf[i * nf + j], rf[j], acc);
+      fp[warp * n + i] = acc;
+    }
+    __syncthreads();
+    for (int i = tid; i < n; i += RR_T) s[i] -= double(sum_f(i));
     __syncthreads();
   }
-  if (tid == 0) eval[0] = theta;
-  for (int i = tid; i < n; i += RR_T) evec[i] = s[i];
+  if (tid < n) evec[tid] = s[tid];  // the thread's own entry
 }
 
 }  // namespace
 
 size_t rr_lowest_smem(int n) {
-  return size_t(n) * n * 8 + 2 * size_t(n) * (n + 1) * 4 + 8 + 3 * size_t(n) * 8;
+  return size_t(n) * (n + 1) * 16 + size_t(n) * ((1 + RR_G) * 8 + (1 + RR_G) * 4);
 }
 
 int rr_lowest_f64(const double* A, int n, int ld, double* eval, double* evec, cudaStream_t st) {
@@ -415,11 +480,11 @@ int rr_lowest_f64_batched(const double* A, int n, int ld, int64_t sA, double* ev
   static std::atomic<bool> attr{false};  // idempotent setup; threads may race to it
   const size_t smem = rr_lowest_smem(RW_MAX);
   if (!attr.load()) {
-    TNX_CUDA(cudaFuncSetAttribute(rr_lowest_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    TNX_CUDA(cudaFuncSetAttribute(rr_lowest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     attr.store(true);
   }
   profile_mark(KF_EIGH, st, true);
-  rr_lowest_warp_kernel<<<batch, RR_T, rr_lowest_smem(n), st>>>(A, n, ld, eval, evec, sA, sE, sV, active);
+  rr_lowest_kernel<<<batch, RR_T, rr_lowest_smem(n), st>>>(A, n, ld, eval, evec, sA, sE, sV, active);
   profile_mark(KF_EIGH, st, false);
   TNX_LAUNCH_CHECK();
   return TNX_OK;

@@ -236,7 +236,7 @@ int eigh_small_f64_ld(const double* A, const int64_t* offsets, const int* sizes,
 // single n x n matrix with leading dimension ld; evecs as [n][keep], work 2*n*n doubles
 int eigh_small_f64_uniform(const double* A, int n, int ld, int keep, double* evals, double* evecs,
                            double* work, cudaStream_t st);
-// lowest eigenpair of one n x n (n <= 64) matrix, one warp: FP32 Jacobi + FP64 refinement
+// lowest eigenpair of one n x n (n <= 64) matrix: FP32 Jacobi + FP64 refinement
 int rr_lowest_f64(const double* A, int n, int ld, double* eval, double* evec, cudaStream_t st);
 // the same for `batch` matrices at A + b sA (results at eval + b sE, evec + b sV); blocks whose
 // active[b] is 0 return at once (active may be null)
