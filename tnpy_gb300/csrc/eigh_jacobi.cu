@@ -1,12 +1,30 @@
 // Dense symmetric eigensolver, one CTA per matrix: parallel cyclic Jacobi (round-robin
 // ordering, n/2 disjoint rotations per round), FP64.
 //
-// Used for the Davidson Rayleigh-Ritz problem (size <= max_basis), the dense
-// effective-Hamiltonian path of FiniteDMRG.one_site_solver (tnpy/finite_dmrg.py:108-110,
-// linalg.eigh at tnpy/linalg.py:42-61, N < 200) and tSDRG blocks (np.linalg.eigh at
-// tnpy/tsdrg.py:584). Jacobi is chosen for these small problems because it needs no
-// tridiagonal stage, reaches full FP64 accuracy and keeps every rotation of a round
+// Used for the dense effective-Hamiltonian path of FiniteDMRG.one_site_solver
+// (tnpy/finite_dmrg.py:108-110, linalg.eigh at tnpy/linalg.py:42-61, N < 200) and tSDRG blocks
+// (np.linalg.eigh at tnpy/tsdrg.py:584). Jacobi is chosen for these small problems because it needs
+// no tridiagonal stage, reaches full FP64 accuracy and keeps every rotation of a round
 // independent, so all threads of the CTA work on one round at a time.
+//
+// What bounds it: an FP64 instruction holds its sub-partition's pipe for 64 clocks (2 FMAs per clock
+// and SM), also in the one warp that computes a round's angles, where square roots and divisions
+// are dozens of them. So
+//   * A and V live in shared memory up to n = 112 (odd row stride), in the workspace above;
+//   * an angle is an FP32 tangent (approximate reciprocal and root, exponents aligned by integer
+//     arithmetic) taken to FP64 accuracy by two corrections against a_pq t^2 + d t - a_pq = 0, and
+//     c = 1 / sqrt(1 + t^2) from an FP32 seed by one third-order step: 17 FP64 instructions, where
+//     the divisions and roots took over 60;
+//   * only the upper triangle of A is held and updated, a 2 x 2 block (pair k, pair l) by one thread
+//     (columns, then rows, as the two-pass form), diagonal blocks by a_pp -= t a_pq, a_qq += t a_pq;
+//   * the blocks that change are queued first (n <= 64), so that their threads fill whole warps: a
+//     warp's FP64 instruction costs the same with one active lane, and a conserved quantity leaves
+//     most blocks zero;
+//   * V of round r is updated while warp 0 computes the angles of round r + 1, by the warps of the
+//     other three sub-partitions, so it does not wait for warp 0's pipe: two barriers a round.
+// 128 tSDRG blocks of 64 x 64 (one conserved quantity): 3.02 ms with A and V in the workspace, exact
+// angles and full passes over A, 1.00 ms so (1.25 ms without the queue); 64 random dense 64 x 64
+// matrices 7.9 and 3.0 ms; one 199 x 199 156 and 128 ms.
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -18,154 +36,317 @@ namespace {
 
 constexpr int EJ_THREADS = 512;
 constexpr int EJ_MAX_SWEEPS = 40;
+constexpr int EJ_MAX_N = 1024;   // largest matrix
+constexpr int EJ_SHARED_N = 112;  // largest matrix whose A and V fit in shared memory
 
-// round-robin (circle method) position j of round r for np (even) players
-__device__ __forceinline__ int rr_player(int j, int r, int np) {
-  return j == 0 ? 0 : 1 + (j - 1 + r) % (np - 1);
+// row stride in shared memory: odd, so that a column's entries fall on distinct banks
+__host__ __device__ constexpr int ej_ld(int n) { return n | 1; }
+constexpr size_t ej_smem_bytes(int n) { return size_t(2) * n * ej_ld(n) * sizeof(double); }
+
+// double <-> float by integer operations (the conversions run on the FP64 pipe): truncated to 24
+// bits, zero below 2^-126; |x| < 2^127
+__device__ __forceinline__ float ej_float(double x) {
+  const unsigned hi = unsigned(__double2hiint(x)), lo = unsigned(__double2loint(x));
+  const int e = int((hi >> 20) & 0x7ffu) - 896;
+  return e <= 0 ? 0.f : __uint_as_float((hi & 0x80000000u) | (unsigned(e) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
+}
+__device__ __forceinline__ double ej_double(float x) {
+  const unsigned u = __float_as_uint(x), m = u & 0x7fffffffu;
+  if (m < 0x00800000u) return 0.0;
+  return __hiloint2double(int((u & 0x80000000u) | ((m >> 3) + (896u << 20))), int(m << 29));
+}
+// x 2^-e for |x| 2^-e < 2^1023; zero where it would be subnormal
+__device__ __forceinline__ double ej_scale(double x, int e) {
+  const int hi = __double2hiint(x), ex = ((hi >> 20) & 0x7ff) - e;
+  return ex <= 0 ? 0.0 : __hiloint2double(hi - (e << 20), __double2loint(x));
+}
+
+// Rotation that zeroes a_pq: t = tan, c, s with |t| <= 1; d = a_qq - a_pp (d = 0: t = 1)
+__device__ __forceinline__ void ej_angle(double apq, double d, double& t, double& c, double& s) {
+  const int ea = (__double2hiint(apq) >> 20) & 0x7ff, ed = (__double2hiint(d) >> 20) & 0x7ff;
+  const int e = max(ea, ed) - 1023;  // both below 2 after the scaling, the larger one above 1
+  const double a1 = ej_scale(apq, e), d1 = ej_scale(d, e);
+  const float af = ej_float(a1), df = ej_float(d1), a2 = 2.f * af;
+  float tf = 1.f;
+  double tt = 1.0;
+  if ((__double_as_longlong(d1) << 1) != 0) {
+    const float h = fmaf(df, df, a2 * a2);
+    const unsigned sign = unsigned(__double2hiint(d1)) & 0x80000000u;
+    tf = __uint_as_float(sign | 0x3f800000u) * __fdividef(a2, fmaf(h, rsqrtf(h), fabsf(df)));
+    // corrections against f(t) = a_pq t^2 + d t - a_pq, f' = 2 a_pq t + d
+    const float inv = __fdividef(1.f, fmaf(a2, tf, df));
+    tt = ej_double(tf);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const double f = fma(fma(a1, tt, d1), tt, -a1);
+      tt -= ej_double(ej_float(f) * inv);
+    }
+  }
+  const double y = ej_double(rsqrtf(fmaf(tf, tf, 1.f)));
+  const double r = fma(-fma(tt, tt, 1.0), y * y, 1.0);  // 1 - (1 + t^2) y^2
+  c = fma(y * r, fma(0.375, r, 0.5), y);
+  s = tt * c;
+  t = tt;
+}
+
+// round-robin (circle method) pair k of round r for np (even) players, p < q
+__device__ __forceinline__ void ej_pair(int k, int r, int np, int& p, int& q) {
+  const int m1 = np - 1;
+  p = k - 1 + r;
+  q = np - 2 - k + r;
+  p = k == 0 ? 0 : 1 + (p >= m1 ? p - m1 : p);
+  q = 1 + (q >= m1 ? q - m1 : q);
+  if (p > q) {
+    const int t = p;
+    p = q;
+    q = t;
+  }
 }
 
 // A: matrix b at A + offsets[b], leading dimension lds[b] (or sizes[b] when lds == null).
-// work: per matrix 2*max_size^2 doubles (copy of A and the rotation accumulator V).
+// work (matrices beyond EJ_SHARED_N): per matrix 2*max_size^2 doubles (copy of A and the rotation
+// accumulator V).
 __global__ void __launch_bounds__(EJ_THREADS) jacobi_eigh_kernel(
     const double* __restrict__ A_all, const int64_t* __restrict__ offsets, const int* __restrict__ sizes,
     const int* __restrict__ lds, int n_uniform, int ld_uniform, int max_size, int keep,
     double* __restrict__ evals, double* __restrict__ evecs, double* __restrict__ work) {
+  extern __shared__ double ej_sm[];
   const int b = blockIdx.x;
   const int n = sizes ? sizes[b] : n_uniform;
   const int lda = lds ? lds[b] : (sizes ? n : ld_uniform);
   const double* Ain = A_all + (offsets ? offsets[b] : int64_t(b) * ld_uniform * n_uniform);
-  double* A = work + size_t(b) * 2 * size_t(max_size) * max_size;
-  double* V = A + size_t(max_size) * max_size;
-  const int tid = threadIdx.x, nt = blockDim.x;
+  const bool shared = max_size <= EJ_SHARED_N;
+  const int ld = shared ? ej_ld(n) : n;
+  double* A = shared ? ej_sm : work + size_t(b) * 2 * size_t(max_size) * max_size;
+  double* V = A + (shared ? size_t(n) * ld : size_t(max_size) * max_size);
+  const int tid = threadIdx.x, nt = EJ_THREADS, lane = tid & 31, warp = tid >> 5;
+  constexpr int NW = EJ_THREADS / 32;
 
-  __shared__ double sc[512], ss[512];
-  __shared__ int sp[512], sq[512];
-  __shared__ double red[EJ_THREADS / 32];
-  __shared__ int s_rot;
+  // rotations of the current and the previous round
+  __shared__ double sc[2][EJ_MAX_N / 2], ss[2][EJ_MAX_N / 2];
+  __shared__ int16_t sp[2][EJ_MAX_N / 2], sq[2][EJ_MAX_N / 2];
+  __shared__ double red[NW];
+  __shared__ uint16_t queue[32 * 31 / 2];  // blocks to update (n <= 64)
+  __shared__ int s_count;
+  __shared__ int s_any[2];  // whether the round rotates anything
+  __shared__ int s_rot;     // whether the sweep did
   __shared__ double s_fro;
 
   if (n <= 0) return;
-  // copy A (ld = n) and V = I
   double fro = 0.0;
   for (int e = tid; e < n * n; e += nt) {
-    int i = e / n, j = e % n;
-    double v = Ain[size_t(i) * lda + j];
-    A[e] = v;
-    V[e] = (i == j) ? 1.0 : 0.0;
-    fro += v * v;
+    const int i = e / n, j = e - i * n;
+    const double v = Ain[size_t(i) * lda + j];
+    A[i * ld + j] = v;  // the strict lower triangle is not used
+    V[i * ld + j] = (i == j) ? 1.0 : 0.0;
+    fro = fma(v, v, fro);
   }
   for (int o = 16; o > 0; o >>= 1) fro += __shfl_xor_sync(0xffffffffu, fro, o);
-  if ((tid & 31) == 0) red[tid >> 5] = fro;
+  if (lane == 0) red[warp] = fro;
   __syncthreads();
   if (tid == 0) {
     double t = 0.0;
-    for (int w = 0; w < nt / 32; ++w) t += red[w];
+    for (int w = 0; w < NW; ++w) t += red[w];
     s_fro = sqrt(t);
   }
   __syncthreads();
   // off-diagonal entries below the rounding noise of the rotations (~eps*||A||) are left alone,
-  // so that a sweep can end without any rotation
-  const double abs_floor = 1e-300 + 2e-16 * s_fro;
+  // so that a sweep can end without any rotation (compared as integers: both are positive)
+  const long long floor_bits = __double_as_longlong(1e-300 + 2e-16 * s_fro);
 
+  const int np = n + (n & 1), npairs = np / 2;
+  // V <- V J with the rotations of buffer u, pairs slot, slot + slots, ...
+  auto update_v = [&](int u, int slot, int slots) {
+    for (int l = slot; l < npairs; l += slots) {
+      const double s = ss[u][l];
+      if ((__double_as_longlong(s) << 1) == 0) continue;
+      const double c = sc[u][l];
+      const int p = sp[u][l], q = sq[u][l];
+      for (int j = lane; j < n; j += 32) {
+        const double vp = V[j * ld + p], vq = V[j * ld + q];
+        V[j * ld + p] = fma(c, vp, -s * vq);
+        V[j * ld + q] = fma(s, vp, c * vq);
+      }
+    }
+  };
+  auto at = [&](int i, int j) -> double& { return i < j ? A[i * ld + j] : A[j * ld + i]; };
+  auto bits = [](double x) { return static_cast<unsigned long long>(__double_as_longlong(x)) << 1; };  // 0 for +-0
+  // whether block (k, l) changes: one of the pairs rotates and the block is not all zero (a conserved
+  // quantity keeps most of A exactly zero)
+  auto active = [&](int u, int k, int l) {
+    if ((bits(ss[u][k]) | bits(ss[u][l])) == 0) return false;
+    const int pk = sp[u][k], qk = sq[u][k], pl = sp[u][l], ql = sq[u][l];
+    const bool row2 = qk < n, col2 = ql < n;  // the padding player of an odd n has no entries
+    unsigned long long z = bits(at(pk, pl));
+    if (col2) z |= bits(at(pk, ql));
+    if (row2) z |= bits(at(qk, pl));
+    if (row2 && col2) z |= bits(at(qk, ql));
+    return z != 0;
+  };
+  auto update_block = [&](int u, int k, int l) {
+    const double sk = ss[u][k], sl = ss[u][l];
+    const int pk = sp[u][k], qk = sq[u][k], pl = sp[u][l], ql = sq[u][l];
+    const bool row2 = qk < n, col2 = ql < n;
+    double a = at(pk, pl), b2 = col2 ? at(pk, ql) : 0.0, c2 = row2 ? at(qk, pl) : 0.0,
+           d2 = row2 && col2 ? at(qk, ql) : 0.0;
+    if (bits(sl)) {
+      const double c = sc[u][l], a0 = a, c0 = c2;
+      a = fma(c, a0, -sl * b2);
+      b2 = fma(sl, a0, c * b2);
+      c2 = fma(c, c0, -sl * d2);
+      d2 = fma(sl, c0, c * d2);
+    }
+    if (bits(sk)) {
+      const double c = sc[u][k], a0 = a, b0 = b2;
+      a = fma(c, a0, -sk * c2);
+      c2 = fma(sk, a0, c * c2);
+      b2 = fma(c, b0, -sk * d2);
+      d2 = fma(sk, b0, c * d2);
+    }
+    at(pk, pl) = a;
+    if (col2) at(pk, ql) = b2;
+    if (row2) at(qk, pl) = c2;
+    if (row2 && col2) at(qk, ql) = d2;
+  };
   if (n > 1) {
-    const int np = n + (n & 1);
-    const int npairs = np / 2;
+    bool pending = false;  // the previous round's rotations still to be applied to V
+    int u = 0;
     for (int sweep = 0; sweep < EJ_MAX_SWEEPS; ++sweep) {
       if (tid == 0) s_rot = 0;
-      __syncthreads();
-      for (int r = 0; r < np - 1; ++r) {
-        // rotation parameters for every pair of this round
-        for (int k = tid; k < npairs; k += nt) {
-          int p = rr_player(k, r, np), q = rr_player(np - 1 - k, r, np);
-          if (p > q) { int t = p; p = q; q = t; }
-          double c = 1.0, s = 0.0;
-          if (q < n) {
-            const double apq = A[p * n + q];
-            const double app = A[p * n + p], aqq = A[q * n + q];
-            if (fabs(apq) > abs_floor && fabs(apq) > 1e-16 * sqrt(fabs(app * aqq))) {
-              const double theta = (aqq - app) / (2.0 * apq);
-              const double t = (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(1.0 + theta * theta));
-              c = 1.0 / sqrt(1.0 + t * t);
-              s = t * c;
-              s_rot = 1;
+      if (npairs > 32) __syncthreads();  // other warps than the first set it too
+      for (int r = 0; r < np - 1; ++r, u ^= 1) {
+        // rotations of this round by the first warps, V of the round before by the others: with few
+        // pairs warp 0 alone, and V on the other three sub-partitions (warp mod 4 != 0)
+        if (tid < ((npairs + 31) & ~31)) {
+          const int k = tid;
+          bool rot = false;
+          if (k < npairs) {
+            int p, q;
+            ej_pair(k, r, np, p, q);
+            double c = 1.0, s = 0.0;
+            if (q < n) {
+              const double apq = A[p * ld + q];
+              const long long ab = __double_as_longlong(apq) & 0x7fffffffffffffffLL;
+              if (ab > floor_bits && ab < 0x7ff0000000000000LL) {
+                double t;
+                const double app = A[p * ld + p], aqq = A[q * ld + q];
+                ej_angle(apq, aqq - app, t, c, s);
+                A[p * ld + p] = fma(-t, apq, app);
+                A[q * ld + q] = fma(t, apq, aqq);
+                A[p * ld + q] = 0.0;
+                rot = true;
+              }
+            }
+            sp[u][k] = int16_t(p);
+            sq[u][k] = int16_t(q);
+            sc[u][k] = c;
+            ss[u][k] = s;
+          }
+          const bool any = __any_sync(0xffffffffu, rot);
+          if (npairs <= 32) {
+            if (tid == 0) {
+              s_any[u] = any;
+              s_count = 0;
             }
           }
-          sp[k] = p; sq[k] = q; sc[k] = c; ss[k] = s;
+          if (any && lane == 0) s_rot = 1;
+        }
+        if (npairs <= 32) {
+          if (pending && (warp & 3) != 0) update_v(u ^ 1, warp - 1 - (warp >> 2), NW - NW / 4);
+        } else if (pending) {
+          update_v(u ^ 1, warp, NW);
         }
         __syncthreads();
-        // A <- A P (columns p, q of every row)
-        for (int e = tid; e < npairs * n; e += nt) {
-          int k = e / n, i = e % n;
-          double s = ss[k];
-          if (s == 0.0) continue;
-          int p = sp[k], q = sq[k];
-          double c = sc[k];
-          double aip = A[i * n + p], aiq = A[i * n + q];
-          A[i * n + p] = c * aip - s * aiq;
-          A[i * n + q] = s * aip + c * aiq;
+        if (npairs <= 32 && !s_any[u]) {  // nothing rotates: no update of A, nor of V
+          pending = false;
+          continue;
         }
-        __syncthreads();
-        // A <- P^T A (rows p, q of every column); V <- V P
-        for (int e = tid; e < npairs * n; e += nt) {
-          int k = e / n, j = e % n;
-          double s = ss[k];
-          if (s == 0.0) continue;
-          int p = sp[k], q = sq[k];
-          double c = sc[k];
-          double apj = A[p * n + j], aqj = A[q * n + j];
-          A[p * n + j] = c * apj - s * aqj;
-          A[q * n + j] = s * apj + c * aqj;
-          double vjp = V[j * n + p], vjq = V[j * n + q];
-          V[j * n + p] = c * vjp - s * vjq;
-          V[j * n + q] = s * vjp + c * vjq;
-        }
-        __syncthreads();
-        for (int k = tid; k < npairs; k += nt)
-          if (ss[k] != 0.0) {
-            A[sp[k] * n + sq[k]] = 0.0;
-            A[sq[k] * n + sp[k]] = 0.0;
+        pending = true;
+        // A <- J^T A J above the diagonal: blocks (rows of pair k, columns of pair l), k < l; rows k
+        // and npairs - 1 - k together have npairs - 1 blocks
+        for (int w = warp; w < (npairs + 1) / 2; w += NW) {
+          const int k2 = npairs - 1 - w, n1 = npairs - 1 - w, n2 = k2 > w ? w : 0;
+          for (int x = lane; x < ((n1 + n2 + 31) & ~31); x += 32) {
+            const int k = x < n1 ? w : k2, l = x < n1 ? w + 1 + x : k2 + 1 + (x - n1);
+            const bool act = x < n1 + n2 && active(u, k, l);
+            if (npairs > 32) {
+              if (act) update_block(u, k, l);
+              continue;
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, act);
+            int base = 0;
+            if (lane == 0 && m) base = atomicAdd(&s_count, __popc(m));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (act) queue[base + __popc(m & ((1u << lane) - 1))] = uint16_t(k << 8 | l);
           }
+        }
+        if (npairs <= 32) {
+          __syncthreads();
+          for (int i = tid; i < s_count; i += nt) update_block(u, queue[i] >> 8, queue[i] & 255);
+        }
         __syncthreads();
       }
-      if (s_rot == 0) break;
-      __syncthreads();
+      const int rot = s_rot;
+      __syncthreads();  // every thread has read the flag before the next sweep clears it
+      if (rot == 0) break;
     }
+    if (pending) update_v(u ^ 1, warp, NW);
+    __syncthreads();
   }
-  // ascending order: rank of each diagonal entry (ties broken by index)
+  // ascending order: rank of each diagonal entry (ties broken by index), by its sortable bits
+  __shared__ int16_t rank[EJ_MAX_N];
+  auto key = [&](int i) {
+    long long k = __double_as_longlong(A[i * ld + i] + 0.0);  // -0 becomes +0
+    return k < 0 ? k ^ 0x7fffffffffffffffLL : k;
+  };
   double* ev_out = evals + size_t(b) * keep;
   double* vec_out = evecs + size_t(b) * max_size * keep;
   for (int i = tid; i < n; i += nt) {
-    const double di = A[i * n + i];
-    int rank = 0;
+    const long long di = key(i);
+    int rk = 0;
     for (int j = 0; j < n; ++j) {
-      const double dj = A[j * n + j];
-      rank += (dj < di) || (dj == di && j < i);
+      const long long dj = key(j);
+      rk += (dj < di) || (dj == di && j < i);
     }
-    if (rank < keep) {
-      ev_out[rank] = di;
-      for (int row = 0; row < n; ++row) vec_out[size_t(row) * keep + rank] = V[row * n + i];
-    }
+    rank[i] = int16_t(rk);
+    if (rk < keep) ev_out[rk] = A[i * ld + i];
+  }
+  __syncthreads();
+  for (int e = tid; e < n * n; e += nt) {
+    const int row = e / n, i = e - row * n;
+    if (rank[i] < keep) vec_out[size_t(row) * keep + rank[i]] = V[row * ld + i];
   }
 }
 
+}  // namespace
+
+namespace {
+int launch_jacobi(const double* A, const int64_t* offsets, const int* sizes, const int* lds, int n, int ld, int batch,
+                  int max_size, int keep, double* evals, double* evecs, double* work, cudaStream_t st) {
+  const size_t smem = max_size <= EJ_SHARED_N ? ej_smem_bytes(max_size) : 0;
+  static std::atomic<bool> attr{false};  // idempotent setup; threads may race to it
+  if (!attr.load()) {
+    TNX_CUDA(cudaFuncSetAttribute(jacobi_eigh_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  int(ej_smem_bytes(EJ_SHARED_N))));
+    attr.store(true);
+  }
+  jacobi_eigh_kernel<<<batch, EJ_THREADS, smem, st>>>(A, offsets, sizes, lds, n, ld, max_size, keep, evals, evecs,
+                                                      work);
+  TNX_LAUNCH_CHECK();
+  return TNX_OK;
+}
 }  // namespace
 
 int eigh_small_f64_ld(const double* A, const int64_t* offsets, const int* sizes, const int* lds,
                       int batch, int max_size, int keep, double* evals, double* evecs, double* work,
                       cudaStream_t st) {
   if (batch <= 0) return TNX_OK;
-  jacobi_eigh_kernel<<<batch, EJ_THREADS, 0, st>>>(A, offsets, sizes, lds, 0, 0, max_size, keep, evals,
-                                                   evecs, work);
-  TNX_LAUNCH_CHECK();
-  return TNX_OK;
+  return launch_jacobi(A, offsets, sizes, lds, 0, 0, batch, max_size, keep, evals, evecs, work, st);
 }
 
 int eigh_small_f64_uniform(const double* A, int n, int ld, int keep, double* evals, double* evecs,
                            double* work, cudaStream_t st) {
-  jacobi_eigh_kernel<<<1, EJ_THREADS, 0, st>>>(A, nullptr, nullptr, nullptr, n, ld, n, keep, evals, evecs,
-                                               work);
-  TNX_LAUNCH_CHECK();
-  return TNX_OK;
+  return launch_jacobi(A, nullptr, nullptr, nullptr, n, ld, 1, n, keep, evals, evecs, work, st);
 }
 
 int eigh_small_f64(double* A, const int64_t* offsets, const int* sizes, int batch, int max_size,
