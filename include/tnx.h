@@ -292,9 +292,10 @@ int tnx_tsdrg_project(const double* const* w1, const double* const* w2, const do
 
 /* Lowest-keep eigenpairs of tSDRG block Hamiltonians H = sum_w W1_b[0,w] (x) W2_b[w,dr2-1]
  * (TreeTensorNetworkSDRG.block_eigen_solver, tnpy/tsdrg.py:569-592) without forming H:
- * Chebyshev-filtered subspace iteration on the Kronecker matvec (FP32 for TNX_DF64 /
- * TNX_BF16X3, FP64 for TNX_FP64) followed by an FP64 Rayleigh-Ritz refinement, one CTA per
- * block. meta[5b..5b+4] = m1, m2, dr2, k, p (node dimensions m1, m2 <= 32, k kept pairs,
+ * Chebyshev-filtered subspace iteration on the Kronecker matvec in FP32, then, for TNX_FP64, FP64
+ * outer steps (product, Rayleigh-Ritz, residual to 1e-13 of the spectrum; the correction of each
+ * vector from the residual in FP32), for TNX_DF64 / TNX_BF16X3 one FP64 Rayleigh-Ritz, one CTA
+ * (or a cluster of up to eight) per block. meta[5b..5b+4] = m1, m2, dr2, k, p (node dimensions m1, m2 <= 32, k kept pairs,
  * p = subspace size with k <= p <= min(m1 m2, 48)); D <= 6; keep >= every k.
  * evals: batch x keep; evecs: batch x (max_m x keep) row-major, like tnx_eigh_batched;
  * iters (device, may be null): filter iterations per block, or a negative count for a block

@@ -29,6 +29,7 @@
 
 #include <atomic>
 
+#include "jacobi.cuh"
 #include "tnx_internal.cuh"
 
 namespace tnx {
@@ -42,66 +43,6 @@ constexpr int EJ_SHARED_N = 112;  // largest matrix whose A and V fit in shared 
 // row stride in shared memory: odd, so that a column's entries fall on distinct banks
 __host__ __device__ constexpr int ej_ld(int n) { return n | 1; }
 constexpr size_t ej_smem_bytes(int n) { return size_t(2) * n * ej_ld(n) * sizeof(double); }
-
-// double <-> float by integer operations (the conversions run on the FP64 pipe): truncated to 24
-// bits, zero below 2^-126; |x| < 2^127
-__device__ __forceinline__ float ej_float(double x) {
-  const unsigned hi = unsigned(__double2hiint(x)), lo = unsigned(__double2loint(x));
-  const int e = int((hi >> 20) & 0x7ffu) - 896;
-  return e <= 0 ? 0.f : __uint_as_float((hi & 0x80000000u) | (unsigned(e) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
-}
-__device__ __forceinline__ double ej_double(float x) {
-  const unsigned u = __float_as_uint(x), m = u & 0x7fffffffu;
-  if (m < 0x00800000u) return 0.0;
-  return __hiloint2double(int((u & 0x80000000u) | ((m >> 3) + (896u << 20))), int(m << 29));
-}
-// x 2^-e for |x| 2^-e < 2^1023; zero where it would be subnormal
-__device__ __forceinline__ double ej_scale(double x, int e) {
-  const int hi = __double2hiint(x), ex = ((hi >> 20) & 0x7ff) - e;
-  return ex <= 0 ? 0.0 : __hiloint2double(hi - (e << 20), __double2loint(x));
-}
-
-// Rotation that zeroes a_pq: t = tan, c, s with |t| <= 1; d = a_qq - a_pp (d = 0: t = 1)
-__device__ __forceinline__ void ej_angle(double apq, double d, double& t, double& c, double& s) {
-  const int ea = (__double2hiint(apq) >> 20) & 0x7ff, ed = (__double2hiint(d) >> 20) & 0x7ff;
-  const int e = max(ea, ed) - 1023;  // both below 2 after the scaling, the larger one above 1
-  const double a1 = ej_scale(apq, e), d1 = ej_scale(d, e);
-  const float af = ej_float(a1), df = ej_float(d1), a2 = 2.f * af;
-  float tf = 1.f;
-  double tt = 1.0;
-  if ((__double_as_longlong(d1) << 1) != 0) {
-    const float h = fmaf(df, df, a2 * a2);
-    const unsigned sign = unsigned(__double2hiint(d1)) & 0x80000000u;
-    tf = __uint_as_float(sign | 0x3f800000u) * __fdividef(a2, fmaf(h, rsqrtf(h), fabsf(df)));
-    // corrections against f(t) = a_pq t^2 + d t - a_pq, f' = 2 a_pq t + d
-    const float inv = __fdividef(1.f, fmaf(a2, tf, df));
-    tt = ej_double(tf);
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const double f = fma(fma(a1, tt, d1), tt, -a1);
-      tt -= ej_double(ej_float(f) * inv);
-    }
-  }
-  const double y = ej_double(rsqrtf(fmaf(tf, tf, 1.f)));
-  const double r = fma(-fma(tt, tt, 1.0), y * y, 1.0);  // 1 - (1 + t^2) y^2
-  c = fma(y * r, fma(0.375, r, 0.5), y);
-  s = tt * c;
-  t = tt;
-}
-
-// round-robin (circle method) pair k of round r for np (even) players, p < q
-__device__ __forceinline__ void ej_pair(int k, int r, int np, int& p, int& q) {
-  const int m1 = np - 1;
-  p = k - 1 + r;
-  q = np - 2 - k + r;
-  p = k == 0 ? 0 : 1 + (p >= m1 ? p - m1 : p);
-  q = 1 + (q >= m1 ? q - m1 : q);
-  if (p > q) {
-    const int t = p;
-    p = q;
-    q = t;
-  }
-}
 
 // A: matrix b at A + offsets[b], leading dimension lds[b] (or sizes[b] when lds == null).
 // work (matrices beyond EJ_SHARED_N): per matrix 2*max_size^2 doubles (copy of A and the rotation
@@ -159,7 +100,7 @@ __global__ void __launch_bounds__(EJ_THREADS) jacobi_eigh_kernel(
   auto update_v = [&](int u, int slot, int slots) {
     for (int l = slot; l < npairs; l += slots) {
       const double s = ss[u][l];
-      if ((__double_as_longlong(s) << 1) == 0) continue;
+      if (jac::bits(s) == 0) continue;
       const double c = sc[u][l];
       const int p = sp[u][l], q = sq[u][l];
       for (int j = lane; j < n; j += 32) {
@@ -170,17 +111,16 @@ __global__ void __launch_bounds__(EJ_THREADS) jacobi_eigh_kernel(
     }
   };
   auto at = [&](int i, int j) -> double& { return i < j ? A[i * ld + j] : A[j * ld + i]; };
-  auto bits = [](double x) { return static_cast<unsigned long long>(__double_as_longlong(x)) << 1; };  // 0 for +-0
   // whether block (k, l) changes: one of the pairs rotates and the block is not all zero (a conserved
   // quantity keeps most of A exactly zero)
   auto active = [&](int u, int k, int l) {
-    if ((bits(ss[u][k]) | bits(ss[u][l])) == 0) return false;
+    if ((jac::bits(ss[u][k]) | jac::bits(ss[u][l])) == 0) return false;
     const int pk = sp[u][k], qk = sq[u][k], pl = sp[u][l], ql = sq[u][l];
     const bool row2 = qk < n, col2 = ql < n;  // the padding player of an odd n has no entries
-    unsigned long long z = bits(at(pk, pl));
-    if (col2) z |= bits(at(pk, ql));
-    if (row2) z |= bits(at(qk, pl));
-    if (row2 && col2) z |= bits(at(qk, ql));
+    unsigned long long z = jac::bits(at(pk, pl));
+    if (col2) z |= jac::bits(at(pk, ql));
+    if (row2) z |= jac::bits(at(qk, pl));
+    if (row2 && col2) z |= jac::bits(at(qk, ql));
     return z != 0;
   };
   auto update_block = [&](int u, int k, int l) {
@@ -189,14 +129,14 @@ __global__ void __launch_bounds__(EJ_THREADS) jacobi_eigh_kernel(
     const bool row2 = qk < n, col2 = ql < n;
     double a = at(pk, pl), b2 = col2 ? at(pk, ql) : 0.0, c2 = row2 ? at(qk, pl) : 0.0,
            d2 = row2 && col2 ? at(qk, ql) : 0.0;
-    if (bits(sl)) {
+    if (jac::bits(sl)) {
       const double c = sc[u][l], a0 = a, c0 = c2;
       a = fma(c, a0, -sl * b2);
       b2 = fma(sl, a0, c * b2);
       c2 = fma(c, c0, -sl * d2);
       d2 = fma(sl, c0, c * d2);
     }
-    if (bits(sk)) {
+    if (jac::bits(sk)) {
       const double c = sc[u][k], a0 = a, b0 = b2;
       a = fma(c, a0, -sk * c2);
       c2 = fma(sk, a0, c * c2);
@@ -222,7 +162,7 @@ __global__ void __launch_bounds__(EJ_THREADS) jacobi_eigh_kernel(
           bool rot = false;
           if (k < npairs) {
             int p, q;
-            ej_pair(k, r, np, p, q);
+            jac::pair_of(k, r, np, p, q);
             double c = 1.0, s = 0.0;
             if (q < n) {
               const double apq = A[p * ld + q];
@@ -230,7 +170,7 @@ __global__ void __launch_bounds__(EJ_THREADS) jacobi_eigh_kernel(
               if (ab > floor_bits && ab < 0x7ff0000000000000LL) {
                 double t;
                 const double app = A[p * ld + p], aqq = A[q * ld + q];
-                ej_angle(apq, aqq - app, t, c, s);
+                jac::angle(apq, aqq - app, t, c, s);
                 A[p * ld + p] = fma(-t, apq, app);
                 A[q * ld + q] = fma(t, apq, aqq);
                 A[p * ld + q] = 0.0;
@@ -465,12 +405,8 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restric
     for (int sweep = 0; sweep < 30; ++sweep) {
       for (int rnd = 0; rnd < np - 1; ++rnd) {
         if (tid < npairs) {
-          // round robin: 0 stays, the others turn by one player a round
-          const int m1 = np - 1;
-          int p = tid - 1 + rnd, q = np - 2 - tid + rnd;
-          p = tid == 0 ? 0 : 1 + (p >= m1 ? p - m1 : p);
-          q = 1 + (q >= m1 ? q - m1 : q);
-          if (p > q) { int t = p; p = q; q = t; }
+          int p, q;
+          jac::pair_of(tid, rnd, np, p, q);
           float c = 1.f, sn = 0.f;
           if (q < n) {
             const float apq = Af[p * nf + q], app = Af[p * nf + p], aqq = Af[q * nf + q];
