@@ -309,95 +309,6 @@ __global__ void bfill_kernel(int* __restrict__ a, int B, int v) {
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < B; b += gridDim.x * blockDim.x) a[b] = v;
 }
 
-// ---- batched Householder QR in shared memory (one CTA per chain) ---------------------------
-// M (m x n, m >= n) = Q R. trans = 0: M is the row-major m x n matrix at A_b; trans = 1: M is
-// the transpose of the row-major n x m matrix at A_b. Q (m x n) overwrites A_b in the same
-// layout (trans = 1 writes Q^T); R (n x n, upper triangular, row-major) goes to R_b.
-// Shared memory: the panel a and the Q accumulator q, column-major, 2 m n doubles.
-constexpr int QT = 256;
-
-__global__ void __launch_bounds__(QT) bqr_kernel(double* __restrict__ A, int64_t sA, int m, int n, int trans,
-                                                double* __restrict__ Rout, int64_t sR) {
-  extern __shared__ double smq[];
-  double* a = smq;          // m x n column-major: a[j*m + i]
-  double* q = smq + m * n;  // m x n column-major
-  __shared__ double tau[128];
-  const int b = blockIdx.x;
-  double* Ab = A + b * sA;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = QT / 32;
-  for (int e = tid; e < m * n; e += QT) {
-    const int j = e / m, i = e % m;
-    a[e] = trans ? Ab[int64_t(j) * m + i] : Ab[int64_t(i) * n + j];
-    q[e] = (i == j) ? 1.0 : 0.0;
-  }
-  __syncthreads();
-  for (int j = 0; j < n; ++j) {
-    double* cj = a + j * m;
-    if (warp == 0) {
-      double sg = 0.0;
-      for (int i = j + 1 + lane; i < m; i += 32) sg = fma(cj[i], cj[i], sg);
-      const double alpha = cj[j];  // every lane reads it before the shuffles below
-      for (int o = 16; o > 0; o >>= 1) sg += __shfl_xor_sync(0xffffffffu, sg, o);
-      double t = 0.0, scale = 0.0, beta = alpha;
-      if (sg > 0.0) {
-        const double nrm = sqrt(fma(alpha, alpha, sg));
-        beta = alpha >= 0.0 ? -nrm : nrm;
-        t = (beta - alpha) / beta;
-        scale = 1.0 / (alpha - beta);
-      }
-      for (int i = j + 1 + lane; i < m; i += 32) cj[i] *= scale;
-      __syncwarp();
-      if (lane == 0) {
-        cj[j] = beta;
-        tau[j] = t;
-      }
-    }
-    __syncthreads();
-    const double tj = tau[j];
-    if (tj != 0.0) {
-      for (int c = j + 1 + warp; c < n; c += nw) {
-        double* cc = a + c * m;
-        const double top = cc[j];  // read by every lane before lane 0 rewrites it
-        double w = 0.0;
-        for (int i = j + 1 + lane; i < m; i += 32) w = fma(cj[i], cc[i], w);
-        for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-        w = tj * (w + top);
-        if (lane == 0) cc[j] -= w;
-        for (int i = j + 1 + lane; i < m; i += 32) cc[i] = fma(-w, cj[i], cc[i]);
-      }
-    }
-    __syncthreads();
-  }
-  // Q = H_0 H_1 ... H_{n-1} I[:, :n], applied from the last reflector
-  for (int j = n - 1; j >= 0; --j) {
-    const double tj = tau[j];
-    const double* cj = a + j * m;
-    if (tj != 0.0) {
-      for (int c = j + warp; c < n; c += nw) {
-        double* qc = q + c * m;
-        const double top = qc[j];
-        double w = 0.0;
-        for (int i = j + 1 + lane; i < m; i += 32) w = fma(cj[i], qc[i], w);
-        for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-        w = tj * (w + top);
-        if (lane == 0) qc[j] -= w;
-        for (int i = j + 1 + lane; i < m; i += 32) qc[i] = fma(-w, cj[i], qc[i]);
-      }
-    }
-    __syncthreads();
-  }
-  for (int e = tid; e < m * n; e += QT) {
-    const int j = e / m, i = e % m;
-    if (trans) Ab[int64_t(j) * m + i] = q[e];
-    else Ab[int64_t(i) * n + j] = q[e];
-  }
-  double* Rb = Rout + b * sR;
-  for (int e = tid; e < n * n; e += QT) {
-    const int i = e / n, c = e % n;
-    Rb[e] = i <= c ? a[c * m + i] : 0.0;
-  }
-}
-
 // ---- batched matvec --------------------------------------------------------------------
 struct BDims {
   int64_t chi_l, d, chi_r, dl, dr;
@@ -745,10 +656,7 @@ int tnx_batched_gauge_move(int direction, double* A_site, int64_t sA, double* A_
   cudaStream_t st = as_stream(stream);
   double* Rm = static_cast<double*>(workspace);
   double* tmp = reinterpret_cast<double*>(static_cast<char*>(workspace) + align_up(size_t(batch) * nn * nn * 8));
-  const size_t smem = size_t(2 * m * nn) * sizeof(double);
-  TNX_CUDA(cudaFuncSetAttribute(bqr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-  bqr_kernel<<<batch, QT, smem, st>>>(A_site, sA, int(m), int(nn), direction == 1 ? 0 : 1, Rm, nn * nn);
-  TNX_LAUNCH_CHECK();
+  TNX_TRY(qr_small(A_site, sA, A_site, sA, Rm, nn * nn, m, nn, direction == 1 ? 0 : 1, batch, st));
   const bool df = use_df64(precision);
   const int64_t other = direction == 1 ? chi_r * d * chi_other : chi_other * d * chi_l;
   const size_t ozb = direction == 1 ? boz_bytes(chi_r, d * chi_other, chi_r, batch)

@@ -1096,6 +1096,12 @@ int form_q_wy(int64_t m, int64_t n, const WyWs& y, double* Q, bool q_rowmajor, c
 
 using namespace tnx;
 
+// One CTA (or a cluster that shares Q) with the matrix in shared memory, FP64 in every precision form,
+// while the 16-CTA panels have less to gain from their spread than they lose to their barriers:
+// gauge move, kernels only, 32 x 16 61 us against 85 (FP64 panels) and 94 (double-FP32), 64 x 32 129
+// against 158 and 165, 128 x 64 367 against 335 and 306; three launches against twelve.
+static bool small_qr(int64_t m, int64_t n) { return n <= 32 && m <= 256; }
+
 extern "C" {
 
 size_t tnx_qr_workspace_bytes(int64_t m, int64_t n) { return qr_layout(m, n, nullptr, nullptr); }
@@ -1112,6 +1118,7 @@ int tnx_qr(const double* M, int64_t m, int64_t n, double* Q, double* R, void* wo
     return TNX_ERR_WORKSPACE;
   }
   cudaStream_t st = as_stream(stream);
+  if (small_qr(m, n)) return qr_small(M, 0, Q, 0, R, 0, m, n, 0, 1, st);
   dim3 tb(32, 8);
   transpose_kernel<<<dim3(unsigned((n + 31) / 32), unsigned((m + 31) / 32)), tb, 0, st>>>(M, m, n, w.F);
   TNX_LAUNCH_CHECK();
@@ -1170,6 +1177,19 @@ int tnx_gauge_move(int direction, double* A_site, double* A_nb, int64_t chi_l, i
   WyWs wys{};
   if (wy) wy_layout(m, n, after_tmp + align_up(gauge_oz_bytes(direction, chi_l, d, chi_r, chi_other)), &wys);
   cudaStream_t st = as_stream(stream);
+  if (small_qr(m, n)) {
+    // Q over the site in its own layout (direction -1: the site is psi^T row-major), R, then the
+    // neighbour: A_next <- R A_next, or A_prev <- A_prev R^T
+    TNX_TRY(qr_small(A_site, 0, A_site, 0, Rb, 0, m, n, direction == 1 ? 0 : 1, 1, st));
+    if (direction == 1)
+      TNX_TRY(gemm_fp64_class(false, false, false, n, d * chi_other, n, 1.0, Rb, n, 0, A_nb, d * chi_other, 0, 0.0, tmp,
+                              d * chi_other, 0, 1, st));
+    else
+      TNX_TRY(gemm_fp64_class(false, false, true, chi_other * d, n, n, 1.0, A_nb, n, 0, Rb, n, 0, 0.0, tmp, n, 0, 1,
+                              st));
+    TNX_CUDA(cudaMemcpyAsync(A_nb, tmp, nb_elems * 8, cudaMemcpyDeviceToDevice, st));
+    return TNX_OK;
+  }
   dim3 tb(32, 8);
   if (direction == 1) {
     // psi (chi_l d x chi_r) row-major -> column-major
