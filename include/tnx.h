@@ -132,7 +132,7 @@ int tnx_env_update(int direction, const double* E_in, const double* A, const dou
  * runs split-BF16 matvecs on FP32 vectors to a residual of ~3e-6 |theta|; an anchored phase
  * then continues from the Ritz vector x with one FP64-class product H x per anchor (exact
  * first row of the projected matrix, split-BF16 products for the corrections) until the
- * FP64-class residual is below max(tol, 2e-7) |theta|. */
+ * FP64-class residual is below max(tol, 2e-7) |theta| (5e-8 for sites of up to 8192 elements). */
 size_t tnx_davidson1_workspace_bytes(int64_t chi_l, int64_t d, int64_t chi_r, int64_t dl,
                                      int64_t dr, int max_basis, int precision);
 int tnx_davidson1(const double* L, const double* W, const double* R, double* x, int64_t chi_l,
