@@ -64,7 +64,13 @@ __device__ __forceinline__ void angle(double apq, double d, double& t, double& c
   const float af = to_float(a1), df = to_float(d1), a2 = 2.f * af;
   float tf = 1.f;
   double tt = 1.0;
-  if (bits(d1) != 0) {
+  if (ed - ea > 30) {
+    // t = a_pq / d to FP64 accuracy (the next term is (a_pq / d)^2 < 2^-60 of it), by an FP32 seed of
+    // 1 / d and one third-order step: a_pq itself may lie far below FP32's range here
+    const double z = to_double(__fdividef(1.f, df)), r = fma(-d1, z, 1.0);
+    tt = a1 * fma(z * r, 1.0 + r, z);
+    tf = 0.f;
+  } else if (bits(d1) != 0) {
     const float h = fmaf(df, df, a2 * a2);
     const unsigned sign = unsigned(__double2hiint(d1)) & 0x80000000u;
     tf = __uint_as_float(sign | 0x3f800000u) * __fdividef(a2, fmaf(h, rsqrtf(h), fabsf(df)));
