@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         for (int h = 0; h < 2; ++h)
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            if (out_fp64) sd[lr * (CW + 1) + h * 32 + j] = double(__uint_as_float(r[h][j]));
+            if (out_fp64) sd[lr * (CW + 1) + h * 32 + j] = float_to_double(__uint_as_float(r[h][j]));
             else sf[lr * (CW + 1) + h * 32 + j] = __uint_as_float(r[h][j]);
           }
       }
@@ -195,27 +195,100 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 }
 
 // ---------------------------------------------------------------- operand preparation
-// dst_hi/lo[c][r] (row pitch ldp) = split(src[r][c]) for r < rows; zeros for rows <= r < ldp.
-// src is row-major rows x cols (FP64).
-template <typename T>
-__global__ void split_transpose_kernel(const T* __restrict__ src, int64_t rows, int64_t cols,
-                                       __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo,
-                                       int64_t ldp) {
-  __shared__ double tile[32][33];
-  const int64_t r0 = int64_t(blockIdx.y) * 32, c0 = int64_t(blockIdx.x) * 32;
-  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-    const int64_t r = r0 + k, c = c0 + threadIdx.x;
-    tile[k][threadIdx.x] = (r < rows && c < cols) ? double(src[r * cols + c]) : 0.0;
+// hi = v rounded to BF16, lo = v - hi (exact in FP64) rounded to BF16, as bit patterns: integer
+// arithmetic on the 53-bit significand, because a conversion or an addition holds the FP64 pipe for
+// 64 clocks a warp. Round to nearest even, subnormal results and overflow included; Inf and NaN as
+// the conversions give them (lo NaN).
+__device__ __forceinline__ uint32_t round_bf16(uint64_t sig, int e, uint32_t sign) {
+  // sign * sig * 2^e, sig < 2^54, to BF16
+  if (sig == 0) return sign << 15;
+  const int p = 63 - __clzll(static_cast<long long>(sig));
+  int ef = e + p + 127;                  // exponent field of a normal result
+  int drop = ef > 0 ? p - 7 : p - 6 - ef;  // bits below the last kept one; a subnormal result keeps fewer
+  uint64_t q;
+  if (drop <= 0) {
+    q = sig << -drop;  // -drop <= 7
+  } else if (drop > 54) {
+    q = 0;
+  } else {
+    const uint64_t half = (1ull << (drop - 1)) - 1 + ((sig >> drop) & 1);
+    q = (sig + half) >> drop;
   }
-  __syncthreads();
-  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-    const int64_t c = c0 + k, r = r0 + threadIdx.x;
-    if (c < cols && r < ldp) {
-      const double v = tile[threadIdx.x][k];
-      const __nv_bfloat16 h = __double2bfloat16(v);
-      hi[c * ldp + r] = h;
-      lo[c * ldp + r] = __double2bfloat16(v - double(__bfloat162float(h)));
+  // q carries the implicit bit of a normal result, which adds one to the exponent field below
+  const uint32_t r = ef > 0 ? (uint32_t(ef - 1) << 7) + uint32_t(q) : uint32_t(q);
+  return (sign << 15) | (r < 0x7f80u ? r : 0x7f80u);
+}
+__device__ __forceinline__ void split_bf16(double v, uint32_t& hi, uint32_t& lo) {
+  const uint64_t u = static_cast<uint64_t>(__double_as_longlong(v));
+  const uint32_t sign = uint32_t(u >> 63);
+  const int eb = int(u >> 52) & 0x7ff;
+  const uint64_t m = u & ((1ull << 52) - 1);
+  if (eb - 896 < 8 || eb - 896 >= 254) {  // near or outside BF16's normal range
+    if (eb == 2047) {
+      hi = m ? 0x7fffu : (sign << 15) | 0x7f80u;
+      lo = 0x7fffu;
+      return;
     }
+    const uint64_t sig = eb ? m | (1ull << 52) : m;
+    const int e = (eb ? eb : 1) - 1075;
+    hi = round_bf16(sig, e, sign);
+    if ((hi & 0x7fffu) == 0x7f80u) {  // overflow: v - Inf
+      lo = ((sign ^ 1u) << 15) | 0x7f80u;
+      return;
+    }
+    // hi as an integer multiple of 2^e (its last bit is at 2^-133 or above, e may be far below)
+    const int hf = int(hi >> 7) & 0xff;
+    const uint64_t hs = (hi & 0x7fu) | (hf ? 0x80u : 0u);
+    const int he = (hf ? hf : 1) - 134 - e;  // hi = hs 2^(he + e); hs == 0 where he is out of range
+    const uint64_t hv = hs ? hs << he : 0;
+    lo = sig >= hv ? round_bf16(sig - hv, e, sign) : round_bf16(hv - sig, e, sign ^ 1u);
+    return;
+  }
+  // normal hi, and lo normal or zero: its leading bit is at 2^-52 of v or above, which the margin of 8
+  // in the exponent leaves to round_bf16's general form
+  const uint64_t sig = m | (1ull << 52);
+  const uint64_t q = (sig + ((1ull << 44) - 1) + ((sig >> 45) & 1)) >> 45;  // 128 .. 256
+  hi = (sign << 15) | ((uint32_t(eb - 897) << 7) + uint32_t(q));
+  const int64_t d = int64_t(sig - (q << 45));  // |d| <= 2^44
+  lo = round_bf16(uint64_t(d < 0 ? -d : d), eb - 1075, d < 0 ? sign ^ 1u : sign);
+  if (d == 0) lo = 0;  // v - hi = +0
+}
+__device__ __forceinline__ void split_bf16(float v, uint32_t& hi, uint32_t& lo) {
+  const __nv_bfloat16 h = __float2bfloat16_rn(v);
+  hi = __bfloat16_as_ushort(h);
+  lo = __bfloat16_as_ushort(__float2bfloat16_rn(v - __bfloat162float(h)));
+}
+
+// dst_hi/lo[c][r] (row pitch ldp, even) = split(src[r][c]) for r < rows; zeros for rows <= r < ldp.
+// src is row-major rows x cols. Bound by memory (8 bytes read, 4 written an element) once the
+// split stays off the FP64 pipe: L, R and x of a chi = 1024 site 101 us with conversions, 58 us so.
+template <typename T>
+__global__ void __launch_bounds__(256) split_transpose_kernel(const T* __restrict__ src, int64_t rows, int64_t cols,
+                                                             __nv_bfloat16* __restrict__ hi,
+                                                             __nv_bfloat16* __restrict__ lo, int64_t ldp) {
+  __shared__ T tile[64][33];
+  const int64_t r0 = int64_t(blockIdx.y) * 64, c0 = int64_t(blockIdx.x) * 32;
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  T x[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int64_t r = r0 + ty + 8 * i, c = c0 + tx;
+    x[i] = (r < rows && c < cols) ? src[r * cols + c] : T(0);
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) tile[ty + 8 * i][tx] = x[i];
+  __syncthreads();
+  const int64_t r = r0 + 2 * tx;
+  if (r >= ldp) return;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int64_t c = c0 + ty + 8 * i;
+    if (c >= cols) continue;
+    uint32_t h0, l0, h1, l1;
+    split_bf16(tile[2 * tx][ty + 8 * i], h0, l0);
+    split_bf16(tile[2 * tx + 1][ty + 8 * i], h1, l1);
+    *reinterpret_cast<uint32_t*>(hi + c * ldp + r) = h0 | h1 << 16;
+    *reinterpret_cast<uint32_t*>(lo + c * ldp + r) = l0 | l1 << 16;
   }
 }
 
@@ -225,10 +298,10 @@ __global__ void split_pad_kernel(const double* __restrict__ src, int64_t rows, i
   for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < rows * ldp;
        e += int64_t(gridDim.x) * blockDim.x) {
     const int64_t r = e / ldp, c = e % ldp;
-    const double v = c < cols ? src[r * cols + c] : 0.0;
-    const __nv_bfloat16 h = __double2bfloat16(v);
-    hi[e] = h;
-    lo[e] = __double2bfloat16(v - double(__bfloat162float(h)));
+    uint32_t h, l;
+    split_bf16(c < cols ? src[r * cols + c] : 0.0, h, l);
+    hi[e] = __ushort_as_bfloat16(uint16_t(h));
+    lo[e] = __ushort_as_bfloat16(uint16_t(l));
   }
 }
 
@@ -326,7 +399,7 @@ void* align1024(void* p) {
 }
 
 dim3 tgrid(int64_t rows, int64_t cols) {
-  return dim3(unsigned((cols + 31) / 32), unsigned((rows + 31) / 32));
+  return dim3(unsigned((cols + 31) / 32), unsigned((rows + 63) / 64));
 }
 
 }  // namespace

@@ -142,6 +142,15 @@ __device__ __forceinline__ void split_df(double x, float& hi, float& lo) {
   lo = __uint_as_float(lb);
 }
 
+// float -> double by integer operations (a conversion holds the FP64 pipe as an addition does); Inf and
+// NaN keep their kind, a subnormal becomes zero
+__device__ __forceinline__ double float_to_double(float x) {
+  const unsigned u = __float_as_uint(x), m = u & 0x7fffffffu;
+  const unsigned base = m >= 0x7f800000u ? (1792u << 20) : (896u << 20);
+  return m < 0x00800000u ? __hiloint2double(int(u & 0x80000000u), 0)
+                         : __hiloint2double(int((u & 0x80000000u) | ((m >> 3) + base)), int(m << 29));
+}
+
 // (h, l) -> the nearest double of h + l (two conversions and one FP64 add)
 __device__ __forceinline__ double join_df(float h, float l) { return double(h) + double(l); }
 
