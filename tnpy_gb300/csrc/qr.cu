@@ -24,6 +24,7 @@
 #include <mutex>
 #include <string>
 
+#include "householder.cuh"
 #include "tnx_internal.cuh"
 #include "qr_panel_df.cuh"
 
@@ -165,7 +166,13 @@ __global__ void __launch_bounds__(QT) panel_kernel(double* __restrict__ F, int64
 // Each step: one thread derives the column's scalars; phase A forms v = scale * x_jj and the
 // updated column jj+1 once per row (FP64 arithmetic is scarce on this part); phase B (before
 // the barrier arrives) updates columns c > jj+1 and forms the partial dots; phase C (between
-// arrive and wait) stores v and column jj+1 and extends T on rank 0.
+// arrive and wait) stores v and column jj+1. The rows of T are dealt out over the CTAs, a warp each.
+//
+// What bounds it: the chain of a column, in FP64 instructions of 64 clocks a warp. The partials of a
+// column's 64 sums (norm and dots right of the pivot, T dots left of it) are added by four threads
+// each, the scalars take 20 instructions (reflector), a row of T seven, behind the scalars and on other
+// sub-partitions. 128 x 64: 304 us with sums in one thread each, exact root and divisions, and all of T
+// by one thread a row on rank 0; 225 us so.
 constexpr int PT = 256;  // threads per CTA of the cluster panel kernel
 
 __device__ __forceinline__ void cluster_arrive_release() {
@@ -186,9 +193,11 @@ __global__ void __launch_bounds__(PT) panel_cl_kernel(double* __restrict__ F, in
   double* vr = pl + NB * ld;      // reflector of the current column over this CTA's rows
   double* vnr = vr + ld;          // next column after the current reflector
   __shared__ double slot[2][3 * NB];  // s[NB] partial dots, piv[NB] pivot row, z[NB] T dots
+  constexpr int NR = NB / CL;  // rows of T held by each CTA: a = q, q + CL, ...
+  static_assert(NB % CL == 0, "panel shape");
   __shared__ double S[NB], P[NB], Z[NB], taus[NB], sc[4];
-  __shared__ double Ts[NB][NB + 1];  // T factor, rank 0 only, row a held by thread a
-  const int tid = threadIdx.x, ci = tid / TPC, h = tid % TPC;
+  __shared__ double Tr[NR][NB];
+  const int tid = threadIdx.x, ci = tid / TPC, h = tid % TPC, warp = tid >> 5, lane = tid & 31;
   const int64_t mp = m - j0;
   const int64_t rpc = (mp + CL - 1) / CL;
   const int64_t r0 = int64_t(q) * rpc;  // first panel row of this CTA
@@ -197,6 +206,22 @@ __global__ void __launch_bounds__(PT) panel_cl_kernel(double* __restrict__ F, in
     const int c = e / rows, r = e % rows;
     pl[c * ld + r] = F[(j0 + c) * m + j0 + r0 + r];
   }
+  // column k of this warp's row of T: T[a][k] = -tau_k sum_{a <= c < k} T[a][c] z_c, T[k][k] = tau_k
+  // (warps 1, 2, 3, 5, 6, 7 take rows 0, 1, ..: not on the sub-partition of warp 0)
+  auto extend_t = [&](int k) {
+    if ((warp & 3) == 0) return;
+    for (int row = warp - 1 - (warp >> 2); row < NR; row += PT / 32 - PT / 128) {
+      const int a = q + CL * row;
+      if (a < k) {
+        double t = 0.0;
+        for (int c = a + lane; c < k; c += 32) t = fma(Tr[row][c], Z[c], t);
+        t = warp_sum(t);
+        if (lane == 0) Tr[row][k] = -taus[k] * t;
+      } else if (a == k && lane == 0) {
+        Tr[row][k] = taus[k];
+      }
+    }
+  };
   __syncthreads();
   // partials of pivot 0: s[c] = sum_{row > 0} x_0 x_c, pivot row 0 from rank 0
   {
@@ -221,39 +246,39 @@ __global__ void __launch_bounds__(PT) panel_cl_kernel(double* __restrict__ F, in
   for (int jj = 0; jj < nb; ++jj) {
     const int par = jj & 1;
     const int owner = int(jj / rpc);
-    if (tid < NB) {
-      const int c = tid;
-      if (c >= jj && c < nb) {
-        double t = 0.0;
+    // S[c] (c >= jj) and Z[c] (c < jj - 1): sum over the ranks by the TPC threads of column c
+    {
+      const bool right = ci >= jj && ci < nb, left = ci < jj - 1;
+      double t = 0.0, piv = 0.0;
+      if (right || left) {
+        const double* from = &slot[par][right ? ci : 2 * NB + ci];
+        if (h == 0 && right) piv = *cluster.map_shared_rank(&slot[par][NB + ci], owner);
 #pragma unroll
-        for (int qq = 0; qq < CL; ++qq) t += cluster.map_shared_rank(&slot[par][0], qq)[c];
-        S[c] = t;
-        P[c] = cluster.map_shared_rank(&slot[par][NB], owner)[c];
+        for (int qq = 0; qq < CL; qq += TPC)
+          if (qq + h < CL) t += *cluster.map_shared_rank(from, qq + h);
       }
-    } else if (tid < 2 * NB && q == 0) {
-      const int a = tid - NB;
-      if (a < jj - 1) {
-        double t = 0.0;
 #pragma unroll
-        for (int qq = 0; qq < CL; ++qq) t += cluster.map_shared_rank(&slot[par][2 * NB], qq)[a];
-        Z[a] = t;
+      for (int o = TPC / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (h == 0) {
+        if (right) {
+          S[ci] = t;
+          P[ci] = piv;
+        } else if (left) {
+          Z[ci] = t;
+        }
       }
     }
     __syncthreads();
-    // column scalars once (FP64 sqrt and divisions are slow on this part's FP64 pipe)
-    if (tid == 0) {
-      const double sigma = S[jj], alpha = P[jj];
-      double tj = 0.0, beta = alpha, scale = 0.0;
-      if (sigma != 0.0) {
-        const double nrm = sqrt(alpha * alpha + sigma);
-        beta = alpha >= 0.0 ? -nrm : nrm;
-        tj = (beta - alpha) / beta;
-        scale = 1.0 / (alpha - beta);
-      }
+    // column scalars once; meanwhile, on the other sub-partitions' pipes, column jj - 1 of T
+    if (warp != 0) {
+      if (jj >= 1) extend_t(jj - 1);
+    } else if (tid == 0) {
+      double tj, beta, scale;
+      reflector(P[jj], S[jj], beta, tj, scale);
       sc[0] = tj;
       sc[1] = beta;
       sc[2] = scale;
-      sc[3] = jj + 1 < nb ? tj * (P[jj + 1] + scale * S[jj + 1]) : 0.0;  // w of column jj+1
+      sc[3] = jj + 1 < nb ? tj * fma(scale, S[jj + 1], P[jj + 1]) : 0.0;  // w of column jj+1
       taus[jj] = tj;
     }
     __syncthreads();
@@ -286,7 +311,7 @@ __global__ void __launch_bounds__(PT) panel_cl_kernel(double* __restrict__ F, in
           if (r >= rs && r < rows) acc = fma(vnr[r], vnr[r], acc);
         }
       } else if (ci > jj) {
-        const double wc = tj * (P[ci] + scale * S[ci]);
+        const double wc = tj * fma(scale, S[ci], P[ci]);
         if (lj >= 0 && lj < rows && lj % TPC == h) xc[lj] -= wc;  // v_jj[jj] = 1
         if (own_ln) {
           const double val = xc[ln] - wc * vr[ln];
@@ -323,55 +348,37 @@ __global__ void __launch_bounds__(PT) panel_cl_kernel(double* __restrict__ F, in
         xj[r] = r == lj ? beta : vr[r];
         if (has_next) xn[r] = vnr[r];
       }
-      if (q == 0 && jj >= 1 && tid < jj) {
-        const int k = jj - 1, a = tid;
-        if (a == k) {
-          Ts[k][k] = taus[k];
-        } else {
-          double t = 0.0;
-          for (int c = a; c < k; ++c) t = fma(Ts[a][c], Z[c], t);
-          Ts[a][k] = -taus[k] * t;
-        }
-      }
     }
     // the next gather rewrites S, P and Z, which phase C of other threads still reads
     __syncthreads();
     cluster_wait_acquire();
   }
   // last T column from the final exchange
-  if (q == 0 && tid >= NB && tid < 2 * NB) {
-    const int a = tid - NB;
-    if (a < nb - 1) {
-      double t = 0.0;
+  {
+    double t = 0.0;
+    if (ci < nb - 1) {
 #pragma unroll
-      for (int qq = 0; qq < CL; ++qq) t += cluster.map_shared_rank(&slot[nb & 1][2 * NB], qq)[a];
-      Z[a] = t;
+      for (int qq = 0; qq < CL; qq += TPC)
+        if (qq + h < CL) t += *cluster.map_shared_rank(&slot[nb & 1][2 * NB + ci], qq + h);
     }
+#pragma unroll
+    for (int o = TPC / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (ci < nb - 1 && h == 0) Z[ci] = t;
   }
   __syncthreads();
-  if (q == 0 && tid < nb) {
-    const int k = nb - 1, a = tid;
-    if (a == k) {
-      Ts[k][k] = taus[k];
-    } else {
-      double t = 0.0;
-      for (int c = a; c < k; ++c) t = fma(Ts[a][c], Z[c], t);
-      Ts[a][k] = -taus[k] * t;
-    }
-  }
+  extend_t(nb - 1);
   __syncthreads();
-  if (q == 0) {
-    for (int e = tid; e < NB * NB; e += PT) {
-      const int b = e / NB, a = e % NB;  // T_out column-major, ld NB
-      T_out[e] = (a <= b && b < nb) ? Ts[a][b] : 0.0;
-    }
+  for (int e = tid; e < NR * NB; e += PT) {
+    const int i = e / NB, b = e % NB, a = q + CL * i;  // T_out column-major, ld NB
+    T_out[b * NB + a] = (a <= b && b < nb) ? Tr[i][b] : 0.0;
+  }
+  if (q == 0)
     for (int b = tid; b < NB; b += PT) tau_out[b] = b < nb ? taus[b] : 0.0;
-  }
   for (int e = tid; e < nb * rows; e += PT) {
     const int c = e / rows, r = e % rows;
     F[(j0 + c) * m + j0 + r0 + r] = pl[c * ld + r];
   }
-  // no CTA leaves while rank 0 may still read its slots
+  // no CTA leaves while another may still read its slots
   cluster_arrive_release();
   cluster_wait_acquire();
 }

@@ -91,24 +91,19 @@ __device__ __forceinline__ void acc(df2& c, df2 a, df2 b) {
   c.l = __fadd_rn(c.l, __fadd_rn(s.l, pe));
 }
 __device__ __forceinline__ df2 norm(df2 c) { return two_sum(c.h, c.l); }
-// 1 / sqrt(t), t > 0: rsqrtf seed, two Newton steps y += y (1 - t y^2) / 2 on the
-// double-FP32 residual (seed error ~2^-22 -> ~2^-44 -> the format's ~2^-47)
+// 1 / sqrt(t), t > 0: rsqrtf seed y (error ~2^-22) and one third-order step y + y (e / 2 + 3 e^2 / 8) on the
+// double-FP32 residual e = 1 - t y^2, accurate to ~2^-47 absolutely: the correction, ~2^-22 of y, is
+// enough in FP32
 __device__ __forceinline__ df2 rsqrt_df(df2 t) {
-  df2 y = {rsqrtf(t.h), 0.f};
-  for (int it = 0; it < 2; ++it) {
-    const df2 e = fms({1.f, 0.f}, t, mul(y, y));
-    y = add(y, {__fmul_rn(__fmul_rn(0.5f, y.h), e.h), 0.f});
-  }
-  return y;
+  const float y = rsqrtf(t.h), yy = __fmul_rn(y, y);
+  const df2 e = fms({1.f, 0.f}, t, {yy, fmaf(y, y, -yy)});
+  return fast_two_sum(y, __fmul_rn(__fmul_rn(y, e.h), fmaf(0.375f, e.h, 0.5f)));
 }
-// 1 / b: approximate FP32 reciprocal seed, two Newton steps z += z (1 - b z)
+// 1 / b: approximate FP32 reciprocal seed z and one third-order step z + z (e + e^2), e = 1 - b z
 __device__ __forceinline__ df2 rcp_df(df2 b) {
-  df2 z = {__fdividef(1.f, b.h), 0.f};
-  for (int it = 0; it < 2; ++it) {
-    const df2 e = fms({1.f, 0.f}, b, z);
-    z = add(z, {__fmul_rn(z.h, e.h), 0.f});
-  }
-  return z;
+  const float z = __fdividef(1.f, b.h);
+  const df2 e = fms({1.f, 0.f}, b, {z, 0.f});
+  return fast_two_sum(z, __fmul_rn(__fmul_rn(z, e.h), 1.f + e.h));
 }
 __device__ __forceinline__ df2 shfl_xor(df2 x, int o) {
   return {__shfl_xor_sync(0xffffffffu, x.h, o), __shfl_xor_sync(0xffffffffu, x.l, o)};
@@ -245,6 +240,21 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
     X[c * ld + r] = split_scaled(F[(j0 + c) * m + j0 + r0 + r], cexp[c]);
   }
   for (int e = tid; e < NR * NB; e += DPT) Tr[e / NB][e % NB] = {0.f, 0.f};
+  // column k of the row of T that warp 1 .. NR holds: T[a][k] = -tau_k sum_{a <= c < k} T[a][c] z_c, T[k][k] = tau_k
+  auto extend_t = [&](int k) {
+    const int row = warp - 1, a = q + CL * row;
+    if (k < 0) return;
+    if (a < k) {
+      df2 t = {0.f, 0.f};
+      for (int c = a + lane; c < k; c += 32) acc(t, Tr[row][c], Z[c]);
+      t = norm(t);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t = add(t, shfl_xor(t, o));
+      if (lane == 0) Tr[row][k] = neg(mul(taus[k], t));
+    } else if (a == k && lane == 0) {
+      Tr[row][k] = taus[k];
+    }
+  };
   __syncthreads();
   // partials of pivot 0: x_0 . x_c below row 0, and pivot row 0 (rank 0)
   {
@@ -287,7 +297,10 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
     __syncthreads();
     PANEL_STAMP(1);
     // ---- column scalars (one thread; every CTA derives the same bits)
-    if (tid == 0) {
+    if (warp >= 1 && warp <= NR) {
+      // meanwhile: column k = jj - 1 of the held rows of T, T[a][k] = -tau_k sum_{a <= c < k} T[a][c] z_c
+      extend_t(jj - 1);
+    } else if (tid == 0) {
       const df2 sigma = S[jj], alpha = P[jj];
       df2 tj = {0.f, 0.f}, beta = alpha, scale = {0.f, 0.f};
       if (sigma.h != 0.f || sigma.l != 0.f) {
@@ -381,27 +394,12 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
     PANEL_STAMP(4);
     cluster_arrive_release();
     __syncthreads();
-    // ---- phase C: store v_jj (beta at the pivot) and column jj + 1; extend the held rows of
-    // T by column k = jj - 1: T[a][k] = -tau_k sum_{a <= c < k} T[a][c] z_c, T[k][k] = tau_k
+    // ---- phase C: store v_jj (beta at the pivot) and column jj + 1
     {
       const df2 beta = sc[1];
       for (int r = rA + tid; r < rows; r += DPT) {
         xj[r] = r == lj ? beta : V[r];
         if (has_next) xj[r + ld] = N[r];
-      }
-      const int k = jj - 1;
-      if (k >= 0 && warp < NR) {
-        const int a = q + CL * warp;
-        if (a < k) {
-          df2 t = {0.f, 0.f};
-          for (int c = a + lane; c < k; c += 32) acc(t, Tr[warp][c], Z[c]);
-          t = norm(t);
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) t = add(t, shfl_xor(t, o));
-          if (lane == 0) Tr[warp][k] = neg(mul(taus[k], t));
-        } else if (a == k && lane == 0) {
-          Tr[warp][k] = taus[k];
-        }
       }
     }
     // the next gather rewrites S, P and Z, which phase C still reads
@@ -415,22 +413,7 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
     if (a < nb - 1) Z[a] = tree_sum<CL>(cluster, &slot[nb & 1][2][0], a);
   }
   __syncthreads();
-  {
-    const int k = nb - 1;
-    if (warp < NR) {
-      const int a = q + CL * warp;
-      if (a < k) {
-        df2 t = {0.f, 0.f};
-        for (int c = a + lane; c < k; c += 32) acc(t, Tr[warp][c], Z[c]);
-        t = norm(t);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t = add(t, shfl_xor(t, o));
-        if (lane == 0) Tr[warp][k] = neg(mul(taus[k], t));
-      } else if (a == k && lane == 0) {
-        Tr[warp][k] = taus[k];
-      }
-    }
-  }
+  if (warp >= 1 && warp <= NR) extend_t(nb - 1);
   __syncthreads();
   // T (column-major, ld NB): this CTA's rows; tau from rank 0
   for (int e = tid; e < NR * NB; e += DPT) {

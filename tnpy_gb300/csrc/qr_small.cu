@@ -26,7 +26,7 @@
 
 #include <atomic>
 
-#include "jacobi.cuh"
+#include "householder.cuh"
 #include "tnx_internal.cuh"
 
 namespace cg = cooperative_groups;
@@ -50,34 +50,6 @@ inline int qs_ld(int64_t m, int64_t n) {
 __device__ __forceinline__ double lanes_sum(double v, int top) {
   for (int o = top; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
-}
-
-// Reflector of a column with pivot alpha and sigma = squares below it: beta, tau, scale (v = scale x)
-__device__ __forceinline__ void reflector(double alpha, double sigma, double& beta, double& tau, double& scale) {
-  tau = scale = 0.0;
-  beta = alpha;
-  if (!(sigma > 0.0)) return;
-  const double t2 = fma(alpha, alpha, sigma);
-  const int ex = (__double2hiint(t2) >> 20) & 0x7ff;
-  if (ex == 2047) {  // Inf or NaN in the column
-    const double nrm = sqrt(t2);
-    beta = alpha >= 0.0 ? -nrm : nrm;
-    tau = (beta - alpha) / beta;
-    scale = 1.0 / (alpha - beta);
-    return;
-  }
-  // t2 = s 2^e with even e and s in [1, 4): nrm = s y, y = 1 / sqrt(s)
-  const int e = (ex - 1023) & ~1, h = e / 2;
-  const double s = jac::scale_exp(t2, e), y = jac::rsqrt_exact(s), a = jac::scale_exp(fabs(alpha), h);
-  double nrm = s * y;
-  nrm = fma(0.5 * y, fma(-nrm, nrm, s), nrm);  // correctly rounded but for rare ties
-  tau = fma(a, y, 1.0);
-  // 1 / (|alpha| + nrm): FP32 seed, one third-order step
-  const double d = a + nrm, z = jac::to_double(__fdividef(1.f, jac::to_float(d))), r = fma(-d, z, 1.0);
-  const double inv = jac::scale_exp(fma(z * r, 1.0 + r, z), h);
-  nrm = jac::scale_exp(nrm, -h);
-  beta = alpha >= 0.0 ? -nrm : nrm;
-  scale = alpha >= 0.0 ? inv : -inv;
 }
 
 // Power of two that keeps the squares of a column in range: 1 unless alpha^2 + sigma, formed from the
