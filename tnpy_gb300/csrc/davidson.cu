@@ -11,11 +11,13 @@
 //   4. solves it for the lowest pair (Jacobi Rayleigh-Ritz, FP32 + FP64 correction),
 //   5. forms the Ritz vector, the residual r = H x - theta x and its norm, and the next
 //      direction t = r / (diag(H) - theta) (diagonal preconditioner).
-// The host loop reads three scalars per expansion to decide convergence. With the
+// The host loop reads a few scalars per expansion (once, from mapped host memory, for vectors of up to
+// DC_MAX elements) to decide convergence. With the
 // split-BF16 matvec a second, anchored phase takes the residual from the split-BF16
 // floor to FP64-class accuracy: one FP64-class matvec (tensor-core Ozaki GEMMs where large,
 // double-FP32 otherwise) per anchor; a start vector already near that floor goes to the
 // anchored phase after one matvec (see davidson1).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -23,7 +25,10 @@
 #include <type_traits>
 #include <vector>
 
+#include "jacobi.cuh"
 #include "tnx_internal.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace tnx {
 namespace {
@@ -304,6 +309,283 @@ inline int nchunk_for(int64_t n) {
   return int(c < 1 ? 1 : c);
 }
 
+// ---- one expansion's vector work in three cluster kernels (vectors of up to DC_MAX elements) -------
+//
+// For small sites an expansion is a chain of launches: 20 kernels of 2-7 us with their gaps and two host
+// reads, around one matvec and one Rayleigh-Ritz step. These kernels do the same arithmetic on one
+// cluster of eight CTAs, each holding its share of the vectors, with the sums over CTAs through
+// distributed shared memory in rank order: Gram-Schmidt with both norms, the DGKS gate and the scaling;
+// the new column of the projected matrix; the Ritz vector, residual and correction, which also puts
+// the expansion's scalars where the host reads them once. A direction that vanished against the basis
+// becomes zero there and is undone on the host. chi = 32 (2048 elements), per expansion: 191 us
+// before, 106 us so. Above DC_MAX the eight SMs' FP64 pipes cost more than the launches (one pass over 24
+// vectors takes 32 DC_MAX / 2 clocks of FMAs).
+constexpr int DC_CL = 8, DC_T = 512, DC_W = DC_T / 32;
+constexpr int64_t DC_MAX = 16384;
+constexpr int DC_PER = int(DC_MAX / DC_CL);  // elements of a vector per CTA
+
+struct Slice {
+  int64_t i0;
+  int len;
+  __device__ Slice(int64_t n, int rank) {
+    const int64_t per = (n + DC_CL - 1) / DC_CL;
+    i0 = rank * per;
+    len = int(i0 >= n ? 0 : (n - i0 < per ? n - i0 : per));
+  }
+};
+
+__device__ __forceinline__ double dc_warp_sum(double v) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// part[j] = this CTA's share of V_j . w (w in shared memory), one warp per j
+template <typename T>
+__device__ void dc_dots(const T* __restrict__ V, int64_t ldv, int k, const T* w, const Slice& s, double* part) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int j = warp; j < k; j += DC_W) {
+    const T* v = V + int64_t(j) * ldv + s.i0;
+    T a0 = T(0), a1 = T(0);
+    int i = lane;
+    for (; i + 32 < s.len; i += 64) {
+      a0 = fma(v[i], w[i], a0);
+      a1 = fma(v[i + 32], w[i + 32], a1);
+    }
+    if (i < s.len) a0 = fma(v[i], w[i], a0);
+    const double t = dc_warp_sum(double(a0) + double(a1));
+    if (lane == 0) part[j] = t;
+  }
+}
+
+// this CTA's sum of v over its threads into part[0]
+__device__ __forceinline__ void dc_block_sum(double v, double* red, double* part) {
+  v = dc_warp_sum(v);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    double t = threadIdx.x < DC_W ? red[threadIdx.x] : 0.0;
+    for (int o = DC_W / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (threadIdx.x == 0) part[0] = t;
+  }
+}
+
+// the same by one warp, in all its lanes: lane r takes rank r (every FP64 instruction of all 16 warps
+// would be four queued on each sub-partition's pipe)
+__device__ __forceinline__ double dc_total_warp(cg::cluster_group& cl, double* part, int j) {
+  const int lane = threadIdx.x & 31;
+  double t = cl.map_shared_rank(part, lane % DC_CL)[j];
+  for (int o = DC_CL / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
+}
+
+// sum over the ranks of their part[j]
+__device__ __forceinline__ double dc_total(cg::cluster_group& cl, double* part, int j) {
+  double t = 0.0;
+#pragma unroll
+  for (int r = 0; r < DC_CL; ++r) t += cl.map_shared_rank(part, r)[j];
+  return t;
+}
+
+// V[k] <- t orthogonalised against V[0..k) (second pass by the DGKS criterion) and scaled; nrm2[0], nrm2[1] = |t|^2
+// before and after; a vanished or non-finite direction becomes zero
+template <typename T>
+__global__ void __launch_bounds__(DC_T) dc_expand_kernel(T* __restrict__ V, int64_t n, int k, const T* __restrict__ t,
+                                                         double* __restrict__ nrm2) {
+  cg::cluster_group cl = cg::this_cluster();
+  const Slice s(n, int(cl.block_rank()));
+  __shared__ T w[DC_PER];
+  __shared__ double part[3][MAXB + 1], red[DC_W];
+  __shared__ T hs[MAXB];
+  double sq = 0.0;
+  for (int i = threadIdx.x; i < s.len; i += DC_T) {
+    const T x = t[s.i0 + i];
+    w[i] = x;
+    sq += double(x) * double(x);
+  }
+  dc_block_sum(sq, red, &part[0][MAXB]);
+  __syncthreads();
+  dc_dots(V, n, k, w, s, part[0]);
+  cl.sync();
+  __shared__ double s_before, s_after, s_f;
+  __shared__ int s_again;
+  const int warp = threadIdx.x >> 5;
+  if (warp == DC_W - 1) {
+    const double t = dc_total_warp(cl, part[0], MAXB);
+    s_before = s_after = t;  // every lane the same value
+  }
+  for (int pass = 0; pass < 2 && k > 0; ++pass) {
+    if (pass == 1) {
+      if (!s_again) break;  // uniform over the cluster: the same sums in every CTA
+      dc_dots(V, n, k, w, s, part[1]);
+      cl.sync();
+    }
+    if (threadIdx.x < k) hs[threadIdx.x] = T(dc_total(cl, part[pass], threadIdx.x));
+    __syncthreads();
+    sq = 0.0;
+    for (int i = threadIdx.x; i < s.len; i += DC_T) {
+      T acc = w[i];
+#pragma unroll 8
+      for (int j = 0; j < k; ++j) acc = fma(-hs[j], V[int64_t(j) * n + s.i0 + i], acc);
+      w[i] = acc;
+      sq += double(acc) * double(acc);
+    }
+    // each pass's sums have a slot of their own: slower CTAs may still read the one before
+    dc_block_sum(sq, red, &part[1 + pass][MAXB]);
+    cl.sync();
+    if (warp == 0) {
+      const double after = dc_total_warp(cl, part[1 + pass], MAXB);
+      s_after = after;
+      s_again = after < 0.5 * s_before;
+    }
+    __syncthreads();
+  }
+  __syncthreads();
+  if (warp == 0) {
+    const double before = s_before, after = s_after;
+    double f = 0.0;
+    if (after > 1e-26 * before && after > 0.0 && after < INFINITY) {
+      const int ex = (__double2hiint(after) >> 20) & 0x7ff, e = (ex - 1023) & ~1;
+      f = ex == 0 ? 1.0 / sqrt(after) : jac::scale_exp(jac::rsqrt_exact(jac::scale_exp(after, e)), e / 2);
+    }
+    s_f = f;
+    if (cl.block_rank() == 0 && threadIdx.x == 0) {
+      nrm2[0] = before;
+      nrm2[1] = after;
+    }
+  }
+  __syncthreads();
+  const bool ok = jac::bits(s_f) != 0;
+  const T f = T(s_f);
+  T* out = V + int64_t(k) * n + s.i0;
+  for (int i = threadIdx.x; i < s.len; i += DC_T) out[i] = ok ? w[i] * f : T(0);
+  cl.sync();  // no CTA leaves while another may still read its sums
+}
+
+// Hm[j][k] = Hm[k][j] = V_j . av for j <= k; with av0 (AV[0], exact) entry 0 is av0 . V_k instead
+template <typename T>
+__global__ void __launch_bounds__(DC_T) dc_project_kernel(const T* __restrict__ V, int64_t n, int k,
+                                                          const T* __restrict__ av, const T* __restrict__ av0,
+                                                          double* __restrict__ Hm, int mb) {
+  cg::cluster_group cl = cg::this_cluster();
+  const Slice s(n, int(cl.block_rank()));
+  __shared__ T w[DC_PER];
+  __shared__ double part[MAXB];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < s.len; i += DC_T) w[i] = av[s.i0 + i];
+  __syncthreads();
+  dc_dots(V, n, k + 1, w, s, part);
+  if (av0 && warp == 0 && k > 0) {  // the warp that took j = 0 takes it again
+    const T* vk = V + int64_t(k) * n + s.i0;
+    T a = T(0);
+    for (int i = lane; i < s.len; i += 32) a = fma(av0[s.i0 + i], vk[i], a);
+    const double t = dc_warp_sum(double(a));
+    if (lane == 0) part[0] = t;
+  }
+  cl.sync();
+  if (cl.block_rank() == 0 && threadIdx.x <= k) {
+    const double t = dc_total(cl, part, threadIdx.x);
+    Hm[int64_t(threadIdx.x) * mb + k] = t;
+    Hm[int64_t(k) * mb + threadIdx.x] = t;
+  }
+  cl.sync();
+}
+
+// What the host reads of an expansion: theta, |r|^2, |t|^2 before and after, the tensor-core wait flag
+// and the Ritz coefficients
+struct DavHost {
+  double theta, rn2, before, after, flag, s[MAXB];
+};
+
+// ritz_kernel on the cluster; host (mapped memory, may be null) gets the scalars
+template <typename T>
+__global__ void __launch_bounds__(DC_T) dc_ritz_kernel(const T* __restrict__ V, const T* __restrict__ AV, int64_t n,
+                                                       int k, const double* __restrict__ sv,
+                                                       const double* __restrict__ theta_p, const T* __restrict__ diag,
+                                                       int precond, T* __restrict__ x, T* __restrict__ ax,
+                                                       T* __restrict__ t, double* __restrict__ rn2,
+                                                       const double* __restrict__ nrm2, const int* __restrict__ flag,
+                                                       DavHost* host) {
+  cg::cluster_group cl = cg::this_cluster();
+  const Slice s(n, int(cl.block_rank()));
+  __shared__ T ss[MAXB];
+  __shared__ double part[1], red[DC_W];
+  if (threadIdx.x < k) ss[threadIdx.x] = T(sv[threadIdx.x]);
+  __syncthreads();
+  const T theta = T(theta_p[0]);
+  double sq = 0.0;
+  for (int q = threadIdx.x; q < s.len; q += DC_T) {
+    const int64_t i = s.i0 + q;
+    T xv = T(0), av = T(0);
+#pragma unroll 4
+    for (int j = 0; j < k; ++j) {
+      xv = fma(ss[j], V[int64_t(j) * n + i], xv);
+      av = fma(ss[j], AV[int64_t(j) * n + i], av);
+    }
+    const T r = av - theta * xv;
+    x[i] = xv;
+    ax[i] = av;
+    T tv = r;
+    if (precond) {
+      T den = diag[i] - theta;
+      const T floor = T(1e-2);
+      if (abs(den) < floor) den = den >= T(0) ? floor : -floor;
+      tv = r / den;
+    }
+    t[i] = tv;
+    sq += double(r) * double(r);
+  }
+  dc_block_sum(sq, red, part);
+  cl.sync();
+  if (cl.block_rank() == 0) {
+    const double total = threadIdx.x < 32 ? dc_total_warp(cl, part, 0) : 0.0;
+    if (threadIdx.x == 0) {
+      rn2[0] = total;
+      if (host) {
+        host->theta = theta_p[0];
+        host->rn2 = total;
+        host->before = nrm2[0];
+        host->after = nrm2[1];
+        host->flag = flag && flag[0] ? 1.0 : 0.0;
+      }
+    }
+    if (host && threadIdx.x < k) host->s[threadIdx.x] = sv[threadIdx.x];
+  }
+  cl.sync();
+}
+
+template <typename... P, typename... A>
+int launch_dc(void (*kernel)(P...), cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = DC_CL;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(DC_CL);
+  cfg.blockDim = dim3(DC_T);
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  TNX_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+  TNX_LAUNCH_CHECK();
+  return TNX_OK;
+}
+
+// Page-locked host memory that the device writes an expansion's scalars to: one block per host thread
+// for as long as the thread lives (a call owns it only while it runs, and waits for its stream).
+int dav_host(DavHost** out) {
+  struct Holder {
+    DavHost* p = nullptr;
+    ~Holder() {
+      if (p) cudaFreeHost(p);
+    }
+  };
+  thread_local Holder h;
+  if (!h.p) TNX_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&h.p), sizeof(DavHost), cudaHostAllocPortable | cudaHostAllocMapped));
+  *out = h.p;
+  return TNX_OK;
+}
+
 struct DavWs {
   double *V, *AV, *x, *ax, *t, *diag, *Hm, *Hwork, *evals, *evecs, *jwork, *part, *scal;
   double *xp, *axp;  // second vector of a GD+1 restart (previous Ritz vector, orthogonalised)
@@ -482,8 +764,41 @@ int davidson1(const double* L, const double* W, const double* R, double* x_io, i
 
   // Rayleigh-Ritz on V[0..k), Ritz vector x, AV-combination ax, residual norm and the next
   // direction t; reads theta, ||r|| and the Ritz coefficient of V[0] back to the host.
-  auto rayleigh_ritz = [&](const auto& vs) -> int {
+  DavHost* hp = nullptr;
+  TNX_TRY(dav_host(&hp));
+  const bool small = n <= DC_MAX;  // the expansion's vector work on one cluster
+  auto ritz_small = [&](const auto& vs, int kk, DavHost* to) -> int {
+    using T = std::remove_pointer_t<decltype(vs.V)>;
+    return launch_dc(dc_ritz_kernel<T>, st, vs.V, vs.AV, n, kk, w.evecs, w.evals, vs.diag, precond, vs.x, vs.ax, vs.t,
+                     rn2, nrm2, dflag, to);
+  };
+  // `fell_in` (small sites' expansions): the new direction vanished, the step is undone
+  auto rayleigh_ritz = [&](const auto& vs, bool* fell_in = nullptr) -> int {
     TNX_TRY(rr_lowest_f64(w.Hm, k, mb, w.evals, w.evecs, st));
+    if (small) {
+      TNX_TRY(ritz_small(vs, k, hp));
+      TNX_CUDA(cudaStreamSynchronize(st));
+      if (hp->flag != 0.0) {
+        set_error("tnx_davidson1: a bounded wait in the tensor-core matvec expired");
+        return TNX_ERR_TIMEOUT;
+      }
+      if (fell_in && (!(hp->after > 1e-26 * hp->before) || !(hp->after > 0.0) || !std::isfinite(hp->after))) {
+        *fell_in = true;
+        return TNX_OK;
+      }
+      std::swap(s_prev, s_cur);
+      prev_k = cur_k;
+      std::copy(hp->s, hp->s + k, s_cur.begin());
+      cur_k = k;
+      theta = hp->theta;
+      rnorm = sqrt(fmax(hp->rn2, 0.0));
+      c0 = hp->s[0];
+      if (!std::isfinite(theta) || !std::isfinite(rnorm)) {
+        set_error("tnx_davidson1: non-finite Ritz value or residual");
+        return TNX_ERR_INVALID_ARG;
+      }
+      return TNX_OK;
+    }
     ritz_kernel<<<nch, DT, 0, st>>>(vs.V, vs.AV, n, k, w.evecs, w.evals, vs.diag, precond, vs.x, vs.ax, vs.t, n,
                                     w.part, nch);
     TNX_LAUNCH_CHECK();
@@ -521,6 +836,26 @@ int davidson1(const double* L, const double* W, const double* R, double* x_io, i
     using T = std::remove_pointer_t<decltype(vs.V)>;
     *fell_in = false;
     T* vk = vs.V + int64_t(k) * n;
+    if (small) {
+      T* avk = vs.AV + int64_t(k) * n;
+      TNX_TRY(launch_dc(dc_expand_kernel<T>, st, vs.V, n, k, vs.t, nrm2));
+      TNX_TRY(matvec(vk, avk));
+      TNX_TRY(launch_dc(dc_project_kernel<T>, st, vs.V, n, k, avk, anchored && k > 0 ? vs.AV : nullptr, w.Hm, mb));
+      ++k;
+      TNX_TRY(rayleigh_ritz(vs, fell_in));
+      if (!*fell_in) {
+        ++iters;
+        return TNX_OK;
+      }
+      // the zero direction took the last row of the projected matrix: back to the basis without it, its
+      // Ritz pair and its vectors
+      if (--k == 0) {
+        set_error("tnx_davidson1: zero or non-finite start vector");
+        return TNX_ERR_INVALID_ARG;
+      }
+      TNX_TRY(rr_lowest_f64(w.Hm, k, mb, w.evals, w.evecs, st));
+      return ritz_small(vs, k, nullptr);
+    }
     TNX_CUDA(cudaMemcpyAsync(vk, vs.t, n * sizeof(T), cudaMemcpyDeviceToDevice, st));
     TNX_TRY(dots<T>(vk, n, 1, vk, n, w.part, nrm2, 1, nullptr, 0, st));
     for (int pass = 0; pass < 2 && k > 0; ++pass) {
