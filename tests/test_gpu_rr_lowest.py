@@ -21,3 +21,49 @@ def test_lowest_pair(n, scale):
     assert abs(e - w[0]) <= 8 * n * 2.0 ** -53 * norm
     assert abs(np.linalg.norm(v) - 1.0) <= 8 * n * 2.0 ** -53
     assert np.linalg.norm(a @ v - e * v) <= 16 * n * 2.0 ** -53 * norm
+
+
+def _form(form, n):
+    rng = np.random.RandomState(n)
+    if form == "diagonal":
+        return np.diag(rng.permutation(np.linspace(-2.0, 3.0, n)))
+    if form == "twice":  # every eigenvalue twice
+        m = rng.standard_normal((n // 2, n // 2))
+        return np.kron(np.eye(2), m + m.T)
+    a = np.diag(np.arange(n) - 5.0)
+    if form == "arrow":
+        a[-1, :-1] = a[:-1, -1] = rng.standard_normal(n - 1)
+    if form == "dense":
+        t = rng.standard_normal((n, n))
+        a = t + t.T
+    if form == "weak":  # the first vector solves it to 1e-9
+        t = rng.standard_normal((n - 1, n - 1))
+        a[1:, 1:] += 0.1 * (t + t.T)
+        a[0, 1:] = a[1:, 0] = 1e-9 * rng.standard_normal(n - 1)
+        a[0, 0] = -20.0
+    return a
+
+
+@pytest.mark.parametrize("n", [2, 6, 18, 32, 40, 64])
+@pytest.mark.parametrize("form", ["zero", "ones", "diagonal", "twice", "arrow", "dense", "weak"])
+@pytest.mark.parametrize("scale", [1.0, 1e-140, 1e140])
+def test_davidson_over_the_whole_space(n, form, scale):
+    """A basis that grows to the whole space: projected matrices of every size up to n."""
+    a = {"zero": np.zeros((n, n)), "ones": np.ones((n, n))}.get(form)
+    a = scale * (_form(form, n) if a is None else a)
+    w = np.linalg.eigvalsh(a)
+    norm = max(abs(w[0]), abs(w[-1]))
+    one = torch.ones((1, 1, 1), dtype=torch.float64, device="cuda")
+    x = torch.from_numpy(np.random.RandomState(n + 1).standard_normal((n, 1, 1))).cuda()
+    e, rn, its, ok = K.davidson1(torch.from_numpy(a).cuda().reshape(n, 1, n), one.reshape(1, 1, 1, 1), one, x,
+                                 tol=1e-11 if scale == 1.0 else 0.0, max_iter=200, max_basis=64)
+    v = x.cpu().numpy().ravel()
+    assert abs(np.linalg.norm(v) - 1.0) <= 1e-13
+    r = np.linalg.norm(a @ v - e * v)
+    # the reported residual is the true one, and the value is its own Rayleigh quotient
+    assert abs(r - rn) <= 64 * n * 2.0 ** -53 * norm
+    assert abs(e - v @ a @ v) <= 64 * n * 2.0 ** -53 * norm
+    if ok and scale == 1.0:  # an eigenpair; the lowest one where the start and the form let a Davidson reach it
+        assert r <= 2e-11 * max(1.0, abs(e))
+        gap = e - w[0] if form not in ("diagonal", "weak") else np.abs(e - w).min()
+        assert gap <= 2e-11 * max(1.0, abs(e))

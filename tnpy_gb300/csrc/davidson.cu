@@ -8,7 +8,7 @@
 //      second pass when the first removed more than half of its norm: DGKS),
 //   2. applies H (FP64, double-FP32 or split-BF16 tensor-core matvec),
 //   3. extends the projected matrix V^T H V (FP64 dots),
-//   4. solves it for the lowest pair (Jacobi Rayleigh-Ritz, FP32 + FP64 correction),
+//   4. solves it for the lowest pair (FP32 tridiagonal form + FP64 correction),
 //   5. forms the Ritz vector, the residual r = H x - theta x and its norm, and the next
 //      direction t = r / (diag(H) - theta) (diagonal preconditioner).
 // The host loop reads a few scalars per expansion (once, from mapped host memory, for vectors of up to
@@ -774,7 +774,7 @@ int davidson1(const double* L, const double* W, const double* R, double* x_io, i
   };
   // `fell_in` (small sites' expansions): the new direction vanished, the step is undone
   auto rayleigh_ritz = [&](const auto& vs, bool* fell_in = nullptr) -> int {
-    TNX_TRY(rr_lowest_f64(w.Hm, k, mb, w.evals, w.evecs, st));
+    TNX_TRY(rr_lowest_tri(w.Hm, k, mb, w.evals, w.evecs, st));
     if (small) {
       TNX_TRY(ritz_small(vs, k, hp));
       TNX_CUDA(cudaStreamSynchronize(st));
@@ -827,6 +827,32 @@ int davidson1(const double* L, const double* W, const double* R, double* x_io, i
     return TNX_OK;
   };
 
+  // The sign of a Ritz vector that leaves its basis is that of the Jacobi Rayleigh-Ritz step: where
+  // the two steps may differ in it (see rr_lowest_tri), that step and the combination are done again.
+  auto settle_sign = [&](const auto& vs) -> int {
+    using T = std::remove_pointer_t<decltype(vs.V)>;
+    for (int j = 0; j < cur_k; ++j)
+      if (s_cur[j] * s_cur[j] >= 0.99) return TNX_OK;
+    const std::vector<double> tri(s_cur.begin(), s_cur.begin() + k);
+    for (auto solve : {rr_lowest_f64, rr_lowest_tri}) {
+      TNX_TRY(solve(w.Hm, k, mb, w.evals, w.evecs, st));
+      if (small) {
+        TNX_TRY(ritz_small(vs, k, nullptr));
+      } else {
+        ritz_kernel<T><<<nch, DT, 0, st>>>(vs.V, vs.AV, n, k, w.evecs, w.evals, vs.diag, precond, vs.x, vs.ax, vs.t, n,
+                                           w.part, nch);
+        TNX_LAUNCH_CHECK();
+      }
+      TNX_CUDA(cudaMemcpyAsync(s_cur.data(), w.evecs, size_t(k) * 8, cudaMemcpyDeviceToHost, st));
+      TNX_CUDA(cudaStreamSynchronize(st));
+      // beyond FP32's range, and for a double eigenvalue, the sweeps may end at another vector: not that one
+      double dot = 0.0;
+      for (int j = 0; j < k; ++j) dot += s_cur[j] * tri[j];
+      if (fabs(dot) > 0.5) break;
+    }
+    return TNX_OK;
+  };
+
   // One expansion: t -> V[k] (classical Gram-Schmidt, second pass by the DGKS criterion),
   // AV[k] = H V[k], column k of V^T H V, Rayleigh-Ritz. With `anchored`, V[0] is a vector whose
   // product AV[0] = H V[0] is FP64-class exact, and row 0 of the projected matrix is taken as
@@ -853,7 +879,7 @@ int davidson1(const double* L, const double* W, const double* R, double* x_io, i
         set_error("tnx_davidson1: zero or non-finite start vector");
         return TNX_ERR_INVALID_ARG;
       }
-      TNX_TRY(rr_lowest_f64(w.Hm, k, mb, w.evals, w.evecs, st));
+      TNX_TRY(rr_lowest_tri(w.Hm, k, mb, w.evals, w.evecs, st));
       return ritz_small(vs, k, nullptr);
     }
     TNX_CUDA(cudaMemcpyAsync(vk, vs.t, n * sizeof(T), cudaMemcpyDeviceToDevice, st));
@@ -892,6 +918,7 @@ int davidson1(const double* L, const double* W, const double* R, double* x_io, i
   // thick restart with the current Ritz vector
   auto restart = [&](const auto& vs) -> int {
     using T = std::remove_pointer_t<decltype(vs.V)>;
+    TNX_TRY(settle_sign(vs));
     TNX_CUDA(cudaMemcpyAsync(vs.V, vs.x, n * sizeof(T), cudaMemcpyDeviceToDevice, st));
     TNX_CUDA(cudaMemcpyAsync(vs.AV, vs.ax, n * sizeof(T), cudaMemcpyDeviceToDevice, st));
     restart_kernel<<<1, 1, 0, st>>>(w.Hm, w.evals, w.evecs);
@@ -910,6 +937,7 @@ int davidson1(const double* L, const double* W, const double* R, double* x_io, i
   auto restart_plus = [&](const auto& vs) -> int {
     using T = std::remove_pointer_t<decltype(vs.V)>;
     if (prev_k != k - 1 || cur_k != k || k < 2) return restart(vs);
+    TNX_TRY(settle_sign(vs));
     double dot = 0.0;
     for (int j = 0; j < k - 1; ++j) dot += s_cur[j] * s_prev[j];
     double sp[MAXB], nrm = 0.0;
@@ -1028,6 +1056,7 @@ int davidson1(const double* L, const double* W, const double* R, double* x_io, i
       ++restarts;
     }
   }
+  if (!start_anchored) TNX_TRY(f32 ? settle_sign(v32) : settle_sign(v64));
   phase1 = iters;
   if (mixed) {
     // Anchored phase. One double-FP32 matvec gives AV[0] = H x exactly for the current Ritz
@@ -1109,6 +1138,7 @@ int davidson1(const double* L, const double* W, const double* R, double* x_io, i
           ++restarts;
         }
       }
+      TNX_TRY(settle_sign(v64));
       if (converged || iters >= max_iter) break;
     }
   }

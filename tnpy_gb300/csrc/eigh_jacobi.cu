@@ -342,9 +342,9 @@ int tnx_eigh_batched(double* A, const int64_t* offsets, const int* sizes, int ba
 //
 // A round of the sweep is two barriers long: the angles (one thread per pair), then every 2 x 2
 // block (pair k, pair l) of A <- J^T A J by one thread, columns first as in the two-pass form, so
-// each entry sees the operations of the two-pass form. A random 24 x 24 matrix: 211 us with a pass and a barrier each for
-// columns, rows and zeroing, exact divisions and the correction in FP64, 87 us so; 64 x 64: 1.90 ms
-// and 0.54 ms; the mean over a chi = 32 eigensolve's 68 problems 93 and 50 us.
+// each entry sees the operations of the two-pass form; a round without a rotation ends at the first
+// barrier. A random 24 x 24 matrix: 211 us with a pass and a barrier each for columns, rows and zeroing,
+// exact divisions and the correction in FP64, 80 us so; 64 x 64: 1.90 ms and 0.47 ms.
 // ---------------------------------------------------------------------------------------
 namespace tnx {
 namespace {
@@ -375,11 +375,10 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restric
   float* Vf = Af + n * nf;                                // n x (n+1) FP32
   float* rf = Vf + n * nf;                                // n: residual
   float* fp = rf + n;                                     // partial projections, RR_G x n
-  __shared__ float cs[32], ss[32];
-  __shared__ int pp[32], qq[32];
+  __shared__ float4 rot[32];  // c, s and (as integers) p, q of a pair
   __shared__ float red[RR_T / 32];
   __shared__ double redd[RR_T / 32];
-  __shared__ int s_any, s_imin;
+  __shared__ int s_imin;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float fro = 0.f;
   for (int e = tid; e < n * n; e += RR_T) {
@@ -393,7 +392,6 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restric
   }
   for (int o = 16; o > 0; o >>= 1) fro += __shfl_xor_sync(0xffffffffu, fro, o);
   if (lane == 0) red[warp] = fro;
-  if (tid == 0) s_any = 0;
   __syncthreads();
   fro = 0.f;
   for (int w = 0; w < RR_T / 32; ++w) fro += red[w];
@@ -403,7 +401,9 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restric
     const int np = n + (n & 1), npairs = np / 2;
     const int tx = tid & 15, ty = tid >> 4;
     for (int sweep = 0; sweep < 30; ++sweep) {
+      bool any = false;
       for (int rnd = 0; rnd < np - 1; ++rnd) {
+        bool turns = false;
         if (tid < npairs) {
           int p, q;
           jac::pair_of(tid, rnd, np, p, q);
@@ -417,21 +417,24 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restric
               const float t = copysignf(__fdividef(1.f, fmaf(h2, rsqrtf(h2), fabsf(th))), th);
               c = rsqrtf(fmaf(t, t, 1.f));
               sn = t * c;
-              s_any = 1;
+              turns = true;
             }
           }
-          pp[tid] = p; qq[tid] = q; cs[tid] = c; ss[tid] = sn;
+          rot[tid] = make_float4(c, sn, __int_as_float(p), __int_as_float(q));
         }
-        __syncthreads();
+        if (!__syncthreads_or(turns)) continue;  // nothing to apply: straight to the next round's angles
+        any = true;
         // A <- J^T (A J): block (rows of pair k, columns of pair l); the padding player of an odd n
         // (index n) has no entries
         for (int k = ty; k < npairs; k += RR_T / 16) {
-          const float sk = ss[k], ck = cs[k];
-          const int pk = pp[k], qk = qq[k];
+          const float4 rk = rot[k];
+          const float sk = rk.y, ck = rk.x;
+          const int pk = __float_as_int(rk.z), qk = __float_as_int(rk.w);
           for (int l = tx; l < npairs; l += 16) {
-            const float sl = ss[l], cl = cs[l];
+            const float4 rl = rot[l];
+            const float sl = rl.y, cl = rl.x;
             if (sk == 0.f && sl == 0.f) continue;
-            const int pl = pp[l], ql = qq[l];
+            const int pl = __float_as_int(rl.z), ql = __float_as_int(rl.w);
             const bool row2 = qk < n, col2 = ql < n;
             float* r0 = Af + pk * nf;
             float* r1 = Af + qk * nf;
@@ -455,9 +458,10 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restric
         }
         // V <- V J
         for (int l = ty; l < npairs; l += RR_T / 16) {
-          const float sl = ss[l], cl = cs[l];
+          const float4 rl = rot[l];
+          const float sl = rl.y, cl = rl.x;
           if (sl == 0.f) continue;
-          const int pl = pp[l], ql = qq[l];
+          const int pl = __float_as_int(rl.z), ql = __float_as_int(rl.w);
           for (int j = tx; j < n; j += 16) {
             const float va = Vf[j * nf + pl], vb = Vf[j * nf + ql];
             Vf[j * nf + pl] = cl * va - sl * vb;
@@ -466,12 +470,7 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restric
         }
         __syncthreads();
       }
-      // every thread reads the flag before thread 0 clears it for the next sweep
-      const int any = s_any;
-      __syncthreads();
       if (!any) break;
-      if (tid == 0) s_any = 0;
-      __syncthreads();
     }
   }
   // lowest FP32 eigenvalue (the first of equal ones), by warp 0
@@ -540,10 +539,7 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restric
     }
     __syncthreads();
     const double nn = redd[0] + redd[1];
-    // 1 / sqrt(nn) from an FP32 seed by two Newton steps
-    double inv = double(rsqrtf(float(nn)));
-    inv = inv * fma(-0.5 * nn * inv, inv, 1.5);
-    inv = inv * fma(-0.5 * nn * inv, inv, 1.5);
+    const double inv = jac::rsqrt_exact(nn);  // nn is 1 to FP32 accuracy
     const double theta = (redd[2] + redd[3]) * (inv * inv);
     if (tid < n) s[tid] = si * inv;
     if (step == 3) {
@@ -602,6 +598,472 @@ int rr_lowest_f64_batched(const double* A, int n, int ld, int64_t sA, double* ev
   }
   profile_mark(KF_EIGH, st, true);
   rr_lowest_kernel<<<batch, RR_T, rr_lowest_smem(n), st>>>(A, n, ld, eval, evec, sA, sE, sV, active);
+  profile_mark(KF_EIGH, st, false);
+  TNX_LAUNCH_CHECK();
+  return TNX_OK;
+}
+
+}  // namespace tnx
+
+// ---------------------------------------------------------------------------------------
+// The lowest pair by way of a tridiagonal form (n <= 64), for a Davidson's Rayleigh-Ritz steps: four
+// warps. Only one pair is wanted, so FP32 finds that one: Householder reflectors (a lane holds a row in
+// registers, one warp per 32 rows; as many warps apply the reflectors to the rows of Q at the same
+// time), 32 Sturm sequences at a time around the lowest eigenvalue, and its vector from the twisted
+// factorisation of T - lambda. FP64 then refines the pair against the given matrix,
+//   s <- s - Q x,  (T - lambda) x = Q^T r without row and column k,  r = A s - theta s,
+// where k is the twist index: T - lambda without it is positive definite, and its factors are there
+// already. A step contracts the error by ~(FP32 error) / gap, and the steps go on until the next one
+// would be below FP64 rounding (two as a rule, six at most). Only s, r, theta and the norm are FP64;
+// the correction's relative error of ~1e-6 is what T and Q leave it anyway. theta gains s . r, whose
+// FP32 rounding shrinks with r. A random 24 x 24 matrix: 80 us in the kernel above, 27 us here; 64 x 64:
+// 471 and 76 us; the mean over a chi = 32 eigensolve's 68 problems 45 and 20 us.
+//
+// The vector's largest entry is positive. The sweeps above give their vector the same sign where
+// the square of that entry is at least 0.99 (none of 4.7 million random problems of 3 to 24 rows
+// differed; 1 in 13000 did between 0.9 and 0.99).
+// ---------------------------------------------------------------------------------------
+namespace tnx {
+namespace {
+
+constexpr int RT_T = 128;
+
+__device__ __forceinline__ float rr_sum(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// x 2^-e; zero for zero and where it would be subnormal
+__device__ __forceinline__ double rr_scale(double x, int e) {
+  return (__double2hiint(x) & 0x7ff00000) == 0 ? 0.0 : jac::scale_exp(x, e);
+}
+
+template <int NR>
+__global__ void __launch_bounds__(RT_T) rr_tri_kernel(const double* __restrict__ A, int n, int ld,
+                                                      double* __restrict__ eval, double* __restrict__ evec) {
+  constexpr int LR = NR / 32;  // rows per lane of one warp
+  constexpr int QS = NR + 1;   // row stride of Q (conflict-free along rows and columns)
+  extern __shared__ double sm_d[];
+  const int nf = n + 1;
+  double* Ad = sm_d;                                   // n x (n+1) FP64
+  float* Vs = reinterpret_cast<float*>(Ad + n * nf);   // reflector k in row k
+  float* Q = Vs + NR * NR;                             // first the scaled matrix, then Q
+  __shared__ __align__(16) float xrow[2][NR], pw[NR];
+  __shared__ float td[NR], te[NR], cs[NR], red[2];
+  __shared__ float2 tde[NR];                           // diagonal, square of the off-diagonal before it
+  __shared__ float2 fm[2][NR];                         // pivots' reciprocals and multipliers, from both ends
+  __shared__ float piv[2][NR], gv[NR], yv[NR], zv[NR], dv[NR];
+  __shared__ double sd[NR], rp[3][NR];
+  __shared__ unsigned s_max[RT_T / 32];
+  __shared__ int s_done;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+
+  // the matrix, and the power of two that brings its Frobenius norm to at most one
+  unsigned mx = 0;
+  for (int i = warp; i < n; i += RT_T / 32)
+    for (int j = lane; j < n; j += 32) {
+      const double v = A[int64_t(i) * ld + j];
+      Ad[i * nf + j] = v;
+      mx = max(mx, unsigned(__double2hiint(v)) & 0x7fffffffu);
+    }
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if (lane == 0) s_max[warp] = mx;
+  __syncthreads();
+  mx = max(max(s_max[0], s_max[1]), max(s_max[2], s_max[3]));
+  const int ex = int(mx >> 20) - 1022 + (NR == 32 ? 5 : 6);
+  for (int i = warp; i < NR; i += RT_T / 32)
+#pragma unroll
+    for (int j = lane; j < NR; j += 32)
+      Q[i * QS + j] = i < n && j < n ? jac::to_float(rr_scale(Ad[i * nf + j], ex)) : 0.f;
+  __syncthreads();
+
+  // ---- tridiagonal form: warps [0, LR) hold the rows of A, warps [LR, 2 LR) those of Q
+  const bool is_a = warp < LR, is_q = !is_a && warp < 2 * LR;
+  const int row = (is_a ? warp : warp - LR) * 32 + lane;
+  float a[NR];
+  if (is_a) {
+#pragma unroll
+    for (int j = 0; j < NR; ++j) a[j] = Q[row * QS + j];
+  } else {
+#pragma unroll
+    for (int j = 0; j < NR; ++j) a[j] = j == row ? 1.f : 0.f;
+  }
+  auto sync_a = [] {  // among the warps of A
+    if (LR == 1) __syncwarp();
+    else __syncthreads();
+  };
+  for (int k = 0; k < n; ++k) {
+    float* xr = xrow[k & 1];
+    if (is_a && row == k) {
+#pragma unroll
+      for (int j = 0; j < NR; j += 4) *reinterpret_cast<float4*>(xr + j) = make_float4(a[j], a[j + 1], a[j + 2], a[j + 3]);
+    }
+    sync_a();
+    if (tid == 0) td[k] = xr[k];
+    if (k >= n - 2) {
+      if (tid == 0) te[k] = k == n - 2 ? xr[n - 1] : 0.f;
+      continue;
+    }
+    float vi = 0.f, c = 0.f;
+    if (is_a) {  // the reflector, by each warp of A for itself
+      const float alpha = xr[k + 1];
+      float sq = 0.f;
+#pragma unroll
+      for (int j = lane; j < NR; j += 32) sq += j > k + 1 ? xr[j] * xr[j] : 0.f;
+      sq = rr_sum(sq);
+      float beta = alpha;
+      if (sq > 1e-22f) {  // entries below 1e-11 of the norm count as zero
+        const float h = fmaf(alpha, alpha, sq), nr = h * rsqrtf(h);
+        beta = -copysignf(nr, alpha);
+        c = __fdividef(1.f, nr * (nr + fabsf(alpha)));
+        vi = row > k + 1 ? xr[row] : (row == k + 1 ? alpha - beta : 0.f);
+      }
+      Vs[k * NR + row] = vi;
+      if (tid == 0) {
+        te[k] = beta;
+        cs[k] = c;
+      }
+    }
+    __syncthreads();
+    const float* v = Vs + k * NR;
+    auto times_v = [&] {
+      float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
+#pragma unroll
+      for (int j = 0; j < NR; j += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(v + j);
+        p0 = fmaf(a[j], x.x, p0);
+        p1 = fmaf(a[j + 1], x.y, p1);
+        p2 = fmaf(a[j + 2], x.z, p2);
+        p3 = fmaf(a[j + 3], x.w, p3);
+      }
+      return (p0 + p1) + (p2 + p3);
+    };
+    float p = 0.f, dot = 0.f;
+    if (is_a) {
+      p = c * times_v();
+      dot = rr_sum(p * vi);
+    }
+    if (LR == 2) {
+      if (is_a) pw[row] = p;
+      if (is_a && lane == 0) red[warp] = dot;
+      __syncthreads();
+    }
+    if (is_a) {
+      if (LR == 1) {
+        const float wi = fmaf(-0.5f * c * dot, vi, p);
+        pw[row] = wi;
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < NR; j += 4) {
+          const float4 x = *reinterpret_cast<const float4*>(v + j), w = *reinterpret_cast<const float4*>(pw + j);
+          a[j] = fmaf(-vi, w.x, fmaf(-wi, x.x, a[j]));
+          a[j + 1] = fmaf(-vi, w.y, fmaf(-wi, x.y, a[j + 1]));
+          a[j + 2] = fmaf(-vi, w.z, fmaf(-wi, x.z, a[j + 2]));
+          a[j + 3] = fmaf(-vi, w.w, fmaf(-wi, x.w, a[j + 3]));
+        }
+      } else {
+        const float kk = 0.5f * c * (red[0] + red[1]), wi = fmaf(-kk, vi, p);
+        const float ui = fmaf(-kk, vi, wi);  // a - v_i w_j - w_i v_j = a - v_i p_j - (w_i - K v_i) v_j
+#pragma unroll
+        for (int j = 0; j < NR; j += 4) {
+          const float4 x = *reinterpret_cast<const float4*>(v + j), q = *reinterpret_cast<const float4*>(pw + j);
+          a[j] = fmaf(-vi, q.x, fmaf(-ui, x.x, a[j]));
+          a[j + 1] = fmaf(-vi, q.y, fmaf(-ui, x.y, a[j + 1]));
+          a[j + 2] = fmaf(-vi, q.z, fmaf(-ui, x.z, a[j + 2]));
+          a[j + 3] = fmaf(-vi, q.w, fmaf(-ui, x.w, a[j + 3]));
+        }
+      }
+    } else if (is_q) {  // Q <- Q (1 - c v v^T)
+      const float y = cs[k] * times_v();
+#pragma unroll
+      for (int j = 0; j < NR; j += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(v + j);
+        a[j] = fmaf(-y, x.x, a[j]);
+        a[j + 1] = fmaf(-y, x.y, a[j + 1]);
+        a[j + 2] = fmaf(-y, x.z, a[j + 2]);
+        a[j + 3] = fmaf(-y, x.w, a[j + 3]);
+      }
+    }
+  }
+  if (is_q) {  // the scaled matrix in its place was read before the loop's first barrier
+#pragma unroll
+    for (int j = 0; j < NR; ++j) Q[row * QS + j] = a[j];
+  }
+  __syncthreads();
+
+  // ---- lowest eigenvalue of T and the factors, by warp 0
+  double sv[LR], theta = 0.0;
+  float z[LR], nrm = 0.f;
+  int kt = 0;
+  auto q_times = [&](const float* x, int i) {  // row i of Q
+    float t0 = 0.f, t1 = 0.f, t2 = 0.f, t3 = 0.f;
+#pragma unroll
+    for (int j = 0; j < NR; j += 4) {
+      t0 = fmaf(Q[i * QS + j], x[j], t0);
+      t1 = fmaf(Q[i * QS + j + 1], x[j + 1], t1);
+      t2 = fmaf(Q[i * QS + j + 2], x[j + 2], t2);
+      t3 = fmaf(Q[i * QS + j + 3], x[j + 3], t3);
+    }
+    return (t0 + t1) + (t2 + t3);
+  };
+  if (warp == 0) {
+    float lo = 3e38f, hi = 3e38f;
+#pragma unroll
+    for (int i = lane; i < NR; i += 32) {
+      if (i < n) {
+        const float dd = td[i], e0 = i > 0 ? te[i - 1] : 0.f, off = fabsf(e0) + fabsf(te[i]);
+        lo = fminf(lo, dd - off);
+        hi = fminf(hi, dd);
+        nrm = fmaxf(nrm, fabsf(dd) + off);
+        tde[i] = make_float2(dd, e0 * e0);
+      }
+      zv[i] = dv[i] = gv[i] = 0.f;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+      hi = fminf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+      nrm = fmaxf(nrm, __shfl_xor_sync(0xffffffffu, nrm, o));
+    }
+    __syncwarp();
+    lo -= 1e-6f * nrm;
+    // 33^5 parts of at most twice the norm: 5e-8 of it. A sequence of leading minors (rescaled every
+    // four, the norm is at most one) stays positive below the lowest eigenvalue.
+    for (int pass = 0; pass < 5; ++pass) {
+      const float h = (hi - lo) * (1.f / 33.f), x = fmaf(h, float(lane + 1), lo);
+      float p0 = 1.f, p1 = 1.f, mn = 1.f;
+      for (int i = 0; i < n; i += 4) {
+        const float f = __uint_as_float((254u << 23) - (__float_as_uint(p1) & 0x7f800000u));
+        p0 *= f;
+        p1 *= f;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (i + u < n) {
+            const float2 t = tde[i + u];
+            const float p2 = fmaf(t.x - x, p1, -t.y * p0);
+            p0 = p1;
+            p1 = p2;
+            mn = fminf(mn, p2);
+          }
+        }
+      }
+      const unsigned below = __ballot_sync(0xffffffffu, mn > 0.f);
+      const int f = below == 0xffffffffu ? 32 : __ffs(~below) - 1;  // first lane at or above it
+      const float l0 = lo;
+      if (f > 0) lo = fmaf(h, float(f), l0);
+      if (f < 32) hi = fmaf(h, float(f + 1), l0);
+    }
+    // pivots of T - lo from the top (lane 0) and from the bottom (lane 1); those before the twist are
+    // positive, and below the rounding of T they mean nothing
+    const float floor = fmaxf(1e-6f * nrm, 1e-30f);
+    if (lane < 2) {
+      float prev = 0.f;  // off-diagonal squared / pivot
+      for (int t = 0; t < n; ++t) {
+        const int i = lane == 0 ? t : n - 1 - t;
+        const float p = (td[i] - lo) - prev;
+        const float r = __fdividef(1.f, fmaxf(p, floor));
+        const float e = lane == 0 ? te[i] : (i > 0 ? te[i - 1] : 0.f);
+        piv[lane][i] = p;
+        fm[lane][i] = make_float2(r, -e * r);
+        prev = e * e * r;
+      }
+    }
+    __syncwarp();
+    float gm = 3e38f;
+#pragma unroll
+    for (int i = lane; i < NR; i += 32)
+      if (i < n) {
+        const float g = fabsf(piv[0][i] + piv[1][i] - (td[i] - lo));
+        if (g < gm) {
+          gm = g;
+          kt = i;
+        }
+      }
+    for (int o = 16; o > 0; o >>= 1) {
+      const float og = __shfl_xor_sync(0xffffffffu, gm, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, kt, o);
+      if (og < gm || (og == gm && oi < kt)) {
+        gm = og;
+        kt = oi;
+      }
+    }
+    if (lane < 2) {
+      float x = 1.f;
+      if (lane == 0) zv[kt] = 1.f;
+      const int m = lane == 0 ? kt : n - 1 - kt, step = lane == 0 ? -1 : 1;
+#pragma unroll 4
+      for (int t = 1; t <= m; ++t) {
+        const int i = kt + t * step;
+        x *= fm[lane][i].y;
+        zv[i] = x;
+      }
+    }
+    __syncwarp();
+    float zz = 0.f;
+#pragma unroll
+    for (int u = 0; u < LR; ++u) {
+      z[u] = zv[lane + 32 * u];
+      zz = fmaf(z[u], z[u], zz);
+    }
+    const float zi = rsqrtf(rr_sum(zz));
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < LR; ++u) zv[lane + 32 * u] = z[u] *= zi;
+    __syncwarp();
+    float sf[LR], big = -1.f, val = 0.f;
+#pragma unroll
+    for (int u = 0; u < LR; ++u) {
+      sf[u] = q_times(zv, lane + 32 * u);
+      if (fabsf(sf[u]) > big) {
+        big = fabsf(sf[u]);
+        val = sf[u];
+      }
+    }
+    int at = lane;
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ob = __shfl_xor_sync(0xffffffffu, big, o), ov = __shfl_xor_sync(0xffffffffu, val, o);
+      const int oa = __shfl_xor_sync(0xffffffffu, at, o);
+      if (ob > big || (ob == big && oa < at)) {
+        big = ob;
+        val = ov;
+        at = oa;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < LR; ++u) sd[lane + 32 * u] = sv[u] = jac::to_double(copysignf(1.f, val) * sf[u]);
+    theta = rr_scale(jac::to_double(lo), -ex);
+  }
+  __syncthreads();
+
+  // ---- refinement: warps 1-3 form A s, warp 0 the norm and the correction
+  float dn_prev = 1.f;
+  for (int step = 0; step < 6; ++step) {
+    double nn = 0.0;
+    if (warp > 0) {
+#pragma unroll
+      for (int i = lane; i < NR; i += 32)
+        if (i < n) {
+          double acc = 0.0;
+          for (int j = warp - 1; j < n; j += 3) acc = fma(Ad[i * nf + j], sd[j], acc);
+          rp[warp - 1][i] = acc;
+        }
+    } else {
+#pragma unroll
+      for (int u = 0; u < LR; ++u) nn = fma(sv[u], sv[u], nn);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) nn += __shfl_xor_sync(0xffffffffu, nn, o);
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const float inn = __fdividef(1.f, jac::to_float(nn));
+      float rf[LR], sf[LR], rho = 0.f;
+#pragma unroll
+      for (int u = 0; u < LR; ++u) {
+        const int i = lane + 32 * u;
+        const double y = i < n ? (rp[0][i] + rp[1][i]) + rp[2][i] : 0.0;
+        rf[u] = jac::to_float(rr_scale(fma(-theta, sv[u], y), ex));
+        sf[u] = jac::to_float(sv[u]);
+        rho = fmaf(rf[u], sf[u], rho);
+      }
+      rho = rr_sum(rho) * inn;
+      theta += rr_scale(jac::to_double(rho), -ex);
+#pragma unroll
+      for (int u = 0; u < LR; ++u) yv[lane + 32 * u] = fmaf(-rho, sf[u], rf[u]);
+      __syncwarp();
+#pragma unroll
+      for (int u = 0; u < LR; ++u) {  // Q^T r
+        float t0 = 0.f, t1 = 0.f;
+#pragma unroll
+        for (int i = 0; i < NR; i += 2) {
+          t0 = fmaf(Q[i * QS + lane + 32 * u], yv[i], t0);
+          t1 = fmaf(Q[(i + 1) * QS + lane + 32 * u], yv[i + 1], t1);
+        }
+        gv[lane + 32 * u] = t0 + t1;
+      }
+      __syncwarp();
+      if (lane < 2) {  // lane 0 the rows above the twist, lane 1 those below
+        const int m = lane == 0 ? kt : n - 1 - kt, first = lane == 0 ? 0 : n - 1, up = lane == 0 ? 1 : -1;
+        float x = 0.f, mu = 0.f;
+#pragma unroll 4
+        for (int t = 0; t < m; ++t) {
+          const int i = first + t * up;
+          x = fmaf(mu, x, gv[i]);
+          const float2 f = fm[lane][i];
+          yv[i] = x * f.x;
+          mu = f.y;
+        }
+        x = 0.f;
+#pragma unroll 4
+        for (int t = 1; t <= m; ++t) {
+          const int i = kt - t * up;
+          x = fmaf(fm[lane][i].y, x, yv[i]);
+          dv[i] = x;
+        }
+        if (lane == 0) dv[kt] = 0.f;
+      }
+      __syncwarp();
+      float d[LR], zd = 0.f, dd = 0.f;
+#pragma unroll
+      for (int u = 0; u < LR; ++u) {
+        d[u] = dv[lane + 32 * u];
+        zd = fmaf(d[u], z[u], zd);
+      }
+      zd = rr_sum(zd);
+      __syncwarp();
+#pragma unroll
+      for (int u = 0; u < LR; ++u) {
+        d[u] = fmaf(-zd, z[u], d[u]);
+        dd = fmaf(d[u], d[u], dd);
+        dv[lane + 32 * u] = d[u];
+      }
+      dd = rr_sum(dd);
+      __syncwarp();
+      const double inv = jac::rsqrt_exact(nn);
+      const bool last = step == 5;
+#pragma unroll
+      for (int u = 0; u < LR; ++u) {
+        const double c = last ? 0.0 : jac::to_double(q_times(dv, lane + 32 * u));
+        sd[lane + 32 * u] = sv[u] = (sv[u] - c) * inv;
+      }
+      // the next correction would be about dd / dn_prev; rho's own rounding is 1e-7 of it
+      const float dn = sqrtf(dd);
+      const bool done = last || (fabsf(rho) <= 1e-9f * nrm && (dd <= 2e-16f * dn_prev || dn <= 1e-15f));
+      dn_prev = dn;
+      if (lane == 0) s_done = done;
+      if (done) {
+        if (lane == 0) eval[0] = theta;
+#pragma unroll
+        for (int u = 0; u < LR; ++u)
+          if (lane + 32 * u < n) evec[lane + 32 * u] = sv[u];
+      }
+    }
+    __syncthreads();
+    if (s_done) break;
+  }
+}
+
+size_t rr_tri_smem(int n, int nr) { return size_t(n) * (n + 1) * 8 + size_t(nr) * (2 * nr + 1) * 4; }
+
+}  // namespace
+
+int rr_lowest_tri(const double* A, int n, int ld, double* eval, double* evec, cudaStream_t st) {
+  if (n > RW_MAX) {
+    set_error("rr_lowest_tri: n=%d > %d", n, RW_MAX);
+    return TNX_ERR_SHAPE;
+  }
+  profile_mark(KF_EIGH, st, true);
+  if (n <= 32) {
+    rr_tri_kernel<32><<<1, RT_T, rr_tri_smem(n, 32), st>>>(A, n, ld, eval, evec);
+  } else {
+    static std::atomic<bool> attr{false};  // idempotent setup; threads may race to it
+    if (!attr.load()) {
+      TNX_CUDA(cudaFuncSetAttribute(rr_tri_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    int(rr_tri_smem(RW_MAX, 64))));
+      attr.store(true);
+    }
+    rr_tri_kernel<64><<<1, RT_T, rr_tri_smem(n, 64), st>>>(A, n, ld, eval, evec);
+  }
   profile_mark(KF_EIGH, st, false);
   TNX_LAUNCH_CHECK();
   return TNX_OK;

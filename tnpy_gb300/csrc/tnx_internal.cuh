@@ -253,6 +253,8 @@ int eigh_small_f64_uniform(const double* A, int n, int ld, int keep, double* eva
                            double* work, cudaStream_t st);
 // lowest eigenpair of one n x n (n <= 64) matrix: FP32 Jacobi + FP64 refinement
 int rr_lowest_f64(const double* A, int n, int ld, double* eval, double* evec, cudaStream_t st);
+// the same, faster; the vector's sign is by its largest entry
+int rr_lowest_tri(const double* A, int n, int ld, double* eval, double* evec, cudaStream_t st);
 // the same for `batch` matrices at A + b sA (results at eval + b sE, evec + b sV); blocks whose
 // active[b] is 0 return at once (active may be null)
 int rr_lowest_f64_batched(const double* A, int n, int ld, int64_t sA, double* eval, int64_t sE, double* evec,
