@@ -487,9 +487,13 @@ size_t qr_layout(int64_t m, int64_t n, void* base, QrWs* w) {
   return off;
 }
 
-// Leading dimension of a CTA's panel rows: a multiple of 16 doubles plus the threads per column,
-// so the TPC row-interleaved threads of 16 / TPC neighbouring columns hit distinct banks.
-inline int panel_ld(int64_t rpc, int tpc) { return int((rpc + 15) / 16 * 16 + tpc); }
+// Leading dimension of a CTA's panel rows. FP64: a multiple of 16 doubles plus the threads per column,
+// so the TPC row-interleaved threads of 16 / TPC neighbouring columns hit distinct banks. Double-FP32:
+// odd, for the threads that take one row of all columns.
+template <bool DF>
+int panel_ld(int64_t rpc, int nb) {
+  return DF ? int(rpc | 1) : int((rpc + 15) / 16 * 16 + PT / nb);
+}
 
 // One-time attribute setup of a cluster panel instantiation: largest dynamic shared memory it
 // may use and whether a cluster of CL CTAs with that much shared memory can be scheduled.
@@ -499,9 +503,16 @@ struct PanelKernelInfo {
 };
 
 // DF selects the double-FP32 panel (FP64-class modes), otherwise the FP64 one
-using PanelFn = void (*)(double*, int64_t, int64_t, int, int, double*, double*);
+template <bool DF>
+struct PanelFn {
+  using type = void (*)(double*, int64_t, int64_t, int, int, double*, double*);
+};
+template <>
+struct PanelFn<true> {
+  using type = void (*)(double*, int64_t, int64_t, int, int, int, double*, double*);
+};
 template <int NB, int CL, bool DF>
-PanelFn panel_fn() {
+typename PanelFn<DF>::type panel_fn() {
   if constexpr (DF) return qrdf::panel_df_kernel<NB, CL>;
   else return panel_cl_kernel<NB, CL>;
 }
@@ -515,7 +526,7 @@ const PanelKernelInfo& panel_info() {
   static PanelKernelInfo info;
   static std::once_flag once;
   std::call_once(once, [] {
-    PanelFn k = panel_fn<NB, CL, DF>();
+    const auto k = panel_fn<NB, CL, DF>();
     cudaFuncAttributes fa{};
     int dev = 0, optin = 0;
     if (cudaFuncGetAttributes(&fa, k) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess ||
@@ -551,10 +562,29 @@ const PanelKernelInfo& panel_info() {
   return info;
 }
 
+// dynamic shared memory of a panel CTA with row stride ld
+template <int NB, int CL, bool DF>
+size_t panel_smem(int ld, bool push) {
+  if constexpr (DF) return qrdf::panel_df_smem_bytes<NB, CL>(ld, push);
+  else return size_t(NB + 2) * ld * sizeof(double);
+}
+
 template <int NB, int CL, bool DF>
 int launch_panel(double* F, int64_t m, int64_t j0, int nb, double* tau, double* T, cudaStream_t st) {
   const int64_t rpc = (m - j0 + CL - 1) / CL;
-  const int ld = panel_ld(rpc, panel_threads<DF>() / NB);
+  int ld = panel_ld<DF>(rpc, NB), mode = 0;
+  size_t smem = panel_smem<NB, CL, DF>(ld, false);
+  if constexpr (DF) {
+    const size_t most = panel_info<NB, CL, DF>().max_dyn;
+    const int padded = panel_ld<DF>(rpc + qrdf::PAD_ROWS, NB);
+    if (panel_smem<NB, CL, DF>(padded, true) <= most) {
+      ld = padded;
+      mode = qrdf::PUSH | qrdf::PAD;
+    } else if (panel_smem<NB, CL, DF>(ld, true) <= most) {
+      mode = qrdf::PUSH;
+    }
+    smem = panel_smem<NB, CL, DF>(ld, mode != 0);
+  }
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -563,11 +593,15 @@ int launch_panel(double* F, int64_t m, int64_t j0, int nb, double* tau, double* 
   at[0].val.clusterDim.z = 1;
   cfg.gridDim = dim3(CL);
   cfg.blockDim = dim3(panel_threads<DF>());
-  cfg.dynamicSmemBytes = size_t(NB + 2) * ld * sizeof(double);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  TNX_CUDA(cudaLaunchKernelEx(&cfg, panel_fn<NB, CL, DF>(), F, m, j0, nb, ld, tau, T));
+  if constexpr (DF) {
+    TNX_CUDA(cudaLaunchKernelEx(&cfg, panel_fn<NB, CL, DF>(), F, m, j0, nb, ld, mode, tau, T));
+  } else {
+    TNX_CUDA(cudaLaunchKernelEx(&cfg, panel_fn<NB, CL, DF>(), F, m, j0, nb, ld, tau, T));
+  }
   TNX_LAUNCH_CHECK();
   return TNX_OK;
 }
@@ -588,7 +622,7 @@ template <int NB, int CL, bool DF>
 bool panel_fits(int64_t m) {
   const PanelKernelInfo& info = panel_info<NB, CL, DF>();
   const int64_t rpc = (m + CL - 1) / CL;
-  return info.ok && size_t(NB + 2) * panel_ld(rpc, panel_threads<DF>() / NB) * sizeof(double) <= info.max_dyn;
+  return info.ok && panel_smem<NB, CL, DF>(panel_ld<DF>(rpc, NB), false) <= info.max_dyn;
 }
 
 PanelPlan plan_panels(int64_t m, bool df) {

@@ -1,8 +1,7 @@
 // Double-FP32 cluster panel of the Householder QR, for the FP64-class precision modes.
 //
 // Same algorithm as the FP64 cluster panel in qr.cu (rows of the panel split over the CTAs of
-// one thread-block cluster, one cluster barrier per column, exchange of partial sums through
-// distributed shared memory, LAPACK dgeqr2 reflectors and the forward/columnwise dlarft T
+// one thread-block cluster, one exchange of partial sums per column through distributed shared memory, LAPACK dgeqr2 reflectors and the forward/columnwise dlarft T
 // factor), with every per-element operation in double-FP32 arithmetic on the FP32 pipe. On
 // this part the FP64 pipe issues about 2 FMA per clock per SM against 128 for FP32, and in the
 // FP64 kernel the per-column update of the remaining panel columns is bound by it.
@@ -10,8 +9,7 @@
 // Numbers are (hi, lo) float pairs (relative error ~2^-47 per operation, the standard model
 // with u ~ 2^-47, so the factorisation stays backward stable at that level). The layout and
 // schedule are chosen for short dependency chains on the FP32 pipe:
-//   * 512 threads, 8 per panel column interleaved over rows, two independent accumulators,
-//     (hi, lo) pairs interleaved in shared memory;
+//   * 16 warps, each with four panel columns, (hi, lo) pairs interleaved in shared memory;
 //     dot products accumulate compensated (hi, lo) sums renormalised once at the end;
 //   * the CL partial sums of a column are added as a fixed binary tree (every CTA derives
 //     bitwise-identical column scalars);
@@ -19,7 +17,7 @@
 //     double-FP32 (tau = 1 + |alpha| / norm needs no division; scale = sign / (norm tau) one
 //     refined reciprocal), not FP64 square root and division;
 //   * the T factor is distributed: CTA q extends rows a = q (mod CL) of T, so no CTA carries
-//     a serial triangular product on the critical path.
+//     a serial triangular product on the critical path, and two columns behind.
 // Columns are scaled by powers of two at load (largest entry of each panel column near 2^32)
 // so that squares and products of small entries stay inside the FP32 exponent range; QR of
 // A D with D a power-of-two diagonal has the same reflectors and R D, so R entries are
@@ -30,10 +28,14 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
+#include "tc_ptx.cuh"
+
+// time stamps of the phases, taken by thread TNX_PANEL_PROBE
 #ifdef TNX_PANEL_PROBE
 #define PANEL_STAMP(k) \
-  if (threadIdx.x == 0 && stamps) stamps[(q * 64 + jj) * 8 + (k)] = clock64()
+  if (threadIdx.x == TNX_PANEL_PROBE && stamps) stamps[(q * 64 + jj) * 8 + (k)] = clock64()
 #else
 #define PANEL_STAMP(k)
 #endif
@@ -42,8 +44,15 @@ namespace tnx {
 namespace qrdf {
 
 namespace cg = cooperative_groups;
+using tc::mbar_expect_tx;
+using tc::mbar_init;
+using tc::mbar_wait;
+using tc::smem_u32;
 
 constexpr int DPT = 512;  // threads per CTA
+constexpr int PUSH = 1;   // sums are stored to every rank, to be awaited at a counting barrier
+constexpr int PAD = 2;    // the row stride has PAD_ROWS zero rows below the CTA's own
+constexpr int PAD_ROWS = 64;
 
 struct df2 {
   float h, l;
@@ -149,57 +158,74 @@ __device__ __forceinline__ void cluster_wait_acquire() {
   asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory");
 }
 
-// Sum of the CL partials slot(rank)[idx] over the cluster, as a fixed binary tree
-template <int CL>
-__device__ __forceinline__ df2 tree_sum(cg::cluster_group& cluster, const df2* slot, int idx) {
-  df2 v[CL];
-#pragma unroll
-  for (int r = 0; r < CL; ++r) v[r] = cluster.map_shared_rank(slot, r)[idx];
-#pragma unroll
-  for (int s = 1; s < CL; s <<= 1)
-#pragma unroll
-    for (int r = 0; r + s < CL; r += 2 * s) v[r] = add(v[r], v[r + s]);
-  return v[0];
+// 8 bytes into the shared memory of `rank` at this CTA's address `at`, counted by that CTA's barrier `bar`
+__device__ __forceinline__ void send_async(uint32_t at, df2 x, uint32_t bar, int rank) {
+  asm volatile(
+      "{\n .reg .b32 a, b;\n mapa.shared::cluster.u32 a, %0, %4;\n mapa.shared::cluster.u32 b, %3, %4;\n"
+      " st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [a], {%1, %2}, [b];\n}\n" ::"r"(at),
+      "f"(x.h), "f"(x.l), "r"(bar), "r"(rank)
+      : "memory");
 }
 
-// Dynamic shared memory bytes of one CTA: (hi, lo) pairs of the panel [NB][ld], of v and of
-// the next column [ld] each (interleaved pairs: one 64-bit access per operand; with ld = TPC
-// (mod 16) the two column groups of a half-warp fall on disjoint banks)
-template <int NB>
-constexpr size_t panel_df_smem_bytes(int ld) {
-  return size_t(NB + 2) * size_t(ld) * sizeof(df2);
+// Dynamic shared memory bytes of one CTA: (hi, lo) pairs of the panel [NB][ld] (interleaved pairs: one
+// 64-bit access per operand) and the exchange of two steps, sums [ranks][NB] and the pivot row [NB]: with `push` every rank's
+// sums, without it this rank's, which the others read.
+template <int NB, int CL>
+constexpr size_t panel_df_smem_bytes(int ld, bool push) {
+  return (size_t(NB) * size_t(ld) + 2 * size_t(NB) * ((push ? CL : 1) + 1)) * sizeof(df2);
 }
 
 // Factor panel columns [j0, j0+nb) of the column-major m x n matrix F (ld = m), rows >= j0:
 // on exit R on/above the diagonal, the reflectors below it (unit diagonal implicit), tau, and T
 // (column-major, ld NB, upper triangular; zero outside [0, nb)) with H_j0..H_{j0+nb-1} =
 // I - V T V^T. `ld` is the CTA's shared-memory row stride (>= rows per CTA).
+//
+// What bounds a column: the chain exchange - scalars - reflector - update, of which the update's arithmetic
+// is under a third. So
+//   * a CTA stores its sums to every rank (PUSH), counted by a barrier in the receiver's shared memory: a
+//     cluster barrier, whose release and acquire took 2400 cycles a column, is not needed, and the sums
+//     are read at local latency. Panels too tall for that buffer read them from the ranks;
+//   * warp 0 takes the two sums that the scalars need straight from the exchange while others fetch the rest;
+//   * v and column jj+1 are formed in place; threads that stand for the columns meanwhile compute the
+//     factors of the update and send the next pivot row; T follows two columns behind;
+//   * in the update a warp has its columns whole: v and the next column are read once for four columns,
+//     and no warp goes through the update, the norm and the T dots one after the other. Zero rows below
+//     the CTA's own (PAD, where they fit) spare it the bounds checks, a third of its instructions.
+// The 16 panels of a 2048 x 1024 matrix: 280 us each with five block barriers and a cluster barrier a
+// column, 254 us so. 256 or 1024 threads: a quarter slower.
 template <int NB, int CL>
 __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, int64_t m, int64_t j0, int nb, int ld,
-                                                       double* __restrict__ tau_out, double* __restrict__ T_out
+                                                       int mode, double* __restrict__ tau_out,
+                                                       double* __restrict__ T_out
 #ifdef TNX_PANEL_PROBE
                                                        ,
                                                        long long* stamps
 #endif
 ) {
-  constexpr int TPC = DPT / NB;  // threads per panel column
-  constexpr int NR = NB / CL;    // rows of T held by each CTA
-  static_assert(NB % CL == 0 && TPC >= 2 && TPC <= 32 && (TPC & (TPC - 1)) == 0, "panel shape");
+  constexpr int NW = DPT / 32, CPW = NB / NW;  // warp w works on columns w, w + NW, ...: CPW of them
+  constexpr int GL = 32 / CPW;                 // lanes that end up with a column's sum
+  constexpr int NR = NB / CL;                  // rows of T held by each CTA
+  static_assert(NB % CL == 0 && NB <= 64 && CPW >= 1 && CPW * NW == NB && 2 * CL <= 32 && 4 + NR <= NW, "panel shape");
   cg::cluster_group cluster = cg::this_cluster();
   const int q = int(cluster.block_rank());
   extern __shared__ df2 pd[];
   df2* X = pd;                        // [NB][ld] panel rows of this CTA, column-major
-  df2* V = pd + NB * ld;              // reflector of the current column over this CTA's rows
-  df2* N = V + ld;                    // next column after the current reflector
-  __shared__ df2 slot[2][3][NB];      // exchange: partial dots, pivot row, partial T dots
+  const bool push = mode & PUSH, pad = mode & PAD;
+  df2* part = pd + NB * ld;           // exchange [2][push ? CL : 1][NB]: dots (right of the column) and T dots (left)
+  const int pr = push ? CL : 1;
+  df2* prow = part + 2 * pr * NB;     // [2][NB] pivot row (pushed, or the owner's)
   __shared__ unsigned long long smax[NB];
-  __shared__ df2 S[NB], P[NB], Z[NB], taus[NB], sc[4];
+  __shared__ df2 W[NB], Z[2][NB], taus[NB], sc[4];  // W: factors of the current reflector in the columns right of it
   __shared__ df2 Tr[NR][NB];          // rows q, q + CL, ... of T
   __shared__ int cexp[NB];
-  const int tid = threadIdx.x, ci = tid / TPC, h = tid % TPC, warp = tid >> 5, lane = tid & 31;
+  __shared__ __align__(8) uint64_t bars[2];  // arrival of a step's sums (push)
+  __shared__ int s_dead;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int ci = warp + NW * (lane / GL), h = lane % GL;
+  constexpr int CT = 64;  // threads CT .. CT + NB - 1 stand for the columns before and after the scalars
   const int64_t mp = m - j0;
-  const int64_t rpc = (mp + CL - 1) / CL;
-  const int64_t r0 = int64_t(q) * rpc;
+  const int rpc = int((mp + CL - 1) / CL);
+  const int r0 = q * rpc;
   const int rows = int(r0 >= mp ? 0 : (mp - r0 < rpc ? mp - r0 : rpc));
 #ifdef TNX_PANEL_PROBE
   int jj = 0;
@@ -208,15 +234,24 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
   // ---- column scales: largest |entry| of each panel column over the cluster (integer max of
   // the magnitude bits), exponent chosen so that it lands in [2^31, 2^32)
   {
+    const uint32_t bar = smem_u32(bars);
+    if (push && tid == 0) {
+      s_dead = 0;
+      mbar_init(bar, 1);
+      mbar_init(bar + 8, 1);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      mbar_expect_tx(bar, uint32_t(8 * nb * (CL + 1)));
+      mbar_expect_tx(bar + 8, uint32_t(8 * ((nb - 1) * CL + nb - 1)));
+    }
     unsigned long long mx = 0;
     if (ci < nb)
-      for (int r = h; r < rows; r += TPC) {
+      for (int r = h; r < rows; r += GL) {
         const unsigned long long b =
             static_cast<unsigned long long>(__double_as_longlong(F[(j0 + ci) * m + j0 + r0 + r])) & 0x7fffffffffffffffull;
         mx = b > mx ? b : mx;
       }
 #pragma unroll
-    for (int o = TPC / 2; o > 0; o >>= 1) {
+    for (int o = GL / 2; o > 0; o >>= 1) {
       const unsigned long long t = __shfl_xor_sync(0xffffffffu, mx, o);
       mx = t > mx ? t : mx;
     }
@@ -239,14 +274,17 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
     const int c = e / rows, r = e % rows;
     X[c * ld + r] = split_scaled(F[(j0 + c) * m + j0 + r0 + r], cexp[c]);
   }
+  if (pad)
+    for (int e = tid; e < NB * PAD_ROWS; e += DPT) X[(e / PAD_ROWS) * ld + rows + e % PAD_ROWS] = {0.f, 0.f};
   for (int e = tid; e < NR * NB; e += DPT) Tr[e / NB][e % NB] = {0.f, 0.f};
-  // column k of the row of T that warp 1 .. NR holds: T[a][k] = -tau_k sum_{a <= c < k} T[a][c] z_c, T[k][k] = tau_k
+  // column k of the rows of T held by warps 4 .. 4 + NR - 1: T[a][k] = -tau_k sum_{a <= c < k} T[a][c] z_c,
+  // T[k][k] = tau_k
   auto extend_t = [&](int k) {
-    const int row = warp - 1, a = q + CL * row;
+    const int row = warp - 4, a = q + CL * row;
     if (k < 0) return;
     if (a < k) {
       df2 t = {0.f, 0.f};
-      for (int c = a + lane; c < k; c += 32) acc(t, Tr[row][c], Z[c]);
+      for (int c = a + lane; c < k; c += 32) acc(t, Tr[row][c], Z[k & 1][c]);
       t = norm(t);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) t = add(t, shfl_xor(t, o));
@@ -255,25 +293,90 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
       Tr[row][k] = taus[k];
     }
   };
+  // a column's sum, held by the GL lanes of column ci, into the exchange
+  auto send_sum = [&](int buf, df2 sum) {
+    if (push) {
+#pragma unroll
+      for (int r = h; r < CL; r += GL)
+        send_async(smem_u32(&part[(buf * CL + q) * NB + ci]), sum, smem_u32(&bars[buf]), r);
+    } else if (h == 0) {
+      part[buf * NB + ci] = sum;
+    }
+  };
+  // column c's entry in the next pivot row
+  auto send_pivot = [&](int buf, int c, df2 piv) {
+    if (push) {
+      const uint32_t at = smem_u32(&prow[buf * NB + c]), bar = smem_u32(&bars[buf]);
+#pragma unroll 4
+      for (int r = 0; r < CL; ++r) send_async(at, piv, bar, r);
+    } else {
+      prow[buf * NB + c] = piv;
+    }
+  };
+  // before the exchange of step `step` is read
+  auto await = [&](int step) {
+    if (push && !mbar_wait(smem_u32(&bars[step & 1]), (step >> 1) & 1)) s_dead = 1;
+  };
+  auto exchange = [&] {
+    if (!push) {
+      cluster_arrive_release();
+      cluster_wait_acquire();
+    }
+  };
+  auto partial = [&](int buf, int r, int idx) {
+    return push ? part[(buf * CL + r) * NB + idx] : cluster.map_shared_rank(part, r)[buf * NB + idx];
+  };
+  // sum of the CL partials idx as a fixed binary tree
+  auto tree_sum = [&](int buf, int idx) {
+    df2 v[CL];
+#pragma unroll
+    for (int r = 0; r < CL; ++r) v[r] = partial(buf, r, idx);
+#pragma unroll
+    for (int s = 1; s < CL; s <<= 1)
+#pragma unroll
+      for (int r = 0; r + s < CL; r += 2 * s) v[r] = add(v[r], v[r + s]);
+    return v[0];
+  };
+  auto pivot = [&](int buf, int owner, int idx) {
+    return push ? prow[buf * NB + idx] : cluster.map_shared_rank(prow, owner)[buf * NB + idx];
+  };
+  auto from_lane = [&](df2 x, int l) {
+    return df2{__shfl_sync(0xffffffffu, x.h, l), __shfl_sync(0xffffffffu, x.l, l)};
+  };
+  // sums of the warp's columns over its lanes: the GL lanes of column ci get that of ci
+  auto reduce = [&](df2* a) {
+    int o = 16;
+#pragma unroll
+    for (int n = CPW; n > 1; n >>= 1, o >>= 1)
+#pragma unroll
+      for (int i = 0; i < n / 2; ++i) {
+        const bool up = lane & o;
+        const df2 give = up ? a[i] : a[i + n / 2], keep = up ? a[i + n / 2] : a[i];
+        a[i] = add(keep, shfl_xor(give, o));
+      }
+#pragma unroll
+    for (o = GL / 2; o > 0; o >>= 1) a[0] = add(a[0], shfl_xor(a[0], o));
+    return a[0];
+  };
   __syncthreads();
   // partials of pivot 0: x_0 . x_c below row 0, and pivot row 0 (rank 0)
   {
-    df2 a0 = {0.f, 0.f};
-    if (ci < nb) {
-      const int rs = r0 > 0 ? 0 : 1;
-      for (int r = rs + ((h - rs) % TPC + TPC) % TPC; r < rows; r += TPC)
-        acc(a0, X[r], X[ci * ld + r]);
-    }
-    a0 = norm(a0);
+    df2 a[CPW];
 #pragma unroll
-    for (int o = TPC / 2; o > 0; o >>= 1) a0 = add(a0, shfl_xor(a0, o));
-    if (ci < nb && h == 0) {
-      slot[0][0][ci] = a0;
-      if (r0 == 0 && rows > 0) slot[0][1][ci] = X[ci * ld];
+    for (int k = 0; k < CPW; ++k) a[k] = {0.f, 0.f};
+    for (int r = lane; r < rows; r += 32) {
+      const df2 x0 = r0 + r > 0 ? X[r] : df2{0.f, 0.f};
+#pragma unroll
+      for (int k = 0; k < CPW; ++k)
+        if (warp + NW * k < nb) acc(a[k], x0, X[(warp + NW * k) * ld + r]);
     }
+#pragma unroll
+    for (int k = 0; k < CPW; ++k) a[k] = norm(a[k]);
+    const df2 sum = reduce(a);
+    if (ci < nb) send_sum(0, sum);
+    if (r0 == 0 && rows > 0 && tid < nb) send_pivot(0, tid, X[tid * ld]);
   }
-  cluster_arrive_release();
-  cluster_wait_acquire();
+  exchange();
 
 #ifndef TNX_PANEL_PROBE
   for (int jj = 0; jj < nb; ++jj) {
@@ -282,152 +385,180 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
 #endif
     PANEL_STAMP(0);
     const int par = jj & 1;
-    const int owner = int(jj / rpc);
-    // ---- gather: S[c] (c >= jj), pivot row P[c], T dots Z[a] = v_a . v_{jj-1} (a < jj - 1)
-    if (tid < NB) {
-      const int c = tid;
-      if (c >= jj && c < nb) {
-        S[c] = tree_sum<CL>(cluster, &slot[par][0][0], c);
-        P[c] = cluster.map_shared_rank(&slot[par][1][0], owner)[c];
-      }
-    } else if (tid < 2 * NB) {
-      const int a = tid - NB;
-      if (a < jj - 1) Z[a] = tree_sum<CL>(cluster, &slot[par][2][0], a);
-    }
-    __syncthreads();
-    PANEL_STAMP(1);
-    // ---- column scalars (one thread; every CTA derives the same bits)
-    if (warp >= 1 && warp <= NR) {
-      // meanwhile: column k = jj - 1 of the held rows of T, T[a][k] = -tau_k sum_{a <= c < k} T[a][c] z_c
-      extend_t(jj - 1);
-    } else if (tid == 0) {
-      const df2 sigma = S[jj], alpha = P[jj];
+    const int owner = jj / rpc;
+    const bool has_next = jj + 1 < nb;
+    const int lj = jj - r0, ln = lj + 1;  // local rows of pivots jj and jj + 1 (outside [0, rows) on other CTAs)
+    const bool has_lj = lj >= 0 && lj < rows, has_ln = ln >= 0 && ln < rows;
+    df2 sum_c = {0.f, 0.f}, piv_c = {0.f, 0.f}, xl_j = {0.f, 0.f}, xl_c = {0.f, 0.f};
+    if (warp == 0) {
+      await(jj);
+      if (push && lane == 0 && jj + 2 <= nb)  // the buffer's next use, for step jj + 2
+        mbar_expect_tx(smem_u32(&bars[par]), uint32_t(8 * ((nb - 1) * CL + nb - 2 - jj)));
+      // ---- column scalars, from the sums of columns jj and jj + 1 (the halves of 2 CL lanes)
+      const int c = jj + (((lane / CL) & 1) && has_next ? 1 : 0);
+      df2 t = partial(par, lane % CL, c);
+      const df2 alpha = pivot(par, owner, jj), pn = pivot(par, owner, has_next ? jj + 1 : jj);
+#pragma unroll
+      for (int o = 1; o < CL; o <<= 1) t = add(t, shfl_xor(t, o));
+      const df2 sigma = from_lane(t, 0), sn = from_lane(t, CL);
       df2 tj = {0.f, 0.f}, beta = alpha, scale = {0.f, 0.f};
       if (sigma.h != 0.f || sigma.l != 0.f) {
         // nrm = sqrt(alpha^2 + sigma) through y = 1 / nrm: tau = (beta - alpha) / beta =
         // 1 + |alpha| y, scale = 1 / (alpha - beta) = sign(alpha) y / tau
-        const df2 t = add(mul(alpha, alpha), sigma);
-        const df2 y = rsqrt_df(t);
-        const df2 nrm = mul(t, y);
+        const df2 t2 = add(mul(alpha, alpha), sigma);
+        const df2 y = rsqrt_df(t2);
+        const df2 nrm = mul(t2, y);
         const bool pos = alpha.h > 0.f || (alpha.h == 0.f && alpha.l >= 0.f);
         beta = pos ? neg(nrm) : nrm;
         tj = add({1.f, 0.f}, mul(pos ? alpha : neg(alpha), y));
         const df2 sy = mul(y, rcp_df(tj));
         scale = pos ? sy : neg(sy);
       }
-      sc[0] = tj;
-      sc[1] = beta;
-      sc[2] = scale;
-      sc[3] = jj + 1 < nb ? mul(tj, add(P[jj + 1], mul(scale, S[jj + 1]))) : df2{0.f, 0.f};
-      taus[jj] = tj;
+      const df2 wn = has_next ? mul(tj, add(pn, mul(scale, sn))) : df2{0.f, 0.f};
+      if (lane == 0) {
+        sc[0] = tj;
+        sc[1] = beta;
+        sc[2] = scale;
+        sc[3] = wn;
+        taus[jj] = tj;
+      }
+    } else if (tid >= CT && tid < CT + NB) {
+      // ---- meanwhile: sum and pivot entry of column c >= jj + 2, T dots Z[a] = v_a . v_{jj-1} (a < jj - 1)
+      const int c = tid - CT;
+      await(jj);
+      if (c > jj + 1 && c < nb) {
+        sum_c = tree_sum(par, c);
+        piv_c = pivot(par, owner, c);
+      } else if (c < jj - 1) {
+        Z[par ^ 1][c] = tree_sum(par, c);
+      }
+      if (has_ln && c < nb) {  // row jj + 1 before the update
+        xl_j = X[jj * ld + ln];
+        xl_c = X[c * ld + ln];
+      }
+    } else if (warp >= 4 && warp < 4 + NR) {
+      extend_t(jj - 2);
+    }
+    __syncthreads();
+    PANEL_STAMP(1);
+    if (push && s_dead) break;
+    const df2 tj = sc[0], scale = sc[2];
+    const int rA = lj > 0 ? lj : 0;
+    df2* xj = X + jj * ld;
+    df2* xn = xj + ld;
+    // ---- phase A: v = scale x_jj below the pivot (beta at it, where v is 1), next column updated by it
+    {
+      const df2 wn = sc[3], beta = sc[1];
+      for (int r = rA + tid; r < rows; r += DPT) {
+        const bool at = r == lj;
+        const df2 v = at ? df2{1.f, 0.f} : mul(scale, xj[r]);
+        if (has_next) xn[r] = fms(xn[r], wn, v);
+        xj[r] = at ? beta : v;
+      }
+    }
+    // meanwhile: the columns' factors, and the next pivot row on its way
+    if (tid >= CT && tid < CT + NB) {
+      const int c = tid - CT;
+      if (c > jj && c < nb) {
+        const df2 w = c == jj + 1 ? sc[3] : mul(tj, add(piv_c, mul(scale, sum_c)));
+        W[c] = w;
+        if (has_lj && c > jj + 1) X[c * ld + lj] = add(X[c * ld + lj], neg(w));  // v_jj[jj] = 1
+        if (has_ln) {
+          const df2 p = fms(xl_c, w, mul(scale, xl_j));
+          if (c > jj + 1) X[c * ld + ln] = p;
+          send_pivot(par ^ 1, c, p);
+        }
+      } else if (c < jj && (has_lj || has_ln)) {  // the pivots' rows of the T dots
+        df2 z = {0.f, 0.f};
+        if (has_lj) z = X[c * ld + lj];
+        if (has_ln) acc(z, xl_c, mul(scale, xl_j));
+        W[c] = norm(z);
+      }
     }
     __syncthreads();
     PANEL_STAMP(2);
-    const df2 tj = sc[0], scale = sc[2], wn = sc[3];
-    const bool has_next = jj + 1 < nb;
-    const int64_t lj = jj - r0;  // local row of pivot jj (outside [0, rows) on other CTAs)
-    const int rA = int(lj > 0 ? lj : 0);
-    df2* xj = X + jj * ld;
-    // ---- phase A: v = scale x_jj below the pivot (1 at it), next column updated by it
-    for (int r = rA + tid; r < rows; r += DPT) {
-      const df2 v = r == lj ? df2{1.f, 0.f} : mul(scale, xj[r]);
-      V[r] = v;
-      if (has_next) N[r] = fms(xj[r + ld], wn, v);
-    }
-    __syncthreads();
-    PANEL_STAMP(3);
     // ---- phase B: update columns c > jj + 1 and the partial dots of step jj + 1 (norm of
-    // column jj + 1 below its pivot, its dots with c > jj + 1), pivot row jj + 1, T dots
-    df2 a0 = {0.f, 0.f}, a1 = {0.f, 0.f};
-    const int64_t ln = lj + 1;
-    const bool own_ln = ln >= 0 && ln < rows && int(ln % TPC) == h;
-    const int rB = int(lj + 2 > 0 ? lj + 2 : 0);
-    const int rB0 = rB + ((h - rB) % TPC + TPC) % TPC;  // first row >= rB held by this thread
-    df2(*nxt)[NB] = slot[par ^ 1];
-    if (ci < nb && ci > jj + 1) {
-      df2* xc = X + ci * ld;
-      const df2 wc = mul(tj, add(P[ci], mul(scale, S[ci])));
-      if (lj >= 0 && lj < rows && int(lj % TPC) == h) xc[lj] = add(xc[lj], neg(wc));  // v_jj[jj] = 1
-      if (own_ln) {
-        const df2 t = fms(xc[ln], wc, V[ln]);
-        xc[ln] = t;
-        nxt[1][ci] = t;
-      }
-      int r = rB0;
-      for (; r + TPC < rows; r += 2 * TPC) {
-        const df2 t0 = fms(xc[r], wc, V[r]);
-        const df2 t1 = fms(xc[r + TPC], wc, V[r + TPC]);
-        xc[r] = t0;
-        xc[r + TPC] = t1;
-        acc(a0, N[r], t0);
-        acc(a1, N[r + TPC], t1);
-      }
-      if (r < rows) {
-        const df2 t0 = fms(xc[r], wc, V[r]);
-        xc[r] = t0;
-        acc(a0, N[r], t0);
-      }
-    } else if (ci == jj + 1 && ci < nb) {
-      if (own_ln) nxt[1][ci] = N[ln];
-      int r = rB0;
-      for (; r + TPC < rows; r += 2 * TPC) {
-        acc(a0, N[r], N[r]);
-        acc(a1, N[r + TPC], N[r + TPC]);
-      }
-      if (r < rows) acc(a0, N[r], N[r]);
-    } else if (ci < jj) {
-      const df2* xc = X + ci * ld;
-      int r = rA + ((h - rA) % TPC + TPC) % TPC;
-      for (; r + TPC < rows; r += 2 * TPC) {
-        acc(a0, xc[r], V[r]);
-        acc(a1, xc[r + TPC], V[r + TPC]);
-      }
-      if (r < rows) acc(a0, xc[r], V[r]);
-    }
-    df2 a = add(norm(a0), norm(a1));
+    // column jj + 1 below its pivot, its dots with c > jj + 1), T dots. A lane has rows lane, lane + 32, ..
+    // of all the warp's columns, two at a time, from the first row below both pivots on
+    df2 a[CPW], wk[CPW];
 #pragma unroll
-    for (int o = TPC / 2; o > 0; o >>= 1) a = add(a, shfl_xor(a, o));
-    if (h == 0 && ci < nb) {
-      if (ci > jj) nxt[0][ci] = a;
-      else if (ci < jj) nxt[2][ci] = a;
+    for (int k = 0; k < CPW; ++k) {
+      a[k] = {0.f, 0.f};
+      wk[k] = W[warp + NW * k];  // not used left of the update
+    }
+    PANEL_STAMP(3);
+    auto two_rows = [&](int r, auto whole) {
+      constexpr bool all = decltype(whole)::value;  // both rows exist (or are zero rows of the padding)
+      const int r1 = r + 32;
+      const bool i0 = all || r < rows, i1 = all || r1 < rows;
+      const df2 zero = {0.f, 0.f};
+      const df2 v0 = i0 ? xj[r] : zero, v1 = i1 ? xj[r1] : zero;
+      const df2 d0 = i0 && has_next ? xn[r] : zero, d1 = i1 && has_next ? xn[r1] : zero;
+#pragma unroll
+      for (int k = 0; k < CPW; ++k) {
+        const int c = warp + NW * k;
+        df2* xc = X + c * ld;
+        if (c >= nb || c == jj) continue;
+        if (c == jj + 1) {
+          acc(a[k], d0, d0);
+          acc(a[k], d1, d1);
+          continue;
+        }
+        const df2 x0 = i0 ? xc[r] : zero, x1 = i1 ? xc[r1] : zero;
+        if (c > jj) {
+          const df2 t0 = fms(x0, wk[k], v0), t1 = fms(x1, wk[k], v1);
+          if (i0) xc[r] = t0;
+          if (i1) xc[r1] = t1;
+          acc(a[k], d0, t0);
+          acc(a[k], d1, t1);
+        } else {
+          acc(a[k], x0, v0);
+          acc(a[k], x1, v1);
+        }
+      }
+    };
+    for (int r = lj + 2 > 0 ? lj + 2 : 0; r < rows; r += 64) {
+      if (pad || r + 64 <= rows) two_rows(r + lane, std::true_type{});
+      else two_rows(r + lane, std::false_type{});
     }
     PANEL_STAMP(4);
-    cluster_arrive_release();
-    __syncthreads();
-    // ---- phase C: store v_jj (beta at the pivot) and column jj + 1
-    {
-      const df2 beta = sc[1];
-      for (int r = rA + tid; r < rows; r += DPT) {
-        xj[r] = r == lj ? beta : V[r];
-        if (has_next) xj[r + ld] = N[r];
-      }
-    }
-    // the next gather rewrites S, P and Z, which phase C still reads
-    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < CPW; ++k) a[k] = norm(a[k]);
+    df2 sum = reduce(a);
+    if (ci < jj && (has_lj || has_ln)) sum = add(sum, W[ci]);
     PANEL_STAMP(5);
-    cluster_wait_acquire();
+    if (ci < nb && ci != jj) send_sum(par ^ 1, sum);
+    PANEL_STAMP(6);
+    exchange();
+    PANEL_STAMP(7);
   }
-  // last T column k = nb - 1 from the final exchange
-  if (tid >= NB && tid < 2 * NB) {
-    const int a = tid - NB;
-    if (a < nb - 1) Z[a] = tree_sum<CL>(cluster, &slot[nb & 1][2][0], a);
+  // the last two columns of T, the last one from the final exchange
+  __syncthreads();
+  if (tid < NB) {
+    if (!s_dead) await(nb);
+    if (tid < nb - 1) Z[(nb - 1) & 1][tid] = tree_sum(nb & 1, tid);
+  } else if (warp >= 4 && warp < 4 + NR) {
+    extend_t(nb - 2);
   }
   __syncthreads();
-  if (warp >= 1 && warp <= NR) extend_t(nb - 1);
+  if (warp >= 4 && warp < 4 + NR) extend_t(nb - 1);
   __syncthreads();
   // T (column-major, ld NB): this CTA's rows; tau from rank 0
   for (int e = tid; e < NR * NB; e += DPT) {
     const int i = e / NB, b = e % NB, a = q + CL * i;
     T_out[b * NB + a] = (a <= b && b < nb) ? join_df(Tr[i][b].h, Tr[i][b].l) : 0.0;
   }
+  const bool dead = push && s_dead;  // a bounded wait ran out: NaN, so that no caller takes the result
   if (q == 0)
     for (int b = tid; b < NB; b += DPT) tau_out[b] = b < nb ? join_df(taus[b].h, taus[b].l) : 0.0;
+  const double nan = __longlong_as_double(0x7ff8000000000000LL);
   // panel back to F: R entries (panel row <= column) rescaled, reflectors as they are
   for (int e = tid; e < nb * rows; e += DPT) {
     const int c = e / rows, r = e % rows;
     const df2 v = X[c * ld + r];
-    F[(j0 + c) * m + j0 + r0 + r] = r0 + r <= c ? join_scaled(v, cexp[c]) : join_df(v.h, v.l);
+    F[(j0 + c) * m + j0 + r0 + r] = dead ? nan : (r0 + r <= c ? join_scaled(v, cexp[c]) : join_df(v.h, v.l));
   }
+  if (dead) __nanosleep(1000000);  // stores of this CTA may still be on their way to others
   // no CTA leaves while another may still read its slots
   cluster_arrive_release();
   cluster_wait_acquire();
