@@ -13,9 +13,9 @@
 // L and R are re-laid out once per site as K-major split operands (Davidson reuses them for
 // every matvec of the site); x is re-laid out per matvec.
 //
-// GEMM kernel: one 128 x BN output tile per CTA, 6 warps:
+// GEMM kernels: one 128 x 128 output tile per CTA, or 256 x BN per pair of CTAs; 6 warps:
 //   warp 0  TMA producer (cp.async.bulk.tensor, 128B swizzle, 64-wide K slabs, 4-stage ring)
-//   warp 1  TMEM allocation + single-thread tcgen05.mma issue (kind::f16, BF16 in, FP32 acc)
+//   warp 1  TMEM allocation + tcgen05.mma issue by one lane (kind::f16, BF16 in, FP32 acc)
 //   warps 2-5 epilogue: tcgen05.ld of the FP32 accumulator, staged through shared memory in
 //             64-column chunks, stored as FP32 or FP64 row segments
 // Every mbarrier wait is bounded (~2 s of clock); on expiry the kernel raises a flag in
@@ -42,7 +42,62 @@ constexpr int BK = 64;  // 64 bf16 = 128 bytes = one swizzle atom row
 constexpr int STAGES = 4;
 constexpr int GEMM_THREADS = 192;
 
-// ---------------------------------------------------------------- GEMM kernel
+// ---------------------------------------------------------------- GEMM kernels
+// Accumulator of the tile at (m0, n0) in tensor memory -> out, by warps 2 .. 5 through shared memory at stg, the
+// 32 rows of a warp 64 columns at a time: in pairs of columns, whose 66-word (FP64: 132-word) row stride
+// is free of conflicts, and out again as row segments of 64 columns by the same warp
+constexpr int CW = 64, LD_OUT = CW + 2;                      // columns of a chunk and their row stride
+constexpr uint32_t STAGING_BYTES = BM * LD_OUT * sizeof(double);  // of the four warps' chunks, in the stage ring
+template <int BN, typename T>
+__device__ __forceinline__ void store_tile_as(uint32_t tmem, uint8_t* stg, int m0, int n0, int M, int N,
+                                              T* __restrict__ out, int64_t ldc) {
+  struct alignas(2 * sizeof(T)) T2 {
+    T a, b;
+  };
+  constexpr int LD = LD_OUT;
+  const int quad = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;  // TMEM lanes 32*quad .. 32*quad+31
+  T* rows = reinterpret_cast<T*>(stg) + quad * 32 * LD;
+  auto val = [](uint32_t x) {
+    if constexpr (sizeof(T) == 8) return float_to_double(__uint_as_float(x));
+    else return __uint_as_float(x);
+  };
+  const int left = M - m0 - quad * 32;  // rows of this warp inside the matrix
+  const bool pairs = ldc % 2 == 0 && reinterpret_cast<uintptr_t>(out) % (2 * sizeof(T)) == 0;
+#pragma unroll 1
+  for (int c0 = 0; c0 < BN; c0 += CW) {
+    uint32_t r[2][32];
+    tmem_ld32_async(tmem + (uint32_t(quad * 32) << 16) + uint32_t(c0), r[0]);
+    tmem_ld32_async(tmem + (uint32_t(quad * 32) << 16) + uint32_t(c0 + 32), r[1]);
+    tmem_ld_wait();
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int j = 0; j < 32; j += 2)
+        *reinterpret_cast<T2*>(rows + lane * LD + h * 32 + j) = T2{val(r[h][j]), val(r[h][j + 1])};
+    __syncwarp();
+    const int c = n0 + c0 + 2 * lane;
+    T* dst = out + int64_t(m0 + quad * 32) * ldc + c;
+    const T* src = rows + 2 * lane;
+    if (pairs && c + 1 < N) {
+#pragma unroll 8
+      for (int i = 0; i < 32; ++i)
+        if (i < left) *reinterpret_cast<T2*>(dst + i * ldc) = *reinterpret_cast<const T2*>(src + i * LD);
+    } else {
+      for (int i = 0; i < 32 && i < left; ++i) {
+        if (c < N) dst[i * ldc] = src[i * LD];
+        if (c + 1 < N) dst[i * ldc + 1] = src[i * LD + 1];
+      }
+    }
+    __syncwarp();  // the chunk is out before the next one is staged
+  }
+}
+template <int BN>
+__device__ __forceinline__ void store_tile(uint32_t tmem, uint8_t* stg, int m0, int n0, int M, int N, void* out,
+                                           int64_t ldc, int out_fp64) {
+  if (out_fp64) store_tile_as<BN>(tmem, stg, m0, n0, M, N, static_cast<double*>(out), ldc);
+  else store_tile_as<BN>(tmem, stg, m0, n0, M, N, static_cast<float*>(out), ldc);
+}
+
 // C[M, N] = sum_k A[m, k] B[n, k] over the three split products; A*, B* are K-major BF16
 // with row pitch Kp (a multiple of 64). out: FP32 or FP64, row-major with leading dim ldc.
 template <int BN>
@@ -55,12 +110,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   constexpr uint32_t B_BYTES = BN * BK * 2;
   constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr uint32_t TMEM_COLS = BN < 32 ? 32 : BN;
+  static_assert(STAGES * STAGE_BYTES >= STAGING_BYTES, "the epilogue stages a chunk in the ring");
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], accum_bar;
   __shared__ uint32_t tmem_base_sh;
-  __shared__ int abort_sh, epi_fail_sh;
+  __shared__ int abort_sh;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   const int kblocks = Kp / BK;
@@ -73,7 +129,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     }
     mbar_init(smem_u32(&accum_bar), 1);
     abort_sh = 0;
-    epi_fail_sh = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -84,7 +139,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
-  const uint32_t tmem = tmem_base_sh;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base_sh, 0);
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer
@@ -114,77 +169,48 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         mbar_wait(smem_u32(&full_bar[it % STAGES]), (it / STAGES) & 1);
     }
   } else if (warp == 1) {
-    // ------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = instr_desc_bf16(BM, BN);
-      bool ok = true;
-      for (int it = 0; it < total; ++it) {
-        const int s = it % STAGES;
-        const uint32_t ph = (it / STAGES) & 1;
-        if (!mbar_wait(smem_u32(&full_bar[s]), ph) || *((volatile int*)&abort_sh)) {
-          atomicExch(err_flag, 1);
-          abort_sh = 1;
-          ok = false;
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint32_t sa = base + s * STAGE_BYTES, sb = sa + A_BYTES;
-#pragma unroll
-        for (int kk = 0; kk < BK / 16; ++kk) {
-          const uint64_t ad = smem_desc_sw128(sa + kk * 32);
-          const uint64_t bd = smem_desc_sw128(sb + kk * 32);
-          mma_bf16(tmem, ad, bd, idesc, (it > 0 || kk > 0) ? 1u : 0u);
-        }
-        mma_commit(smem_u32(&empty_bar[s]));
+    // ------------------------------------------------ MMA issuer: the whole warp runs the loop, so that descriptors
+    // and addresses stay in uniform registers; one lane issues (by one lane's loop a slab took 600 clocks to
+    // issue, more than its products take)
+    constexpr uint32_t idesc = instr_desc_bf16(BM, BN);
+    const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
+    const uint64_t desc0 = smem_desc_sw128(base);
+    const bool one = elect_one();
+    bool ok = true;
+    int s = 0;
+    uint32_t ph = 0;
+    for (int it = 0; it < total; ++it) {
+      if (!mbar_wait(full0 + 8 * s, ph)) {
+        if (one) atomicExch(err_flag, 1);
+        abort_sh = 1;
+        ok = false;
+        break;
       }
-      if (ok) mma_commit(smem_u32(&accum_bar));
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      // addresses sit in the descriptors in units of 16 bytes
+      const uint64_t ad = desc0 + uint32_t(s) * (STAGE_BYTES >> 4), bd = ad + (A_BYTES >> 4);
+      if (one) {
+#pragma unroll
+        for (int kk = 0; kk < BK / 16; ++kk)
+          mma_bf16(tmem, ad + 2 * kk, bd + 2 * kk, idesc, (it > 0 || kk > 0) ? 1u : 0u);
+        mma_commit(empty0 + 8 * s);
+      }
+      if (++s == STAGES) {
+        s = 0;
+        ph ^= 1;
+      }
     }
+    if (ok && one) mma_commit(smem_u32(&accum_bar));
   } else {
     // ------------------------------------------------ epilogue (warps 2..5)
     // The accumulator goes out in 64-column chunks through shared memory (the stage ring is free
     // once the accumulator is complete): a thread holds one row of the tile in TMEM, and storing
     // from there would write 32 rows per warp instruction; from shared memory every warp store
     // covers 32 consecutive columns of one row.
-    const int quad = warp & 3;  // TMEM lanes 32*quad .. 32*quad+31
-    const int lr = quad * 32 + lane, et = threadIdx.x - 64;
     const bool ok = mbar_wait(smem_u32(&accum_bar), 0);
-    if (!ok) {
-      if (lane == 0) atomicExch(err_flag, 1);
-      epi_fail_sh = 1;
-    }
+    if (!ok && lane == 0) atomicExch(err_flag, 1);
     asm volatile("tcgen05.fence::after_thread_sync;");
-    constexpr int CW = 64;  // columns per chunk; the FP64 chunk [BM][CW + 1] is 66.5 KB
-    uint8_t* stg = smem_raw + (base - smem_u32(smem_raw));
-    float* sf = reinterpret_cast<float*>(stg);
-    double* sd = reinterpret_cast<double*>(stg);
-#pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += CW) {
-      if (ok) {
-        uint32_t r[2][32];
-        tmem_ld32_async(tmem + (uint32_t(quad * 32) << 16) + uint32_t(c0), r[0]);
-        tmem_ld32_async(tmem + (uint32_t(quad * 32) << 16) + uint32_t(c0 + 32), r[1]);
-        tmem_ld_wait();
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            if (out_fp64) sd[lr * (CW + 1) + h * 32 + j] = float_to_double(__uint_as_float(r[h][j]));
-            else sf[lr * (CW + 1) + h * 32 + j] = __uint_as_float(r[h][j]);
-          }
-      }
-      asm volatile("bar.sync 1, 128;" ::: "memory");  // the four epilogue warps
-      if (!epi_fail_sh) {
-        for (int idx = et; idx < BM * CW; idx += 128) {
-          const int rr = idx / CW, cc = idx % CW;
-          if (m0 + rr < M && n0 + c0 + cc < N) {
-            const int64_t o = int64_t(m0 + rr) * ldc + n0 + c0 + cc;
-            if (out_fp64) static_cast<double*>(out)[o] = sd[rr * (CW + 1) + cc];
-            else static_cast<float*>(out)[o] = sf[rr * (CW + 1) + cc];
-          }
-        }
-      }
-      asm volatile("bar.sync 1, 128;" ::: "memory");  // the chunk is out before the next one is staged
-    }
+    if (ok) store_tile<BN>(tmem, smem_raw + (base - smem_u32(smem_raw)), m0, n0, M, N, out, ldc, out_fp64);
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
@@ -192,6 +218,156 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   if (warp == 1) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
   }
+}
+
+// The same product with 256 x BN tiles by pairs of CTAs (cta_group::2): each holds its 128 rows of A and
+// half of the tile's rows of B, so an SM takes in 128 + BN / 2 rows a K slab for 128 x BN products where
+// the kernel above takes 128 + BN, at about 64 bytes a clock. Every output sums the same products in the
+// same order as above.
+//
+// ST stages of SL slabs of 64; MINB CTAs on an SM. What bounded the kernel was neither: waiting for a stage,
+// issuing its four products and the commit took the issuing lane 600 clocks a slab, whose products take 256
+// (BN = 128) to 512. Run by the whole warp with uniform operands, and with two slabs a stage, it is
+// below that; two CTAs on an SM hide it too, and one's stores run beside the other's products where tiles
+// outnumber the SMs. chi = 1024: 5120 x 2048 x 1024 89 us by single CTAs with 128 x 256 tiles, 54 us
+// with <192, 3, 1, 2> here; 2048 x 1024 x 5120 85 us with 128 x 128 tiles, 52 us with <128, 4, 2, 1>. The
+// epilogue's row segments in place of element by element made 8 us of each.
+template <int BN, int ST, int SL, int MINB>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, MINB)
+    bf16x3_pair_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant__ CUtensorMap ta_lo,
+                       const __grid_constant__ CUtensorMap tb_hi, const __grid_constant__ CUtensorMap tb_lo,
+                       int M, int N, int Kp, int tiles_n, void* __restrict__ out, int64_t ldc, int out_fp64,
+                       int* __restrict__ err_flag) {
+  constexpr uint32_t A_BYTES = BM * BK * 2;
+  constexpr uint32_t B_BYTES = BN / 2 * BK * 2;
+  constexpr uint32_t SLAB_BYTES = A_BYTES + B_BYTES, STAGE_BYTES = SL * SLAB_BYTES;
+  constexpr uint32_t TMEM_COLS = BN <= 128 ? 128 : 256;
+  static_assert(ST * STAGE_BYTES >= STAGING_BYTES, "the epilogue stages a chunk in the ring");
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t full_bar[ST], empty_bar[ST], accum_bar;  // full: rank 0's, for both
+  __shared__ uint32_t tmem_base_sh;
+  __shared__ int abort_sh;
+
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank();
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const int tile = blockIdx.x >> 1;
+  const int m0 = (tile / tiles_n * 2 + int(rank)) * BM, n0 = tile % tiles_n * BN;
+  const int kblocks = Kp / BK;
+  const int ksteps = (kblocks + SL - 1) / SL, total = 3 * ksteps;  // stages of SL slabs; the last of a product may be short
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < ST; ++s) {
+      mbar_init(smem_u32(&full_bar[s]), 1);
+      mbar_init(smem_u32(&empty_bar[s]), 1);
+    }
+    mbar_init(smem_u32(&accum_bar), 1);
+    abort_sh = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_sh)),
+                 "r"(TMEM_COLS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  cluster_sync_all();  // both CTAs' barriers and tensor memory are there
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base_sh, 0);
+
+  if (warp == 0) {
+    // ------------------------------------------------ TMA producer of this CTA's rows
+    if (lane == 0) {
+      int issued = 0, s = 0;
+      uint32_t ph = 0;
+      const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar), fb0 = rank_addr(full0, 0);
+      const int nb0 = n0 + int(rank) * (BN / 2);
+      bool ok = true;
+      for (int seg = 0; seg < 3 && ok; ++seg) {
+        const CUtensorMap* ma = seg == 2 ? &ta_lo : &ta_hi;
+        const CUtensorMap* mb = seg == 1 ? &tb_lo : &tb_hi;
+        for (int kb = 0; kb < kblocks; kb += SL) {
+          if ((issued >= ST && !mbar_wait(empty0 + 8 * s, ph ^ 1)) || *((volatile int*)&abort_sh)) {
+            if (!*((volatile int*)&abort_sh)) atomicExch(err_flag, 1);
+            abort_sh = 1;
+            ok = false;
+            break;
+          }
+          const uint32_t sa = base + s * STAGE_BYTES;
+          const int slabs = kblocks - kb < SL ? kblocks - kb : SL;
+          if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * SLAB_BYTES * slabs);
+#pragma unroll
+          for (int i = 0; i < SL; ++i)
+            if (i < slabs) {
+              tma_load_2d_pair(sa + i * SLAB_BYTES, ma, fb0 + 8 * s, (kb + i) * BK, m0);
+              tma_load_2d_pair(sa + i * SLAB_BYTES + A_BYTES, mb, fb0 + 8 * s, (kb + i) * BK, nb0);
+            }
+          ++issued;
+          if (++s == ST) {
+            s = 0;
+            ph ^= 1;
+          }
+        }
+      }
+      // drain: wait (bounded) until every copy that rank 0 counts has landed before the CTAs can exit
+      if (rank == 0)
+        for (int it = issued - ST < 0 ? 0 : issued - ST; it < issued; ++it)
+          mbar_wait(smem_u32(&full_bar[it % ST]), (it / ST) & 1);
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------ MMA issuer (rank 0). The whole warp runs the loop, so that
+    // descriptors and addresses stay in uniform registers; one lane issues
+    if (rank == 0) {
+      constexpr uint32_t idesc = instr_desc_bf16(2 * BM, BN);
+      const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
+      const uint64_t desc0 = smem_desc_sw128(base);
+      const bool one = elect_one();
+      bool ok = true;
+      int s = 0, left = kblocks;
+      uint32_t ph = 0;
+      for (int it = 0; it < total; ++it) {
+        if (!mbar_wait(full0 + 8 * s, ph)) {
+          if (one) atomicExch(err_flag, 1);
+          abort_sh = 1;
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        // addresses sit in the descriptors in units of 16 bytes
+        const uint64_t ad = desc0 + uint32_t(s) * (STAGE_BYTES >> 4), bd = ad + (A_BYTES >> 4);
+        if (one) {
+#pragma unroll
+          for (int i = 0; i < SL; ++i)
+            if (i < left)
+#pragma unroll
+              for (int kk = 0; kk < BK / 16; ++kk)
+                mma_bf16_pair(tmem, ad + i * (SLAB_BYTES >> 4) + 2 * kk, bd + i * (SLAB_BYTES >> 4) + 2 * kk, idesc,
+                              (it > 0 || i > 0 || kk > 0) ? 1u : 0u);
+          mma_commit_pair(empty0 + 8 * s);
+        }
+        left = left > SL ? left - SL : kblocks;
+        if (++s == ST) {
+          s = 0;
+          ph ^= 1;
+        }
+      }
+      if (ok && one) mma_commit_pair(smem_u32(&accum_bar));
+    }
+  } else {
+    // ------------------------------------------------ epilogue of this CTA's rows (warps 2..5)
+    const bool ok = mbar_wait(smem_u32(&accum_bar), 0);
+    if (!ok && lane == 0) atomicExch(err_flag, 1);
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    if (ok) store_tile<BN>(tmem, smem_raw + (base - smem_u32(smem_raw)), m0, n0, M, N, out, ldc, out_fp64);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  cluster_sync_all();  // nothing reads the other CTA's shared or tensor memory any more
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  if (warp == 1)
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+  cluster_sync_all();
 }
 
 // ---------------------------------------------------------------- operand preparation
@@ -355,6 +531,62 @@ int launch_gemm(const __nv_bfloat16* a_hi, const __nv_bfloat16* a_lo, const __nv
   return TNX_OK;
 }
 
+template <int BN, int ST, int SL, int MINB>
+int launch_pair(const __nv_bfloat16* a_hi, const __nv_bfloat16* a_lo, const __nv_bfloat16* b_hi,
+                const __nv_bfloat16* b_lo, int M, int N, int Kp, void* out, int64_t ldc, bool out_fp64, int* err_flag,
+                cudaStream_t st, int64_t k_real) {
+  CUtensorMap mah, mal, mbh, mbl;
+  TNX_TRY(make_map(&mah, a_hi, M, Kp, BM));
+  TNX_TRY(make_map(&mal, a_lo, M, Kp, BM));
+  TNX_TRY(make_map(&mbh, b_hi, N, Kp, BN / 2));
+  TNX_TRY(make_map(&mbl, b_lo, N, Kp, BN / 2));
+  const size_t smem = size_t(ST) * SL * (BM + BN / 2) * BK * 2 + 1024;
+  static std::atomic<bool> attr_set{false};  // idempotent setup; threads may race to it
+  if (!attr_set.load()) {
+    TNX_CUDA(cudaFuncSetAttribute(bf16x3_pair_kernel<BN, ST, SL, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  int(smem)));
+    attr_set.store(true);
+  }
+  const int tn = (N + BN - 1) / BN, tm = (M + 2 * BM - 1) / (2 * BM);
+  profile_mark(KF_TC_GEMM, st, true);
+  bf16x3_pair_kernel<BN, ST, SL, MINB><<<2 * tn * tm, GEMM_THREADS, smem, st>>>(mah, mal, mbh, mbl, M, N, Kp, tn, out, ldc,
+                                                                            out_fp64 ? 1 : 0, err_flag);
+  profile_mark(KF_TC_GEMM, st, false);
+  profile_work(KF_TC_GEMM, 2.0 * M * N * double(k_real),
+               2.0 * 2.0 * (double(M) + N) * Kp * 3 + double(M) * N * (out_fp64 ? 8 : 4));
+  TNX_LAUNCH_CHECK();
+  return TNX_OK;
+}
+
+// C = A B^T in the split products by variant v: 0 one CTA a tile of 128 x 128, 1 - 3 pairs with 256 x 128, 192, 256
+int split_gemm(int v, const __nv_bfloat16* a_hi, const __nv_bfloat16* a_lo, const __nv_bfloat16* b_hi,
+               const __nv_bfloat16* b_lo, int64_t M, int64_t N, int64_t Kp, void* out, int64_t ldc, bool out_fp64,
+               int* err_flag, cudaStream_t st, int64_t k_real) {
+  const int m = int(M), n = int(N), k = int(Kp);
+  switch (v) {
+    case 0: return launch_gemm<128>(a_hi, a_lo, b_hi, b_lo, m, n, k, out, ldc, out_fp64, err_flag, st, k_real);
+    case 1: return launch_pair<128, 4, 2, 1>(a_hi, a_lo, b_hi, b_lo, m, n, k, out, ldc, out_fp64, err_flag, st, k_real);
+    case 2: return launch_pair<192, 3, 1, 2>(a_hi, a_lo, b_hi, b_lo, m, n, k, out, ldc, out_fp64, err_flag, st, k_real);
+    default: return launch_pair<256, 3, 2, 1>(a_hi, a_lo, b_hi, b_lo, m, n, k, out, ldc, out_fp64, err_flag, st, k_real);
+  }
+}
+constexpr int SPLIT_VARIANTS = 4;
+// Variant where no timing is possible or wanted: rows taken in by the busiest SM, (tiles a SM or pair) x
+// (rows a slab)
+int split_rule(int64_t M, int64_t N) {
+  const int64_t m1 = (M + 127) / 128, m2 = (M + 255) / 256;
+  const int64_t sms = 152;
+  auto waves = [](int64_t tiles, int64_t slots) { return (tiles + slots - 1) / slots; };
+  const int64_t cost[SPLIT_VARIANTS] = {waves(m1 * ((N + 127) / 128), sms) * 256,
+                                        waves(m2 * ((N + 127) / 128), sms / 2) * 192,
+                                        waves(m2 * ((N + 191) / 192), sms / 2) * 224,
+                                        waves(m2 * ((N + 255) / 256), sms / 2) * 256};
+  int best = 0;
+  for (int v = 1; v < SPLIT_VARIANTS; ++v)
+    if (cost[v] < cost[best]) best = v;
+  return best;
+}
+
 inline int64_t pad64(int64_t k) { return (k + 63) / 64 * 64; }
 
 struct MixedLayout {
@@ -483,16 +715,12 @@ int mixed_apply_t(const double* W, const T* x, T* y, int64_t chi_l, int64_t d, i
   // B1[(s c)][a] = x[a][(s c)]
   split_transpose_kernel<T><<<tgrid(m.K1p, m.N1), tb, 0, st>>>(x, chi_l, m.N1, m.b1h, m.b1l, m.K1p);
   TNX_LAUNCH_CHECK();
-  // step 1: T1 (FP32) = A1 . B1^T; 128 x 256 or 128 x 128 tiles, autotuned per shape
+  // step 1: T1 (FP32) = A1 . B1^T; tiles autotuned per shape
   {
     auto run = [&](int v) -> int {
-      if (v == 0)
-        return launch_gemm<256>(m.a1h, m.a1l, m.b1h, m.b1l, int(m.M1), int(m.N1), int(m.K1p), m.T1, m.N1, false,
-                                m.flag, st, chi_l);
-      return launch_gemm<128>(m.a1h, m.a1l, m.b1h, m.b1l, int(m.M1), int(m.N1), int(m.K1p), m.T1, m.N1, false,
-                              m.flag, st, chi_l);
+      return split_gemm(v, m.a1h, m.a1l, m.b1h, m.b1l, m.M1, m.N1, m.K1p, m.T1, m.N1, false, m.flag, st, chi_l);
     };
-    TNX_TRY(autotuned(TuneKey{3, m.M1, m.N1, m.K1p, 0, 0}, 2, m.N1 >= 256 ? 0 : 1, m.N1 >= 256, st, run));
+    TNX_TRY(autotuned(TuneKey{3, m.M1, m.N1, m.K1p, 0, 0}, SPLIT_VARIANTS, split_rule(m.M1, m.N1), m.N1 >= 256, st, run));
   }
   // step 2: MPO contraction into the split A3 operand, [(a',s')][(c,v)] with row pitch K3p (wcontract.cuh)
   TNX_TRY((wc::launch_left<float>(m.T1, 0, W, 0, wc::OutSplit{m.a3h, m.a3l}, 0, chi_l, d, chi_r, dl, dr, m.K3p, 1,
@@ -500,13 +728,11 @@ int mixed_apply_t(const double* W, const T* x, T* y, int64_t chi_l, int64_t d, i
   // step 3: y = A3 . B3^T (FP32 accumulators written as T); tiles autotuned per shape
   {
     auto run = [&](int v) -> int {
-      if (v == 0)
-        return launch_gemm<256>(m.a3h, m.a3l, m.b3h, m.b3l, int(m.M3), int(m.N3), int(m.K3p), y, m.N3,
-                                sizeof(T) == 8, m.flag, st, chi_r * dr);
-      return launch_gemm<128>(m.a3h, m.a3l, m.b3h, m.b3l, int(m.M3), int(m.N3), int(m.K3p), y, m.N3,
-                              sizeof(T) == 8, m.flag, st, chi_r * dr);
+      return split_gemm(v, m.a3h, m.a3l, m.b3h, m.b3l, m.M3, m.N3, m.K3p, y, m.N3, sizeof(T) == 8, m.flag, st,
+                        chi_r * dr);
     };
-    TNX_TRY(autotuned(TuneKey{3, m.M3, m.N3, m.K3p, int64_t(sizeof(T)), 0}, 2, 1, m.N3 >= 256, st, run));
+    TNX_TRY(autotuned(TuneKey{3, m.M3, m.N3, m.K3p, int64_t(sizeof(T)), 0}, SPLIT_VARIANTS, split_rule(m.M3, m.N3),
+                      m.N3 >= 256, st, run));
   }
   return TNX_OK;
 }
@@ -580,10 +806,7 @@ int tnx_gemm_bf16x3(int64_t m, int64_t n, int64_t k, const double* A, const doub
   TNX_LAUNCH_CHECK();
   split_pad_kernel<<<152 * 4, 256, 0, st>>>(B, n, k, bh, bl, kp);
   TNX_LAUNCH_CHECK();
-  if (n >= 256)
-    TNX_TRY(launch_gemm<256>(ah, al, bh, bl, int(m), int(n), int(kp), C, n, true, flag, st, k));
-  else
-    TNX_TRY(launch_gemm<128>(ah, al, bh, bl, int(m), int(n), int(kp), C, n, true, flag, st, k));
+  TNX_TRY(split_gemm(split_rule(m, n), ah, al, bh, bl, m, n, kp, C, n, true, flag, st, k));
   int host_flag = 0;
   TNX_CUDA(cudaMemcpyAsync(&host_flag, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
   TNX_CUDA(cudaStreamSynchronize(st));
