@@ -19,9 +19,9 @@
 // double-FP32 summation (~2^-46 of the running sum): FP64-class where rows and columns do not
 // span many decades; at the tensor cores' rate divided by 36.
 //
-// Kernel: one 128 x 64 output tile per CTA, 10 warps: warp 0 TMA producer (all 2 S slice tiles of
+// Kernel: 128 x 64 output tiles, 10 warps: warp 0 TMA producer (all 2 S slice tiles of
 // a 32-deep K block per stage, 2 stages of 96 KB, 64-byte swizzle), warp 1 TMEM allocation (512
-// columns: eight 64-column group accumulators) and single-thread tcgen05.mma issue of the 36
+// columns: eight 64-column group accumulators) and tcgen05.mma issue of the 36
 // slice products per K block as 12 MMAs per 16-deep step (slice q of A against the B slices
 // 0..7-q at once, N up to 256), warps 2-9 epilogue (two per TMEM lane quarter, 32 columns
 // each). All
@@ -45,6 +45,7 @@ constexpr int OZ_S = 8;                         // slices per operand
 constexpr int OZ_BM = 128, OZ_BN = 64, OZ_BK = 32;  // BK = 32 bf16 = one 64-byte swizzle row
 constexpr int OZ_KC = 480;                      // K values per exact accumulation chunk
 constexpr int OZ_STAGES = 2;                    // a stage holds all 2 S slice tiles of one K block
+constexpr int OZ_PARTS = 3;                      // parts in which a stage is freed
 constexpr int OZ_EPI_WARPS = 8;                 // two per TMEM lane quarter, 32 columns each
 constexpr int OZ_THREADS = 64 + 32 * OZ_EPI_WARPS;
 constexpr uint32_t OZ_TMEM_COLS = 512;
@@ -212,45 +213,78 @@ __global__ void __launch_bounds__(256) oz_slice_kernel(const double* __restrict_
 // 16-deep step: A slice q against B slices 0..7-q in MMAs of N <= 256 (2, 2, 2, 2, 1, 1, 1, 1 for
 // q = 0..7), 12 MMAs instead of 36, each A slice read from shared memory once or twice instead of
 // 8 - q times.
-// Batch and split-K: blockIdx.z = bz * nsplit + sz. Chain bz reads its slice planes at plane rows
-// (bz * S + q) * Mp (A) / (bz * S + q) * Np (B) and its exponents at ea + bz Mp / eb + bz Np;
+// Batch and split-K: a work item is a tile of plane z = bz * nsplit + sz. Chain bz reads its slice planes at plane
+// rows (bz * S + q) * Mp (A) / (bz * S + q) * Np (B) and its exponents at ea + bz Mp / eb + bz Np;
 // split sz covers K blocks [sz kbs, (sz + 1) kbs). With nsplit == 1 the CTA writes
 // C + bz sC = alpha P + beta C; otherwise the unscaled partial P to part[(sz * batch + bz) M N]
 // (row-major, ld N), which oz_split_reduce_kernel sums in split order.
+//
+// One CTA an SM takes items until there are none: the producer draws them from a counter (a fixed share
+// would leave the work of SMs that a concurrent kernel holds to the end) and hands them on through a
+// queue of two. So the ring fills for the next tile, and its products run, while the epilogue warps
+// are still at the FP64 sums and stores of this one; only the drain of the accumulators, which take all of
+// tensor memory, stops the products (a tenth of the time at K = 1024). The whole MMA warp runs the issue loop, with
+// descriptors in uniform registers. The products go by slices of A, so that a stage is freed in three parts
+// (A slices 0-1, 2-3, 4-7 with the B slices that no later one meets) and the next block's copies start while it is
+// still in use: 96 KB at about 64 bytes a clock and their latency take longer than the 2304 clocks of a block's
+// products. 5120 x 2048 x 1024: 567 us with a launch of one CTA a tile and a one-lane issue loop, 485 us
+// persistent, 458 us with stages freed in parts.
 __global__ void __launch_bounds__(OZ_THREADS, 1)
     oz_gemm_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, int M, int N,
                    int Kp, int Mp, int Np, const int* __restrict__ ea, const int* __restrict__ eb, double alpha,
-                   double beta, double* __restrict__ C, int64_t ldc, int* __restrict__ err_flag, int batch,
-                   int nsplit, int kbs, int64_t sC, double* __restrict__ part, const int* __restrict__ mask) {
+                   double beta, double* __restrict__ C, int64_t ldc, int* __restrict__ err_flag,
+                   int* __restrict__ counter, int batch, int nsplit, int kbs, int64_t sC, double* __restrict__ part,
+                   const int* __restrict__ mask) {
   constexpr uint32_t A_TILE = OZ_BM * OZ_BK * 2, B_TILE = OZ_BN * OZ_BK * 2;
   constexpr uint32_t STAGE_BYTES = OZ_S * (A_TILE + B_TILE);
   extern __shared__ uint8_t smem_raw[];
-  __shared__ uint64_t full_bar[OZ_STAGES], empty_bar[OZ_STAGES], chunk_full, chunk_empty;
+  __shared__ uint64_t full_bar[OZ_STAGES], empty_bar[OZ_STAGES][OZ_PARTS], chunk_full, chunk_empty, q_full[2], q_empty[2];
   __shared__ uint32_t tmem_base_sh;
-  __shared__ int abort_sh, epi_fail_sh;
-  const int bz = int(blockIdx.z) / nsplit, sz = int(blockIdx.z) % nsplit;
-  if (mask && !mask[bz]) return;  // uniform over the CTA, before any barrier or TMEM allocation
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __shared__ int abort_sh, queue[2];
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const int m0 = blockIdx.y * OZ_BM, n0 = blockIdx.x * OZ_BN;
+  const int tiles_n = Np / OZ_BN, tiles = tiles_n * (Mp / OZ_BM), items = tiles * batch * nsplit;
   const int kb_all = Kp / OZ_BK;
-  const int kb0 = sz * kbs, kb1 = min(kb_all, kb0 + kbs);
-  const int kblocks = kb1 > kb0 ? kb1 - kb0 : 0;
   const int kb_per_chunk = OZ_KC / OZ_BK;
-  const int nchunks = (kblocks + kb_per_chunk - 1) / kb_per_chunk;
-  const int a_row0 = bz * OZ_S * Mp, b_row0 = bz * OZ_S * Np;
-  ea += int64_t(bz) * Mp;
-  eb += int64_t(bz) * Np;
+  struct Item {
+    int bz, sz, m0, n0, kb0, kblocks;
+  };
+  auto item = [&](int t) {
+    Item w;
+    const int z = t / tiles, r = t - z * tiles;
+    w.bz = z / nsplit;
+    w.sz = z - w.bz * nsplit;
+    w.m0 = r / tiles_n * OZ_BM;
+    w.n0 = r % tiles_n * OZ_BN;
+    w.kb0 = w.sz * kbs;
+    const int kb1 = min(kb_all, w.kb0 + kbs);
+    w.kblocks = kb1 > w.kb0 ? kb1 - w.kb0 : 0;
+    return w;
+  };
+  // w-th item of this CTA for a warp that consumes the queue; -1: no more (or a wait that ran out)
+  auto next_item = [&](int w) {
+    if (!mbar_wait(smem_u32(&q_full[w & 1]), (w >> 1) & 1)) {
+      if (lane == 0) atomicExch(err_flag, 1);
+      abort_sh = 1;
+      return -1;
+    }
+    const int t = __shfl_sync(0xffffffffu, queue[w & 1], 0);
+    if (lane == 0) mbar_arrive(smem_u32(&q_empty[w & 1]));
+    return t;
+  };
 
   if (threadIdx.x == 0) {
     for (int st = 0; st < OZ_STAGES; ++st) {
       mbar_init(smem_u32(&full_bar[st]), 1);
-      mbar_init(smem_u32(&empty_bar[st]), 1);
+      for (int i = 0; i < OZ_PARTS; ++i) mbar_init(smem_u32(&empty_bar[st][i]), 1);
     }
     mbar_init(smem_u32(&chunk_full), 1);
     mbar_init(smem_u32(&chunk_empty), OZ_EPI_WARPS);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&q_full[i]), 1);
+      mbar_init(smem_u32(&q_empty[i]), 1 + OZ_EPI_WARPS);
+    }
     abort_sh = 0;
-    epi_fail_sh = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -261,79 +295,110 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
-  const uint32_t tmem = tmem_base_sh;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base_sh, 0);
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer: one K block per stage
     if (lane == 0) {
-      int issued = 0;
-      for (int kb = 0; kb < kblocks; ++kb) {
-        const int st = kb % OZ_STAGES;
-        const uint32_t ph = (kb / OZ_STAGES) & 1;
-        if (kb >= OZ_STAGES && !mbar_wait(smem_u32(&empty_bar[st]), ph ^ 1)) {
+      int issued = 0, t = blockIdx.x;
+      bool ok = true;
+      for (int w = 0; ok; ++w) {
+        while (t < items && mask && !mask[t / tiles / nsplit]) t = int(gridDim.x) + atomicAdd(counter, 1);
+        if (w >= 2 && !mbar_wait(smem_u32(&q_empty[w & 1]), ((w >> 1) & 1) ^ 1)) {
           atomicExch(err_flag, 1);
           abort_sh = 1;
           break;
         }
-        if (*((volatile int*)&abort_sh)) break;
-        const uint32_t sa = base + st * STAGE_BYTES, sb = sa + OZ_S * A_TILE;
-        const uint32_t fb = smem_u32(&full_bar[st]);
-        mbar_expect_tx(fb, STAGE_BYTES);
-        for (int q = 0; q < OZ_S; ++q) {
-          tma_load_2d(sa + q * A_TILE, &ta, fb, (kb0 + kb) * OZ_BK, a_row0 + q * Mp + m0);
-          tma_load_2d(sb + q * B_TILE, &tb, fb, (kb0 + kb) * OZ_BK, b_row0 + q * Np + n0);
+        queue[w & 1] = t < items ? t : -1;
+        mbar_arrive(smem_u32(&q_full[w & 1]));
+        if (t >= items) break;
+        const Item it = item(t);
+        t = int(gridDim.x) + atomicAdd(counter, 1);
+        const int a_row = it.bz * OZ_S * Mp + it.m0, b_row = it.bz * OZ_S * Np + it.n0;
+        for (int kb = 0; kb < it.kblocks; ++kb) {
+          const int st = issued % OZ_STAGES;
+          const uint32_t ph = (issued / OZ_STAGES) & 1;
+          const uint32_t sa = base + st * STAGE_BYTES, sb = sa + OZ_S * A_TILE;
+          const uint32_t fb = smem_u32(&full_bar[st]);
+#pragma unroll
+          for (int i = 0; i < OZ_PARTS; ++i) {
+            if (ok && issued >= OZ_STAGES && !mbar_wait(smem_u32(&empty_bar[st][i]), ph ^ 1)) {
+              atomicExch(err_flag, 1);
+              abort_sh = 1;
+            }
+            ok = ok && !*((volatile int*)&abort_sh);
+            if (!ok) break;
+            if (i == 0) mbar_expect_tx(fb, STAGE_BYTES);
+            // A slices q0 .. q1 - 1 and the B slices that no later one meets
+            const int q0 = 2 * i, q1 = i == 2 ? OZ_S : 2 * i + 2;
+#pragma unroll
+            for (int q = q0; q < q1; ++q) {
+              tma_load_2d(sa + q * A_TILE, &ta, fb, (it.kb0 + kb) * OZ_BK, a_row + q * Mp);
+              const int t = OZ_S - 1 - q;
+              tma_load_2d(sb + t * B_TILE, &tb, fb, (it.kb0 + kb) * OZ_BK, b_row + t * Np);
+            }
+          }
+          ++issued;  // also a block given up half way: its wait below runs out long after its copies have landed
+          if (!ok) break;
         }
-        ++issued;
       }
       for (int kb = issued - OZ_STAGES < 0 ? 0 : issued - OZ_STAGES; kb < issued; ++kb)
         mbar_wait(smem_u32(&full_bar[kb % OZ_STAGES]), (kb / OZ_STAGES) & 1);
     }
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      bool ok = true;
-      for (int c = 0; c < nchunks && ok; ++c) {
+    const uint64_t desc0 = smem_desc_sw64(base);
+    const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
+    const bool one = elect_one();
+    int block = 0, chunk = 0;  // K blocks and chunks of all items so far
+    bool ok = true;
+    for (int w = 0; ok; ++w) {
+      const int t = next_item(w);
+      if (t < 0) break;
+      const int kblocks = item(t).kblocks;
+      for (int kb = 0; kb < kblocks && ok; ++chunk) {
         // the epilogue must have read the previous chunk's accumulators
-        if (c > 0 && !mbar_wait(smem_u32(&chunk_empty), (c - 1) & 1)) {
-          atomicExch(err_flag, 1);
-          abort_sh = 1;
+        if (chunk > 0 && !mbar_wait(smem_u32(&chunk_empty), (chunk - 1) & 1)) {
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;");
-        const int kb_end = min(kblocks, (c + 1) * kb_per_chunk);
-        for (int kb = c * kb_per_chunk; kb < kb_end; ++kb) {
-          const int st = kb % OZ_STAGES;
-          const uint32_t ph = (kb / OZ_STAGES) & 1;
-          if (!mbar_wait(smem_u32(&full_bar[st]), ph) || *((volatile int*)&abort_sh)) {
-            atomicExch(err_flag, 1);
-            abort_sh = 1;
+        const int kb_end = min(kblocks, kb + kb_per_chunk);
+        for (bool chunk_start = true; kb < kb_end; ++kb, ++block, chunk_start = false) {
+          const int st = block % OZ_STAGES;
+          if (!mbar_wait(full0 + 8 * st, (block / OZ_STAGES) & 1)) {
             ok = false;
             break;
           }
           asm volatile("tcgen05.fence::after_thread_sync;");
-          const uint32_t sa = base + st * STAGE_BYTES, sb = sa + OZ_S * A_TILE;
-          const bool chunk_start = kb == c * kb_per_chunk;
-#pragma unroll
-          for (int kk = 0; kk < OZ_BK / 16; ++kk) {
+          // addresses sit in the descriptors in units of 16 bytes
+          const uint64_t da = desc0 + uint32_t(st) * (STAGE_BYTES >> 4), db = da + (OZ_S * A_TILE >> 4);
+          if (one) {
 #pragma unroll
             for (int q = 0; q < OZ_S; ++q) {
-              const uint64_t ad = smem_desc_sw64(sa + q * A_TILE + kk * 32);
 #pragma unroll
-              for (int t0 = 0; t0 < OZ_S - q; t0 += 4) {
-                // slice pairs (q, t0) .. (q, t0 + w - 1) into groups q + t0 .. q + t0 + w - 1; the two
-                // MMAs of (q = 0, kk = 0) cover all eight groups and start a chunk's sums
-                const int w = OZ_S - q - t0 < 4 ? OZ_S - q - t0 : 4;
-                const uint64_t bd = smem_desc_sw64(sb + t0 * B_TILE + kk * 32);
-                mma_bf16(tmem + uint32_t((q + t0) * OZ_BN), ad, bd, instr_desc_bf16(OZ_BM, OZ_BN * w),
-                         (chunk_start && kk == 0 && q == 0) ? 0u : 1u);
+              for (int kk = 0; kk < OZ_BK / 16; ++kk) {
+                const uint64_t ad = da + q * (A_TILE >> 4) + 2 * kk;
+#pragma unroll
+                for (int t0 = 0; t0 < OZ_S - q; t0 += 4) {
+                  // slice pairs (q, t0) .. (q, t0 + w - 1) into groups q + t0 .. q + t0 + w - 1; the two
+                  // MMAs of (q = 0, kk = 0) cover all eight groups and start a chunk's sums
+                  const int w = OZ_S - q - t0 < 4 ? OZ_S - q - t0 : 4;
+                  mma_bf16(tmem + uint32_t((q + t0) * OZ_BN), ad, db + t0 * (B_TILE >> 4) + 2 * kk,
+                           instr_desc_bf16(OZ_BM, OZ_BN * w), (chunk_start && kk == 0 && q == 0) ? 0u : 1u);
+                }
               }
+              if (q == 1 || q == 3 || q == OZ_S - 1)
+                mma_commit(empty0 + 8 * (st * OZ_PARTS + (q == 1 ? 0 : q == 3 ? 1 : 2)));
             }
           }
-          mma_commit(smem_u32(&empty_bar[st]));
         }
-        if (ok) mma_commit(smem_u32(&chunk_full));
+        if (ok && one) mma_commit(smem_u32(&chunk_full));
       }
+    }
+    if (!ok) {
+      if (one) atomicExch(err_flag, 1);
+      abort_sh = 1;
     }
   } else {
     // ------------------------------------------------ epilogue (warps 2..9): tile row = lane of
@@ -341,75 +406,89 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     // quarter)
     const int quad = warp & 3;
     const int cb = (warp - 2) / 4 * 32;
-    float hi[32], lo[32];
-#pragma unroll
-    for (int j = 0; j < 32; ++j) hi[j] = lo[j] = 0.f;
-    bool ok = true;
-    for (int c = 0; c < nchunks; ++c) {
-      if (!mbar_wait(smem_u32(&chunk_full), c & 1)) {
-        if (lane == 0) atomicExch(err_flag, 1);
-        ok = false;
-        break;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;");
-#pragma unroll 1
-      for (int g = 0; g < OZ_S; g += 2) {  // two groups' loads in flight per wait
-        uint32_t r[2][32];
-        tmem_ld32_async(tmem + (uint32_t(quad * 32) << 16) + uint32_t(g * OZ_BN + cb), r[0]);
-        tmem_ld32_async(tmem + (uint32_t(quad * 32) << 16) + uint32_t((g + 1) * OZ_BN + cb), r[1]);
-        tmem_ld_wait();
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const float scale = __uint_as_float(uint32_t(127 - 7 * (g + h + 2)) << 23);  // 2^-7(g+h+2)
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float v = __uint_as_float(r[h][j]) * scale;  // exact: power-of-two scaling
-            float sum, err;
-            two_sum_f(hi[j], v, sum, err);
-            hi[j] = sum;
-            lo[j] += err;
-          }
-        }
-      }
-      asm volatile("tcgen05.fence::before_thread_sync;");
-      __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&chunk_empty)) : "memory");
-    }
+    // a finished tile goes out through shared memory of the warp's own, 8 columns at a time, so that the
+    // global stores are row segments: a thread holds one row of 32 columns
+    constexpr int OW = 8, OLD = OW + 1;
+    double* Cs = reinterpret_cast<double*>(smem_raw + (base - smem_u32(smem_raw)) + OZ_STAGES * STAGE_BYTES) +
+                 (warp - 2) * 32 * OLD;
     const bool unit = alpha == 1.0;
-    // the finished tile goes through shared memory (the stage buffers are free once the last
-    // chunk's MMAs are done), so that the global stores are whole row segments: a thread owns one
-    // row of 32 columns in TMEM, and storing from there would write 32 rows per warp instruction
-    if (!ok) epi_fail_sh = 1;
-    double* Cs = reinterpret_cast<double*>(smem_raw + (base - smem_u32(smem_raw)));  // [BM][BN + 1]
-    if (ok) {
-      const int lr = quad * 32 + lane;
-      const int er = row_scale_exp(ea[m0 + lr]);  // ea and eb are padded to Mp and Np entries
-      const bool row_nonfinite = ea[m0 + lr] == 2047;  // the row holds Inf / NaN: its slices are not the value
-      const int* ebc = eb + n0 + cb;
+    int chunk = 0;
+    bool ok = true;
+    for (int w = 0; ok; ++w) {
+      const int t = next_item(w);
+      if (t < 0) break;
+      const Item it = item(t);
+      const int nchunks = (it.kblocks + kb_per_chunk - 1) / kb_per_chunk;
+      float hi[32], lo[32];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        // one FP64 addition an output; conversions and the power of two by integer arithmetic
-        double v = scale_pow2(float_to_double(hi[j]) + float_to_double(lo[j]), er + row_scale_exp(ebc[j]));
-        if (row_nonfinite || ebc[j] == 2047) v = __longlong_as_double(0x7ff8000000000000LL);
-        Cs[lr * (OZ_BN + 1) + cb + j] = v;
-      }
-    }
-    asm volatile("bar.sync 1, %0;" ::"n"(32 * OZ_EPI_WARPS) : "memory");  // the epilogue warps only
-    if (!epi_fail_sh) {
-      const int et = threadIdx.x - 64;
-      double* out = nsplit == 1 ? C + int64_t(bz) * sC : part + (int64_t(sz) * batch + bz) * M * N;
-      const int64_t ldo = nsplit == 1 ? ldc : N;
-      for (int idx = et; idx < OZ_BM * OZ_BN; idx += 32 * OZ_EPI_WARPS) {
-        const int r = idx / OZ_BN, c = idx % OZ_BN;
-        if (m0 + r < M && n0 + c < N) {
-          double v = Cs[r * (OZ_BN + 1) + c];
-          double* o = out + int64_t(m0 + r) * ldo + n0 + c;
-          if (nsplit == 1) {
-            if (!unit) v *= alpha;
-            if (beta != 0.0) v = fma(beta, *o, v);
-          }
-          *o = v;
+      for (int j = 0; j < 32; ++j) hi[j] = lo[j] = 0.f;
+      for (int c = 0; c < nchunks; ++c, ++chunk) {
+        if (!mbar_wait(smem_u32(&chunk_full), chunk & 1)) {
+          if (lane == 0) atomicExch(err_flag, 1);
+          ok = false;
+          break;
         }
+        asm volatile("tcgen05.fence::after_thread_sync;");
+#pragma unroll 1
+        for (int g = 0; g < OZ_S; g += 2) {  // two groups' loads in flight per wait
+          uint32_t r[2][32];
+          tmem_ld32_async(tmem + (uint32_t(quad * 32) << 16) + uint32_t(g * OZ_BN + cb), r[0]);
+          tmem_ld32_async(tmem + (uint32_t(quad * 32) << 16) + uint32_t((g + 1) * OZ_BN + cb), r[1]);
+          tmem_ld_wait();
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const float scale = __uint_as_float(uint32_t(127 - 7 * (g + h + 2)) << 23);  // 2^-7(g+h+2)
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const float v = __uint_as_float(r[h][j]) * scale;  // exact: power-of-two scaling
+              float sum, err;
+              two_sum_f(hi[j], v, sum, err);
+              hi[j] = sum;
+              lo[j] += err;
+            }
+          }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&chunk_empty));
+      }
+      if (!ok) break;
+      // ea and eb are padded to Mp and Np entries
+      const int row = it.m0 + quad * 32 + lane, col0 = it.n0 + cb;
+      const int ear = ea[int64_t(it.bz) * Mp + row];
+      const int* ebc = eb + int64_t(it.bz) * Np + col0;
+      const int er = row_scale_exp(ear);
+      const bool row_nonfinite = ear == 2047;  // the row holds Inf / NaN: its slices are not the value
+      double* out = nsplit == 1 ? C + int64_t(it.bz) * sC : part + (int64_t(it.sz) * batch + it.bz) * M * N;
+      const int64_t ldo = nsplit == 1 ? ldc : N;
+      const int r0 = it.m0 + quad * 32 + (lane >> 3), cc = lane & 7;
+#pragma unroll
+      for (int p = 0; p < 32 / OW; ++p) {
+#pragma unroll
+        for (int j = 0; j < OW; ++j) {
+          const int e = ebc[p * OW + j];
+          // one FP64 addition an output; conversions and the power of two by integer arithmetic
+          double v = scale_pow2(float_to_double(hi[p * OW + j]) + float_to_double(lo[p * OW + j]), er + row_scale_exp(e));
+          if (row_nonfinite || e == 2047) v = __longlong_as_double(0x7ff8000000000000LL);
+          Cs[lane * OLD + j] = v;
+        }
+        __syncwarp();
+        const int c = col0 + p * OW + cc;
+        if (c < N)
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int r = r0 + 4 * i;
+            if (r < M) {
+              double v = Cs[((lane >> 3) + 4 * i) * OLD + cc];
+              double* o = out + int64_t(r) * ldo + c;
+              if (nsplit == 1) {
+                if (!unit) v *= alpha;
+                if (beta != 0.0) v = fma(beta, *o, v);
+              }
+              *o = v;
+            }
+          }
+        __syncwarp();
       }
     }
   }
@@ -453,7 +532,7 @@ size_t oz_layout(int64_t m, int64_t n, int64_t k, int64_t batch, int nsplit, voi
   size_t off = 0;
   auto take = [&](size_t bytes) { size_t r = off; off += align_up(bytes); return r; };
   const size_t osa = take(size_t(batch) * OZ_S * o.Mp * o.Kp * 2), osb = take(size_t(batch) * OZ_S * o.Np * o.Kp * 2),
-               oea = take(size_t(batch) * o.Mp * 4), oeb = take(size_t(batch) * o.Np * 4), ofl = take(4),
+               oea = take(size_t(batch) * o.Mp * 4), oeb = take(size_t(batch) * o.Np * 4), ofl = take(8),
                opt = take(nsplit > 1 ? size_t(nsplit) * batch * m * n * 8 : 0);
   if (base && L) {
     char* b = static_cast<char*>(base);
@@ -468,7 +547,10 @@ size_t oz_layout(int64_t m, int64_t n, int64_t k, int64_t batch, int nsplit, voi
   return off;
 }
 
-size_t oz_smem_bytes() { return size_t(OZ_STAGES) * OZ_S * (OZ_BM * OZ_BK * 2 + OZ_BN * OZ_BK * 2) + 1024; }
+// stage ring, the epilogue warps' 32 x 9 doubles each, and slack for the alignment
+size_t oz_smem_bytes() {
+  return size_t(OZ_STAGES) * OZ_S * (OZ_BM * OZ_BK * 2 + OZ_BN * OZ_BK * 2) + OZ_EPI_WARPS * 32 * 9 * 8 + 1024;
+}
 
 }  // namespace
 
@@ -499,8 +581,8 @@ int gemm_oz_ex(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha, 
   // op(A)(i, kk): ta ? A[kk lda + i] : A[i lda + kk];  op(B) column j: tb ? B[j ldb + kk] : B[kk ldb + j]
   const int64_t a_rs = ta ? 1 : lda, a_ks = ta ? lda : 1;
   const int64_t b_rs = tb ? ldb : 1, b_ks = tb ? 1 : ldb;
-  // row maxima (atomicMax into zeroed arrays) and the error flag: ea, eb and flag are consecutive
-  TNX_CUDA(cudaMemsetAsync(L.ea, 0, reinterpret_cast<char*>(L.flag + 1) - reinterpret_cast<char*>(L.ea), st));
+  // row maxima (atomicMax into zeroed arrays), the error flag and the item counter: ea, eb and flag are consecutive
+  TNX_CUDA(cudaMemsetAsync(L.ea, 0, reinterpret_cast<char*>(L.flag + 2) - reinterpret_cast<char*>(L.ea), st));
   const unsigned kscan = unsigned((k + OZ_SCAN_K - 1) / OZ_SCAN_K), bzs = unsigned(batch);
   auto rowmax = [&](const double* src, int64_t rows, int64_t rs, int64_t ks, int* e, int64_t s_src, int64_t pad) {
     const dim3 grid(kscan, unsigned(pad / 32), bzs);
@@ -533,13 +615,16 @@ int gemm_oz_ex(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha, 
   const int kb_all = int(L.Kp / OZ_BK);
   const int kbs = (kb_all + nsplit - 1) / nsplit;
   nsplit = (kb_all + kbs - 1) / kbs;  // no empty splits
-  dim3 grid(unsigned(L.Np / OZ_BN), unsigned(L.Mp / OZ_BM), unsigned(batch * nsplit));
+  const int64_t items = (L.Np / OZ_BN) * (L.Mp / OZ_BM) * batch * nsplit;
+  TNX_CHECK_SHAPE(items < (int64_t(1) << 30), "gemm_oz: too many tiles");
+  const unsigned grid = unsigned(std::min<int64_t>(items, 152));
   // profiler family: the large products (environment updates, anchor matvecs, the gauge move's
   // X, Q and R A) apart from the narrow ones (a side of 128 or less, split K, batches)
   const int fam = (nsplit > 1 || batch > 1 || m <= 128 || n <= 128 || k <= 128) ? KF_OZ_NARROW : KF_OZ_GEMM;
   profile_mark(fam, st, true);
   oz_gemm_kernel<<<grid, OZ_THREADS, smem, st>>>(ma, mb, int(m), int(n), int(L.Kp), int(L.Mp), int(L.Np), L.ea, L.eb,
-                                                 alpha, beta, C, ldc, L.flag, batch, nsplit, kbs, sC, L.part, mask);
+                                                 alpha, beta, C, ldc, L.flag, L.flag + 1, batch, nsplit, kbs, sC, L.part,
+                                                 mask);
   TNX_LAUNCH_CHECK();
   if (nsplit > 1) {
     const int64_t mn = m * n;
