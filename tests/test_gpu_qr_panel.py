@@ -28,3 +28,20 @@ def test_gauge_move_with_double_fp32_panels(half, n, graded):
     rl = np.linalg.qr(a)[1]
     assert np.all(np.sign(np.diag(r)) == np.sign(np.diag(rl)))
     assert np.abs(np.tril(r, -1)).max() <= tol * np.abs(r).max()
+
+
+@pytest.mark.parametrize("m,n", [(34, 34), (257, 20), (300, 64), (130, 129), (1000, 65), (2050, 97), (6400, 34), (6890, 33)])
+@pytest.mark.parametrize("kind", ["normal", "zero_columns", "graded"])
+def test_qr_with_fp64_panels(m, n, kind):
+    a = np.random.RandomState(m + n).standard_normal((m, n))
+    if kind == "zero_columns":
+        a[:, ::3] = 0.0
+    elif kind == "graded":
+        a *= np.logspace(0, -140, n)
+    q, r = (t.cpu().numpy() for t in K.qr(torch.from_numpy(a).cuda()))
+    tol = 20 * m * 2.0 ** -53  # Householder: a few m u, columnwise
+    assert np.abs(q.T @ q - np.eye(n)).max() <= tol
+    assert np.all(np.tril(r, -1) == 0.0)
+    assert np.all(np.linalg.norm(q @ r - a, axis=0) <= tol * np.linalg.norm(a, axis=0) + 1e-300)
+    if kind == "normal":
+        assert np.all(np.sign(np.diag(r)) == np.sign(np.diag(np.linalg.qr(a)[1])))

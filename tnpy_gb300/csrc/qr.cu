@@ -153,68 +153,135 @@ __global__ void __launch_bounds__(QT) panel_kernel(double* __restrict__ F, int64
 }
 
 // Cluster form of the panel factorisation: the panel's rows are split over CL CTAs of one
-// thread-block cluster, each holding its rows in shared memory. Column jj costs ONE cluster
-// barrier: before it, every CTA publishes in its exchange slot the partial dot products of
+// thread-block cluster, each holding its rows in shared memory. Column jj costs ONE
+// exchange: before it, every CTA publishes the partial dot products of
 // column jj (below its pivot) with every column c >= jj (c = jj gives the norm), the pivot
 // row jj (its owner only) and the partial dot products v_a . v_{jj-1} that extend the
-// compact-WY T factor by one column (LAPACK dlarft recurrence, forward/columnwise). After the
-// barrier each CTA sums the CL partials in rank order, so all CTAs derive bitwise-identical
+// compact-WY T factor by one column (LAPACK dlarft recurrence, forward/columnwise). After
+// it each CTA sums the CL partials in rank order, so all CTAs derive bitwise-identical
 // beta, tau and v^T x_c = x_c[jj] + scale * sum_{i>jj} x_jj[i] x_c[i] without a second
 // exchange, update their rows, and compute the next column's partials in the same pass.
-// Slots are double-buffered, so the barrier of step jj also orders the reads of step jj-1.
+// The exchange is double-buffered: a CTA sends step jj+1's sums only after it has every rank's of step
+// jj, which a rank sends after it has read step jj-1's.
 //
-// Each step: one thread derives the column's scalars; phase A forms v = scale * x_jj and the
-// updated column jj+1 once per row (FP64 arithmetic is scarce on this part); phase B (before
-// the barrier arrives) updates columns c > jj+1 and forms the partial dots; phase C (between
-// arrive and wait) stores v and column jj+1. The rows of T are dealt out over the CTAs, a warp each.
+// Each step: one warp derives the column's scalars; phase A forms v = scale * x_jj and the
+// updated column jj+1 in place, once per row (FP64 arithmetic is scarce on this part), while 64 threads that
+// stand for the columns form the factors of the update and send the next pivot row; phase B updates
+// columns c > jj+1 and forms the partial dots. The rows of T are dealt out over the CTAs, a warp each, and
+// follow two columns behind.
 //
-// What bounds it: the chain of a column, in FP64 instructions of 64 clocks a warp. The partials of a
-// column's 64 sums (norm and dots right of the pivot, T dots left of it) are added by four threads
-// each, the scalars take 20 instructions (reflector), a row of T seven, behind the scalars and on other
-// sub-partitions. 128 x 64: 304 us with sums in one thread each, exact root and divisions, and all of T
-// by one thread a row on rank 0; 225 us so.
+// What bounds it: the chain of a column, in FP64 instructions of 64 clocks a warp: the two sums that the
+// scalars need are added by 16 lanes each, straight from the exchange, the other sums by one thread each
+// meanwhile, the scalars take 20 instructions (reflector); none of it shares warp 0's
+// sub-partition. The sums go to every rank's shared memory, counted by a barrier there (qr_panel_df.cuh);
+// panels too tall for that buffer read them from the ranks after a cluster barrier. 128 x 64: 304 us with sums in
+// one thread each, exact root and divisions, and all of T by one thread a row on rank 0; 225 us with
+// those spread out; 134 us without copies of v and the next column and with the sums sent.
 constexpr int PT = 256;  // threads per CTA of the cluster panel kernel
 
-__device__ __forceinline__ void cluster_arrive_release() {
-  asm volatile("barrier.cluster.arrive.release;\n" ::: "memory");
-}
-__device__ __forceinline__ void cluster_wait_acquire() {
-  asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory");
+using qrdf::cluster_arrive_release;
+using qrdf::cluster_wait_acquire;
+using tc::mbar_expect_tx;
+using tc::mbar_init;
+using tc::mbar_wait;
+using tc::smem_u32;
+
+// dynamic shared memory of a CTA: panel [NB][ld] and the exchange of two steps, sums [ranks][NB] (with `push`
+// every rank's, without it this rank's) and pivot row [NB]
+template <int NB, int CL>
+constexpr size_t panel_cl_smem_bytes(int ld, bool push) {
+  return (size_t(NB) * ld + 2 * size_t(NB) * ((push ? CL : 1) + 1)) * sizeof(double);
 }
 
 template <int NB, int CL>
 __global__ void __launch_bounds__(PT) panel_cl_kernel(double* __restrict__ F, int64_t m, int64_t j0, int nb,
-                                                      int ld, double* __restrict__ tau_out,
+                                                      int ld, int mode, double* __restrict__ tau_out,
                                                       double* __restrict__ T_out) {
   constexpr int TPC = PT / NB;  // threads per panel column, interleaved over rows
   cg::cluster_group cluster = cg::this_cluster();
   const int q = int(cluster.block_rank());
-  extern __shared__ double pl[];  // [NB][ld] column-major panel rows of this CTA, then vr[ld], vnr[ld]
-  double* vr = pl + NB * ld;      // reflector of the current column over this CTA's rows
-  double* vnr = vr + ld;          // next column after the current reflector
-  __shared__ double slot[2][3 * NB];  // s[NB] partial dots, piv[NB] pivot row, z[NB] T dots
-  constexpr int NR = NB / CL;  // rows of T held by each CTA: a = q, q + CL, ...
-  static_assert(NB % CL == 0, "panel shape");
-  __shared__ double S[NB], P[NB], Z[NB], taus[NB], sc[4];
+  const bool push = mode & qrdf::PUSH;
+  extern __shared__ double pl[];  // [NB][ld] column-major panel rows of this CTA
+  double* part = pl + NB * ld;    // exchange [2][push ? CL : 1][NB]: dots (right of the column) and T dots (left)
+  double* prow = part + 2 * (push ? CL : 1) * NB;  // [2][NB] pivot row
+  constexpr int NR = NB / CL;     // rows of T held by each CTA: a = q, q + CL, ...
+  constexpr int CT = 64;          // threads CT .. CT + NB - 1 stand for the columns
+  static_assert(NB % CL == 0 && 2 * CL <= 32 && NB <= 64 && PT == 256, "panel shape");
+  __shared__ double W[NB], Z[2][NB], taus[NB], sc[4];
   __shared__ double Tr[NR][NB];
+  __shared__ __align__(8) uint64_t bars[2];
+  __shared__ int s_dead;
   const int tid = threadIdx.x, ci = tid / TPC, h = tid % TPC, warp = tid >> 5, lane = tid & 31;
   const int64_t mp = m - j0;
-  const int64_t rpc = (mp + CL - 1) / CL;
-  const int64_t r0 = int64_t(q) * rpc;  // first panel row of this CTA
+  const int rpc = int((mp + CL - 1) / CL);
+  const int r0 = q * rpc;  // first panel row of this CTA
   const int rows = int(r0 >= mp ? 0 : (mp - r0 < rpc ? mp - r0 : rpc));
+  if (push && tid == 0) {
+    s_dead = 0;
+    mbar_init(smem_u32(&bars[0]), 1);
+    mbar_init(smem_u32(&bars[1]), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    mbar_expect_tx(smem_u32(&bars[0]), uint32_t(8 * nb * (CL + 1)));
+    mbar_expect_tx(smem_u32(&bars[1]), uint32_t(8 * (nb - 1) * (CL + 1)));
+  }
   for (int e = tid; e < nb * rows; e += PT) {
     const int c = e / rows, r = e % rows;
     pl[c * ld + r] = F[(j0 + c) * m + j0 + r0 + r];
   }
-  // column k of this warp's row of T: T[a][k] = -tau_k sum_{a <= c < k} T[a][c] z_c, T[k][k] = tau_k
-  // (warps 1, 2, 3, 5, 6, 7 take rows 0, 1, ..: not on the sub-partition of warp 0)
+  // a column's sum, held by the TPC threads of column ci, into the exchange
+  auto send_sum = [&](int buf, double sum) {
+    if (push) {
+#pragma unroll
+      for (int r = h; r < CL; r += TPC)
+        qrdf::send_async(smem_u32(&part[(buf * CL + q) * NB + ci]), sum, smem_u32(&bars[buf]), r);
+    } else if (h == 0) {
+      part[buf * NB + ci] = sum;
+    }
+  };
+  // column c's entry in the next pivot row
+  auto send_pivot = [&](int buf, int c, double piv) {
+    if (push) {
+#pragma unroll 4
+      for (int r = 0; r < CL; ++r) qrdf::send_async(smem_u32(&prow[buf * NB + c]), piv, smem_u32(&bars[buf]), r);
+    } else {
+      prow[buf * NB + c] = piv;
+    }
+  };
+  // before the exchange of step `step` is read
+  auto await = [&](int step) {
+    if (push && !mbar_wait(smem_u32(&bars[step & 1]), (step >> 1) & 1)) s_dead = 1;
+  };
+  auto exchange = [&] {
+    if (!push) {
+      cluster_arrive_release();
+      cluster_wait_acquire();
+    }
+  };
+  auto partial = [&](int buf, int r, int idx) {
+    return push ? part[(buf * CL + r) * NB + idx] : cluster.map_shared_rank(part, r)[buf * NB + idx];
+  };
+  auto pivot = [&](int buf, int owner, int idx) {
+    return push ? prow[buf * NB + idx] : cluster.map_shared_rank(prow, owner)[buf * NB + idx];
+  };
+  // sum over the ranks by one thread, in rank order
+  auto sum_ranks = [&](int buf, int idx) {
+    double v[CL];
+#pragma unroll
+    for (int r = 0; r < CL; ++r) v[r] = partial(buf, r, idx);
+    double t = v[0];
+#pragma unroll
+    for (int r = 1; r < CL; ++r) t += v[r];
+    return t;
+  };
+  // column k of the rows of T: T[a][k] = -tau_k sum_{a <= c < k} T[a][c] z_c, T[k][k] = tau_k (warps 1, 5, 6, 7: not on
+  // the sub-partition of warp 0)
   auto extend_t = [&](int k) {
-    if ((warp & 3) == 0) return;
-    for (int row = warp - 1 - (warp >> 2); row < NR; row += PT / 32 - PT / 128) {
+    if (k < 0 || !(warp == 1 || warp >= 5)) return;
+    for (int row = warp == 1 ? 0 : warp - 4; row < NR; row += 4) {
       const int a = q + CL * row;
       if (a < k) {
         double t = 0.0;
-        for (int c = a + lane; c < k; c += 32) t = fma(Tr[row][c], Z[c], t);
+        for (int c = a + lane; c < k; c += 32) t = fma(Tr[row][c], Z[k & 1][c], t);
         t = warp_sum(t);
         if (lane == 0) Tr[row][k] = -taus[k] * t;
       } else if (a == k && lane == 0) {
@@ -222,7 +289,8 @@ __global__ void __launch_bounds__(PT) panel_cl_kernel(double* __restrict__ F, in
       }
     }
   };
-  __syncthreads();
+  cluster_arrive_release();  // the barriers are there before anything is sent
+  cluster_wait_acquire();
   // partials of pivot 0: s[c] = sum_{row > 0} x_0 x_c, pivot row 0 from rank 0
   {
     double acc = 0.0;
@@ -236,138 +304,128 @@ __global__ void __launch_bounds__(PT) panel_cl_kernel(double* __restrict__ F, in
     }
 #pragma unroll
     for (int o = TPC / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (ci < nb && h == 0) {
-      slot[0][ci] = acc;
-      if (r0 == 0 && rows > 0) slot[0][NB + ci] = pl[ci * ld];
-    }
+    if (ci < nb) send_sum(0, acc);
+    if (r0 == 0 && rows > 0 && tid < nb) send_pivot(0, tid, pl[tid * ld]);
   }
-  cluster_arrive_release();
-  cluster_wait_acquire();
+  exchange();
   for (int jj = 0; jj < nb; ++jj) {
     const int par = jj & 1;
-    const int owner = int(jj / rpc);
-    // S[c] (c >= jj) and Z[c] (c < jj - 1): sum over the ranks by the TPC threads of column c
-    {
-      const bool right = ci >= jj && ci < nb, left = ci < jj - 1;
-      double t = 0.0, piv = 0.0;
-      if (right || left) {
-        const double* from = &slot[par][right ? ci : 2 * NB + ci];
-        if (h == 0 && right) piv = *cluster.map_shared_rank(&slot[par][NB + ci], owner);
+    const int owner = jj / rpc;
+    const bool has_next = jj + 1 < nb;
+    const int lj = jj - r0, ln = lj + 1;  // local rows of pivots jj and jj + 1 (outside [0, rows) on other CTAs)
+    const bool has_lj = lj >= 0 && lj < rows, has_ln = ln >= 0 && ln < rows;
+    double* xj = pl + jj * ld;
+    double* xn = xj + ld;
+    double sum_c = 0.0, piv_c = 0.0, xl_j = 0.0, xl_c = 0.0;
+    if (warp == 0) {
+      await(jj);
+      if (push && lane == 0 && jj + 2 <= nb)  // the buffer's next use, for step jj + 2
+        mbar_expect_tx(smem_u32(&bars[par]), uint32_t(8 * ((nb - 1) * CL + nb - 2 - jj)));
+      // column scalars, from the sums of columns jj and jj + 1 (the halves of 2 CL lanes)
+      double t = partial(par, lane % CL, jj + (((lane / CL) & 1) && has_next ? 1 : 0));
+      const double alpha = pivot(par, owner, jj), pn = pivot(par, owner, has_next ? jj + 1 : jj);
 #pragma unroll
-        for (int qq = 0; qq < CL; qq += TPC)
-          if (qq + h < CL) t += *cluster.map_shared_rank(from, qq + h);
+      for (int o = 1; o < CL; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      const double sigma = __shfl_sync(0xffffffffu, t, 0), sn = __shfl_sync(0xffffffffu, t, CL);
+      double tj, beta, scale;
+      reflector(alpha, sigma, beta, tj, scale);
+      if (lane == 0) {
+        sc[0] = tj;
+        sc[1] = beta;
+        sc[2] = scale;
+        taus[jj] = tj;
       }
-#pragma unroll
-      for (int o = TPC / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if (h == 0) {
-        if (right) {
-          S[ci] = t;
-          P[ci] = piv;
-        } else if (left) {
-          Z[ci] = t;
+      const double wn = has_next ? tj * fma(scale, sn, pn) : 0.0;  // w of column jj + 1
+      if (lane == 0) sc[3] = wn;
+    } else if (tid >= CT && tid < CT + NB) {
+      // meanwhile: sum and pivot entry of column c >= jj + 2, T dots Z[a] = v_a . v_{jj-1} (a < jj - 1)
+      const int c = tid - CT;
+      await(jj);
+      if (c > jj + 1 && c < nb) {
+        sum_c = sum_ranks(par, c);
+        piv_c = pivot(par, owner, c);
+      } else if (c < jj - 1) {
+        Z[par ^ 1][c] = sum_ranks(par, c);
+      }
+      if (has_ln && c > jj && c < nb) {  // row jj + 1 before the update
+        xl_j = xj[ln];
+        xl_c = pl[c * ld + ln];
+      }
+    } else {
+      extend_t(jj - 2);
+    }
+    __syncthreads();
+    if (push && s_dead) break;
+    const double tj = sc[0], scale = sc[2];
+    // ---- phase A: v_jj = scale * x_jj below the pivot (beta at it, where v is 1) and the updated column jj+1
+    {
+      const double beta = sc[1], wn = sc[3];
+      for (int r = (lj > 0 ? lj : 0) + tid; r < rows; r += PT) {
+        const bool at = r == lj;
+        const double v = at ? 1.0 : scale * xj[r];
+        if (has_next) xn[r] -= wn * v;
+        xj[r] = at ? beta : v;
+      }
+    }
+    // meanwhile: the columns' factors, rows jj and jj + 1 of them, and the next pivot row on its way
+    if (tid >= CT && tid < CT + NB) {
+      const int c = tid - CT;
+      if (c > jj && c < nb) {
+        const double w = c == jj + 1 ? sc[3] : tj * fma(scale, sum_c, piv_c);
+        W[c] = w;
+        if (has_lj && c > jj + 1) pl[c * ld + lj] -= w;  // v_jj[jj] = 1
+        if (has_ln) {
+          const double p = xl_c - w * (scale * xl_j);
+          if (c > jj + 1) pl[c * ld + ln] = p;
+          send_pivot(par ^ 1, c, p);
         }
       }
     }
     __syncthreads();
-    // column scalars once; meanwhile, on the other sub-partitions' pipes, column jj - 1 of T
-    if (warp != 0) {
-      if (jj >= 1) extend_t(jj - 1);
-    } else if (tid == 0) {
-      double tj, beta, scale;
-      reflector(P[jj], S[jj], beta, tj, scale);
-      sc[0] = tj;
-      sc[1] = beta;
-      sc[2] = scale;
-      sc[3] = jj + 1 < nb ? tj * fma(scale, S[jj + 1], P[jj + 1]) : 0.0;  // w of column jj+1
-      taus[jj] = tj;
-    }
-    __syncthreads();
-    const double tj = sc[0], beta = sc[1], scale = sc[2], wn = sc[3];
-    const bool has_next = jj + 1 < nb;
-    double* nxt = slot[par ^ 1];
-    double* xj = pl + jj * ld;
-    double* xn = pl + (jj + 1) * ld;
-    const int64_t lj = jj - r0;  // local row of pivot jj (outside [0, rows) if another CTA holds it)
-    // ---- phase A: v_jj = scale * x_jj below the pivot (1 at it) and the updated column jj+1,
-    // once per row
-    for (int r = int(lj > 0 ? lj : 0) + tid; r < rows; r += PT) {
-      const double v = r == lj ? 1.0 : scale * xj[r];
-      vr[r] = v;
-      if (has_next) vnr[r] = xn[r] - wn * v;
-    }
-    __syncthreads();
-    // ---- phase B: update columns c > jj+1, partial dots of column jj+1 with c >= jj+1 below
-    // pivot jj+1 (norm at c = jj+1), pivot row jj+1, T dots v_c . v_jj for c < jj
+    // ---- phase B: update columns c > jj+1 below both pivots, partial dots of column jj+1 with c >= jj+1 below
+    // pivot jj+1 (norm at c = jj+1), T dots v_c . v_jj for c < jj
     double acc = 0.0;
     if (ci < nb && ci != jj) {
       double* xc = pl + ci * ld;
-      const int64_t ln = lj + 1;
-      const bool own_ln = ln >= 0 && ln < rows && ln % TPC == h;
-      if (ci == jj + 1) {
-        if (own_ln) nxt[NB + ci] = vnr[ln];
-        const int rs = int(lj + 2 > 0 ? lj + 2 : 0);
-        for (int i = rs / TPC; i * TPC < rows; ++i) {
-          const int r = i * TPC + h;
-          if (r >= rs && r < rows) acc = fma(vnr[r], vnr[r], acc);
-        }
-      } else if (ci > jj) {
-        const double wc = tj * fma(scale, S[ci], P[ci]);
-        if (lj >= 0 && lj < rows && lj % TPC == h) xc[lj] -= wc;  // v_jj[jj] = 1
-        if (own_ln) {
-          const double val = xc[ln] - wc * vr[ln];
-          xc[ln] = val;
-          nxt[NB + ci] = val;  // pivot row of step jj+1
-        }
-        const int rs = int(lj + 2 > 0 ? lj + 2 : 0);
+      if (ci > jj) {
+        const double wc = W[ci];
+        const int rs = lj + 2 > 0 ? lj + 2 : 0;
         for (int i = rs / TPC; i * TPC < rows; ++i) {
           const int r = i * TPC + h;
           if (r < rs || r >= rows) continue;
-          const double val = xc[r] - wc * vr[r];
-          xc[r] = val;
-          acc = fma(vnr[r], val, acc);
+          double val = xc[r];
+          if (ci > jj + 1) {
+            val -= wc * xj[r];
+            xc[r] = val;
+          }
+          acc = fma(xn[r], val, acc);
         }
       } else {
-        const int rs = int(lj > 0 ? lj : 0);
+        const int rs = lj > 0 ? lj : 0;
         for (int i = rs / TPC; i * TPC < rows; ++i) {
           const int r = i * TPC + h;
-          if (r >= rs && r < rows) acc = fma(xc[r], vr[r], acc);
+          if (r >= rs && r < rows) acc = fma(xc[r], r == lj ? 1.0 : xj[r], acc);
         }
       }
     }
 #pragma unroll
     for (int o = TPC / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (ci < nb && ci != jj && h == 0) {
-      if (ci > jj) nxt[ci] = acc;
-      else nxt[2 * NB + ci] = acc;
-    }
-    cluster_arrive_release();
-    __syncthreads();
-    // ---- phase C: store v_jj and beta, the updated column jj+1, extend T by column jj-1
-    {
-      for (int r = int(lj > 0 ? lj : 0) + tid; r < rows; r += PT) {
-        xj[r] = r == lj ? beta : vr[r];
-        if (has_next) xn[r] = vnr[r];
-      }
-    }
-    // the next gather rewrites S, P and Z, which phase C of other threads still reads
-    __syncthreads();
-    cluster_wait_acquire();
+    if (ci < nb && ci != jj) send_sum(par ^ 1, acc);
+    exchange();
   }
-  // last T column from the final exchange
-  {
-    double t = 0.0;
-    if (ci < nb - 1) {
-#pragma unroll
-      for (int qq = 0; qq < CL; qq += TPC)
-        if (qq + h < CL) t += *cluster.map_shared_rank(&slot[nb & 1][2 * NB + ci], qq + h);
-    }
-#pragma unroll
-    for (int o = TPC / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (ci < nb - 1 && h == 0) Z[ci] = t;
+  __syncthreads();
+  // the last two columns of T, the last one from the final exchange
+  if (tid >= CT && tid < CT + NB) {
+    const int c = tid - CT;
+    if (!(push && s_dead)) await(nb);
+    if (c < nb - 1) Z[(nb - 1) & 1][c] = sum_ranks(nb & 1, c);
+  } else {
+    extend_t(nb - 2);
   }
   __syncthreads();
   extend_t(nb - 1);
   __syncthreads();
+  const bool dead = push && s_dead;  // a bounded wait ran out: NaN, so that no caller takes the result
   for (int e = tid; e < NR * NB; e += PT) {
     const int i = e / NB, b = e % NB, a = q + CL * i;  // T_out column-major, ld NB
     T_out[b * NB + a] = (a <= b && b < nb) ? Tr[i][b] : 0.0;
@@ -376,8 +434,9 @@ __global__ void __launch_bounds__(PT) panel_cl_kernel(double* __restrict__ F, in
     for (int b = tid; b < NB; b += PT) tau_out[b] = b < nb ? taus[b] : 0.0;
   for (int e = tid; e < nb * rows; e += PT) {
     const int c = e / rows, r = e % rows;
-    F[(j0 + c) * m + j0 + r0 + r] = pl[c * ld + r];
+    F[(j0 + c) * m + j0 + r0 + r] = dead ? __longlong_as_double(0x7ff8000000000000LL) : pl[c * ld + r];
   }
+  if (dead) __nanosleep(1000000);  // stores of this CTA may still be on their way to others
   // no CTA leaves while another may still read its slots
   cluster_arrive_release();
   cluster_wait_acquire();
@@ -503,16 +562,9 @@ struct PanelKernelInfo {
 };
 
 // DF selects the double-FP32 panel (FP64-class modes), otherwise the FP64 one
-template <bool DF>
-struct PanelFn {
-  using type = void (*)(double*, int64_t, int64_t, int, int, double*, double*);
-};
-template <>
-struct PanelFn<true> {
-  using type = void (*)(double*, int64_t, int64_t, int, int, int, double*, double*);
-};
+using PanelFn = void (*)(double*, int64_t, int64_t, int, int, int, double*, double*);
 template <int NB, int CL, bool DF>
-typename PanelFn<DF>::type panel_fn() {
+PanelFn panel_fn() {
   if constexpr (DF) return qrdf::panel_df_kernel<NB, CL>;
   else return panel_cl_kernel<NB, CL>;
 }
@@ -526,7 +578,7 @@ const PanelKernelInfo& panel_info() {
   static PanelKernelInfo info;
   static std::once_flag once;
   std::call_once(once, [] {
-    const auto k = panel_fn<NB, CL, DF>();
+    PanelFn k = panel_fn<NB, CL, DF>();
     cudaFuncAttributes fa{};
     int dev = 0, optin = 0;
     if (cudaFuncGetAttributes(&fa, k) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess ||
@@ -566,25 +618,22 @@ const PanelKernelInfo& panel_info() {
 template <int NB, int CL, bool DF>
 size_t panel_smem(int ld, bool push) {
   if constexpr (DF) return qrdf::panel_df_smem_bytes<NB, CL>(ld, push);
-  else return size_t(NB + 2) * ld * sizeof(double);
+  else return panel_cl_smem_bytes<NB, CL>(ld, push);
 }
 
 template <int NB, int CL, bool DF>
 int launch_panel(double* F, int64_t m, int64_t j0, int nb, double* tau, double* T, cudaStream_t st) {
   const int64_t rpc = (m - j0 + CL - 1) / CL;
   int ld = panel_ld<DF>(rpc, NB), mode = 0;
-  size_t smem = panel_smem<NB, CL, DF>(ld, false);
-  if constexpr (DF) {
-    const size_t most = panel_info<NB, CL, DF>().max_dyn;
-    const int padded = panel_ld<DF>(rpc + qrdf::PAD_ROWS, NB);
-    if (panel_smem<NB, CL, DF>(padded, true) <= most) {
-      ld = padded;
-      mode = qrdf::PUSH | qrdf::PAD;
-    } else if (panel_smem<NB, CL, DF>(ld, true) <= most) {
-      mode = qrdf::PUSH;
-    }
-    smem = panel_smem<NB, CL, DF>(ld, mode != 0);
+  const size_t most = panel_info<NB, CL, DF>().max_dyn;
+  const int padded = DF ? panel_ld<DF>(rpc + qrdf::PAD_ROWS, NB) : ld;
+  if (DF && panel_smem<NB, CL, DF>(padded, true) <= most) {
+    ld = padded;
+    mode = qrdf::PUSH | qrdf::PAD;
+  } else if (panel_smem<NB, CL, DF>(ld, true) <= most) {
+    mode = qrdf::PUSH;
   }
+  const size_t smem = panel_smem<NB, CL, DF>(ld, mode != 0);
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -597,11 +646,7 @@ int launch_panel(double* F, int64_t m, int64_t j0, int nb, double* tau, double* 
   cfg.stream = st;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  if constexpr (DF) {
-    TNX_CUDA(cudaLaunchKernelEx(&cfg, panel_fn<NB, CL, DF>(), F, m, j0, nb, ld, mode, tau, T));
-  } else {
-    TNX_CUDA(cudaLaunchKernelEx(&cfg, panel_fn<NB, CL, DF>(), F, m, j0, nb, ld, tau, T));
-  }
+  TNX_CUDA(cudaLaunchKernelEx(&cfg, panel_fn<NB, CL, DF>(), F, m, j0, nb, ld, mode, tau, T));
   TNX_LAUNCH_CHECK();
   return TNX_OK;
 }

@@ -167,6 +167,14 @@ __device__ __forceinline__ void send_async(uint32_t at, df2 x, uint32_t bar, int
       : "memory");
 }
 
+__device__ __forceinline__ void send_async(uint32_t at, double x, uint32_t bar, int rank) {
+  asm volatile(
+      "{\n .reg .b32 a, b;\n mapa.shared::cluster.u32 a, %0, %3;\n mapa.shared::cluster.u32 b, %2, %3;\n"
+      " st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [a], %1, [b];\n}\n" ::"r"(at),
+      "l"(__double_as_longlong(x)), "r"(bar), "r"(rank)
+      : "memory");
+}
+
 // Dynamic shared memory bytes of one CTA: (hi, lo) pairs of the panel [NB][ld] (interleaved pairs: one
 // 64-bit access per operand) and the exchange of two steps, sums [ranks][NB] and the pivot row [NB]: with `push` every rank's
 // sums, without it this rank's, which the others read.
