@@ -193,14 +193,14 @@ constexpr size_t panel_cl_smem_bytes(int ld, bool push) {
   return (size_t(NB) * ld + 2 * size_t(NB) * ((push ? CL : 1) + 1)) * sizeof(double);
 }
 
-template <int NB, int CL>
+template <int NB, int CL, int MODE>
 __global__ void __launch_bounds__(PT) panel_cl_kernel(double* __restrict__ F, int64_t m, int64_t j0, int nb,
-                                                      int ld, int mode, double* __restrict__ tau_out,
+                                                      int ld, double* __restrict__ tau_out,
                                                       double* __restrict__ T_out) {
   constexpr int TPC = PT / NB;  // threads per panel column, interleaved over rows
   cg::cluster_group cluster = cg::this_cluster();
   const int q = int(cluster.block_rank());
-  const bool push = mode & qrdf::PUSH;
+  constexpr bool push = MODE & qrdf::PUSH;
   extern __shared__ double pl[];  // [NB][ld] column-major panel rows of this CTA
   double* part = pl + NB * ld;    // exchange [2][push ? CL : 1][NB]: dots (right of the column) and T dots (left)
   double* prow = part + 2 * (push ? CL : 1) * NB;  // [2][NB] pivot row
@@ -562,11 +562,11 @@ struct PanelKernelInfo {
 };
 
 // DF selects the double-FP32 panel (FP64-class modes), otherwise the FP64 one
-using PanelFn = void (*)(double*, int64_t, int64_t, int, int, int, double*, double*);
-template <int NB, int CL, bool DF>
+using PanelFn = void (*)(double*, int64_t, int64_t, int, int, double*, double*);
+template <int NB, int CL, bool DF, int MODE>
 PanelFn panel_fn() {
-  if constexpr (DF) return qrdf::panel_df_kernel<NB, CL>;
-  else return panel_cl_kernel<NB, CL>;
+  if constexpr (DF) return qrdf::panel_df_kernel<NB, CL, MODE>;
+  else return panel_cl_kernel<NB, CL, MODE & qrdf::PUSH>;
 }
 template <bool DF>
 constexpr int panel_threads() {
@@ -578,35 +578,46 @@ const PanelKernelInfo& panel_info() {
   static PanelKernelInfo info;
   static std::once_flag once;
   std::call_once(once, [] {
-    PanelFn k = panel_fn<NB, CL, DF>();
-    cudaFuncAttributes fa{};
     int dev = 0, optin = 0;
-    if (cudaFuncGetAttributes(&fa, k) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess ||
+    if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
       cudaGetLastError();
       return;
     }
-    const size_t dyn = size_t(optin) > fa.sharedSizeBytes ? size_t(optin) - fa.sharedSizeBytes : 0;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)) != cudaSuccess ||
-        (CL > 8 && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
-      cudaGetLastError();
-      return;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = CL;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(CL);
-    cfg.blockDim = dim3(panel_threads<DF>());
-    cfg.dynamicSmemBytes = dyn;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
+    size_t dyn = size_t(optin);
     int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      clusters = 0;
+    for (PanelFn k : {panel_fn<NB, CL, DF, 0>(), panel_fn<NB, CL, DF, qrdf::PUSH>(),
+                      panel_fn<NB, CL, DF, qrdf::PUSH | qrdf::PAD>()}) {
+      cudaFuncAttributes fa{};
+      if (cudaFuncGetAttributes(&fa, k) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+      }
+      dyn = std::min(dyn, size_t(optin) > fa.sharedSizeBytes ? size_t(optin) - fa.sharedSizeBytes : 0);
+    }
+    for (PanelFn k : {panel_fn<NB, CL, DF, 0>(), panel_fn<NB, CL, DF, qrdf::PUSH>(),
+                      panel_fn<NB, CL, DF, qrdf::PUSH | qrdf::PAD>()}) {
+      if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)) != cudaSuccess ||
+          (CL > 8 && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
+        cudaGetLastError();
+        return;
+      }
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = CL;
+      at[0].val.clusterDim.y = 1;
+      at[0].val.clusterDim.z = 1;
+      cfg.gridDim = dim3(CL);
+      cfg.blockDim = dim3(panel_threads<DF>());
+      cfg.dynamicSmemBytes = dyn;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        clusters = 0;
+      }
+      if (clusters < 1) return;
     }
     info.max_dyn = dyn;
     info.ok = clusters > 0;
@@ -624,16 +635,19 @@ size_t panel_smem(int ld, bool push) {
 template <int NB, int CL, bool DF>
 int launch_panel(double* F, int64_t m, int64_t j0, int nb, double* tau, double* T, cudaStream_t st) {
   const int64_t rpc = (m - j0 + CL - 1) / CL;
-  int ld = panel_ld<DF>(rpc, NB), mode = 0;
   const size_t most = panel_info<NB, CL, DF>().max_dyn;
-  const int padded = DF ? panel_ld<DF>(rpc + qrdf::PAD_ROWS, NB) : ld;
+  const int padded = panel_ld<DF>(rpc + qrdf::PAD_ROWS, NB);
+  int ld = panel_ld<DF>(rpc, NB);
+  PanelFn k = panel_fn<NB, CL, DF, 0>();
+  size_t smem = panel_smem<NB, CL, DF>(ld, false);
   if (DF && panel_smem<NB, CL, DF>(padded, true) <= most) {
     ld = padded;
-    mode = qrdf::PUSH | qrdf::PAD;
+    k = panel_fn<NB, CL, DF, qrdf::PUSH | qrdf::PAD>();
+    smem = panel_smem<NB, CL, DF>(ld, true);
   } else if (panel_smem<NB, CL, DF>(ld, true) <= most) {
-    mode = qrdf::PUSH;
+    k = panel_fn<NB, CL, DF, qrdf::PUSH>();
+    smem = panel_smem<NB, CL, DF>(ld, true);
   }
-  const size_t smem = panel_smem<NB, CL, DF>(ld, mode != 0);
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -646,7 +660,7 @@ int launch_panel(double* F, int64_t m, int64_t j0, int nb, double* tau, double* 
   cfg.stream = st;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  TNX_CUDA(cudaLaunchKernelEx(&cfg, panel_fn<NB, CL, DF>(), F, m, j0, nb, ld, mode, tau, T));
+  TNX_CUDA(cudaLaunchKernelEx(&cfg, k, F, m, j0, nb, ld, tau, T));
   TNX_LAUNCH_CHECK();
   return TNX_OK;
 }

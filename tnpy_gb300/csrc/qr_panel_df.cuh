@@ -201,10 +201,9 @@ constexpr size_t panel_df_smem_bytes(int ld, bool push) {
 //     the CTA's own (PAD, where they fit) spare it the bounds checks, a third of its instructions.
 // The 16 panels of a 2048 x 1024 matrix: 280 us each with five block barriers and a cluster barrier a
 // column, 254 us so. 256 or 1024 threads: a quarter slower.
-template <int NB, int CL>
+template <int NB, int CL, int MODE>
 __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, int64_t m, int64_t j0, int nb, int ld,
-                                                       int mode, double* __restrict__ tau_out,
-                                                       double* __restrict__ T_out
+                                                       double* __restrict__ tau_out, double* __restrict__ T_out
 #ifdef TNX_PANEL_PROBE
                                                        ,
                                                        long long* stamps
@@ -218,9 +217,9 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
   const int q = int(cluster.block_rank());
   extern __shared__ df2 pd[];
   df2* X = pd;                        // [NB][ld] panel rows of this CTA, column-major
-  const bool push = mode & PUSH, pad = mode & PAD;
+  constexpr bool push = MODE & PUSH, pad = MODE & PAD;
   df2* part = pd + NB * ld;           // exchange [2][push ? CL : 1][NB]: dots (right of the column) and T dots (left)
-  const int pr = push ? CL : 1;
+  constexpr int pr = push ? CL : 1;
   df2* prow = part + 2 * pr * NB;     // [2][NB] pivot row (pushed, or the owner's)
   __shared__ unsigned long long smax[NB];
   __shared__ df2 W[NB], Z[2][NB], taus[NB], sc[4];  // W: factors of the current reflector in the columns right of it
