@@ -420,14 +420,23 @@ __device__ __forceinline__ void split_bf16(double v, uint32_t& hi, uint32_t& lo)
     lo = sig >= hv ? round_bf16(sig - hv, e, sign) : round_bf16(hv - sig, e, sign ^ 1u);
     return;
   }
-  // normal hi, and lo normal or zero: its leading bit is at 2^-52 of v or above, which the margin of 8
-  // in the exponent leaves to round_bf16's general form
-  const uint64_t sig = m | (1ull << 52);
-  const uint64_t q = (sig + ((1ull << 44) - 1) + ((sig >> 45) & 1)) >> 45;  // 128 .. 256
-  hi = (sign << 15) | ((uint32_t(eb - 897) << 7) + uint32_t(q));
-  const int64_t d = int64_t(sig - (q << 45));  // |d| <= 2^44
-  lo = round_bf16(uint64_t(d < 0 ? -d : d), eb - 1075, d < 0 ? sign ^ 1u : sign);
-  if (d == 0) lo = 0;  // v - hi = +0
+  // normal hi: the upper word holds its 8 bits and the half's, the lower one only breaks ties
+  const uint32_t lw = uint32_t(u), hw = (uint32_t(u >> 32) & 0xfffffu) | 0x100000u;
+  const uint32_t q = (hw + 0xfffu + (((hw >> 13) & 1u) | (lw != 0 ? 1u : 0u))) >> 13;  // 128 .. 256
+  hi = (sign << 15) | ((uint32_t(eb - 897) << 7) + q);
+  // v - hi = d 2^(eb - 1075), |d| <= 2^44; its upper 32 bits (t, below them a sticky bit) round to 8 where they
+  // hold 10 and more and the result is normal
+  const uint32_t dh = hw - (q << 13), neg = dh >> 31;
+  const uint64_t d = (uint64_t(dh) << 32) | lw, a = neg ? 0 - d : d;
+  const uint32_t al = uint32_t(a), ah = uint32_t(a >> 32), t = __funnelshift_l(al, ah, 19);
+  const int p = 31 - __clz(int(t)), ef = eb - 1075 + p + 13 + 127;
+  if (p >= 9 && ef > 0) {
+    const int drop = p - 7;
+    const uint32_t r = (t + (1u << (drop - 1)) - 1u + (((t >> drop) & 1u) | ((al << 19) != 0 ? 1u : 0u))) >> drop;
+    lo = ((sign ^ neg) << 15) | ((uint32_t(ef - 1) << 7) + r);
+    return;
+  }
+  lo = a == 0 ? 0 : round_bf16(a, eb - 1075, sign ^ neg);  // v - hi = +0
 }
 __device__ __forceinline__ void split_bf16(float v, uint32_t& hi, uint32_t& lo) {
   const __nv_bfloat16 h = __float2bfloat16_rn(v);
@@ -437,7 +446,8 @@ __device__ __forceinline__ void split_bf16(float v, uint32_t& hi, uint32_t& lo) 
 
 // dst_hi/lo[c][r] (row pitch ldp, even) = split(src[r][c]) for r < rows; zeros for rows <= r < ldp.
 // src is row-major rows x cols. Bound by memory (8 bytes read, 4 written an element) once the
-// split stays off the FP64 pipe: L, R and x of a chi = 1024 site 101 us with conversions, 58 us so.
+// split stays off the FP64 pipe: L, R and x of a chi = 1024 site 101 us with conversions, 58 us with 64-bit
+// integers, 53 us with 32-bit ones.
 template <typename T>
 __global__ void __launch_bounds__(256) split_transpose_kernel(const T* __restrict__ src, int64_t rows, int64_t cols,
                                                              __nv_bfloat16* __restrict__ hi,
