@@ -67,3 +67,40 @@ def test_davidson_over_the_whole_space(n, form, scale):
         assert r <= 2e-11 * max(1.0, abs(e))
         gap = e - w[0] if form not in ("diagonal", "weak") else np.abs(e - w).min()
         assert gap <= 2e-11 * max(1.0, abs(e))
+
+
+@pytest.mark.parametrize("n", [3, 5, 12, 24, 37, 50])
+@pytest.mark.parametrize("seed", [0, 1, 2, 3])
+def test_davidson_sign_is_that_of_jacobi_steps(n, seed):
+    """The generalised solver with B = 1 is the same iteration with a Jacobi Rayleigh-Ritz in every step."""
+    rng = np.random.RandomState(100 * n + seed)
+    a = rng.standard_normal((n, n))
+    a = a + a.T + np.diag(rng.uniform(-1.0, 1.0, n) * 5 * (seed % 2))
+    one = torch.ones((1, 1, 1), dtype=torch.float64, device="cuda")
+    op = (torch.from_numpy(a).cuda().reshape(n, 1, n), one.reshape(1, 1, 1, 1), one)
+    eye = (torch.eye(n, dtype=torch.float64, device="cuda").reshape(n, 1, n), one.reshape(1, 1, 1, 1), one)
+    x = torch.from_numpy(rng.standard_normal((n, 1, 1))).cuda()
+    y = x.clone()
+    K.davidson1(*op, x, tol=1e-9, max_iter=200, max_basis=64)
+    K.gdavidson1(*op, *eye, y, tol=1e-9, max_iter=200, max_basis=64)
+    assert float((x * y).sum()) > 0.9
+
+
+@pytest.mark.parametrize("max_basis", [4, 7, 24])
+@pytest.mark.parametrize("chi", [8, 20])
+def test_davidson_sign_through_restarts(max_basis, chi):
+    """Stacked chains run the same iteration, restarts included, with a Jacobi Rayleigh-Ritz in every step."""
+    g = torch.Generator(device="cuda").manual_seed(chi + max_basis)
+    rand = lambda *s: torch.randn(*s, generator=g, dtype=torch.float64, device="cuda")
+    batch = 4
+    L, R = ((e + e.transpose(1, 3)).contiguous() for e in (rand(batch, chi, 1, chi), rand(batch, chi, 1, chi)))
+    w = torch.diag(torch.tensor([1.0, 0.6], dtype=torch.float64, device="cuda")).reshape(1, 1, 2, 2)
+    x = rand(batch, chi, 2, chi)
+    y = x.clone()
+    K.batched_davidson1(L, w.expand(batch, 1, 1, 2, 2).contiguous(), R, y, tol=1e-10, max_iter=400, max_basis=max_basis)
+    for i in range(batch):
+        xi = x[i].clone()
+        e, rn, its, ok = K.davidson1(L[i], w, R[i], xi, tol=1e-10, max_iter=400, max_basis=max_basis)
+        dot = float((xi * y[i]).sum())
+        if ok and abs(dot) > 0.9:
+            assert dot > 0, (i, its)

@@ -761,6 +761,9 @@ int davidson1(const double* L, const double* W, const double* R, double* x_io, i
   // s_prev is valid when it was computed on the basis V[0..k-1) that the current one extends.
   std::vector<double> s_cur(MAXB, 0.0), s_prev(MAXB, 0.0), hm_host(size_t(MAXB) * MAXB, 0.0);
   int cur_k = 0, prev_k = 0;
+  // of every step since the basis began with first_k vectors (settle_sign)
+  std::vector<double> s_hist(size_t(MAXB + 1) * MAXB, 0.0);
+  int first_k = 0;
 
   // Rayleigh-Ritz on V[0..k), Ritz vector x, AV-combination ax, residual norm and the next
   // direction t; reads theta, ||r|| and the Ritz coefficient of V[0] back to the host.
@@ -789,6 +792,7 @@ int davidson1(const double* L, const double* W, const double* R, double* x_io, i
       std::swap(s_prev, s_cur);
       prev_k = cur_k;
       std::copy(hp->s, hp->s + k, s_cur.begin());
+      std::copy(hp->s, hp->s + k, s_hist.begin() + size_t(k) * MAXB);
       cur_k = k;
       theta = hp->theta;
       rnorm = sqrt(fmax(hp->rn2, 0.0));
@@ -817,6 +821,7 @@ int davidson1(const double* L, const double* W, const double* R, double* x_io, i
       set_error("tnx_davidson1: a bounded wait in the tensor-core matvec expired");
       return TNX_ERR_TIMEOUT;
     }
+    std::copy(s_cur.begin(), s_cur.begin() + k, s_hist.begin() + size_t(k) * MAXB);
     theta = host[0];
     rnorm = sqrt(fmax(host[1], 0.0));
     c0 = host[2];
@@ -827,29 +832,59 @@ int davidson1(const double* L, const double* W, const double* R, double* x_io, i
     return TNX_OK;
   };
 
-  // The sign of a Ritz vector that leaves its basis is that of the Jacobi Rayleigh-Ritz step: where
-  // the two steps may differ in it (see rr_lowest_tri), that step and the combination are done again.
+  // The sign of a Ritz vector that leaves its basis is the one it has when the Jacobi sweeps do every
+  // Rayleigh-Ritz step. Theirs is equivariant: with the basis vectors' signs changed by D they give D s D_w, w being
+  // the index at which they leave the lowest value. So with D_j the sign that basis vector j (made from the
+  // Ritz vector of j vectors) has here against there, eta_j = (sign of the sweeps' s against the one used) D_w
+  // is that of the Ritz vector, and D_j = eta_j. Where the largest entry of s settles both (rr_lowest_tri) nothing is
+  // computed; the other steps since the basis began are solved by the sweeps at once, in one launch.
+  // Also sets s_prev's sign (the restart combines it).
   auto settle_sign = [&](const auto& vs) -> int {
     using T = std::remove_pointer_t<decltype(vs.V)>;
-    for (int j = 0; j < cur_k; ++j)
-      if (s_cur[j] * s_cur[j] >= 0.99) return TNX_OK;
-    const std::vector<double> tri(s_cur.begin(), s_cur.begin() + k);
-    for (auto solve : {rr_lowest_f64, rr_lowest_tri}) {
-      TNX_TRY(solve(w.Hm, k, mb, w.evals, w.evecs, st));
-      if (small) {
-        TNX_TRY(ritz_small(vs, k, nullptr));
-      } else {
-        ritz_kernel<T><<<nch, DT, 0, st>>>(vs.V, vs.AV, n, k, w.evecs, w.evals, vs.diag, precond, vs.x, vs.ax, vs.t, n,
-                                           w.part, nch);
-        TNX_LAUNCH_CHECK();
-      }
-      TNX_CUDA(cudaMemcpyAsync(s_cur.data(), w.evecs, size_t(k) * 8, cudaMemcpyDeviceToHost, st));
-      TNX_CUDA(cudaStreamSynchronize(st));
-      // beyond FP32's range, and for a double eigenvalue, the sweeps may end at another vector: not that one
-      double dot = 0.0;
-      for (int j = 0; j < k; ++j) dot += s_cur[j] * tri[j];
-      if (fabs(dot) > 0.5) break;
+    double eta[MAXB + 1], D[MAXB + 1];
+    int w_at[MAXB + 1];
+    RrSizes open;
+    for (int j = 0; j <= k; ++j) D[j] = eta[j] = 1.0;
+    for (int j = first_k + 1; j <= k; ++j) {
+      const double* s = &s_hist[size_t(j) * MAXB];
+      w_at[j] = 0;
+      for (int i = 1; i < j; ++i)
+        if (fabs(s[i]) > fabs(s[w_at[j]])) w_at[j] = i;
+      if (!(s[w_at[j]] * s[w_at[j]] >= 0.99)) open.n[open.count++] = j;
     }
+    if (open.count > 0) {
+      double* vecs = w.jwork;
+      double* where = w.jwork + int64_t(mb) * mb;
+      TNX_TRY(rr_lowest_f64_leading(w.Hm, mb, open, where + mb, vecs, mb, where, st));
+      std::vector<double> got(size_t(open.count) * mb), at(open.count);
+      TNX_CUDA(cudaMemcpyAsync(got.data(), vecs, got.size() * 8, cudaMemcpyDeviceToHost, st));
+      TNX_CUDA(cudaMemcpyAsync(at.data(), where, at.size() * 8, cudaMemcpyDeviceToHost, st));
+      TNX_CUDA(cudaStreamSynchronize(st));
+      for (int b = 0; b < open.count; ++b) {
+        const int j = open.n[b];
+        double dot = 0.0;
+        for (int i = 0; i < j; ++i) dot += got[size_t(b) * mb + i] * s_hist[size_t(j) * MAXB + i];
+        // beyond FP32's range, and for a double eigenvalue, the sweeps may end at another vector: no sign from them
+        if (!(fabs(dot) > 0.5)) continue;
+        w_at[j] = at[b] >= 0.0 && at[b] < j ? int(at[b]) : w_at[j];
+        eta[j] = dot < 0.0 ? -1.0 : 1.0;
+      }
+    }
+    for (int j = first_k + 1; j <= k; ++j) D[j] = eta[j] *= D[w_at[j]];
+    if (prev_k == k - 1 && prev_k > first_k && eta[prev_k] < 0.0)
+      for (int i = 0; i < prev_k; ++i) s_prev[i] = -s_prev[i];
+    if (eta[k] > 0.0) return TNX_OK;
+    for (int i = 0; i < k; ++i) s_cur[i] = -s_cur[i];
+    std::copy(s_cur.begin(), s_cur.begin() + k, s_hist.begin() + size_t(k) * MAXB);  // settled
+    TNX_CUDA(cudaMemcpyAsync(w.evecs, s_cur.data(), size_t(k) * 8, cudaMemcpyHostToDevice, st));
+    if (small) {
+      TNX_TRY(ritz_small(vs, k, nullptr));
+    } else {
+      ritz_kernel<T><<<nch, DT, 0, st>>>(vs.V, vs.AV, n, k, w.evecs, w.evals, vs.diag, precond, vs.x, vs.ax, vs.t, n,
+                                         w.part, nch);
+      TNX_LAUNCH_CHECK();
+    }
+    TNX_CUDA(cudaStreamSynchronize(st));  // s_cur is host memory that the next step rewrites
     return TNX_OK;
   };
 
@@ -923,7 +958,7 @@ int davidson1(const double* L, const double* W, const double* R, double* x_io, i
     TNX_CUDA(cudaMemcpyAsync(vs.AV, vs.ax, n * sizeof(T), cudaMemcpyDeviceToDevice, st));
     restart_kernel<<<1, 1, 0, st>>>(w.Hm, w.evals, w.evecs);
     TNX_LAUNCH_CHECK();
-    k = 1;
+    k = first_k = 1;
     cur_k = prev_k = 0;
     return TNX_OK;
   };
@@ -971,7 +1006,7 @@ int davidson1(const double* L, const double* W, const double* R, double* x_io, i
     const double h2[4] = {theta, h01, h01, h11};
     TNX_CUDA(cudaMemcpy2DAsync(w.Hm, size_t(mb) * 8, h2, 16, 16, 2, cudaMemcpyHostToDevice, st));
     TNX_CUDA(cudaStreamSynchronize(st));  // h2 / sp are host stack memory
-    k = 2;
+    k = first_k = 2;
     cur_k = prev_k = 0;
     return TNX_OK;
   };
@@ -1089,6 +1124,7 @@ int davidson1(const double* L, const double* W, const double* R, double* x_io, i
       ++anchors;
       TNX_TRY(dots(w.V, n, 1, w.AV, n, w.part, w.Hm, 1, nullptr, 0, st));
       k = 1;
+      first_k = 0;
       precond = 1;
       TNX_TRY(rayleigh_ritz(v64));
       double drift = 0.0;  // sum of |c| over restarts inside this anchor

@@ -27,6 +27,7 @@
 // matrices 7.9 and 3.0 ms; one 199 x 199 156 and 128 ms.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "jacobi.cuh"
@@ -357,12 +358,15 @@ constexpr int RR_G = RR_T / 32;
 // FP32 rounding keeps regenerating off-diagonal entries at ~6e-8 |A|_F, so the sweeps
 // stop once every off-diagonal entry is below 1e-6 |A|_F; the FP64 steps take it from there.
 // Block b solves the matrix at A + b sA into eval[b sE], evec + b sV, and returns at
-// once when active is given and active[b] == 0.
+// once when active is given and active[b] == 0. With `sizes` (count > 0), block b solves the leading block
+// of sizes.n[b] rows of A instead of n, and where[b] is the index at which the sweeps left the lowest value.
 __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restrict__ A, int n, int ld,
                                                          double* __restrict__ eval, double* __restrict__ evec,
                                                          int64_t sA, int64_t sE, int64_t sV,
-                                                         const int* __restrict__ active) {
+                                                         const int* __restrict__ active, const RrSizes sizes,
+                                                         double* __restrict__ where) {
   if (active && !active[blockIdx.x]) return;
+  if (sizes.count > 0) n = sizes.n[blockIdx.x];
   A += int64_t(blockIdx.x) * sA;
   eval += int64_t(blockIdx.x) * sE;
   evec += int64_t(blockIdx.x) * sV;
@@ -493,6 +497,7 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restric
   }
   __syncthreads();
   const int imin = s_imin;
+  if (where && tid == 0) where[blockIdx.x] = double(imin);
   for (int i = tid; i < n; i += RR_T) s[i] = double(Vf[i * nf + imin]);
   __syncthreads();
   const float floor = 1e-6f * fro;
@@ -579,28 +584,41 @@ size_t rr_lowest_smem(int n) {
   return size_t(n) * (n + 1) * 16 + size_t(n) * ((1 + RR_G) * 8 + (1 + RR_G) * 4);
 }
 
-int rr_lowest_f64(const double* A, int n, int ld, double* eval, double* evec, cudaStream_t st) {
-  return rr_lowest_f64_batched(A, n, ld, 0, eval, 0, evec, 0, 1, nullptr, st);
-}
-
-int rr_lowest_f64_batched(const double* A, int n, int ld, int64_t sA, double* eval, int64_t sE, double* evec,
-                          int64_t sV, int batch, const int* active, cudaStream_t st) {
+namespace {
+int launch_rr(const double* A, int n, int ld, int64_t sA, double* eval, int64_t sE, double* evec, int64_t sV, int batch,
+              const int* active, const RrSizes& sizes, double* where, cudaStream_t st) {
   if (n > RW_MAX) {
     set_error("rr_lowest_f64: n=%d > %d", n, RW_MAX);
     return TNX_ERR_SHAPE;
   }
   if (batch <= 0) return TNX_OK;
   static std::atomic<bool> attr{false};  // idempotent setup; threads may race to it
-  const size_t smem = rr_lowest_smem(RW_MAX);
   if (!attr.load()) {
-    TNX_CUDA(cudaFuncSetAttribute(rr_lowest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    TNX_CUDA(cudaFuncSetAttribute(rr_lowest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  int(rr_lowest_smem(RW_MAX))));
     attr.store(true);
   }
   profile_mark(KF_EIGH, st, true);
-  rr_lowest_kernel<<<batch, RR_T, rr_lowest_smem(n), st>>>(A, n, ld, eval, evec, sA, sE, sV, active);
+  rr_lowest_kernel<<<batch, RR_T, rr_lowest_smem(n), st>>>(A, n, ld, eval, evec, sA, sE, sV, active, sizes, where);
   profile_mark(KF_EIGH, st, false);
   TNX_LAUNCH_CHECK();
   return TNX_OK;
+}
+}  // namespace
+
+int rr_lowest_f64(const double* A, int n, int ld, double* eval, double* evec, cudaStream_t st) {
+  return launch_rr(A, n, ld, 0, eval, 0, evec, 0, 1, nullptr, RrSizes{}, nullptr, st);
+}
+
+int rr_lowest_f64_batched(const double* A, int n, int ld, int64_t sA, double* eval, int64_t sE, double* evec,
+                          int64_t sV, int batch, const int* active, cudaStream_t st) {
+  return launch_rr(A, n, ld, sA, eval, sE, evec, sV, batch, active, RrSizes{}, nullptr, st);
+}
+
+int rr_lowest_f64_leading(const double* A, int ld, const RrSizes& sizes, double* eval, double* evec, int64_t sV,
+                          double* where, cudaStream_t st) {
+  return launch_rr(A, *std::max_element(sizes.n, sizes.n + sizes.count), ld, 0, eval, 1, evec, sV, sizes.count, nullptr,
+                   sizes, where, st);
 }
 
 }  // namespace tnx
@@ -619,9 +637,9 @@ int rr_lowest_f64_batched(const double* A, int n, int ld, int64_t sA, double* ev
 // FP32 rounding shrinks with r. A random 24 x 24 matrix: 80 us in the kernel above, 27 us here; 64 x 64:
 // 471 and 76 us; the mean over a chi = 32 eigensolve's 68 problems 45 and 20 us.
 //
-// The vector's largest entry is positive. The sweeps above give their vector the same sign where
-// the square of that entry is at least 0.99 (none of 4.7 million random problems of 3 to 24 rows
-// differed; 1 in 13000 did between 0.9 and 0.99).
+// The vector's largest entry is positive. The sweeps above give their vector the same sign, and leave its
+// value at that entry's index, where the square of the entry is at least 0.99 (none of 4.7 million random problems of
+// 3 to 24 rows differed; 1 in 13000 did between 0.9 and 0.99).
 // ---------------------------------------------------------------------------------------
 namespace tnx {
 namespace {

@@ -253,7 +253,15 @@ int eigh_small_f64_uniform(const double* A, int n, int ld, int keep, double* eva
                            double* work, cudaStream_t st);
 // lowest eigenpair of one n x n (n <= 64) matrix: FP32 Jacobi + FP64 refinement
 int rr_lowest_f64(const double* A, int n, int ld, double* eval, double* evec, cudaStream_t st);
-// the same, faster; the vector's sign is by its largest entry
+// leading blocks of sizes.n[b] rows of A at once, b < sizes.count: eval[b], evec + b sV, and in where[b] the index at
+// which the sweeps left the lowest value
+struct RrSizes {
+  int count = 0;
+  int n[64] = {};
+};
+int rr_lowest_f64_leading(const double* A, int ld, const RrSizes& sizes, double* eval, double* evec, int64_t sV,
+                          double* where, cudaStream_t st);
+// the lowest pair, faster; the vector's sign is by its largest entry
 int rr_lowest_tri(const double* A, int n, int ld, double* eval, double* evec, cudaStream_t st);
 // the same for `batch` matrices at A + b sA (results at eval + b sE, evec + b sV); blocks whose
 // active[b] is 0 return at once (active may be null)
