@@ -6,16 +6,17 @@
 //
 // A dense W costs (dl d)(dr d) FMAs per (a', c) fibre: 1.05e8 at chi = 1024, D = 5, which the FP64
 // pipe (2 FMAs per clock and SM) turns into 170 us against 25 us for the bytes. The MPOs of spin
-// chains are mostly zeros (12 of 100 entries for XXZ), so every output keeps a bit mask of its
+// chains are mostly zeros (12 of 100 entries for XXZ), so every output keeps a list of its
 // nonzero coefficients and runs over those only, in the dense order: the result is bit for bit
 // the dense one, because adding a finite value times zero to the sum changes nothing; a tile
 // that holds Inf or NaN takes the dense sum, where 0 * Inf has to give NaN.
 //
 // A lane owns one fibre and reads its inputs coalesced along c, all of them in flight at once;
 // its shared-memory column only makes them indexable, so the loop needs no barrier. The left
-// form's outputs, strided by dr, go out through the warp's shared memory as contiguous rows.
-// chi = 1024, D = 5, left form: 300 us (FP64) with a dense sum over per-thread arrays in local
-// memory, 69 us so; 100 and 45 us for the split-BF16 operand.
+// form's outputs, strided by dr, go out through the warp's shared memory as contiguous rows, in
+// pairs where they lie aligned. Instructions bound it: chi = 1024, D = 5, left form: 300 us (FP64) with a dense sum
+// over per-thread arrays in local memory, 69 us with bit masks and single outputs, 60 us so; 100, 46 and 35 us
+// for the split-BF16 operand.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -40,6 +41,11 @@ __device__ __forceinline__ bool nonzero(float x) { return (__float_as_uint(x) <<
 struct OutF64 {
   double* p;
   __device__ void at(int64_t i, double v) const { p[i] = v; }
+  // outputs i, i + 1 with even i
+  __device__ bool aligned() const { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+  __device__ void two(int64_t i, const double* v) const {
+    *reinterpret_cast<double2*>(p + i) = *reinterpret_cast<const double2*>(v);
+  }
 };
 struct OutSplit {
   __nv_bfloat16 *hi, *lo;
@@ -48,30 +54,46 @@ struct OutSplit {
     hi[i] = h;
     lo[i] = __float2bfloat16_rn(v - __bfloat162float(h));
   }
+  __device__ bool aligned() const {
+    return ((reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo)) & 3) == 0;
+  }
+  __device__ void two(int64_t i, const float* v) const {
+    const float2 x = *reinterpret_cast<const float2*>(v);
+    const __nv_bfloat162 h = __float22bfloat162_rn(x);
+    *reinterpret_cast<__nv_bfloat162*>(hi + i) = h;
+    *reinterpret_cast<__nv_bfloat162*>(lo + i) =
+        __float22bfloat162_rn(make_float2(x.x - __low2float(h), x.y - __high2float(h)));
+  }
 };
 
-// Shared memory of a CTA of nw warps: offsets [64] of the inputs, masks [64], W as [nout][nin], and
-// per warp the inputs [nin][32] and (left form) the outputs [d][32][dr]; nin, nout <= 64
+// Shared memory of a CTA of nw warps: offsets [64] of the inputs, lengths [64] of the lists, coefficients [nout][nin]
+// with their inputs' places, and per warp the inputs [nin][32] and (left form) the outputs [d][32][dr]; nin,
+// nout <= 64
+__host__ __device__ constexpr int list_len(int nin, int nout) { return (nin * nout + 7) / 8 * 8; }
 template <typename T, bool LEFT>
 __host__ __device__ constexpr size_t smem_bytes(int nin, int nout, int nw) {
-  return 64 * 16 + sizeof(T) * (size_t(nin) * nout + size_t(nw) * 32 * (nin + (LEFT ? nout : 0)));
+  return 64 * 12 + (sizeof(T) + 2) * size_t(list_len(nin, nout)) +
+         sizeof(T) * size_t(nw) * 32 * (nin + (LEFT ? nout : 0));
 }
 
 template <typename T, bool LEFT>
 struct Smem {
-  uint64_t* mask;
   int64_t* off;
+  int* cnt;
   T *w, *in, *out;
+  uint16_t* at;  // of each listed coefficient: element of the warp's inputs, 32 t
   __device__ Smem(unsigned char* raw, int nin, int nout, int warp) {
-    mask = reinterpret_cast<uint64_t*>(raw);
-    off = reinterpret_cast<int64_t*>(mask + 64);
-    w = reinterpret_cast<T*>(off + 64);
-    in = w + nin * nout + warp * 32 * (nin + (LEFT ? nout : 0));
+    off = reinterpret_cast<int64_t*>(raw);
+    cnt = reinterpret_cast<int*>(off + 64);
+    const int len = list_len(nin, nout);
+    at = reinterpret_cast<uint16_t*>(cnt + 64);
+    w = reinterpret_cast<T*>(at + len);
+    in = w + len + warp * 32 * (nin + (LEFT ? nout : 0));
     out = in + nin * 32;
   }
 };
 
-// coefficients of output o = (v or w) * d + s' over inputs t = (w or v) * d + s, their masks, and
+// lists of the coefficients of output o = (v or w) * d + s' over inputs t = (w or v) * d + s, and
 // each input's offset from the fibre's first one
 template <bool LEFT, typename T>
 __device__ void load_w(const Smem<T, LEFT>& s, const double* __restrict__ W, int64_t chi_l, int d, int64_t chi_r,
@@ -85,10 +107,16 @@ __device__ void load_w(const Smem<T, LEFT>& s, const double* __restrict__ W, int
     s.off[t] = LEFT ? ((t / d) * chi_l * d + t % d) * chi_r : int64_t((t % d) * dr + t / d) * chi_r;
   __syncthreads();
   for (int o = threadIdx.x; o < nout; o += blockDim.x) {
-    uint64_t m = 0;
-    for (int t = 0; t < nin; ++t)
-      if (nonzero(s.w[o * nin + t])) m |= 1ull << t;
-    s.mask[o] = m;
+    T* w = s.w + o * nin;
+    int n = 0;
+    for (int t = 0; t < nin; ++t) {
+      const T c = w[t];
+      if (nonzero(c)) {
+        w[n] = c;  // n <= t
+        s.at[o * nin + n++] = uint16_t(32 * t);
+      }
+    }
+    s.cnt[o] = n;
   }
   __syncthreads();
 }
@@ -118,13 +146,20 @@ __device__ __forceinline__ bool stage(const Smem<T, LEFT>& s, const T* __restric
 
 template <bool LEFT, typename T>
 __device__ __forceinline__ T combine(const Smem<T, LEFT>& s, int nin, int o, bool dense, int lane) {
-  uint64_t m = dense ? ~0ull >> (64 - nin) : s.mask[o];
   const T* w = s.w + o * nin;
+  const uint16_t* at = s.at + o * nin;
+  const T* in = s.in + lane;
+  const int n = s.cnt[o];
   T acc = T(0);
-  while (m) {
-    const int t = __ffsll(static_cast<long long>(m)) - 1;
-    m &= m - 1;
-    acc = fma(s.in[t * 32 + lane], w[t], acc);
+  if (!dense) {
+#pragma unroll 2
+    for (int i = 0; i < n; ++i) acc = fma(in[at[i]], w[i], acc);
+  } else {
+    for (int t = 0, i = 0; t < nin; ++t) {
+      const bool listed = i < n && at[i] == 32 * t;
+      acc = fma(in[32 * t], listed ? w[i] : T(0), acc);
+      i += listed;
+    }
   }
   return acc;
 }
@@ -149,6 +184,7 @@ __global__ void left_kernel(const T* __restrict__ T1, int64_t sT1, const double*
   const int64_t total = chi_l * chi_r;
   const int qd = 32 / dr, rd = 32 % dr;  // step of (fibre, v) over 32 consecutive outputs
   const int p0 = lane / dr, v0 = lane - p0 * dr;
+  const bool in_pairs = out.aligned() && ((ldp | ob) & 1) == 0;
   for (int64_t i0 = (int64_t(blockIdx.x) * nw + warp) * 32; i0 < total; i0 += int64_t(gridDim.x) * nw * 32) {
     const int64_t idx = i0 + lane;
     const int64_t ap = quot(idx, chi_r), c = idx - ap * chi_r;
@@ -159,6 +195,17 @@ __global__ void left_kernel(const T* __restrict__ T1, int64_t sT1, const double*
     const int np = total - i0 < 32 ? int(total - i0) : 32;
     // the 32 fibres cover c .. c + 31 of row a' and, past the row's end, the start of the next
     const int64_t ap0 = __shfl_sync(0xffffffffu, ap, 0), c0 = __shfl_sync(0xffffffffu, c, 0);
+    if (in_pairs && c0 + np <= chi_r && ((c0 * dr) & 1) == 0) {
+      const int64_t base = ob + ap0 * d * ldp + c0 * dr;
+      for (int sp = 0; sp < d; ++sp) {
+        const T* res = s.out + sp * 32 * dr;
+        int e = 2 * lane;
+        for (; e + 1 < np * dr; e += 64) out.two(base + sp * ldp + e, res + e);
+        if (e < np * dr) out.at(base + sp * ldp + e, res[e]);
+      }
+      __syncwarp();
+      continue;
+    }
     int p = p0, v = v0;
     for (int e = lane; e < np * dr; e += 32) {
       int64_t pc = c0 + p, pa = ap0;
