@@ -329,7 +329,7 @@ int tnx_eigh_batched(double* A, const int64_t* offsets, const int* sizes, int ba
 }  // extern "C"
 
 // ---------------------------------------------------------------------------------------
-// Lowest eigenpair of small symmetric matrices (n <= 64), one CTA of 256 threads each: the
+// Lowest eigenpair of small symmetric matrices (n <= 64), one CTA each (256 threads, 1024 above 32 rows): the
 // Davidson Rayleigh-Ritz problem and the dense effective Hamiltonians of the chain ends.
 //
 // An FP64 instruction holds its sub-partition's pipe for 64 clocks on GB300 (2 FMAs per clock and
@@ -345,21 +345,22 @@ int tnx_eigh_batched(double* A, const int64_t* offsets, const int* sizes, int ba
 // block (pair k, pair l) of A <- J^T A J by one thread, columns first as in the two-pass form, so
 // each entry sees the operations of the two-pass form; a round without a rotation ends at the first
 // barrier. A random 24 x 24 matrix: 211 us with a pass and a barrier each for columns, rows and zeroing,
-// exact divisions and the correction in FP64, 80 us so; 64 x 64: 1.90 ms and 0.47 ms.
+// exact divisions and the correction in FP64, 80 us so; 64 x 64: 1.90 ms and
+// 0.39 ms (0.47 ms by 256 threads).
 // ---------------------------------------------------------------------------------------
 namespace tnx {
 namespace {
 
 constexpr int RW_MAX = 64;
 
-constexpr int RR_T = 256;  // threads of the Rayleigh-Ritz kernel
-constexpr int RR_G = RR_T / 32;
+constexpr int RR_G = 8;  // warps that share a product of the refinement
 
 // FP32 rounding keeps regenerating off-diagonal entries at ~6e-8 |A|_F, so the sweeps
 // stop once every off-diagonal entry is below 1e-6 |A|_F; the FP64 steps take it from there.
 // Block b solves the matrix at A + b sA into eval[b sE], evec + b sV, and returns at
 // once when active is given and active[b] == 0. With `sizes` (count > 0), block b solves the leading block
 // of sizes.n[b] rows of A instead of n, and where[b] is the index at which the sweeps left the lowest value.
+template <int RR_T>
 __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restrict__ A, int n, int ld,
                                                          double* __restrict__ eval, double* __restrict__ evec,
                                                          int64_t sA, int64_t sE, int64_t sV,
@@ -516,7 +517,7 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restric
   };
   for (int step = 0; step < 4; ++step) {
     // y = A s, then |s|^2 and s . y together (n <= 64: the entries sit in warps 0 and 1)
-    for (int i = lane; i < n; i += 32) {
+    for (int i = warp < RR_G ? lane : n; i < n; i += 32) {
       double acc = 0.0;
       for (int j = warp; j < n; j += RR_G) acc = fma(Ad[i * nf + j], s[j], acc);
       rp[warp * n + i] = acc;
@@ -554,7 +555,7 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restric
     if (tid < n) rf[tid] = float(fma(-theta, si, yi) * inv);
     __syncthreads();
     // f_j = (v_j . r) / (l_j - theta); (near-)degenerate partners keep f_j = 0
-    for (int j = lane; j < n; j += 32) {
+    for (int j = warp < RR_G ? lane : n; j < n; j += 32) {
       float acc = 0.f;
       for (int i = warp; i < n; i += RR_G) acc = fmaf(Vf[i * nf + j], rf[i], acc);
       fp[warp * n + j] = acc;
@@ -566,7 +567,7 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restric
       rf[j] = (j != imin && fabsf(den) >= floor) ? dot / den : 0.f;
     }
     __syncthreads();
-    for (int i = lane; i < n; i += 32) {
+    for (int i = warp < RR_G ? lane : n; i < n; i += 32) {
       float acc = 0.f;
       for (int j = warp; j < n; j += RR_G) acc = fmaf(Vf[i * nf + j], rf[j], acc);
       fp[warp * n + i] = acc;
@@ -594,12 +595,16 @@ int launch_rr(const double* A, int n, int ld, int64_t sA, double* eval, int64_t 
   if (batch <= 0) return TNX_OK;
   static std::atomic<bool> attr{false};  // idempotent setup; threads may race to it
   if (!attr.load()) {
-    TNX_CUDA(cudaFuncSetAttribute(rr_lowest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    TNX_CUDA(cudaFuncSetAttribute(rr_lowest_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   int(rr_lowest_smem(RW_MAX))));
     attr.store(true);
   }
   profile_mark(KF_EIGH, st, true);
-  rr_lowest_kernel<<<batch, RR_T, rr_lowest_smem(n), st>>>(A, n, ld, eval, evec, sA, sE, sV, active, sizes, where);
+  // the blocks of a round, (n / 2)^2 of them and n^2 / 4 entries of V twice, by a thread each
+  if (n <= 32)
+    rr_lowest_kernel<256><<<batch, 256, rr_lowest_smem(n), st>>>(A, n, ld, eval, evec, sA, sE, sV, active, sizes, where);
+  else
+    rr_lowest_kernel<1024><<<batch, 1024, rr_lowest_smem(n), st>>>(A, n, ld, eval, evec, sA, sE, sV, active, sizes, where);
   profile_mark(KF_EIGH, st, false);
   TNX_LAUNCH_CHECK();
   return TNX_OK;
@@ -635,7 +640,7 @@ int rr_lowest_f64_leading(const double* A, int ld, const RrSizes& sizes, double*
 // would be below FP64 rounding (two as a rule, six at most). Only s, r, theta and the norm are FP64;
 // the correction's relative error of ~1e-6 is what T and Q leave it anyway. theta gains s . r, whose
 // FP32 rounding shrinks with r. A random 24 x 24 matrix: 80 us in the kernel above, 27 us here; 64 x 64:
-// 471 and 76 us; the mean over a chi = 32 eigensolve's 68 problems 45 and 20 us.
+// 385 and 76 us; the mean over a chi = 32 eigensolve's 68 problems 45 and 20 us.
 //
 // The vector's largest entry is positive. The sweeps above give their vector the same sign, and leave its
 // value at that entry's index, where the square of the entry is at least 0.99 (none of 4.7 million random problems of
