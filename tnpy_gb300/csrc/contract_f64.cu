@@ -7,6 +7,8 @@
 // Every contraction is L x MPS -> MPO -> R split into two GEMMs (K = chi and K = chi*D)
 // around a small dense MPO step (K = D*d), i.e. 4*chi^3*D*d + 2*chi^2*D^2*d^2 flops.
 #include <cooperative_groups.h>
+
+#include <algorithm>
 #include <cuda_runtime.h>
 
 #include <cstring>
@@ -163,12 +165,13 @@ __global__ void __launch_bounds__(NT) gemm_f64_kernel(int64_t M, int64_t N, int6
 struct F64Plan {
   int tile, nsplit;
   int64_t kslice;
+  double clocks;  // estimate
 };
 
 F64Plan f64_plan(int64_t m, int64_t n, int64_t k, int64_t batch) {
   static const int tiles[3] = {64, 32, 16};
   static const int splits[4] = {1, 2, 4, 8};  // 8: the largest portable cluster
-  F64Plan best{64, 1, (k + GB_K - 1) / GB_K * GB_K};
+  F64Plan best{64, 1, (k + GB_K - 1) / GB_K * GB_K, 0.0};
   double best_cost = 1e300;
   for (int t : tiles) {
     const int64_t my = (m + t - 1) / t, nx = (n + t - 1) / t;
@@ -184,7 +187,7 @@ F64Plan f64_plan(int64_t m, int64_t n, int64_t k, int64_t batch) {
       const double cost = waves * (per + t * t / 2.0) + 2000.0 + (s > 1 ? 3000.0 + waves * t * t / 2.0 : 0.0);
       if (cost < best_cost) {
         best_cost = cost;
-        best = {t, s, ks};
+        best = {t, s, ks, cost};
       }
     }
   }
@@ -217,6 +220,15 @@ int launch_f64(bool ta, bool tb, const F64Plan& p, dim3 grid, int64_t m, int64_t
   return TNX_OK;
 }
 }  // namespace
+
+bool f64_cheaper(int64_t m, int64_t n, int64_t k, int nsplit) {
+  // a double-FP32 product of K slices of kc in 32 x 32 tiles: 560 clocks a step of K in a tile's chain, 200 of an SM's
+  // time once several tiles share it; partial sums in memory where split
+  const int64_t kc = (k + nsplit - 1) / nsplit;
+  const double tiles = double((m + 31) / 32) * double((n + 31) / 32) * nsplit;
+  const double df = std::max(560.0, tiles / 152.0 * 200.0) * double(kc) + 4000.0 + (nsplit > 1 ? 6000.0 : 0.0);
+  return f64_plan(m, n, k, 1).clocks < df;
+}
 
 int gemm_f64(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha, const double* A,
              int64_t lda, int64_t sa, const double* B, int64_t ldb, int64_t sb, double beta,
@@ -269,10 +281,11 @@ __global__ void splitk_reduce_kernel(const double* __restrict__ P, int nsplit, i
 
 int gemm_f64_splitk(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha, const double* A, int64_t lda,
                     const double* B, int64_t ldb, double beta, double* C, int64_t ldc, int nsplit, double* part,
-                    cudaStream_t st, bool df) {
-  // FP64 products split K inside gemm_f64 (clusters), without partials in memory
-  if (!df || nsplit <= 1)
-    return gemm_fp64_class(df, ta, tb, m, n, k, alpha, A, lda, 0, B, ldb, 0, beta, C, ldc, 0, 1, st);
+                    cudaStream_t st, bool df, bool alone) {
+  // FP64 products split K inside gemm_f64 (clusters), without partials in memory; `alone`: nothing of note runs beside
+  // the product, so that clusters are scheduled at once
+  if (!df || nsplit <= 1 || (alone && f64_cheaper(m, n, k, nsplit)))
+    return gemm_fp64_class(df && nsplit <= 1, ta, tb, m, n, k, alpha, A, lda, 0, B, ldb, 0, beta, C, ldc, 0, 1, st);
   const int64_t kc = (k + nsplit - 1) / nsplit;
   nsplit = int((k + kc - 1) / kc);
   const int64_t sa = ta ? kc * lda : kc, sb = tb ? kc : kc * ldb;

@@ -710,14 +710,20 @@ PanelPlan plan_panels(int64_t m, bool df) {
   return {QB, 0, false};
 }
 
+// Rows up to which a panel of the FP64-class modes is factored in FP64 all the same: a column's chain is shorter
+// in FP64 instructions than in double-FP32 sequences, and only the update of taller panels is bound by the FP64
+// pipe. 64 columns of 128, 256, 384 and 512 rows: 157, 175, 195 and 214 us against 191, 193, 195 and 195 us.
+constexpr int64_t FP64_PANEL_ROWS = 320;
+
 int factor_panel(const PanelPlan& pp, double* F, int64_t m, int64_t j0, int nb, double* tau, double* T,
                  cudaStream_t st) {
   profile_mark(KF_QR_PANEL, st, true);
   int rc = TNX_OK;
+  const bool df = pp.df && !(pp.nb == 64 && pp.cl == 16 && m - j0 <= FP64_PANEL_ROWS && panel_fits<64, 16, false>(m - j0));
   if (pp.cl == 0) {
     panel_kernel<<<1, QT, 0, st>>>(F, m, j0, nb, tau, T);
     TNX_LAUNCH_CHECK();
-  } else if (pp.df) {
+  } else if (df) {
     rc = pp.nb == 32   ? launch_panel<32, 16, true>(F, m, j0, nb, tau, T, st)
          : pp.cl == 16 ? launch_panel<64, 16, true>(F, m, j0, nb, tau, T, st)
                        : launch_panel<64, 8, true>(F, m, j0, nb, tau, T, st);
@@ -905,6 +911,9 @@ int apply_panel_t(int64_t m, int64_t mp, int nb, int NB, const double* Vp, const
                   void* oz = nullptr, size_t ozb = 0) {
   if (nc <= 0) return TNX_OK;
   const bool on_oz = df && oz && bulk_on_oz(mp, nc);
+  // the small products of tall matrices stay on the FP32 pipe: they run beside a panel's cluster and Ozaki products,
+  // where FP64 ones, in clusters, gained nothing (chi = 1024 gauge move within 1 %); chi = 100 to 300: 10 % faster
+  const bool alone = m <= 1024;
   // Row-major views: C (column-major mp x nc, ld m) is C^T (nc x mp, ld m), V is V^T (nb x mp).
   // W1 (nb x nc) = V^T C  (short output rows, long K: split over K; finer for narrow C)
   if (on_oz) {
@@ -912,13 +921,18 @@ int apply_panel_t(int64_t m, int64_t mp, int nb, int NB, const double* Vp, const
                        ozb, st));
   } else {
     const int ns = nc <= NB ? qr_nsplit_cap(mp, nb, nc, part_cap) : qr_nsplit(mp);
-    TNX_TRY(gemm_f64_splitk(false, true, nb, nc, mp, 1.0, Vp, mp, C, m, 0.0, W1, nc, ns, part, st, df));
+    TNX_TRY(gemm_f64_splitk(false, true, nb, nc, mp, 1.0, Vp, mp, C, m, 0.0, W1, nc, ns, part, st, df, alone));
   }
   // W2 = T^T W1   (T column-major with ld NB is T^T row-major)
-  TNX_TRY(gemm_fp64_class(df, false, false, nb, nc, nb, 1.0, Tp, NB, 0, W1, nc, 0, 0.0, W2, nc, 0, 1, st));
+  if (df && !alone)
+    TNX_TRY(gemm_df64(false, false, nb, nc, nb, 1.0, Tp, NB, 0, W1, nc, 0, 0.0, W2, nc, 0, 1, st, 0, nullptr));
+  else
+    TNX_TRY(gemm_fp64_class(df, false, false, nb, nc, nb, 1.0, Tp, NB, 0, W1, nc, 0, 0.0, W2, nc, 0, 1, st));
   // C -= V W2, i.e. C^T -= W2^T V^T
   if (on_oz) {
     TNX_TRY(gemm_oz_ex(true, false, nc, mp, nb, -1.0, W2, nc, 0, Vp, mp, 0, 1.0, C, m, 0, 1, 1, nullptr, oz, ozb, st));
+  } else if (df && !alone) {
+    TNX_TRY(gemm_df64(true, false, nc, mp, nb, -1.0, W2, nc, 0, Vp, mp, 0, 1.0, C, m, 0, 1, st, 0, nullptr));
   } else {
     TNX_TRY(gemm_fp64_class(df, true, false, nc, mp, nb, -1.0, W2, nc, 0, Vp, mp, 0, 1.0, C, m, 0, 1, st));
   }
@@ -1051,17 +1065,17 @@ int wy_append_panel(int64_t m, int64_t n, int NB, int64_t j0, int nb, const doub
                        QR_OZ_SPLIT, nullptr, y.oz, y.oz_bytes, st));
   } else {
     TNX_TRY(gemm_f64_splitk(false, true, j0, nb, K, 1.0, y.V + j0, m, y.V + j0 * m + j0, m, 0.0, y.S, nb,
-                            qr_nsplit_cap(K, j0, nb, int64_t(QR_SPLIT_MAX) * n * QBMAX), part, st, true));
+                            qr_nsplit_cap(K, j0, nb, int64_t(QR_SPLIT_MAX) * n * QBMAX), part, st, true, false));
   }
   // Y (j0 x nb, ld nb) = S T_p   (op(B)(k, j) = T_p(k, j) = Tp[j NB + k])
-  TNX_TRY(gemm_fp64_class(true, false, true, j0, nb, nb, 1.0, y.S, nb, 0, Tp, NB, 0, 0.0, y.Y, nb, 0, 1, st));
+  TNX_TRY(gemm_df64(false, true, j0, nb, nb, 1.0, y.S, nb, 0, Tp, NB, 0, 0.0, y.Y, nb, 0, 1, st, 0, nullptr));
   // Tf[0:j0, j0:j0+nb] = -Tf[0:j0, 0:j0] Y  (K = j0 long, nb = 64 wide: split over K)
   if (on_oz) {
     TNX_TRY(gemm_oz_ex(false, false, j0, nb, j0, -1.0, y.Tf, n, 0, y.Y, nb, 0, 0.0, y.Tf + j0, n, 0, 1, QR_OZ_SPLIT,
                        nullptr, y.oz, y.oz_bytes, st));
   } else {
     TNX_TRY(gemm_f64_splitk(false, false, j0, nb, j0, -1.0, y.Tf, n, y.Y, nb, 0.0, y.Tf + j0, n,
-                            qr_nsplit_cap(j0, j0, nb, int64_t(QR_SPLIT_MAX) * n * QBMAX), y.part, st, true));
+                            qr_nsplit_cap(j0, j0, nb, int64_t(QR_SPLIT_MAX) * n * QBMAX), y.part, st, true, false));
   }
   return TNX_OK;
 }

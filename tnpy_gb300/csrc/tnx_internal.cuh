@@ -161,6 +161,8 @@ __device__ __forceinline__ void two_sum_f(float a, float b, float& s, float& e) 
   e = (a - (s - bb)) + (b - bb);
 }
 
+// whether the FP64 GEMM is estimated to be faster than the double-FP32 one (in nsplit slices of K)
+bool f64_cheaper(int64_t m, int64_t n, int64_t k, int nsplit = 1);
 // ---- FP64 GEMM (row-major, optional transposes, strided batch) --------------------
 // k_total > 0 selects split-K: batch z multiplies the K slice [z*k, min((z+1)*k, k_total));
 // bmask (device, batch ints, may be null) skips the batch entries whose mask is 0
@@ -172,7 +174,7 @@ int gemm_f64(bool trans_a, bool trans_b, int64_t m, int64_t n, int64_t k, double
 // nsplit * m * n doubles of partial products
 int gemm_f64_splitk(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha, const double* A, int64_t lda,
                     const double* B, int64_t ldb, double beta, double* C, int64_t ldc, int nsplit, double* part,
-                    cudaStream_t st, bool df = false);
+                    cudaStream_t st, bool df = false, bool alone = true);
 // double-FP32 emulated GEMM (same contract as gemm_f64)
 int gemm_df64(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha, const double* A, int64_t lda,
               int64_t sa, const double* B, int64_t ldb, int64_t sb, double beta, double* C, int64_t ldc, int64_t sc,
