@@ -53,7 +53,8 @@ __device__ __forceinline__ double lanes_sum(double v, int top) {
 }
 
 // Power of two that keeps the squares of a column in range: 1 unless alpha^2 + sigma, formed from the
-// entries as they are, comes out below 2^-823 (or zero) or above 2^877
+// entries as they are, comes out below 2^-823 (or zero) or above 2^877. The column is then multiplied by it
+// before the reflector's own factor: the product of the two overflows where the norm is subnormal
 __device__ __forceinline__ double column_factor(double alpha, double sigma) {
   const int ex = (__double2hiint(fma(alpha, alpha, sigma)) >> 20) & 0x7ff;
   return ex < 200 ? 0x1p700 : (ex > 1900 ? 0x1p-600 : 1.0);
@@ -93,9 +94,12 @@ __global__ void __launch_bounds__(QS_T) qr_small_kernel(const double* A, int64_t
       sg = lanes_sum(sg, 16);
     }
     reflector(x[c] * f, sg, beta, t, scale);
-    beta *= f == 1.0 ? 1.0 : (f > 1.0 ? 0x1p-700 : 0x1p600);
-    scale *= f;
-    for (int i = c + 1 + lane; i < m; i += 32) x[i] *= scale;
+    if (f == 1.0) {
+      for (int i = c + 1 + lane; i < m; i += 32) x[i] *= scale;
+    } else {
+      beta *= f > 1.0 ? 0x1p-700 : 0x1p600;
+      for (int i = c + 1 + lane; i < m; i += 32) x[i] = x[i] * f * scale;
+    }
     __syncwarp();
     if (lane == 0) {
       x[c] = beta;
@@ -147,7 +151,8 @@ __global__ void __launch_bounds__(QS_T) qr_small_kernel(const double* A, int64_t
             if (r > 0 || lane > 0) sg = fma(xr[r] * f, xr[r] * f, sg);
           reflector(alpha * f, lanes_sum(sg, 16), beta, t, scale);
           beta *= f > 1.0 ? 0x1p-700 : 0x1p600;
-          scale *= f;
+#pragma unroll
+          for (int r = 0; r < QS_R; ++r) xr[r] *= f;  // the pivot's entry becomes beta below
         }
 #pragma unroll
         for (int r = 0; r < QS_R; ++r)
