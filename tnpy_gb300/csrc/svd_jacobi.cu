@@ -13,7 +13,7 @@
 // (a zero column pads odd n): each of the ne - 1 rounds rotates ne / 2 disjoint pairs, one CTA
 // per pair; a sweep is ne - 1 launches, and sweeps repeat until a sweep rotates no pair
 // (|g| <= tol sqrt(a b), tol = sqrt(m) * 2^-52) or 40 sweeps pass. The host reads one counter
-// per sweep. Working copies are column-major so that every column is contiguous.
+// and one mark per sweep. Working copies are column-major so that every column is contiguous.
 //
 // What bounds it: the chain of one pair, an FP64 instruction holding its sub-partition's pipe for 64
 // clocks a warp, and the launches. A pair takes four warps (eight above 1024 rows), one to each
@@ -66,7 +66,78 @@ __device__ __forceinline__ void pair_of(int round, int k, int ne, int& p, int& q
   }
 }
 
+// Sums over the CTA of the threads' a, b and g: in lane l of every warp, that of a (l mod 4 = 0), g (1 and 3) or b (2)
 template <int WARPS>
+__device__ __forceinline__ double pair_sums(double a, double b, double g, double (&red)[WARPS][4]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  // lanes 0-15 go on with a, 16-31 with b, then every other eight of them with g
+  const bool hi = lane & 16, mid = lane & 8;
+  double x = hi ? b : a;
+  const double give = hi ? a : b;
+  x += __shfl_xor_sync(0xffffffffu, give, 16);
+  g += __shfl_xor_sync(0xffffffffu, g, 16);
+  double z = mid ? g : x;
+  const double give2 = mid ? x : g;
+  z += __shfl_xor_sync(0xffffffffu, give2, 8);
+  for (int o = 4; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+  if ((lane & 7) == 0) red[w][lane >> 3] = z;  // 0: a, 1 and 3: g, 2: b
+  __syncthreads();
+  double sum = red[0][lane & 3];
+#pragma unroll
+  for (int i = 1; i < WARPS; ++i) sum += red[i][lane & 3];
+  return sum;
+}
+__device__ __forceinline__ void pair_share(double sum, double& a, double& b, double& g) {
+  a = __shfl_sync(0xffffffffu, sum, 0);
+  g = __shfl_sync(0xffffffffu, sum, 1);
+  b = __shfl_sync(0xffffffffu, sum, 2);
+}
+
+// x <- c x - s y, y <- s x + c y
+template <int T>
+__device__ __forceinline__ void turn(double* xs, double* ys, int64_t n, double c, double s) {
+#pragma unroll 4
+  for (int64_t i = threadIdx.x; i < n; i += T) {
+    const double x = xs[i], y = ys[i];
+    xs[i] = fma(c, x, -s * y);
+    ys[i] = fma(s, x, c * y);
+  }
+}
+
+// A squared norm below 2^-TINY_EXP: their product with the tolerance may leave the normal range, and the sums may have
+// lost bits to it. Where neither column is longer than 2^-150 the sums are taken again of the columns times 2^600
+// (the angle does not change); otherwise g is well inside the range. FP64 roots and divisions: a rare case, in an
+// instantiation of its own (47 registers against 32) that takes over once a sweep has met such a pair.
+constexpr int TINY_EXP = 800;
+template <int WARPS>
+__device__ __forceinline__ void tiny_pair(double a, double b, double g, double* cp, double* cq, int64_t m, double* vp,
+                                       double* vq, int ne, float tol, int* rotated, double (&red)[WARPS][4]) {
+  constexpr int T = 32 * WARPS;
+  if (fmax(a, b) < 0x1p-300) {
+    a = b = g = 0.0;
+    for (int64_t i = threadIdx.x; i < m; i += T) {
+      const double x = cp[i] * 0x1p600, y = cq[i] * 0x1p600;
+      a = fma(x, x, a);
+      b = fma(y, y, b);
+      g = fma(x, y, g);
+    }
+    __syncthreads();  // red has been read by all
+    pair_share(pair_sums<WARPS>(a, b, g, red), a, b, g);
+  }
+  if (!(fabs(g) > double(tol) * sqrt(a) * sqrt(b))) return;
+  // t = tan(theta): the smaller root of t^2 + 2 zeta t - 1 = 0, zeta = (b - a) / (2 g)
+  const double zeta = (b - a) / (2.0 * g), az = fabs(zeta);
+  const double t = copysign(az > 1e100 ? 0.5 / az : 1.0 / (az + sqrt(fma(zeta, zeta, 1.0))), zeta);
+  const double c = 1.0 / sqrt(fma(t, t, 1.0)), s = c * t;
+  if (jac::bits(s) == 0) return;
+  if (threadIdx.x == 0) atomicAdd(rotated, 1);
+  turn<T>(cp, cq, m, c, s);
+  if (vp) turn<T>(vp, vq, ne, c, s);
+}
+
+// rotated[0]: rotations of the sweep; rotated[TINY_AT]: set where a pair was left to the form with TINY
+constexpr int TINY_AT = 2;
+template <int WARPS, bool TINY>
 __global__ void __launch_bounds__(32 * WARPS) jac_round_kernel(double* __restrict__ C, int64_t m,
                                                               double* __restrict__ V, int ne, int round, float tol,
                                                               int* __restrict__ rotated) {
@@ -85,34 +156,25 @@ __global__ void __launch_bounds__(32 * WARPS) jac_round_kernel(double* __restric
     b = fma(y, y, b);
     g = fma(x, y, g);
   }
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  {
-    // lanes 0-15 go on with a, 16-31 with b, then every other eight of them with g
-    const bool hi = lane & 16, mid = lane & 8;
-    double x = hi ? b : a;
-    const double give = hi ? a : b;
-    x += __shfl_xor_sync(0xffffffffu, give, 16);
-    g += __shfl_xor_sync(0xffffffffu, g, 16);
-    double z = mid ? g : x;
-    const double give2 = mid ? x : g;
-    z += __shfl_xor_sync(0xffffffffu, give2, 8);
-    for (int o = 4; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
-    if ((lane & 7) == 0) red[w][lane >> 3] = z;  // 0: a, 1 and 3: g, 2: b
-  }
-  __syncthreads();
-  double sum = red[0][lane & 3];
-#pragma unroll
-  for (int i = 1; i < WARPS; ++i) sum += red[i][lane & 3];
+  const double sum = pair_sums<WARPS>(a, b, g, red);
   // the next round's CTAs come in now and wait; triggered any earlier, several rounds of them pile up
   // (1024 columns: 330 against 105 ms)
   asm volatile("griddepcontrol.launch_dependents;");
-  a = __shfl_sync(0xffffffffu, sum, 0);
-  g = __shfl_sync(0xffffffffu, sum, 1);
-  b = __shfl_sync(0xffffffffu, sum, 2);
+  pair_share(sum, a, b, g);
   // |g| > tol sqrt(a b) in FP32, a and b scaled into [1, 4) by even powers of two and g to match; a
-  // squared norm of zero (or subnormal) has no direction to rotate
+  // squared norm of zero has no direction to rotate
   const int xa = (__double2hiint(a) >> 20) & 0x7ff, xb = (__double2hiint(b) >> 20) & 0x7ff;
-  if (xa == 0 || xb == 0 || xa == 2047 || xb == 2047 || jac::bits(g) == 0) return;
+  constexpr int LOW = 1023 - TINY_EXP;
+  if (xa < LOW || xb < LOW || xa == 2047 || xb == 2047 || jac::bits(g) == 0) {
+    if (min(xa, xb) < LOW && max(xa, xb) < 2047 && jac::bits(a) != 0 && jac::bits(b) != 0) {
+      if constexpr (TINY)
+        tiny_pair<WARPS>(a, b, g, cp, cq, m, V ? V + int64_t(p) * ne : nullptr, V ? V + int64_t(q) * ne : nullptr, ne,
+                         tol, rotated, red);
+      else if (threadIdx.x == 0)
+        rotated[TINY_AT] = 1;
+    }
+    return;
+  }
   const int ea = (xa - 1023) & ~1, eb = (xb - 1023) & ~1;
   const float fa = jac::to_float(jac::scale_exp(a, ea)), fb = jac::to_float(jac::scale_exp(b, eb));
   const float fg = fabsf(jac::to_float(jac::scale_exp(g, (ea + eb) / 2)));
@@ -120,22 +182,8 @@ __global__ void __launch_bounds__(32 * WARPS) jac_round_kernel(double* __restric
   double t, c, s;
   jac::angle(g, b - a, t, c, s);
   if (threadIdx.x == 0) atomicAdd(rotated, 1);
-#pragma unroll 4
-  for (int64_t i = threadIdx.x; i < m; i += T) {
-    const double x = cp[i], y = cq[i];
-    cp[i] = fma(c, x, -s * y);
-    cq[i] = fma(s, x, c * y);
-  }
-  if (V) {
-    double* vp = V + int64_t(p) * ne;
-    double* vq = V + int64_t(q) * ne;
-#pragma unroll 4
-    for (int i = threadIdx.x; i < ne; i += T) {
-      const double x = vp[i], y = vq[i];
-      vp[i] = fma(c, x, -s * y);
-      vq[i] = fma(s, x, c * y);
-    }
-  }
+  turn<T>(cp, cq, m, c, s);
+  if (V) turn<T>(V + int64_t(p) * ne, V + int64_t(q) * ne, ne, c, s);
 }
 
 // flip[0] = 1 where the strict upper triangle of the square A carries more of its squared norm than the
@@ -180,21 +228,31 @@ __global__ void __launch_bounds__(1024) jac_orient_kernel(const double* __restri
   }
 }
 
-// sigma_j = |c_j| for j < n
+// sigma_j = |c_j| for j < n, squared times 2^600 where the squares leave the normal range
 __global__ void __launch_bounds__(JT) jac_norms_kernel(const double* __restrict__ C, int64_t m,
                                                       double* __restrict__ sig) {
   __shared__ double red[JT / 32];
   const double* c = C + int64_t(blockIdx.x) * m;
-  double a = 0.0;
-  for (int64_t i = threadIdx.x; i < m; i += JT) a = fma(c[i], c[i], a);
-  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = a;
-  __syncthreads();
-  if (threadIdx.x == 0) {
+  auto sum_of_squares = [&](double f) {
+    double a = 0.0;
+    for (int64_t i = threadIdx.x; i < m; i += JT) {
+      const double x = c[i] * f;
+      a = fma(x, x, a);
+    }
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = a;
+    __syncthreads();
     double t = 0.0;
     for (int i = 0; i < JT / 32; ++i) t += red[i];
-    sig[blockIdx.x] = sqrt(t);
+    return t;
+  };
+  double t = sum_of_squares(1.0), back = 1.0;
+  if (t > 0.0 && t < 0x1p-900) {
+    __syncthreads();
+    t = sum_of_squares(0x1p600);
+    back = 0x1p-600;
   }
+  if (threadIdx.x == 0) sig[blockIdx.x] = sqrt(t) * back;
 }
 
 // order[rank] = j, descending sigma (ties by index): one CTA, rank by counting
@@ -300,17 +358,26 @@ int tnx_svd(const double* A, int64_t m, int64_t n, double* S, double* U, double*
   cfg.attrs = at;
   int sweeps = 0, host_count = 1;
   if (ne >= 2) {
+    auto kernel = m > 1024 ? jac_round_kernel<8, false> : jac_round_kernel<4, false>;
+    bool tiny = false;
+    TNX_CUDA(cudaMemsetAsync(w.counter + TINY_AT, 0, sizeof(int), st));
     for (; sweeps < kMaxSweeps && host_count > 0; ++sweeps) {
       TNX_CUDA(cudaMemsetAsync(w.counter, 0, sizeof(int), st));
       for (int r = 0; r < ne - 1; ++r) {
         // the first round follows a memset or another kernel: plain stream order
         cfg.numAttrs = r > 0 ? 1 : 0;
-        TNX_CUDA(m > 1024 ? cudaLaunchKernelEx(&cfg, jac_round_kernel<8>, w.C, m, w.V, ne, r, tol, w.counter)
-                          : cudaLaunchKernelEx(&cfg, jac_round_kernel<4>, w.C, m, w.V, ne, r, tol, w.counter));
+        TNX_CUDA(cudaLaunchKernelEx(&cfg, kernel, w.C, m, w.V, ne, r, tol, w.counter));
         TNX_LAUNCH_CHECK();
       }
-      TNX_CUDA(cudaMemcpyAsync(&host_count, w.counter, sizeof(int), cudaMemcpyDeviceToHost, st));
+      int seen[TINY_AT + 1];
+      TNX_CUDA(cudaMemcpyAsync(seen, w.counter, sizeof(seen), cudaMemcpyDeviceToHost, st));
       TNX_CUDA(cudaStreamSynchronize(st));
+      host_count = seen[0];
+      if (!tiny && seen[TINY_AT]) {  // a sweep without rotations has left these pairs out
+        tiny = true;
+        kernel = m > 1024 ? jac_round_kernel<8, true> : jac_round_kernel<4, true>;
+        host_count = 1;
+      }
     }
   }
   jac_norms_kernel<<<int(n), JT, 0, st>>>(w.C, m, w.sig);
