@@ -236,10 +236,7 @@ __global__ void __launch_bounds__(EJ_THREADS) jacobi_eigh_kernel(
   }
   // ascending order: rank of each diagonal entry (ties broken by index), by its sortable bits
   __shared__ int16_t rank[EJ_MAX_N];
-  auto key = [&](int i) {
-    long long k = __double_as_longlong(A[i * ld + i] + 0.0);  // -0 becomes +0
-    return k < 0 ? k ^ 0x7fffffffffffffffLL : k;
-  };
+  auto key = [&](int i) { return jac::sort_key(A[i * ld + i]); };
   double* ev_out = evals + size_t(b) * keep;
   double* vec_out = evecs + size_t(b) * max_size * keep;
   for (int i = tid; i < n; i += nt) {

@@ -46,6 +46,16 @@ __device__ __forceinline__ unsigned long long bits(float x) {
   return __float_as_uint(x) << 1;
 }
 
+// integer in the order of x, +-0 equal; NaN beyond the infinities, so that ranks by it are always a permutation
+__device__ __forceinline__ long long sort_key(double x) {
+  const long long k = bits(x) == 0 ? 0 : __double_as_longlong(x);
+  return k < 0 ? k ^ 0x7fffffffffffffffLL : k;
+}
+__device__ __forceinline__ int sort_key(float x) {
+  const int k = bits(x) == 0 ? 0 : __float_as_int(x);
+  return k < 0 ? k ^ 0x7fffffff : k;
+}
+
 // 1 / sqrt(d) for d in FP32's normal range: FP32 seed and one third-order step (error 2^-66 before
 // the last rounding), five FP64 instructions
 __device__ __forceinline__ double rsqrt_exact(double d) {

@@ -421,10 +421,11 @@ __device__ void small_eigh(KSmall<T>& s, int n) {
   if (pending) update_v(u ^ 1, warp, NW);
   if (tid < n) {
     const T di = G[tid * GL + tid];
-    int rank = 0;
+    const auto ki = jac::sort_key(di);
+    int rank = 0;  // by integer keys: order[] is complete also where G holds NaN
     for (int j = 0; j < n; ++j) {
-      const T dj = G[j * GL + j];
-      rank += (dj < di) || (dj == di && j < tid);
+      const auto kj = jac::sort_key(G[j * GL + j]);
+      rank += (kj < ki) || (kj == ki && j < tid);
     }
     s.order[rank] = tid;
     s.theta[rank] = di;
