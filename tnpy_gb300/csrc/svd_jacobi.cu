@@ -255,14 +255,15 @@ __global__ void __launch_bounds__(JT) jac_norms_kernel(const double* __restrict_
   if (threadIdx.x == 0) sig[blockIdx.x] = sqrt(t) * back;
 }
 
-// order[rank] = j, descending sigma (ties by index): one CTA, rank by counting
+// order[rank] = j, descending sigma (ties by index): one CTA, rank by counting, by integer keys so that order[] is
+// complete also where a sigma is NaN
 __global__ void jac_rank_kernel(const double* __restrict__ sig, int n, int* __restrict__ order) {
   for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    const double sj = sig[j];
+    const long long kj = jac::sort_key(sig[j]);
     int r = 0;
     for (int i = 0; i < n; ++i) {
-      const double si = sig[i];
-      r += (si > sj) || (si == sj && i < j);
+      const long long ki = jac::sort_key(sig[i]);
+      r += (ki > kj) || (ki == kj && i < j);
     }
     order[r] = j;
   }
