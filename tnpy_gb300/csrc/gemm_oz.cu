@@ -116,15 +116,6 @@ __global__ void __launch_bounds__(256) oz_rowmax_kernel(const double* __restrict
 
 __device__ __forceinline__ int row_scale_exp(int bmax) { return bmax > 0 ? bmax - 1021 : 0; }
 
-// x 2^e by integer arithmetic on the exponent where x and the result are normal (exact), ldexp
-// (rounded to a subnormal, zero, Inf) otherwise: an FP64 multiplication holds the pipe for 64 clocks a warp
-__device__ __forceinline__ double scale_pow2(double x, int e) {
-  const int hi = __double2hiint(x), ex = (hi >> 20) & 0x7ff;
-  if (ex != 0 && ex != 2047 && ex + e > 0 && ex + e < 2047)
-    return __hiloint2double(hi + (e << 20), __double2loint(x));
-  return ldexp(x, e);
-}
-
 // planes[s][r][k] (row pitch Kp, rows_pad rows per plane) = slice s of X(r, k) 2^-E[r];
 // zero for r >= rows or k >= K.
 //

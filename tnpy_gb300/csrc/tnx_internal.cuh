@@ -151,6 +151,15 @@ __device__ __forceinline__ double float_to_double(float x) {
                          : __hiloint2double(int((u & 0x80000000u) | ((m >> 3) + base)), int(m << 29));
 }
 
+// x 2^e by integer arithmetic on the exponent where x and the result are normal (exact), ldexp
+// (rounded to a subnormal, zero, Inf) otherwise: an FP64 multiplication holds the pipe for 64 clocks a warp
+__device__ __forceinline__ double scale_pow2(double x, int e) {
+  const int hi = __double2hiint(x), ex = (hi >> 20) & 0x7ff;
+  if (ex != 0 && ex != 2047 && ex + e > 0 && ex + e < 2047)
+    return __hiloint2double(hi + (e << 20), __double2loint(x));
+  return ldexp(x, e);
+}
+
 // (h, l) -> the nearest double of h + l (two conversions and one FP64 add)
 __device__ __forceinline__ double join_df(float h, float l) { return double(h) + double(l); }
 

@@ -66,6 +66,7 @@ struct KSmall {
   int16_t sp[2][KP / 2], sq[2][KP / 2];
   int order[KP];
   int flag, any[2], rot;
+  int ea[KD], eb[KD], eh;  // A_w is taken as A_w 2^-ea[w], B_w as B_w 2^-eb[w], H as H 2^-eh: eh = ea[w] + eb[w]
 };
 
 // operands of the products, padded with zeros to W x W: At[w][b1][k1] = A_w[k1][b1],
@@ -593,14 +594,53 @@ __device__ __forceinline__ float hash_unit(uint32_t a, uint32_t b, uint32_t c) {
   return float(h) * (2.0f / 4294967296.0f) - 1.0f;
 }
 
-// A_w = W1[0, w] and B_w = W2[w, dr2 - 1] as padded operands of type T
-template <typename T, int W>
-__device__ Ops<T> load_ops(const double* W1, const double* W2, int m1, int m2, int dr2, int D, T* mem) {
+// Powers of two that bring H to the order of one, so that no Hamiltonian is out of FP32's range: the largest A_w
+// (x) B_w, by its exponents, becomes one. Exact, and every step of the solvers is homogeneous in H. A term with a zero
+// factor is dropped.
+template <typename T>
+__device__ void scale_ops(KSmall<T>& s, const double* W1, const double* W2, int m1, int m2, int dr2, int D) {
+  auto field = [](double x) { return (__double2hiint(x) >> 20) & 0x7ff; };
+  for (int i = threadIdx.x; i < KD; i += KT) s.ea[i] = s.eb[i] = 0;
+  __syncthreads();
+  for (int w = 0; w < D; ++w) {
+    const double* a = W1 + size_t(w) * m1 * m1;  // row 0 of W1
+    const double* b = W2 + (size_t(w) * dr2 + dr2 - 1) * m2 * m2;
+    int xa = 0, xb = 0;
+    for (int e = threadIdx.x; e < m1 * m1; e += KT) xa = max(xa, field(a[e]));
+    for (int e = threadIdx.x; e < m2 * m2; e += KT) xb = max(xb, field(b[e]));
+    xa = __reduce_max_sync(0xffffffffu, xa);
+    xb = __reduce_max_sync(0xffffffffu, xb);
+    if ((threadIdx.x & 31) == 0) {
+      atomicMax(&s.ea[w], xa);
+      atomicMax(&s.eb[w], xb);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int e = -5000;
+    for (int w = 0; w < D; ++w)
+      if (s.ea[w] && s.eb[w]) e = max(e, s.ea[w] + s.eb[w] - 2046);
+    s.eh = e == -5000 ? 0 : e;
+    for (int w = 0; w < D; ++w) {
+      const bool zero = !s.ea[w] || !s.eb[w];
+      s.ea[w] = zero ? 5000 : s.ea[w] - 1023;
+      s.eb[w] = zero ? 5000 : s.eh - s.ea[w];
+    }
+  }
+  __syncthreads();
+}
+
+// A_w = W1[0, w] and B_w = W2[w, dr2 - 1], scaled by scale_ops, as padded operands of type T
+template <typename T, int W, typename S>
+__device__ Ops<T> load_ops(const KSmall<S>& s, const double* W1, const double* W2, int m1, int m2, int dr2, int D,
+                           T* mem) {
   T* bt = mem + D * W * W;
   for (int e = threadIdx.x; e < D * W * W; e += KT) {
     const int w = e / (W * W), b = e / W % W, k = e % W;
-    mem[e] = (b < m1 && k < m1) ? T(W1[(size_t(w) * m1 + k) * m1 + b]) : T(0);  // row 0 of W1
-    bt[e] = (b < m2 && k < m2) ? T(W2[((size_t(w) * dr2 + dr2 - 1) * m2 + k) * m2 + b]) : T(0);
+    const double x = (b < m1 && k < m1) ? W1[(size_t(w) * m1 + k) * m1 + b] : 0.0;  // row 0 of W1
+    const double y = (b < m2 && k < m2) ? W2[((size_t(w) * dr2 + dr2 - 1) * m2 + k) * m2 + b] : 0.0;
+    mem[e] = jac::bits(x) == 0 ? T(0) : T(scale_pow2(x, -s.ea[w]));
+    bt[e] = jac::bits(y) == 0 ? T(0) : T(scale_pow2(y, -s.eb[w]));
   }
   __syncthreads();
   return {mem, bt, m1, m2, D};
@@ -694,7 +734,7 @@ __host__ __device__ constexpr size_t scratch_elems(int max_m, bool lanczos) {
 static_assert(2 * KP * GL + KP <= NW * TILE && KM1 * KM1 <= NW * TILE, "scratch of the small problems");
 
 // FP32 subspace iteration; `nout` of the Ritz vectors go to `out` (FP64, vector-major) and the filter's
-// upper bound to bound[b].
+// upper bound (of the scaled H) to bound[b].
 template <int W>
 __device__ void chfsi(const Team& tm, const double* W1, const double* W2, int m1, int m2, int dr2, int k, int p, int D,
                       int b, float* X, float* Y, int max_outer, int degree, double* out, int nout, float* bound,
@@ -702,7 +742,8 @@ __device__ void chfsi(const Team& tm, const double* W1, const double* W2, int m1
   KSmall<float>& s = *reinterpret_cast<KSmall<float>*>(raw);
   float* mem = reinterpret_cast<float*>(raw + (sizeof(KSmall<float>) + 15) / 16 * 16);
   const int m = m1 * m2;
-  const Ops<float> o = load_ops<float, W>(W1, W2, m1, m2, dr2, D, mem);
+  scale_ops(s, W1, W2, m1, m2, dr2, D);
+  const Ops<float> o = load_ops<float, W>(s, W1, W2, m1, m2, dr2, D, mem);
   float* tiles = mem + ops_elems(W, D);
   const float ub = upper_bound<W>(s, o, b, tiles, tiles + scratch_elems<float>(0, false));
   auto orthonormal = [&] {  // one vector after the other: the first CTA's
@@ -831,7 +872,8 @@ __device__ void polish(const Team& tm, const double* W1, const double* W2, int m
   KSmall<double>& s = *reinterpret_cast<KSmall<double>*>(raw);
   double* mem = reinterpret_cast<double*>(raw + (sizeof(KSmall<double>) + 15) / 16 * 16);
   const int m = m1 * m2;
-  const Ops<double> o = load_ops<double, W>(W1, W2, m1, m2, dr2, D, mem);
+  scale_ops(s, W1, W2, m1, m2, dr2, D);
+  const Ops<double> o = load_ops<double, W>(s, W1, W2, m1, m2, dr2, D, mem);
   double* tiles = mem + ops_elems(W, D);
   float* fmem = reinterpret_cast<float*>(tiles);  // FP32 operands and tiles of the corrections
   int it = 0;
@@ -869,7 +911,7 @@ __device__ void polish(const Team& tm, const double* W1, const double* W2, int m
     if (s.flag) break;
     tm.sync();
     const double a = s.theta[p - 1], c = 0.5 * (a + double(ub)), h = 0.5 * (double(ub) - a) + 1e-30;
-    const Ops<float> of = load_ops<float, W>(W1, W2, m1, m2, dr2, D, fmem);
+    const Ops<float> of = load_ops<float, W>(s, W1, W2, m1, m2, dr2, D, fmem);
     float* ftiles = fmem + ops_elems(W, D);
     const float cf = float(c), ih = float(1.0 / h);
     for_vectors<float, W>(tm, p, ftiles, [&](int j, bool live, int sl, float* tile) {
@@ -929,7 +971,7 @@ __device__ void polish(const Team& tm, const double* W1, const double* W2, int m
     tm.sync();
   }
   if (tm.rank == 0) {
-    if (threadIdx.x < k) ev[threadIdx.x] = s.theta[threadIdx.x];
+    if (threadIdx.x < k) ev[threadIdx.x] = scale_pow2(s.theta[threadIdx.x], s.eh);
     for (int e = threadIdx.x; e < k * m; e += KT) {
       const int row = e / k, i = e % k;
       out[size_t(row) * keep + i] = X[size_t(i) * m + row];
@@ -968,7 +1010,8 @@ template <int W>
 __device__ void ritz64(const Team& tm, KSmall<double>& s, const double* W1, const double* W2, int m1, int m2, int dr2,
                        int k, int D, double* V, double* Z, double* mem) {
   const int m = m1 * m2;
-  const Ops<double> o = load_ops<double, W>(W1, W2, m1, m2, dr2, D, mem);
+  scale_ops(s, W1, W2, m1, m2, dr2, D);
+  const Ops<double> o = load_ops<double, W>(s, W1, W2, m1, m2, dr2, D, mem);
   double* tiles = mem + ops_elems(W, D);
   orthonormalise(s, V, k, m, tiles);
   apply_block<double, W>(tm, o, V, Z, k, tiles);
@@ -1001,7 +1044,7 @@ __global__ void __launch_bounds__(KT) kron_refine_kernel(const double* const* __
   else
     ritz64<32>(tm, s, w1s[b], w2s[b], m1, m2, dr2, k, D, V, Zb, mem);
   double* ev = evals + size_t(b) * keep;
-  for (int i = threadIdx.x; i < k; i += KT) ev[i] = s.theta[i];
+  for (int i = threadIdx.x; i < k; i += KT) ev[i] = scale_pow2(s.theta[i], s.eh);
   double* out = evecs + size_t(b) * max_m * keep;  // [max_m][keep], like tnx_eigh_batched
   for (int e = threadIdx.x; e < k * m; e += KT) {
     const int row = e / k, i = e % k;
