@@ -30,7 +30,7 @@
 // shares a block while the batch leaves SMs idle: 7.7 ms and 168 ms; 4 blocks of m = 1024 1139 and
 // 19 ms. FP64-class precisions (FP32 stage and one Rayleigh-Ritz): 16 blocks 15.8 and 3.9 ms.
 //
-// A product runs one vector (or two, for nodes of at most 16 states) per warp: the lane holds column
+// A product runs one vector (two, for nodes of at most 16 states; four, where one has at most 8) per warp: the lane holds column
 // b2 of X in registers, T = A_w X with A_w read as broadcast vectors, T is turned around through
 // the warp's shared-memory tile, and the lane then holds row k1 of T and of the sum of T B_w^T. A
 // whole filter runs in registers without touching memory in between.
@@ -69,12 +69,17 @@ struct KSmall {
   int ea[KD], eb[KD], eh;  // A_w is taken as A_w 2^-ea[w], B_w as B_w 2^-eb[w], H as H 2^-eh: eh = ea[w] + eb[w]
 };
 
+// A vector as the matrix that a product takes: nr rows (in registers) by nc columns (on lanes), entry (i, j) at
+// i si + j sj. X itself, or X^T where that has the fewer columns.
+struct Shape {
+  int nr, nc, si, sj;
+};
 // operands of the products, padded with zeros to W x W: At[w][b1][k1] = A_w[k1][b1],
-// Bt[w][b2][k2] = B_w[k2][b2]; W = 16 or 32 >= m1, m2
+// Bt[w][b2][k2] = B_w[k2][b2]; W = 16 or 32 >= nr, nc (of X^T: B_w and A_w)
 template <typename T>
-struct Ops {
+struct Ops : Shape {
   const T *at, *bt;
-  int m1, m2, D;
+  int D;
 };
 constexpr int ops_elems(int W, int D) { return 2 * D * W * W; }
 
@@ -139,98 +144,144 @@ __device__ __forceinline__ void load4(const double* p, double (&o)[4]) {
   o[0] = q.x; o[1] = q.y; o[2] = r.x; o[3] = r.y;
 }
 
-// y = sum A_w X B_w^T over w = w0, w0 + wstep, ... for the vector(s) of one warp. W = 16: lanes
-// 0-15 and 16-31 hold a vector each; sl: lane within W; x[b1], y[k1] of column sl; tile: W x (W + 1).
-// Everything runs over the padded W, so that the loads of a step are in flight together.
-template <typename T, int W>
+// How a warp takes vectors: W rows in registers, L lanes a vector, 32 / L vectors at once
+template <int W, int L>
+__device__ __forceinline__ constexpr int tile_stride() { return W == L ? W * (W + 1) : W * L + 8; }
+
+// y = sum A_w X B_w^T over w = w0, w0 + wstep, ... for the vector(s) of one warp; x[b1], y[k1] of column sl =
+// lane mod L; tile: the vector's. With L = W the lane turns to row sl of T = A_w X for the second product and back at
+// the end; with fewer lanes (L = 8) it stays with its column and reads T's rows from the tile. FULL runs over the
+// padded W, so that all loads of a step are in flight together; otherwise the sums and rows stop at the
+// dimensions, eight at a time. Padded to 32 x 32, a (24, 4) pair took over three times its operations, one vector a
+// warp: 600 pairs, 32 kept, FP64-class 52 ms so and 17 ms with L = 8, FP64 245 and 61 ms; 200 of (17, 17) 34 and 21 ms with
+// bounds; 32 x 32 in FP64 is 9 % faster padded, in FP32 2 % slower.
+template <typename T, int W, int L, bool FULL>
 __device__ __forceinline__ void warp_apply(const Ops<T>& o, const T (&x)[W], T (&y)[W], T* tile, int sl, int w0 = 0,
                                            int wstep = 1) {
+  constexpr bool turn = W == L;
+  constexpr int LT = turn ? W + 1 : L;  // row stride of the tile
   T acc[W];
 #pragma unroll
   for (int i = 0; i < W; ++i) acc[i] = T(0);
   for (int w = w0; w < o.D; w += wstep) {
     const T* a = o.at + w * W * W;
 #pragma unroll 1
-    for (int k1 = 0; k1 < W; k1 += 4) {
+    for (int k1 = 0; k1 < (FULL ? W : o.nr); k1 += 4) {
       T t[4] = {T(0), T(0), T(0), T(0)};
 #pragma unroll
-      for (int b1 = 0; b1 < W; ++b1) {
-        T v[4];
-        load4(a + b1 * W + k1, v);
+      for (int b0 = 0; b0 < W; b0 += 8) {
+        if (!FULL && b0 >= o.nr) continue;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) t[i] = fma(v[i], x[b1], t[i]);
+        for (int b1 = b0; b1 < b0 + 8; ++b1) {
+          T v[4];
+          load4(a + b1 * W + k1, v);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) t[i] = fma(v[i], x[b1], t[i]);
+        }
       }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) tile[(k1 + i) * (W + 1) + sl] = t[i];
+      for (int i = 0; i < 4; ++i) tile[(k1 + i) * LT + sl] = t[i];
     }
     __syncwarp();
     const T* bm = o.bt + w * W * W;
+    if constexpr (turn) {
 #pragma unroll 2
-    for (int b2 = 0; b2 < W; ++b2) {
-      const T tr = tile[sl * (W + 1) + b2];
+      for (int b2 = 0; b2 < (FULL ? W : o.nc); ++b2) {
+        const T tr = FULL || sl < o.nr ? tile[sl * LT + b2] : T(0);  // rows beyond were not written
 #pragma unroll
-      for (int k2 = 0; k2 < W; k2 += 4) {
-        T v[4];
-        load4(bm + b2 * W + k2, v);
+        for (int k0 = 0; k0 < W; k0 += 8) {
+          if (!FULL && k0 >= o.nc) continue;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) acc[k2 + i] = fma(tr, v[i], acc[k2 + i]);
+          for (int k2 = k0; k2 < k0 + 8; k2 += 4) {
+            T v[4];
+            load4(bm + b2 * W + k2, v);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[k2 + i] = fma(tr, v[i], acc[k2 + i]);
+          }
+        }
+      }
+    } else {
+#pragma unroll
+      for (int b0 = 0; b0 < L; b0 += 4) {
+        if (b0 >= o.nc) continue;
+        T b[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) b[i] = bm[(b0 + i) * W + sl];
+#pragma unroll
+        for (int k0 = 0; k0 < W; k0 += 4) {
+          if (k0 >= o.nr) continue;
+#pragma unroll
+          for (int k1 = k0; k1 < k0 + 4; ++k1) {
+            T v[4];
+            load4(tile + k1 * LT + b0, v);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[k1] = fma(v[i], b[i], acc[k1]);
+          }
+        }
       }
     }
     __syncwarp();
   }
-  // lane k1, entry k2 -> lane k2, entry k1
+  if constexpr (turn) {
+    // lane k1, entry k2 -> lane k2, entry k1
 #pragma unroll
-  for (int k2 = 0; k2 < W; ++k2) tile[sl * (W + 1) + k2] = acc[k2];
-  __syncwarp();
+    for (int k2 = 0; k2 < W; ++k2) tile[sl * LT + k2] = acc[k2];
+    __syncwarp();
 #pragma unroll
-  for (int k1 = 0; k1 < W; ++k1) y[k1] = tile[k1 * (W + 1) + sl];
-  __syncwarp();
+    for (int k1 = 0; k1 < W; ++k1) y[k1] = tile[k1 * LT + sl];
+    __syncwarp();
+  } else {
+#pragma unroll
+    for (int k1 = 0; k1 < W; ++k1) y[k1] = acc[k1];
+  }
 }
 
-// vector j of X (vector-major) into registers: x[b1] = X_j[b1 m2 + sl]
+// vector j of X (vector-major) into registers, column sl
 template <typename T, int W, typename S>
-__device__ __forceinline__ void load_vec(const S* X, int j, bool live, T (&x)[W], int m1, int m2, int sl) {
-#pragma unroll
-  for (int i = 0; i < W; ++i) x[i] = (live && i < m1 && sl < m2) ? T(X[size_t(j) * m1 * m2 + i * m2 + sl]) : T(0);
-}
-template <typename T, int W>
-__device__ __forceinline__ void store_vec(T* X, int j, bool live, const T (&x)[W], int m1, int m2, int sl) {
+__device__ __forceinline__ void load_vec(const S* X, int j, bool live, T (&x)[W], const Shape& o, int sl) {
 #pragma unroll
   for (int i = 0; i < W; ++i)
-    if (live && i < m1 && sl < m2) X[size_t(j) * m1 * m2 + i * m2 + sl] = x[i];
+    x[i] = (live && i < o.nr && sl < o.nc) ? T(X[size_t(j) * o.nr * o.nc + i * o.si + sl * o.sj]) : T(0);
+}
+template <typename T, int W>
+__device__ __forceinline__ void store_vec(T* X, int j, bool live, const T (&x)[W], const Shape& o, int sl) {
+#pragma unroll
+  for (int i = 0; i < W; ++i)
+    if (live && i < o.nr && sl < o.nc) X[size_t(j) * o.nr * o.nc + i * o.si + sl * o.sj] = x[i];
 }
 
-// f(j, live, sl, tile) for the vectors j < p, one (W = 32) or two (W = 16) per warp of the team; every
+// f(j, live, sl, tile) for the vectors j < p, 32 / L per warp of the team; every
 // lane of the warp calls it, live false past the end
-template <typename T, int W, typename F>
+template <typename T, int W, int L, typename F>
 __device__ __forceinline__ void for_vectors(const Team& tm, int p, T* tiles, F f) {
-  constexpr int PK = 32 / W;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane / W, sl = lane % W;
-  T* tile = tiles + warp * TILE + sub * W * (W + 1);
+  constexpr int PK = 32 / L;
+  static_assert(PK * tile_stride<W, L>() <= TILE, "tiles of a warp's vectors");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane / L, sl = lane % L;
+  T* tile = tiles + warp * TILE + sub * tile_stride<W, L>();
   for (int j0 = (warp * tm.size + tm.rank) * PK; j0 < p; j0 += NW * tm.size * PK) f(j0 + sub, j0 + sub < p, sl, tile);
 }
 
 // Y_j = H X_j for j < p
-template <typename T, int W>
+template <typename T, int W, int L, bool FULL>
 __device__ void apply_block(const Team& tm, const Ops<T>& o, const T* X, T* Y, int p, T* tiles) {
-  for_vectors<T, W>(tm, p, tiles, [&](int j, bool live, int sl, T* tile) {
+  for_vectors<T, W, L>(tm, p, tiles, [&](int j, bool live, int sl, T* tile) {
     T x[W], y[W];
-    load_vec<T, W>(X, j, live, x, o.m1, o.m2, sl);
-    warp_apply<T, W>(o, x, y, tile, sl);
-    store_vec<T, W>(Y, j, live, y, o.m1, o.m2, sl);
+    load_vec<T, W>(X, j, live, x, o, sl);
+    warp_apply<T, W, L, FULL>(o, x, y, tile, sl);
+    store_vec<T, W>(Y, j, live, y, o, sl);
   });
   tm.sync();
 }
 
 // y = H x for one vector in shared memory, the terms w spread over the CTA's warps; part: NW x m
-template <typename T, int W>
+template <typename T, int W, int L, bool FULL>
 __device__ void apply_one(const Ops<T>& o, const T* x, T* y, T* tiles, T* part) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, m = o.m1 * o.m2, sl = lane % W;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, m = o.nr * o.nc, sl = lane % L;
   if (warp < o.D) {
     T xv[W], yv[W];
-    load_vec<T, W>(x, 0, true, xv, o.m1, o.m2, sl);
-    warp_apply<T, W>(o, xv, yv, tiles + warp * TILE + lane / W * W * (W + 1), sl, warp, NW);
-    store_vec<T, W>(part, warp, lane < W, yv, o.m1, o.m2, sl);
+    load_vec<T, W>(x, 0, true, xv, o, sl);
+    warp_apply<T, W, L, FULL>(o, xv, yv, tiles + warp * TILE + lane / L * tile_stride<W, L>(), sl, warp, NW);
+    store_vec<T, W>(part, warp, lane < L, yv, o, sl);
   }
   __syncthreads();
   for (int e = threadIdx.x; e < m; e += KT) {
@@ -630,36 +681,39 @@ __device__ void scale_ops(KSmall<T>& s, const double* W1, const double* W2, int 
   __syncthreads();
 }
 
-// A_w = W1[0, w] and B_w = W2[w, dr2 - 1], scaled by scale_ops, as padded operands of type T
+// A_w = W1[0, w] and B_w = W2[w, dr2 - 1], scaled by scale_ops, as padded operands of type T; for X^T if
+// `transposed`
 template <typename T, int W, typename S>
 __device__ Ops<T> load_ops(const KSmall<S>& s, const double* W1, const double* W2, int m1, int m2, int dr2, int D,
-                           T* mem) {
-  T* bt = mem + D * W * W;
+                           bool transposed, T* mem) {
+  T* at = transposed ? mem + D * W * W : mem;
+  T* bt = transposed ? mem : mem + D * W * W;
   for (int e = threadIdx.x; e < D * W * W; e += KT) {
     const int w = e / (W * W), b = e / W % W, k = e % W;
     const double x = (b < m1 && k < m1) ? W1[(size_t(w) * m1 + k) * m1 + b] : 0.0;  // row 0 of W1
     const double y = (b < m2 && k < m2) ? W2[((size_t(w) * dr2 + dr2 - 1) * m2 + k) * m2 + b] : 0.0;
-    mem[e] = jac::bits(x) == 0 ? T(0) : T(scale_pow2(x, -s.ea[w]));
+    at[e] = jac::bits(x) == 0 ? T(0) : T(scale_pow2(x, -s.ea[w]));
     bt[e] = jac::bits(y) == 0 ? T(0) : T(scale_pow2(y, -s.eb[w]));
   }
   __syncthreads();
-  return {mem, bt, m1, m2, D};
+  const Shape sh = transposed ? Shape{m2, m1, 1, m2} : Shape{m1, m2, m2, 1};
+  return {sh, mem, mem + D * W * W, D};
 }
 
 // Upper end of the spectrum for the filter: 24 Lanczos steps on one vector give the largest
 // Ritz value theta_max; theta_max + |beta_last| (plus 1% of the Ritz range) bounds lambda_max
 // in practice and is far tighter than the norm bound sum_w ||A_w||_inf ||B_w||_inf, which caps
 // it. A tighter damping interval makes every filter application converge faster. mem: (NW + 3) m.
-template <int W>
+template <int W, int L, bool FULL>
 __device__ float upper_bound(KSmall<float>& s, const Ops<float>& o, int b, float* tiles, float* mem) {
   __shared__ double lal[25], lbe[25];
   __shared__ unsigned norm[2 * KD];
-  const int m = o.m1 * o.m2, nl = m < 24 ? m : 24;
+  const int m = o.nr * o.nc, nl = m < 24 ? m : 24;
   if (threadIdx.x < 2 * KD) norm[threadIdx.x] = 0u;
   __syncthreads();
-  for (int r = threadIdx.x; r < o.D * (o.m1 + o.m2); r += KT) {  // row sums
-    const bool a = r < o.D * o.m1;
-    const int q = a ? r : r - o.D * o.m1, mm = a ? o.m1 : o.m2, w = q / mm, k = q % mm;
+  for (int r = threadIdx.x; r < o.D * (o.nr + o.nc); r += KT) {  // row sums
+    const bool a = r < o.D * o.nr;
+    const int q = a ? r : r - o.D * o.nr, mm = a ? o.nr : o.nc, w = q / mm, k = q % mm;
     const float* x = (a ? o.at : o.bt) + w * W * W + k;
     float t = 0.f;
     for (int i = 0; i < mm; ++i) t += fabsf(x[i * W]);
@@ -681,7 +735,7 @@ __device__ float upper_bound(KSmall<float>& s, const Ops<float>& o, int b, float
   float beta = 0.f;
   int steps = 0;
   for (int j = 0; j < nl; ++j) {
-    apply_one<float, W>(o, v, w, tiles, part);
+    apply_one<float, W, L, FULL>(o, v, w, tiles, part);
     float t = 0.f;
     for (int e = threadIdx.x; e < m; e += KT) t = fmaf(w[e], v[e], t);
     const float alpha = bsum(t, s.red);
@@ -735,17 +789,18 @@ static_assert(2 * KP * GL + KP <= NW * TILE && KM1 * KM1 <= NW * TILE, "scratch 
 
 // FP32 subspace iteration; `nout` of the Ritz vectors go to `out` (FP64, vector-major) and the filter's
 // upper bound (of the scaled H) to bound[b].
-template <int W>
+template <int W, int L>
 __device__ void chfsi(const Team& tm, const double* W1, const double* W2, int m1, int m2, int dr2, int k, int p, int D,
                       int b, float* X, float* Y, int max_outer, int degree, double* out, int nout, float* bound,
                       int* iters, unsigned char* raw) {
+  constexpr bool FULL = W == 16;
   KSmall<float>& s = *reinterpret_cast<KSmall<float>*>(raw);
   float* mem = reinterpret_cast<float*>(raw + (sizeof(KSmall<float>) + 15) / 16 * 16);
   const int m = m1 * m2;
   scale_ops(s, W1, W2, m1, m2, dr2, D);
-  const Ops<float> o = load_ops<float, W>(s, W1, W2, m1, m2, dr2, D, mem);
+  const Ops<float> o = load_ops<float, W>(s, W1, W2, m1, m2, dr2, D, L < W && m1 < m2, mem);
   float* tiles = mem + ops_elems(W, D);
-  const float ub = upper_bound<W>(s, o, b, tiles, tiles + scratch_elems<float>(0, false));
+  const float ub = upper_bound<W, L, FULL>(s, o, b, tiles, tiles + scratch_elems<float>(0, false));
   auto orthonormal = [&] {  // one vector after the other: the first CTA's
     if (tm.rank == 0) orthonormalise(s, X, p, m, tiles);
     tm.sync();
@@ -757,7 +812,7 @@ __device__ void chfsi(const Team& tm, const double* W1, const double* W2, int m1
   int it = 0;
   for (; it < max_outer; ++it) {
     // Rayleigh-Ritz: Y = H X, G = X^T Y
-    apply_block<float, W>(tm, o, X, Y, p, tiles);
+    apply_block<float, W, L, FULL>(tm, o, X, Y, p, tiles);
     gram<float, false>(tm, s, X, Y, p, m, tiles);
     small_eigh(s, p);
     rotate(tm, s, X, p, m);
@@ -782,14 +837,14 @@ __device__ void chfsi(const Team& tm, const double* W1, const double* W2, int m1
     // Chebyshev filter of degree `degree` on [a, ub], a = largest Ritz value of the block
     const float a = s.theta[p - 1];
     const float c = 0.5f * (a + ub), h = 0.5f * (ub - a) + 1e-30f;
-    for_vectors<float, W>(tm, p, tiles, [&](int j, bool live, int sl, float* tile) {
+    for_vectors<float, W, L>(tm, p, tiles, [&](int j, bool live, int sl, float* tile) {
       float prev[W], cur[W], hx[W];
-      load_vec<float, W>(X, j, live, prev, m1, m2, sl);
-      load_vec<float, W>(Y, j, live, cur, m1, m2, sl);
+      load_vec<float, W>(X, j, live, prev, o, sl);
+      load_vec<float, W>(Y, j, live, cur, o, sl);
 #pragma unroll
       for (int i = 0; i < W; ++i) cur[i] = (cur[i] - c * prev[i]) / h;
       for (int d = 2; d <= degree; ++d) {
-        warp_apply<float, W>(o, cur, hx, tile, sl);
+        warp_apply<float, W, L, FULL>(o, cur, hx, tile, sl);
 #pragma unroll
         for (int i = 0; i < W; ++i) {
           const float t = 2.f * (hx[i] - c * cur[i]) / h - prev[i];
@@ -797,7 +852,7 @@ __device__ void chfsi(const Team& tm, const double* W1, const double* W2, int m1
           cur[i] = t;
         }
       }
-      store_vec<float, W>(X, j, live, cur, m1, m2, sl);
+      store_vec<float, W>(X, j, live, cur, o, sl);
     });
     tm.sync();
     orthonormal();
@@ -810,6 +865,9 @@ __device__ void chfsi(const Team& tm, const double* W1, const double* W2, int m1
   }
   tm.sync();  // shared memory stays until no CTA reads it
 }
+
+// Where one node has more than 16 states, the lanes a vector takes while the other has no more
+constexpr int NARROW = 8;
 
 // meta[5b..5b+4] = m1, m2, dr2, k, p; the k Ritz vectors go to vec_base, all p when keep_guards
 __global__ void __launch_bounds__(KT) kron_chfsi_kernel(const double* const* __restrict__ w1s,
@@ -828,20 +886,23 @@ __global__ void __launch_bounds__(KT) kron_chfsi_kernel(const double* const* __r
   double* out = vec_base + size_t(b) * vec_stride;
   const int nout = keep_guards ? p : k;
   if (m1 <= 16 && m2 <= 16)
-    chfsi<16>(tm, w1s[b], w2s[b], m1, m2, dr2, k, p, D, b, X, Y, max_outer, degree, out, nout, bounds, out_iters,
-              ksm_raw);
+    chfsi<16, 16>(tm, w1s[b], w2s[b], m1, m2, dr2, k, p, D, b, X, Y, max_outer, degree, out, nout, bounds, out_iters,
+                  ksm_raw);
+  else if (min(m1, m2) <= NARROW)
+    chfsi<32, NARROW>(tm, w1s[b], w2s[b], m1, m2, dr2, k, p, D, b, X, Y, max_outer, degree, out, nout, bounds, out_iters,
+                      ksm_raw);
   else
-    chfsi<32>(tm, w1s[b], w2s[b], m1, m2, dr2, k, p, D, b, X, Y, max_outer, degree, out, nout, bounds, out_iters,
-              ksm_raw);
+    chfsi<32, 32>(tm, w1s[b], w2s[b], m1, m2, dr2, k, p, D, b, X, Y, max_outer, degree, out, nout, bounds, out_iters,
+                  ksm_raw);
 }
 
-// e -= XF (XF^T e) for two vectors per lane group, over the lanes of W
-template <int W>
-__device__ __forceinline__ void project_out(const float* XF, int p, int m1, int m2, int sl, float (&e)[W],
+// e -= XF (XF^T e) for two vectors per group of L lanes
+template <int W, int L>
+__device__ __forceinline__ void project_out(const float* XF, int p, const Shape& o, int sl, float (&e)[W],
                                             float (&f)[W]) {
   for (int i = 0; i < p; ++i) {
     float x[W];
-    load_vec<float, W>(XF, i, true, x, m1, m2, sl);
+    load_vec<float, W>(XF, i, true, x, o, sl);
     float d = 0.f, g = 0.f;
 #pragma unroll
     for (int q = 0; q < W; ++q) {
@@ -849,7 +910,7 @@ __device__ __forceinline__ void project_out(const float* XF, int p, int m1, int 
       g = fmaf(x[q], f[q], g);
     }
 #pragma unroll
-    for (int q = W / 2; q > 0; q >>= 1) {
+    for (int q = L / 2; q > 0; q >>= 1) {
       d += __shfl_xor_sync(0xffffffffu, d, q);
       g += __shfl_xor_sync(0xffffffffu, g, q);
     }
@@ -865,7 +926,7 @@ constexpr int POLISH_STEPS = 48;  // Chebyshev steps of a correction
 constexpr int POLISH_PROJECT = 8;  // steps between projections onto the complement
 
 // FP64 eigenpairs from the FP32 subspace in X (p vectors, vector-major): see the head of the file
-template <int W>
+template <int W, int L, bool FULL>
 __device__ void polish(const Team& tm, const double* W1, const double* W2, int m1, int m2, int dr2, int k, int p,
                        int D, int b, double* X, double* Y, float* XF, float ub, int max_outer, double* ev, double* out,
                        int keep, int* iters, unsigned char* raw) {
@@ -873,17 +934,18 @@ __device__ void polish(const Team& tm, const double* W1, const double* W2, int m
   double* mem = reinterpret_cast<double*>(raw + (sizeof(KSmall<double>) + 15) / 16 * 16);
   const int m = m1 * m2;
   scale_ops(s, W1, W2, m1, m2, dr2, D);
-  const Ops<double> o = load_ops<double, W>(s, W1, W2, m1, m2, dr2, D, mem);
+  const bool transposed = L < W && m1 < m2;
+  const Ops<double> o = load_ops<double, W>(s, W1, W2, m1, m2, dr2, D, transposed, mem);
   double* tiles = mem + ops_elems(W, D);
   float* fmem = reinterpret_cast<float*>(tiles);  // FP32 operands and tiles of the corrections
   int it = 0;
   for (; it < max_outer; ++it) {
-    apply_block<double, W>(tm, o, X, Y, p, tiles);
+    apply_block<double, W, L, FULL>(tm, o, X, Y, p, tiles);
     gram<double, true>(tm, s, X, Y, p, m, tiles);
     if (!small_eigh_general(s, p, tiles)) {  // nearly dependent vectors: orthonormalise them first
       if (tm.rank == 0) orthonormalise(s, X, p, m, tiles);
       tm.sync();
-      apply_block<double, W>(tm, o, X, Y, p, tiles);
+      apply_block<double, W, L, FULL>(tm, o, X, Y, p, tiles);
       gram<double, false>(tm, s, X, Y, p, m, tiles);
       small_eigh(s, p);
     }
@@ -911,10 +973,10 @@ __device__ void polish(const Team& tm, const double* W1, const double* W2, int m
     if (s.flag) break;
     tm.sync();
     const double a = s.theta[p - 1], c = 0.5 * (a + double(ub)), h = 0.5 * (double(ub) - a) + 1e-30;
-    const Ops<float> of = load_ops<float, W>(s, W1, W2, m1, m2, dr2, D, fmem);
+    const Ops<float> of = load_ops<float, W>(s, W1, W2, m1, m2, dr2, D, transposed, fmem);
     float* ftiles = fmem + ops_elems(W, D);
     const float cf = float(c), ih = float(1.0 / h);
-    for_vectors<float, W>(tm, p, ftiles, [&](int j, bool live, int sl, float* tile) {
+    for_vectors<float, W, L>(tm, p, ftiles, [&](int j, bool live, int sl, float* tile) {
       const double th = live ? s.theta[j] : 0.0, nr = live ? s.scal[j] : 0.0;
       const bool work = nr > 0.0;
       const double inv = work ? 1.0 / (nr * h) : 0.0;
@@ -922,8 +984,8 @@ __device__ void polish(const Team& tm, const double* W1, const double* W2, int m
 #pragma unroll
       for (int i = 0; i < W; ++i) {
         r[i] = 0.f;
-        if (work && i < m1 && sl < m2) {
-          const size_t q = size_t(j) * m + i * m2 + sl;
+        if (work && i < o.nr && sl < o.nc) {
+          const size_t q = size_t(j) * m + i * o.si + sl * o.sj;
           r[i] = float(fma(-th, X[q], Y[q]) * inv);
         }
       }
@@ -936,7 +998,7 @@ __device__ void polish(const Team& tm, const double* W1, const double* W2, int m
       }
       for (int n = 1; n < POLISH_STEPS; ++n) {
         const float q1 = 1.f / (2.f * tc - q0);
-        warp_apply<float, W>(of, e, hx, tile, sl);
+        warp_apply<float, W, L, FULL>(of, e, hx, tile, sl);
 #pragma unroll
         for (int i = 0; i < W; ++i) {
           const float t = 2.f * q1 * (fmaf(-cf, e[i], hx[i]) * ih + r[i]) - q1 * q0 * prev[i];
@@ -944,12 +1006,13 @@ __device__ void polish(const Team& tm, const double* W1, const double* W2, int m
           e[i] = t;
         }
         q0 = q1;
-        if ((n + 1) % POLISH_PROJECT == 0) project_out<W>(XF, p, m1, m2, sl, e, prev);
+        if ((n + 1) % POLISH_PROJECT == 0) project_out<W, L>(XF, p, o, sl, e, prev);
       }
       bool finite = true;
 #pragma unroll
       for (int i = 0; i < W; ++i) finite = finite && fabsf(e[i]) < 1e30f;
-      finite = __all_sync(0xffffffffu, finite || !work);
+      const unsigned group = (L == 32 ? ~0u : (1u << (L & 31)) - 1) << (((threadIdx.x & 31) / L) * L);
+      finite = (__ballot_sync(0xffffffffu, finite) & group) == group;
       // x + |r| e, scaled to unit length (e is orthogonal to x)
       double len = 0.0;
       if (work && finite) {
@@ -957,13 +1020,13 @@ __device__ void polish(const Team& tm, const double* W1, const double* W2, int m
         for (int i = 0; i < W; ++i) len = fma(nr * double(e[i]), nr * double(e[i]), len);
       }
 #pragma unroll
-      for (int q = W / 2; q > 0; q >>= 1) len += __shfl_xor_sync(0xffffffffu, len, q);
+      for (int q = L / 2; q > 0; q >>= 1) len += __shfl_xor_sync(0xffffffffu, len, q);
       if (work && finite) {
         const double f = 1.0 / sqrt(1.0 + len);
 #pragma unroll
         for (int i = 0; i < W; ++i)
-          if (i < m1 && sl < m2) {
-            const size_t q = size_t(j) * m + i * m2 + sl;
+          if (i < o.nr && sl < o.nc) {
+            const size_t q = size_t(j) * m + i * o.si + sl * o.sj;
             X[q] = fma(nr, double(e[i]), X[q]) * f;
           }
       }
@@ -999,22 +1062,28 @@ __global__ void __launch_bounds__(KT) kron_polish_kernel(const double* const* __
   double* ev = evals + size_t(b) * keep;
   double* out = evecs + size_t(b) * max_m * keep;  // [max_m][keep], like tnx_eigh_batched
   if (m1 <= 16 && m2 <= 16)
-    polish<16>(tm, w1s[b], w2s[b], m1, m2, dr2, k, p, D, b, X, Y, XF, bounds[b], max_outer, ev, out, keep, out_iters,
-               ksm_raw);
+    polish<16, 16, true>(tm, w1s[b], w2s[b], m1, m2, dr2, k, p, D, b, X, Y, XF, bounds[b], max_outer, ev, out,
+                        keep, out_iters, ksm_raw);
+  else if (min(m1, m2) <= NARROW)
+    polish<32, NARROW, false>(tm, w1s[b], w2s[b], m1, m2, dr2, k, p, D, b, X, Y, XF, bounds[b], max_outer, ev, out,
+                             keep, out_iters, ksm_raw);
+  else if (m1 > 24 && m2 > 24)
+    polish<32, 32, true>(tm, w1s[b], w2s[b], m1, m2, dr2, k, p, D, b, X, Y, XF, bounds[b], max_outer, ev, out,
+                        keep, out_iters, ksm_raw);
   else
-    polish<32>(tm, w1s[b], w2s[b], m1, m2, dr2, k, p, D, b, X, Y, XF, bounds[b], max_outer, ev, out, keep, out_iters,
-               ksm_raw);
+    polish<32, 32, false>(tm, w1s[b], w2s[b], m1, m2, dr2, k, p, D, b, X, Y, XF, bounds[b], max_outer, ev, out,
+                         keep, out_iters, ksm_raw);
 }
 
-template <int W>
+template <int W, int L>
 __device__ void ritz64(const Team& tm, KSmall<double>& s, const double* W1, const double* W2, int m1, int m2, int dr2,
                        int k, int D, double* V, double* Z, double* mem) {
   const int m = m1 * m2;
   scale_ops(s, W1, W2, m1, m2, dr2, D);
-  const Ops<double> o = load_ops<double, W>(s, W1, W2, m1, m2, dr2, D, mem);
+  const Ops<double> o = load_ops<double, W>(s, W1, W2, m1, m2, dr2, D, L < W && m1 < m2, mem);
   double* tiles = mem + ops_elems(W, D);
   orthonormalise(s, V, k, m, tiles);
-  apply_block<double, W>(tm, o, V, Z, k, tiles);
+  apply_block<double, W, L, W == 16>(tm, o, V, Z, k, tiles);
   gram<double, false>(tm, s, V, Z, k, m, tiles);
   small_eigh(s, k);
   rotate(tm, s, V, k, m);
@@ -1040,9 +1109,11 @@ __global__ void __launch_bounds__(KT) kron_refine_kernel(const double* const* __
   double* Zb = scratch + size_t(b) * scratch_stride;
   const Team tm{0, 1};
   if (m1 <= 16 && m2 <= 16)
-    ritz64<16>(tm, s, w1s[b], w2s[b], m1, m2, dr2, k, D, V, Zb, mem);
+    ritz64<16, 16>(tm, s, w1s[b], w2s[b], m1, m2, dr2, k, D, V, Zb, mem);
+  else if (min(m1, m2) <= NARROW)
+    ritz64<32, NARROW>(tm, s, w1s[b], w2s[b], m1, m2, dr2, k, D, V, Zb, mem);
   else
-    ritz64<32>(tm, s, w1s[b], w2s[b], m1, m2, dr2, k, D, V, Zb, mem);
+    ritz64<32, 32>(tm, s, w1s[b], w2s[b], m1, m2, dr2, k, D, V, Zb, mem);
   double* ev = evals + size_t(b) * keep;
   for (int i = threadIdx.x; i < k; i += KT) ev[i] = scale_pow2(s.theta[i], s.eh);
   double* out = evecs + size_t(b) * max_m * keep;  // [max_m][keep], like tnx_eigh_batched
