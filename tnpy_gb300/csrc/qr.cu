@@ -181,6 +181,7 @@ constexpr int PT = 256;  // threads per CTA of the cluster panel kernel
 
 using qrdf::cluster_arrive_release;
 using qrdf::cluster_wait_acquire;
+using tc::mbar_arrive;
 using tc::mbar_expect_tx;
 using tc::mbar_init;
 using tc::mbar_wait;
@@ -218,8 +219,8 @@ __global__ void __launch_bounds__(PT) panel_cl_kernel(double* __restrict__ F, in
   const int rows = int(r0 >= mp ? 0 : (mp - r0 < rpc ? mp - r0 : rpc));
   if (push && tid == 0) {
     s_dead = 0;
-    mbar_init(smem_u32(&bars[0]), 1);
-    mbar_init(smem_u32(&bars[1]), 1);
+    mbar_init(smem_u32(&bars[0]), 1 + PT / 32);
+    mbar_init(smem_u32(&bars[1]), 1 + PT / 32);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     mbar_expect_tx(smem_u32(&bars[0]), uint32_t(8 * nb * (CL + 1)));
     mbar_expect_tx(smem_u32(&bars[1]), uint32_t(8 * (nb - 1) * (CL + 1)));
@@ -247,7 +248,15 @@ __global__ void __launch_bounds__(PT) panel_cl_kernel(double* __restrict__ F, in
       prow[buf * NB + c] = piv;
     }
   };
-  // before the exchange of step `step` is read
+  // A warp's end of the update that sends into buffer buf: its stores to the panel come before this CTA reads what the
+  // barrier guards (the sums order the stores of the lane that sends them alone)
+  auto updated = [&](int buf) {
+    if (push) {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&bars[buf]));
+    }
+  };
+  // before the exchange of step `step`, or the panel as the update before left it, is read
   auto await = [&](int step) {
     if (push && !mbar_wait(smem_u32(&bars[step & 1]), (step >> 1) & 1)) s_dead = 1;
   };
@@ -306,6 +315,7 @@ __global__ void __launch_bounds__(PT) panel_cl_kernel(double* __restrict__ F, in
     for (int o = TPC / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (ci < nb) send_sum(0, acc);
     if (r0 == 0 && rows > 0 && tid < nb) send_pivot(0, tid, pl[tid * ld]);
+    updated(0);
   }
   exchange();
   for (int jj = 0; jj < nb; ++jj) {
@@ -411,6 +421,7 @@ __global__ void __launch_bounds__(PT) panel_cl_kernel(double* __restrict__ F, in
 #pragma unroll
     for (int o = TPC / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (ci < nb && ci != jj) send_sum(par ^ 1, acc);
+    updated(par ^ 1);
     exchange();
   }
   __syncthreads();

@@ -44,6 +44,7 @@ namespace tnx {
 namespace qrdf {
 
 namespace cg = cooperative_groups;
+using tc::mbar_arrive;
 using tc::mbar_expect_tx;
 using tc::mbar_init;
 using tc::mbar_wait;
@@ -225,7 +226,7 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
   __shared__ df2 W[NB], Z[2][NB], taus[NB], sc[4];  // W: factors of the current reflector in the columns right of it
   __shared__ df2 Tr[NR][NB];          // rows q, q + CL, ... of T
   __shared__ int cexp[NB];
-  __shared__ __align__(8) uint64_t bars[2];  // arrival of a step's sums (push)
+  __shared__ __align__(8) uint64_t bars[2];  // arrival of a step's sums and end of the update before it (push)
   __shared__ int s_dead;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ci = warp + NW * (lane / GL), h = lane % GL;
@@ -244,8 +245,8 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
     const uint32_t bar = smem_u32(bars);
     if (push && tid == 0) {
       s_dead = 0;
-      mbar_init(bar, 1);
-      mbar_init(bar + 8, 1);
+      mbar_init(bar, 1 + NW);
+      mbar_init(bar + 8, 1 + NW);
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       mbar_expect_tx(bar, uint32_t(8 * nb * (CL + 1)));
       mbar_expect_tx(bar + 8, uint32_t(8 * ((nb - 1) * CL + nb - 1)));
@@ -320,7 +321,15 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
       prow[buf * NB + c] = piv;
     }
   };
-  // before the exchange of step `step` is read
+  // A warp's end of the update that sends into buffer buf: its stores to the panel come before this CTA reads what the
+  // barrier guards (the sums order the stores of the lane that sends them alone)
+  auto updated = [&](int buf) {
+    if (push) {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&bars[buf]));
+    }
+  };
+  // before the exchange of step `step`, or the panel as the update before left it, is read
   auto await = [&](int step) {
     if (push && !mbar_wait(smem_u32(&bars[step & 1]), (step >> 1) & 1)) s_dead = 1;
   };
@@ -382,6 +391,7 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
     const df2 sum = reduce(a);
     if (ci < nb) send_sum(0, sum);
     if (r0 == 0 && rows > 0 && tid < nb) send_pivot(0, tid, X[tid * ld]);
+    updated(0);
   }
   exchange();
 
@@ -535,6 +545,7 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
     if (ci < jj && (has_lj || has_ln)) sum = add(sum, W[ci]);
     PANEL_STAMP(5);
     if (ci < nb && ci != jj) send_sum(par ^ 1, sum);
+    updated(par ^ 1);
     PANEL_STAMP(6);
     exchange();
     PANEL_STAMP(7);
