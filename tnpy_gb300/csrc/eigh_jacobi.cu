@@ -352,11 +352,18 @@ constexpr int RW_MAX = 64;
 
 constexpr int RR_G = 8;  // warps that share a product of the refinement
 
+// x 2^-e; zero for zero and where it would be subnormal
+__device__ __forceinline__ double rr_scale(double x, int e) {
+  return (__double2hiint(x) & 0x7ff00000) == 0 ? 0.0 : jac::scale_exp(x, e);
+}
+
 // FP32 rounding keeps regenerating off-diagonal entries at ~6e-8 |A|_F, so the sweeps
 // stop once every off-diagonal entry is below 1e-6 |A|_F; the FP64 steps take it from there.
 // Block b solves the matrix at A + b sA into eval[b sE], evec + b sV, and returns at
 // once when active is given and active[b] == 0. With `sizes` (count > 0), block b solves the leading block
 // of sizes.n[b] rows of A instead of n, and where[b] is the index at which the sweeps left the lowest value.
+// The matrix is taken times the power of two that brings its largest entry below one (exact): sweeps and corrections are
+// FP32's. One with Inf or NaN has NaN for its pair.
 template <int RR_T>
 __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restrict__ A, int n, int ld,
                                                          double* __restrict__ eval, double* __restrict__ evec,
@@ -380,16 +387,35 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restric
   __shared__ float4 rot[32];  // c, s and (as integers) p, q of a pair
   __shared__ float red[RR_T / 32];
   __shared__ double redd[RR_T / 32];
+  __shared__ unsigned s_max[RR_T / 32];
   __shared__ int s_imin;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  float fro = 0.f;
+  unsigned mx = 0;
   for (int e = tid; e < n * n; e += RR_T) {
     const int i = e / n, j = e - i * n;
     const double v = A[int64_t(i) * ld + j];
+    Ad[i * nf + j] = v;
+    Vf[i * nf + j] = (i == j) ? 1.f : 0.f;
+    mx = max(mx, unsigned(__double2hiint(v)) & 0x7fffffffu);
+  }
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if (lane == 0) s_max[warp] = mx;
+  __syncthreads();
+  for (int w = 0; w < RR_T / 32; ++w) mx = max(mx, s_max[w]);
+  if (mx >= 0x7ff00000u) {
+    if (tid == 0) eval[0] = __longlong_as_double(0x7ff8000000000000LL);
+    if (tid < n) evec[tid] = __longlong_as_double(0x7ff8000000000000LL);
+    if (where && tid == 0) where[blockIdx.x] = 0.0;
+    return;
+  }
+  const int ex = int(mx >> 20) - 1022;
+  float fro = 0.f;
+  for (int e = tid; e < n * n; e += RR_T) {
+    const int i = e / n, j = e - i * n;
+    const double v = rr_scale(Ad[i * nf + j], ex);
     const float f = float(v);
     Ad[i * nf + j] = v;
     Af[i * nf + j] = f;
-    Vf[i * nf + j] = (i == j) ? 1.f : 0.f;
     fro += f * f;
   }
   for (int o = 16; o > 0; o >>= 1) fro += __shfl_xor_sync(0xffffffffu, fro, o);
@@ -546,7 +572,7 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restric
     const double theta = (redd[2] + redd[3]) * (inv * inv);
     if (tid < n) s[tid] = si * inv;
     if (step == 3) {
-      if (tid == 0) eval[0] = theta;
+      if (tid == 0) eval[0] = scale_pow2(theta, ex);
       break;
     }
     if (tid < n) rf[tid] = float(fma(-theta, si, yi) * inv);
@@ -652,11 +678,6 @@ __device__ __forceinline__ float rr_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
-}
-
-// x 2^-e; zero for zero and where it would be subnormal
-__device__ __forceinline__ double rr_scale(double x, int e) {
-  return (__double2hiint(x) & 0x7ff00000) == 0 ? 0.0 : jac::scale_exp(x, e);
 }
 
 template <int NR>
