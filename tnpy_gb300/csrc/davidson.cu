@@ -662,6 +662,9 @@ int dots(const T* V, int64_t ldv, int k, const T* w, int64_t n, double* part, do
 
 }  // namespace
 
+// root of a squared norm; NaN stays NaN
+inline double norm_of(double squared) { return squared > 0.0 || std::isnan(squared) ? sqrt(squared) : 0.0; }
+
 // Counters of the calling thread's last davidson1 call (tnx_davidson1_stats)
 struct DavStats {
   int phase1 = 0, anchored = 0, anchors = 0, restarts = 0;
@@ -795,7 +798,7 @@ int davidson1(const double* L, const double* W, const double* R, double* x_io, i
       std::copy(hp->s, hp->s + k, s_hist.begin() + size_t(k) * MAXB);
       cur_k = k;
       theta = hp->theta;
-      rnorm = sqrt(fmax(hp->rn2, 0.0));
+      rnorm = norm_of(hp->rn2);
       c0 = hp->s[0];
       if (!std::isfinite(theta) || !std::isfinite(rnorm)) {
         set_error("tnx_davidson1: non-finite Ritz value or residual");
@@ -823,7 +826,7 @@ int davidson1(const double* L, const double* W, const double* R, double* x_io, i
     }
     std::copy(s_cur.begin(), s_cur.begin() + k, s_hist.begin() + size_t(k) * MAXB);
     theta = host[0];
-    rnorm = sqrt(fmax(host[1], 0.0));
+    rnorm = norm_of(host[1]);
     c0 = host[2];
     if (!std::isfinite(theta) || !std::isfinite(rnorm)) {
       set_error("tnx_davidson1: non-finite Ritz value or residual");
@@ -1322,7 +1325,7 @@ int gdavidson1(const double* L, const double* W, const double* R, const double* 
     TNX_CUDA(cudaMemcpyAsync(host + 1, rn2, 8, cudaMemcpyDeviceToHost, st));
     TNX_CUDA(cudaStreamSynchronize(st));
     theta = host[0];
-    rnorm = sqrt(fmax(host[1], 0.0));
+    rnorm = norm_of(host[1]);
     if (!std::isfinite(theta) || !std::isfinite(rnorm)) {
       set_error("tnx_gdavidson1: non-finite Ritz value or residual");
       return TNX_ERR_INVALID_ARG;

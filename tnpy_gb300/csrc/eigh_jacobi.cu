@@ -712,6 +712,11 @@ __global__ void __launch_bounds__(RT_T) rr_tri_kernel(const double* __restrict__
   if (lane == 0) s_max[warp] = mx;
   __syncthreads();
   mx = max(max(s_max[0], s_max[1]), max(s_max[2], s_max[3]));
+  if (mx >= 0x7ff00000u) {  // Inf or NaN, which the scaling below would make finite
+    if (tid == 0) eval[0] = __longlong_as_double(0x7ff8000000000000LL);
+    if (tid < n) evec[tid] = __longlong_as_double(0x7ff8000000000000LL);
+    return;
+  }
   const int ex = int(mx >> 20) - 1022 + (NR == 32 ? 5 : 6);
   for (int i = warp; i < NR; i += RT_T / 32)
 #pragma unroll
