@@ -206,7 +206,8 @@ __global__ void __launch_bounds__(QS_T) qr_small_kernel(const double* A, int64_t
 #pragma unroll 4
       for (int i = j + 1 + h; i < m; i += 8) w = fma(v[i], x[i], w);
       const double top = x[j];
-      w = live ? tj * (lanes_sum(w, 4) + top) : (lanes_sum(w, 4), 0.0);
+      const double dot = lanes_sum(w, 4) + top;  // all lanes take part
+      w = live ? tj * dot : 0.0;
       __syncwarp();
       if (live) {
 #pragma unroll 4
