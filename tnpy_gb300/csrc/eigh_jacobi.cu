@@ -28,7 +28,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 
 #include "jacobi.cuh"
 #include "tnx_internal.cuh"
@@ -262,12 +261,8 @@ namespace {
 int launch_jacobi(const double* A, const int64_t* offsets, const int* sizes, const int* lds, int n, int ld, int batch,
                   int max_size, int keep, double* evals, double* evecs, double* work, cudaStream_t st) {
   const size_t smem = max_size <= EJ_SHARED_N ? ej_smem_bytes(max_size) : 0;
-  static std::atomic<bool> attr{false};  // idempotent setup; threads may race to it
-  if (!attr.load()) {
-    TNX_CUDA(cudaFuncSetAttribute(jacobi_eigh_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  int(ej_smem_bytes(EJ_SHARED_N))));
-    attr.store(true);
-  }
+  static DeviceSet allowed;
+  TNX_CUDA(allow_smem(jacobi_eigh_kernel, ej_smem_bytes(EJ_SHARED_N), allowed));
   jacobi_eigh_kernel<<<batch, EJ_THREADS, smem, st>>>(A, offsets, sizes, lds, n, ld, max_size, keep, evals, evecs,
                                                       work);
   TNX_LAUNCH_CHECK();
@@ -616,12 +611,8 @@ int launch_rr(const double* A, int n, int ld, int64_t sA, double* eval, int64_t 
     return TNX_ERR_SHAPE;
   }
   if (batch <= 0) return TNX_OK;
-  static std::atomic<bool> attr{false};  // idempotent setup; threads may race to it
-  if (!attr.load()) {
-    TNX_CUDA(cudaFuncSetAttribute(rr_lowest_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  int(rr_lowest_smem(RW_MAX))));
-    attr.store(true);
-  }
+  static DeviceSet allowed;
+  TNX_CUDA(allow_smem(rr_lowest_kernel<1024>, rr_lowest_smem(RW_MAX), allowed));
   profile_mark(KF_EIGH, st, true);
   // the blocks of a round, (n / 2)^2 of them and n^2 / 4 entries of V twice, by a thread each
   if (n <= 32)
@@ -1102,12 +1093,8 @@ int rr_lowest_tri(const double* A, int n, int ld, double* eval, double* evec, cu
   if (n <= 32) {
     rr_tri_kernel<32><<<1, RT_T, rr_tri_smem(n, 32), st>>>(A, n, ld, eval, evec);
   } else {
-    static std::atomic<bool> attr{false};  // idempotent setup; threads may race to it
-    if (!attr.load()) {
-      TNX_CUDA(cudaFuncSetAttribute(rr_tri_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(rr_tri_smem(RW_MAX, 64))));
-      attr.store(true);
-    }
+    static DeviceSet allowed;
+    TNX_CUDA(allow_smem(rr_tri_kernel<64>, rr_tri_smem(RW_MAX, 64), allowed));
     rr_tri_kernel<64><<<1, RT_T, rr_tri_smem(n, 64), st>>>(A, n, ld, eval, evec);
   }
   profile_mark(KF_EIGH, st, false);

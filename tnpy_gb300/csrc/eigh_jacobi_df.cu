@@ -19,7 +19,6 @@
 // kernel: the lowest `keep` eigenvalues ascending and their vectors, as FP64.
 #include <cuda_runtime.h>
 
-#include <atomic>
 
 #include "tnx_internal.cuh"
 #include "qr_panel_df.cuh"
@@ -185,11 +184,8 @@ int tnx_eigh_batched_df64(double* A, const int64_t* offsets, const int* sizes, i
   TNX_CHECK_SHAPE(max_size <= EJD_MAX, "double-FP32 eigh: matrices up to %d (got %d)", EJD_MAX, max_size);
   if (batch == 0) return TNX_OK;
   const size_t smem = size_t(2) * EJD_MAX * (EJD_MAX + 1) * sizeof(df2);
-  static std::atomic<bool> attr{false};
-  if (!attr.load()) {
-    TNX_CUDA(cudaFuncSetAttribute(jacobi_eigh_df_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    attr.store(true);
-  }
+  static DeviceSet allowed;
+  TNX_CUDA(allow_smem(jacobi_eigh_df_kernel, smem, allowed));
   cudaStream_t st = as_stream(stream);
   profile_mark(KF_EIGH, st, true);
   jacobi_eigh_df_kernel<<<batch, EJD_THREADS, smem, st>>>(A, offsets, sizes, max_size, keep, evals, evecs);

@@ -31,7 +31,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 
 #include "tc_ptx.cuh"
 #include "tnx_internal.cuh"
@@ -598,11 +597,8 @@ int gemm_oz_ex(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha, 
   TNX_TRY(make_tma_map_bf16(&ma, L.sa, int64_t(batch) * OZ_S * L.Mp, L.Kp, OZ_BK, OZ_BM));
   TNX_TRY(make_tma_map_bf16(&mb, L.sb, int64_t(batch) * OZ_S * L.Np, L.Kp, OZ_BK, OZ_BN));
   const size_t smem = oz_smem_bytes();
-  static std::atomic<bool> attr{false};  // idempotent setup; threads may race to it
-  if (!attr.load()) {
-    TNX_CUDA(cudaFuncSetAttribute(oz_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    attr.store(true);
-  }
+  static DeviceSet allowed;
+  TNX_CUDA(allow_smem(oz_gemm_kernel, smem, allowed));
   const int kb_all = int(L.Kp / OZ_BK);
   const int kbs = (kb_all + nsplit - 1) / nsplit;
   nsplit = (kb_all + kbs - 1) / kbs;  // no empty splits

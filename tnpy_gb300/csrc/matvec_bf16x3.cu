@@ -26,8 +26,6 @@
 
 #include <cstring>
 
-#include <atomic>
-
 #include "tc_ptx.cuh"
 #include "tnx_internal.cuh"
 #include "wcontract.cuh"
@@ -524,11 +522,8 @@ int launch_gemm(const __nv_bfloat16* a_hi, const __nv_bfloat16* a_lo, const __nv
   TNX_TRY(make_map(&mbh, b_hi, N, Kp, BN));
   TNX_TRY(make_map(&mbl, b_lo, N, Kp, BN));
   const size_t smem = gemm_smem_bytes<BN>();
-  static std::atomic<bool> attr_set{false};  // idempotent setup; threads may race to it
-  if (!attr_set.load()) {
-    TNX_CUDA(cudaFuncSetAttribute(bf16x3_gemm_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    attr_set.store(true);
-  }
+  static DeviceSet allowed;
+  TNX_CUDA(allow_smem(bf16x3_gemm_kernel<BN>, smem, allowed));
   dim3 grid(unsigned((N + BN - 1) / BN), unsigned((M + BM - 1) / BM));
   profile_mark(KF_TC_GEMM, st, true);
   bf16x3_gemm_kernel<BN><<<grid, GEMM_THREADS, smem, st>>>(mah, mal, mbh, mbl, M, N, Kp, out, ldc,
@@ -551,12 +546,8 @@ int launch_pair(const __nv_bfloat16* a_hi, const __nv_bfloat16* a_lo, const __nv
   TNX_TRY(make_map(&mbh, b_hi, N, Kp, BN / 2));
   TNX_TRY(make_map(&mbl, b_lo, N, Kp, BN / 2));
   const size_t smem = size_t(ST) * SL * (BM + BN / 2) * BK * 2 + 1024;
-  static std::atomic<bool> attr_set{false};  // idempotent setup; threads may race to it
-  if (!attr_set.load()) {
-    TNX_CUDA(cudaFuncSetAttribute(bf16x3_pair_kernel<BN, ST, SL, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  int(smem)));
-    attr_set.store(true);
-  }
+  static DeviceSet allowed;
+  TNX_CUDA((allow_smem(bf16x3_pair_kernel<BN, ST, SL, MINB>, smem, allowed)));
   const int tn = (N + BN - 1) / BN, tm = (M + 2 * BM - 1) / (2 * BM);
   profile_mark(KF_TC_GEMM, st, true);
   bf16x3_pair_kernel<BN, ST, SL, MINB><<<2 * tn * tm, GEMM_THREADS, smem, st>>>(mah, mal, mbh, mbl, M, N, Kp, tn, out, ldc,

@@ -586,12 +586,19 @@ constexpr int panel_threads() {
 
 template <int NB, int CL, bool DF>
 const PanelKernelInfo& panel_info() {
-  static PanelKernelInfo info;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    int dev = 0, optin = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
+  constexpr int MAXDEV = 64;  // attributes are a device's; beyond it the forms without clusters run
+  static PanelKernelInfo infos[MAXDEV];
+  static std::once_flag once[MAXDEV];
+  static const PanelKernelInfo none;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAXDEV) {
+    cudaGetLastError();
+    return none;
+  }
+  PanelKernelInfo& info = infos[dev];
+  std::call_once(once[dev], [dev, &info] {
+    int optin = 0;
+    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
       cudaGetLastError();
       return;
     }

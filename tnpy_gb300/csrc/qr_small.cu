@@ -24,7 +24,6 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
-#include <atomic>
 
 #include "householder.cuh"
 #include "tnx_internal.cuh"
@@ -237,11 +236,8 @@ __global__ void __launch_bounds__(QS_T) qr_small_kernel(const double* A, int64_t
 int qr_small(const double* A, int64_t sA, double* Q, int64_t sQ, double* R, int64_t sR, int64_t m, int64_t n, int trans,
              int batch, cudaStream_t st) {
   const int ld = qs_ld(m, n);
-  static std::atomic<bool> attr{false};  // idempotent setup; threads may race to it
-  if (!attr.load()) {
-    TNX_CUDA(cudaFuncSetAttribute(qr_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(QS_SMEM)));
-    attr.store(true);
-  }
+  static DeviceSet allowed;
+  TNX_CUDA(allow_smem(qr_small_kernel, QS_SMEM, allowed));
   int team = 8;
   while (team > 1 && (batch * team > 152 || team > (n + 3) / 4)) team /= 2;
   cudaLaunchConfig_t cfg = {};

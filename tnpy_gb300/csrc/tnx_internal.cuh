@@ -10,6 +10,7 @@
 #include <functional>
 
 #include "../../include/tnx.h"
+#include "per_device.cuh"
 
 namespace tnx {
 

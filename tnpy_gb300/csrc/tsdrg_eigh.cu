@@ -37,7 +37,6 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
-#include <atomic>
 #include <type_traits>
 
 #include "jacobi.cuh"
@@ -1160,16 +1159,6 @@ int launch_team(void (*kernel)(P...), int batch, int team, size_t smem, cudaStre
   return TNX_OK;
 }
 
-// largest dynamic shared memory a kernel may use, once per kernel
-template <typename K>
-int opt_in(K kernel, std::atomic<bool>& done, size_t smem) {
-  if (!done.load()) {  // idempotent setup; threads may race to it
-    TNX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    done.store(true);
-  }
-  return TNX_OK;
-}
-
 }  // namespace
 }  // namespace tnx
 
@@ -1209,15 +1198,15 @@ int tnx_tsdrg_block_eigh(const double* const* w1, const double* const* w2, const
   double* vecs = reinterpret_cast<double*>(work + size_t(batch) * per_work);
   double* scr = reinterpret_cast<double*>(reinterpret_cast<char*>(vecs) + size_t(batch) * per_vec);
   const int max_outer = 60, degree = 10;
-  static std::atomic<bool> attr_c{false}, attr_p{false}, attr_r{false};
-  TNX_TRY(opt_in(kron_chfsi_kernel, attr_c, kron_smem<float>(KD, KM1 * KM1, true)));
+  static DeviceSet allowed_c, allowed_p, allowed_r;
+  TNX_CUDA(allow_smem(kron_chfsi_kernel, kron_smem<float>(KD, KM1 * KM1, true), allowed_c));
   const int team = team_for(batch);
   const size_t smem_c = kron_smem<float>(D, max_m, true);
   profile_mark(KF_EIGH, st, true);
   if (fp64) {
     // the FP32 stage leaves all p vectors where the FP64 stage reads them (the first of work's four
     // blocks of p m doubles); its own two FP32 blocks are the last of the four
-    TNX_TRY(opt_in(kron_polish_kernel, attr_p, polish_smem(KD)));
+    TNX_CUDA(allow_smem(kron_polish_kernel, polish_smem(KD), allowed_p));
     float* bounds = reinterpret_cast<float*>(scr);
     float* w32 = reinterpret_cast<float*>(work) + 6 * size_t(KP) * max_m;
     double* w64 = reinterpret_cast<double*>(work);
@@ -1229,7 +1218,7 @@ int tnx_tsdrg_block_eigh(const double* const* w1, const double* const* w2, const
     TNX_TRY(launch_team(kron_chfsi_kernel, batch, team, smem_c, st, w1, w2, meta, D, reinterpret_cast<float*>(work),
                         int64_t(per_work / 4), max_outer, degree, vecs, int64_t(per_vec / 8), 0,
                         static_cast<float*>(nullptr), iters, team));
-    TNX_TRY(opt_in(kron_refine_kernel, attr_r, kron_smem<double>(KD, KM1 * KM1, false)));
+    TNX_CUDA(allow_smem(kron_refine_kernel, kron_smem<double>(KD, KM1 * KM1, false), allowed_r));
     kron_refine_kernel<<<batch, KT, kron_smem<double>(D, max_m, false), st>>>(
         w1, w2, meta, D, vecs, int64_t(per_vec / 8), scr, int64_t(per_scr / 8), evals, keep, evecs, max_m);
     TNX_LAUNCH_CHECK();
