@@ -260,19 +260,14 @@ inline unsigned ctas_for(int64_t total, int nw) {
   return unsigned(b > 152 * 11 ? 152 * 11 : (b < 1 ? 1 : b));
 }
 
-// dynamic shared memory above 48 KB needs an opt-in
-template <typename K>
-int opt_in(K kernel, size_t smem) {
-  if (smem > 48 * 1024) TNX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-  return TNX_OK;
-}
-
+// (internal linkage: a kernel in a header is a translation unit's own, and so is the set of devices that know it)
 template <typename T, typename Out>
-int launch_left(const T* T1, int64_t sT1, const double* W, int64_t sW, Out out, int64_t sT2, int64_t chi_l, int64_t d,
+static int launch_left(const T* T1, int64_t sT1, const double* W, int64_t sW, Out out, int64_t sT2, int64_t chi_l, int64_t d,
                 int64_t chi_r, int64_t dl, int64_t dr, int64_t ldp, int batch, const int* mask, cudaStream_t st) {
   const int nin = int(dl * d), nout = int(dr * d), nw = warps_for<T, true>(nin, nout);
   const size_t smem = smem_bytes<T, true>(nin, nout, nw);
-  TNX_TRY(opt_in(left_kernel<T, Out>, smem));
+  static DeviceSet allowed;
+  TNX_CUDA((allow_smem(left_kernel<T, Out>, smem_bytes<T, true>(64, 64, 4), allowed)));  // no MPO takes more
   left_kernel<T, Out><<<dim3(ctas_for(chi_l * chi_r, nw), unsigned(batch)), 32 * nw, smem, st>>>(
       T1, sT1, W, sW, out, sT2, chi_l, int(d), chi_r, int(dl), int(dr), ldp, mask);
   TNX_LAUNCH_CHECK();
@@ -280,11 +275,12 @@ int launch_left(const T* T1, int64_t sT1, const double* W, int64_t sW, Out out, 
 }
 
 template <typename T>
-int launch_right(const T* T1, int64_t sT1, const double* W, int64_t sW, T* T2, int64_t sT2, int64_t chi_l, int64_t d,
+static int launch_right(const T* T1, int64_t sT1, const double* W, int64_t sW, T* T2, int64_t sT2, int64_t chi_l, int64_t d,
                  int64_t chi_r, int64_t dl, int64_t dr, int batch, cudaStream_t st) {
   const int nin = int(dr * d), nout = int(dl * d), nw = warps_for<T, false>(nin, nout);
   const size_t smem = smem_bytes<T, false>(nin, nout, nw);
-  TNX_TRY(opt_in(right_kernel<T>, smem));
+  static DeviceSet allowed;
+  TNX_CUDA((allow_smem(right_kernel<T>, smem_bytes<T, false>(64, 64, 4), allowed)));
   right_kernel<T><<<dim3(ctas_for(chi_l * chi_r, nw), unsigned(batch)), 32 * nw, smem, st>>>(
       T1, sT1, W, sW, T2, sT2, chi_l, int(d), chi_r, int(dl), int(dr));
   TNX_LAUNCH_CHECK();
