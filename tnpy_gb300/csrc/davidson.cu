@@ -853,6 +853,7 @@ int davidson1(const double* L, const double* W, const double* R, double* x_io, i
       w_at[j] = 0;
       for (int i = 1; i < j; ++i)
         if (fabs(s[i]) > fabs(s[w_at[j]])) w_at[j] = i;
+      eta[j] = s[w_at[j]] < 0.0 ? -1.0 : 1.0;  // positive, but where an earlier settling of this step turned it
       if (!(s[w_at[j]] * s[w_at[j]] >= 0.99)) open.n[open.count++] = j;
     }
     if (open.count > 0) {
