@@ -32,14 +32,6 @@
 
 #include "tc_ptx.cuh"
 
-// time stamps of the phases, taken by thread TNX_PANEL_PROBE
-#ifdef TNX_PANEL_PROBE
-#define PANEL_STAMP(k) \
-  if (threadIdx.x == TNX_PANEL_PROBE && stamps) stamps[(q * 64 + jj) * 8 + (k)] = clock64()
-#else
-#define PANEL_STAMP(k)
-#endif
-
 namespace tnx {
 namespace qrdf {
 
@@ -204,12 +196,7 @@ constexpr size_t panel_df_smem_bytes(int ld, bool push) {
 // column, 254 us so. 256 or 1024 threads: a quarter slower.
 template <int NB, int CL, int MODE>
 __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, int64_t m, int64_t j0, int nb, int ld,
-                                                       double* __restrict__ tau_out, double* __restrict__ T_out
-#ifdef TNX_PANEL_PROBE
-                                                       ,
-                                                       long long* stamps
-#endif
-) {
+                                                       double* __restrict__ tau_out, double* __restrict__ T_out) {
   constexpr int NW = DPT / 32, CPW = NB / NW;  // warp w works on columns w, w + NW, ...: CPW of them
   constexpr int GL = 32 / CPW;                 // lanes that end up with a column's sum
   constexpr int NR = NB / CL;                  // rows of T held by each CTA
@@ -235,9 +222,6 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
   const int rpc = int((mp + CL - 1) / CL);
   const int r0 = q * rpc;
   const int rows = int(r0 >= mp ? 0 : (mp - r0 < rpc ? mp - r0 : rpc));
-#ifdef TNX_PANEL_PROBE
-  int jj = 0;
-#endif
 
   // ---- column scales: largest |entry| of each panel column over the cluster (integer max of
   // the magnitude bits), exponent chosen so that it lands in [2^31, 2^32)
@@ -395,12 +379,7 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
   }
   exchange();
 
-#ifndef TNX_PANEL_PROBE
   for (int jj = 0; jj < nb; ++jj) {
-#else
-  for (jj = 0; jj < nb; ++jj) {
-#endif
-    PANEL_STAMP(0);
     const int par = jj & 1;
     const int owner = jj / rpc;
     const bool has_next = jj + 1 < nb;
@@ -457,7 +436,6 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
       extend_t(jj - 2);
     }
     __syncthreads();
-    PANEL_STAMP(1);
     if (push && s_dead) break;
     const df2 tj = sc[0], scale = sc[2];
     const int rA = lj > 0 ? lj : 0;
@@ -493,7 +471,6 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
       }
     }
     __syncthreads();
-    PANEL_STAMP(2);
     // ---- phase B: update columns c > jj + 1 and the partial dots of step jj + 1 (norm of
     // column jj + 1 below its pivot, its dots with c > jj + 1), T dots. A lane has rows lane, lane + 32, ..
     // of all the warp's columns, two at a time, from the first row below both pivots on
@@ -503,7 +480,6 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
       a[k] = {0.f, 0.f};
       wk[k] = W[warp + NW * k];  // not used left of the update
     }
-    PANEL_STAMP(3);
     auto two_rows = [&](int r, auto whole) {
       constexpr bool all = decltype(whole)::value;  // both rows exist (or are zero rows of the padding)
       const int r1 = r + 32;
@@ -538,17 +514,13 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
       if (pad || r + 64 <= rows) two_rows(r + lane, std::true_type{});
       else two_rows(r + lane, std::false_type{});
     }
-    PANEL_STAMP(4);
 #pragma unroll
     for (int k = 0; k < CPW; ++k) a[k] = norm(a[k]);
     df2 sum = reduce(a);
     if (ci < jj && (has_lj || has_ln)) sum = add(sum, W[ci]);
-    PANEL_STAMP(5);
     if (ci < nb && ci != jj) send_sum(par ^ 1, sum);
     updated(par ^ 1);
-    PANEL_STAMP(6);
     exchange();
-    PANEL_STAMP(7);
   }
   // the last two columns of T, the last one from the final exchange
   __syncthreads();
@@ -584,5 +556,3 @@ __global__ void __launch_bounds__(DPT) panel_df_kernel(double* __restrict__ F, i
 
 }  // namespace qrdf
 }  // namespace tnx
-
-#undef PANEL_STAMP
