@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restric
     for (int j = tid; j < n; j += RR_T) {
       const float den = float(double(Af[j * nf + j]) - theta);
       const float dot = sum_f(j);
-      rf[j] = (j != imin && fabsf(den) >= floor) ? dot / den : 0.f;
+      rf[j] = (j != imin && fabsf(den) > floor) ? dot / den : 0.f;  // the floor of a zero matrix is zero
     }
     __syncthreads();
     for (int i = warp < RR_G ? lane : n; i < n; i += 32) {
