@@ -11,7 +11,8 @@ import ctypes
 from ._lib import check, lib
 
 KINDS = {1: "df64_gemm_tile", 2: "fp64_class_engine", 3: "bf16x3_gemm_tile"}
-VARIANTS = {1: ["64x128/256thr", "32x32/64thr"], 2: ["ozaki_tcgen05", "df64_simt"], 3: ["128x256", "128x128"]}
+VARIANTS = {1: ["64x128/256thr", "32x32/64thr"], 2: ["ozaki_tcgen05", "df64_simt"],
+            3: ["128x128", "256x128/pair", "256x192/pair", "256x256/pair"]}
 
 
 def enable(on: bool = True) -> None:

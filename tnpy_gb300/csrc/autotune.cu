@@ -4,7 +4,7 @@
 // Tuned decisions (kind: key -> candidates):
 //   1 double-FP32 GEMM tile        (trans, m, n, k, batch) -> 64 x 128 tiles / 256 threads, 32 x 32 / 64
 //   2 FP64-class GEMM engine        (trans, m, n, k)        -> tcgen05 Ozaki GEMM, double-FP32 SIMT GEMM
-//   3 split-BF16 tcgen05 GEMM tile  (m, n, k)               -> 128 x 256 tiles, 128 x 128 tiles
+//   3 split-BF16 tcgen05 GEMM tile  (m, n, k, output size)  -> 128 x 128 tiles by a CTA; 256 x 128, 192, 256 by a pair
 // Only calls whose output is overwritten (beta = 0) are tuned, so that running every candidate
 // leaves the same result in place; a call inside a stream capture, or with tuning switched off
 // (tnx_autotune_set(0) or TNX_AUTOTUNE=0), takes the cached choice or the fixed size rule.
