@@ -328,8 +328,10 @@ int tnx_eigh_batched(double* A, const int64_t* offsets, const int* sizes, int ba
 // SM), an FP32 one for one, so the Jacobi sweeps run in FP32 and the lowest pair is then refined
 // against the FP64 matrix,
 //   s <- s - sum_{j != 0} v_j (v_j . r) / (lambda_j - theta),  r = A s - theta s,
-// which contracts the error by ~(FP32 eigenvector error) per step; three steps reach
-// FP64 accuracy for a non-degenerate lowest eigenvalue, and theta = s^T A s is FP64.
+// which contracts the error by ~(FP32 eigenvector error) / (relative gap) per step; three steps reach
+// FP64 accuracy where the lowest eigenvalue is well apart, a closer one takes up to seven, while the
+// corrections shrink (gaps of 1e-3 of the norm, 24 rows: residual 7e-14 after three, 2e-16 so).
+// theta = s^T A s is FP64.
 // Only s, r, theta and the norm are FP64: the correction's relative error of ~1e-6 is what the
 // FP32 eigenvectors leave it anyway, and the next step works it off.
 //
@@ -345,7 +347,8 @@ namespace {
 
 constexpr int RW_MAX = 64;
 
-constexpr int RR_G = 8;  // warps that share a product of the refinement
+constexpr int RR_G = 8;      // warps that share a product of the refinement
+constexpr int RR_STEPS = 7;  // most corrections
 
 // x 2^-e; zero for zero and where it would be subnormal
 __device__ __forceinline__ double rr_scale(double x, int e) {
@@ -533,7 +536,9 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restric
     for (int g = 1; g < RR_G; ++g) t += fp[g * n + i];
     return t;
   };
-  for (int step = 0; step < 4; ++step) {
+  int last = 3;         // the step that ends it
+  float dd_prev = 0.f;  // squared norm of the correction before
+  for (int step = 0;; ++step) {
     // y = A s, then |s|^2 and s . y together (n <= 64: the entries sit in warps 0 and 1)
     for (int i = warp < RR_G ? lane : n; i < n; i += 32) {
       double acc = 0.0;
@@ -566,7 +571,7 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restric
     const double inv = jac::rsqrt_exact(nn);  // nn is 1 to FP32 accuracy
     const double theta = (redd[2] + redd[3]) * (inv * inv);
     if (tid < n) s[tid] = si * inv;
-    if (step == 3) {
+    if (step == last) {
       if (tid == 0) eval[0] = scale_pow2(theta, ex);
       break;
     }
@@ -585,6 +590,14 @@ __global__ void __launch_bounds__(RR_T) rr_lowest_kernel(const double* __restric
       rf[j] = (j != imin && fabsf(den) > floor) ? dot / den : 0.f;  // the floor of a zero matrix is zero
     }
     __syncthreads();
+    if (step > 0) {  // every warp the same sum
+      float dd = lane < n ? rf[lane] * rf[lane] : 0.f;
+      if (lane + 32 < n) dd = fmaf(rf[lane + 32], rf[lane + 32], dd);
+      for (int o = 16; o > 0; o >>= 1) dd += __shfl_xor_sync(0xffffffffu, dd, o);
+      // the next correction would be about dd / dd_prev of this one: another step while that is above rounding
+      if (step == last - 1 && last < RR_STEPS && dd < 0.25f * dd_prev && dd * (dd / dd_prev) > 1e-32f) ++last;
+      dd_prev = dd;
+    }
     for (int i = warp < RR_G ? lane : n; i < n; i += 32) {
       float acc = 0.f;
       for (int j = warp; j < n; j += RR_G) acc = fmaf(Vf[i * nf + j], rf[j], acc);
