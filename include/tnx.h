@@ -68,7 +68,7 @@ int tnx_profile_end(int* launches, double* total_ms, double* flops, double* byte
  * caller's stream (first call of that shape, outside stream capture, output-overwriting calls
  * only) and caching the fastest for the process: the double-FP32 GEMM tile (64 x 128 / 32 x 32),
  * the FP64-class GEMM engine (tcgen05 Ozaki / double-FP32 SIMT) and the split-BF16 tcgen05 GEMM
- * tile (128 x 256 / 128 x 128). On by default; TNX_AUTOTUNE=0 in the environment or
+ * tile (128 x 128 by one CTA; 256 x 128, 192 or 256 by a pair of CTAs). On by default; TNX_AUTOTUNE=0 in the environment or
  * tnx_autotune_set(0) keeps the fixed size rules. tnx_autotune_report writes one line per cached
  * choice, "kind key0..key4 -> variant ms_0 .. ms_(n-1)" (kind 1 / 2 / 3 as listed; -1 ms for a
  * candidate that did not apply), and returns the bytes needed including the terminating zero.

@@ -301,8 +301,9 @@ __global__ void __launch_bounds__(DT) lincomb_kernel(const T* __restrict__ V, co
 }
 
 // CTAs of a vector kernel: one element per thread until two CTAs fill every SM. The FP64 pipe takes
-// a warp's FMA in 64 clocks, so a Ritz vector over 24 basis vectors at n = 2048 took 18 us on 2 CTAs
-// (four elements per thread) and takes 6.5 us on 8.
+// a warp's FMA in 64 clocks, so a pass over 24 basis vectors at n = 2048 took 18 us on 2 CTAs (four elements
+// per thread) and 6.5 us on 8 (the Ritz vector, which is a cluster kernel's at that size by now; the
+// generalised solver and the preparation still use these launches there).
 inline int nchunk_for(int64_t n) {
   int64_t c = (n + DT - 1) / DT;
   if (c > 2 * 152) c = 2 * 152;
@@ -318,8 +319,8 @@ inline int nchunk_for(int64_t n) {
 // the new column of the projected matrix; the Ritz vector, residual and correction, which also puts
 // the expansion's scalars where the host reads them once. A direction that vanished against the basis
 // becomes zero there and is undone on the host. chi = 32 (2048 elements), per expansion: 191 us
-// before, 106 us so. Above DC_MAX the eight SMs' FP64 pipes cost more than the launches (one pass over 24
-// vectors takes 32 DC_MAX / 2 clocks of FMAs).
+// before, 106 us so (63 us with the tridiagonal Rayleigh-Ritz step). Above DC_MAX the eight SMs' FP64 pipes cost
+// more than the launches: one pass over 24 vectors is 24 DC_MAX FMAs at 16 a clock, 1.5 DC_MAX clocks (12 us).
 constexpr int DC_CL = 8, DC_T = 512, DC_W = DC_T / 32;
 constexpr int64_t DC_MAX = 16384;
 constexpr int DC_PER = int(DC_MAX / DC_CL);  // elements of a vector per CTA

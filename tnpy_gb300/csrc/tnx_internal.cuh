@@ -250,7 +250,8 @@ int mixed_apply_f32(const double* W, const float* x, float* y, int64_t chi_l, in
                     int64_t dr, void* scratch, cudaStream_t st);
 int mixed_flag(void* scratch, int64_t chi_l, int64_t d, int64_t chi_r, int64_t dl, int64_t dr, int** flag);
 
-// Householder QR of `batch` matrices in shared memory, one CTA each (m >= n, n <= 128, m n <= 12800):
+// Householder QR of `batch` matrices in shared memory, one CTA each, or a cluster of up to eight while the batch
+// leaves SMs idle (m >= n, n <= 128, m n <= 12800):
 // trans = 0 row-major m x n at A + b sA, trans = 1 its transpose; Q in the same layout (may be A), R
 // (n x n, row-major) at R + b sR
 int qr_small(const double* A, int64_t sA, double* Q, int64_t sQ, double* R, int64_t sR, int64_t m, int64_t n, int trans,

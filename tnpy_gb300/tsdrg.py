@@ -192,7 +192,7 @@ KRON_MAX_P = 48
 def kron_eigh(pairs, chi: int, dev, precision: str = "mixed"):
     """Lowest min(chi, m) eigenpairs of the two-block Hamiltonians of (W1, W2) pairs without
     forming them (Kronecker-sum Chebyshev subspace iteration + FP64 Rayleigh-Ritz, one CTA per
-    block). Returns (evals [batch, keep] device, evecs [batch, max_m, keep] device, ks, iters), iters
+    block, or a cluster of them while the batch leaves SMs idle). Returns (evals [batch, keep] device, evecs [batch, max_m, keep] device, ks, iters), iters
     negative for blocks whose subspace iteration did not converge."""
     D = pairs[0][0].shape[1]
     ms = [(w1.shape[2], w2.shape[2]) for w1, w2 in pairs]
@@ -305,10 +305,11 @@ def _select(c: "_Chain", ev: np.ndarray, vec: torch.Tensor):
 
 
 # Dense block eigensolver: the FP64 Jacobi in every precision mode. The double-FP32 Jacobi
-# ('df64', 2.1x faster per 64-state block) changes, on SU(2)-symmetric chains (h = 0), which
-# members of degenerate multiplets are kept; on the n=128, chi=32 bench chains the resulting
-# trees merge more 32 x 32 blocks, whose Kronecker solves cost more than the Jacobi saves
-# (44.6 against 90 realisations/s), so it is not the default.
+# ('df64', 1.6x faster per 64-state block: 128 of them 1.9 against 3.1 ms) changes, on
+# SU(2)-symmetric chains (h = 0), which members of degenerate multiplets are kept; on the n=128,
+# chi=32 bench chains the resulting trees merge more 32 x 32 blocks, whose Kronecker solves cost
+# more than the Jacobi saves (512 chains, two runs: 77 and 84 against 101 and 130 realisations/s), so it is not
+# the default.
 _dense_precision = "fp64"
 
 
